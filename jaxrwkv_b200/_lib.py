@@ -1,9 +1,13 @@
-"""ctypes binding of libb200wkv.so (the C ABI declared in include/b200wkv.h)."""
+"""ctypes binding of libb200wkv.so (the C ABI declared in include/b200wkv.h), and the loader of the operators'
+native host path (csrc/host_ext.cpp)."""
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libb200wkv.so")
+HOST_PATH = os.path.join(_HERE, "lib", "_b200wkv_host.so")
 
 F32, BF16 = 0, 1
 FLAG_SEQUENTIAL = 1
@@ -42,6 +46,7 @@ PROTOTYPES = {
 }
 
 _lib = None
+_host = None
 
 
 class B200WKVError(RuntimeError):
@@ -63,6 +68,22 @@ def load():
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def host():
+    """The native host path (a Python extension beside the library); loaded once, an error if it was not built."""
+    global _host
+    if _host is None:
+        load()
+        if not os.path.exists(HOST_PATH):
+            raise B200WKVError(f"{HOST_PATH} is missing: build it with `python -m jaxrwkv_b200.build`")
+        import torch  # noqa: F401  (the extension links against its libraries)
+        loader = importlib.machinery.ExtensionFileLoader("_b200wkv_host", HOST_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+        loader.exec_module(module)
+        module.set_error_class(B200WKVError)
+        _host = module
+    return _host
 
 
 def check(status):

@@ -161,6 +161,10 @@ _FUNCS = {ver: _make_functions(ver) for ver in ("6", "5_2", "5")}
 
 def wkv_cuda(version, r, k, v, w, time_first, s, length, new_starts):
     """Differentiable operator; returns (s_out, out)."""
+    if k.is_cuda:
+        native = _lib.host().wkv6(version == "6", r, k, v, w, time_first, s, length, new_starts)
+        if native is not None:                   # None: a transform such as vmap, or arguments that need a closer look
+            return native
     new_s, out, _ = _FUNCS[version][0].apply(r, k, v, w, time_first, s, length, new_starts)
     return new_s, out
 

@@ -1,12 +1,14 @@
 """Build libb200wkv.so in-tree with nvcc for sm_100a:  python -m jaxrwkv_b200.build [--force] [-v]
 
 Every ``csrc/*.cu`` is compiled to an object file of its own (in parallel, only when it or a header
-is newer than the object) and the objects are linked into ``lib/libb200wkv.so``.
+is newer than the object) and the objects are linked into ``lib/libb200wkv.so``.  ``csrc/host_ext.cpp`` becomes ``lib/_b200wkv_host.so``, the
+Python extension with the operators' native host path.
 """
 import glob
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -14,6 +16,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(LIBDIR, "obj")
 OUT = os.path.join(LIBDIR, "libb200wkv.so")
+EXT_SRC = os.path.join(CSRC, "host_ext.cpp")
+EXT_OUT = os.path.join(LIBDIR, "_b200wkv_host.so")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC"]
@@ -39,7 +43,21 @@ def _stale(target, deps):
 
 
 def needs_build():
-    return _stale(OUT, sources() + headers())
+    return _stale(OUT, sources() + headers()) or _stale(EXT_OUT, [EXT_SRC] + headers())
+
+
+def build_host_ext():
+    """Compile csrc/host_ext.cpp against the installed torch and link it to libb200wkv.so beside it."""
+    import torch
+    from torch.utils import cpp_extension as ce
+    inc = ce.include_paths(device_type="cuda") + [sysconfig.get_paths()["include"]]
+    libs = ce.library_paths(device_type="cuda")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [x for d in inc for x in ("-isystem", d)] + ["-o", EXT_OUT, EXT_SRC, "-L", LIBDIR, "-lb200wkv", "-Wl,-rpath,$ORIGIN"]
+    cmd += [x for d in libs for x in ("-L", d)] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    print(" ".join(cmd), file=sys.stderr)
+    subprocess.check_call(cmd)
 
 
 def build(force=False, verbose=False):
@@ -60,6 +78,8 @@ def build(force=False, verbose=False):
     cmd = [nvcc, "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-o", OUT] + [_obj(s) for s in sources()]
     print(" ".join(cmd), file=sys.stderr)
     subprocess.check_call(cmd)
+    if force or _stale(EXT_OUT, [EXT_SRC] + headers()):
+        build_host_ext()
     return OUT
 
 

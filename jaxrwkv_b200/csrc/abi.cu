@@ -291,7 +291,7 @@ int b200wkv7_step_inplace(void* stream, int dtype, int B, int H, int N, const vo
                           const uint32_t* length, const uint8_t* new_starts, void* y) {
     int st = check_dims(dtype, B, 1, H, N);
     if (st != B200WKV_OK) return st;
-    if (!w || !r || !k || !v || !a || !b || !state || !length || !new_starts || !y) return B200WKV_ENULL;
+    if (!w || !r || !k || !v || !a || !b || !state || !y) return B200WKV_ENULL;
     const long long esz = dtype == B200WKV_F32 ? 4 : 2;
     if (state_batch_stride < (long long)H * N * N) return B200WKV_ESHAPE;
     const uintptr_t vec_bits = reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(k) |

@@ -169,7 +169,8 @@ wkv7_step_stream_kernel(int BH, int H, const T* __restrict__ w, const T* __restr
         const int it = it0 + tid;
         if (it < n_my) {
             const int bi = (first + it * stride) / H;
-            sm.flags[(it0 / kFlagBatch) & 1][tid] = (unsigned char)((length[bi] == 0 ? 1 : 0) | (new_starts[bi] != 0 ? 2 : 0));
+            const bool none = length != nullptr && length[bi] == 0, start = new_starts != nullptr && new_starts[bi] != 0;
+            sm.flags[(it0 / kFlagBatch) & 1][tid] = (unsigned char)((none ? 1 : 0) | (start ? 2 : 0));
         }
     };
     // thread c turns channel c of the six vectors of a stage into fp32 (the decay into exp(-exp(w)))

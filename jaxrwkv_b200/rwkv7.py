@@ -231,6 +231,10 @@ def wkv7_step_packed(r, w, k, v, a, b, state, layer, new_starts=None, length=Non
     operator's ``(H, N, N)`` block (rwkv7.py:255, :260).  The kernel reads and writes that block
     where it lies: no slice is copied out or back.  Returns ``out`` shaped like ``r``.
     """
+    if r.is_cuda:
+        native = _lib.host().step_packed(r, w, k, v, a, b, state, layer, new_starts, length)
+        if native is not None:                   # None: arguments that need a closer look
+            return native
     lib = _lib.load()
     shp = r.shape
     B, H, N = shp[0], shp[-2], shp[-1]
@@ -258,6 +262,10 @@ def wkv7_cuda(r, w, k, v, a, b, s, length, new_starts):
     """Differentiable WKV-7 operator (rwkv7.py:442-446).  Tensors are (..., T, H, N) with any
     number of leading batch axes, the state (..., H, N, N); ``length`` and ``new_starts`` may
     carry the same leading axes or be shared.  Returns ``(s_out, out)``."""
+    if k.is_cuda:
+        native = _lib.host().wkv7(r, w, k, v, a, b, s, length, new_starts)
+        if native is not None:                   # None: a transform such as vmap, or arguments that need a closer look
+            return native
     new_s, out, _ = _WKV7.apply(r, w, k, v, a, b, s, length, new_starts)
     return new_s, out
 
