@@ -2,6 +2,7 @@
 #include <initializer_list>
 #include "common.cuh"
 #include "chunk_common.cuh"
+#include "host_calls.h"
 #include "../../include/b200wkv_debug.h"
 
 namespace b200wkv {
@@ -53,12 +54,6 @@ int wkv6_chunk_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
                    int per_token, const void* u, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out,
                    void* residual, const int* residual_mark, void* dr, void* dk, void* dv, void* dw, void* du, void* ds0);
 size_t wkv4_residual_bytes(int B, int T, int C);
-int wkv4_fwd(cudaStream_t st, int dtype, int B, int T, int C, const void* w, const void* u, const void* k, const void* v,
-             const void* s0, const uint32_t* length, const uint8_t* ns, void* s_out, void* y, void* residual);
-int wkv4_bwd(cudaStream_t st, int dtype, int B, int T, int C, const void* w, const void* u, const void* k, const void* v,
-             const void* gy, const uint32_t* length, const uint8_t* ns, const void* gs_new, const void* residual,
-             void* gw, void* gu, void* gk, void* gv, void* gs);
-
 int wkv7_mix_partial_rows(int rows, int C);
 int wkv7_mix_pre_fwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al,
                      const void* v, const void* vf, const void* vl, const void* w0, const void* a0, const void* v0,
@@ -269,7 +264,7 @@ int b200wkv4_fwd(void* stream, int dtype, int B, int T, int C, const void* w, co
     if (!w || !u || !k || !v || !s0 || !length || !new_starts || !s_out || !y) return B200WKV_ENULL;
     if (residual != nullptr && residual_bytes < wkv4_residual_bytes(B, T, C)) return B200WKV_ERESIDUAL;
     (void)flags;
-    return wkv4_fwd((cudaStream_t)stream, dtype, B, T, C, w, u, k, v, s0, length, new_starts, s_out, y, residual);
+    return wkv4_fwd((cudaStream_t)stream, dtype, B, T, C, false, w, u, nullptr, k, v, s0, length, new_starts, s_out, y, residual);
 }
 
 int b200wkv4_bwd(void* stream, int dtype, int B, int T, int C, const void* w, const void* u, const void* k,
@@ -282,8 +277,8 @@ int b200wkv4_bwd(void* stream, int dtype, int B, int T, int C, const void* w, co
         return B200WKV_ENULL;
     if (residual_bytes < wkv4_residual_bytes(B, T, C)) return B200WKV_ERESIDUAL;
     (void)flags;
-    return wkv4_bwd((cudaStream_t)stream, dtype, B, T, C, w, u, k, v, gy, length, new_starts, gs_new, residual, gw, gu,
-                    gk, gv, gs);
+    return wkv4_bwd((cudaStream_t)stream, dtype, B, T, C, false, w, u, nullptr, k, v, gy, length, new_starts, gs_new, residual,
+                    (float*)gw, (float*)gu, nullptr, gk, gv, gs);
 }
 
 int b200wkv7_step_inplace(void* stream, int dtype, int B, int H, int N, const void* w, const void* r, const void* k,

@@ -20,6 +20,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include "../../include/b200wkv.h"
+#include "host_calls.h"
 
 namespace {
 
@@ -49,7 +50,7 @@ Tensor fresh(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
 Tensor fresh_like(const Tensor& t) { return fresh(t.sizes(), t.scalar_type(), t); }
 Tensor bytes(size_t n, const Tensor& like) { return fresh({(int64_t)n}, at::kByte, like); }
 int dtype_code(const Tensor& t) { return t.scalar_type() == at::kFloat ? B200WKV_F32 : B200WKV_BF16; }
-void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
 // The plain case: no functorch transform, no dispatch mode.
 bool plain_mode() {
@@ -281,6 +282,78 @@ struct Wkv6Node : public torch::autograd::Function<Wkv6Node<kPerToken>> {
     }
 };
 
+// ------------------------------------------------------------------------------------------------- RWKV-4
+// k, v (lead, T, C), parameters (C), state (lead, 3, C).  With r (lead, T, C) the result is r * wkv, as the model takes it.
+struct Wkv4 {
+    static constexpr const char* kName = "wkv4";
+    struct Dims {
+        at::IntArrayRef lead;
+        int B, T, C;
+        explicit Dims(const Tensor& k) : lead(k.sizes().slice(0, k.dim() - 2)) {
+            B = (int)c10::multiply_integers(lead);
+            T = (int)k.size(-2); C = (int)k.size(-1);
+        }
+    };
+    // t: k v w u s [r]
+    static bool fits(const Tensor* t, bool with_r) {
+        if (!same_kind(t, with_r ? 6 : 5) || t[0].dim() < 2) return false;
+        const Dims d(t[0]);
+        return t[1].sizes().equals(t[0].sizes()) && sizes_are(t[2], {}, {d.C}) && sizes_are(t[3], {}, {d.C}) &&
+               sizes_are(t[4], d.lead, {3, d.C}) && (!with_r || t[5].sizes().equals(t[0].sizes()));
+    }
+    static std::pair<Tensor, Tensor> forward(const Tensor* t, const Tensor& length, const Tensor& starts, Tensor* residual) {
+        const Tensor& k = t[0];
+        const c10::cuda::CUDAGuard guard(k.device());
+        const Dims d(k);
+        const Flags f(length, starts, d.lead, d.T, k);
+        Tensor c[6];
+        for (int i = 0; i < 6; ++i) c[i] = t[i].defined() ? t[i].contiguous() : t[i];
+        Tensor y = fresh_like(k), s_out = fresh_like(t[4]);
+        if (residual) *residual = bytes(b200wkv4_residual_bytes(dtype_code(k), d.B, d.T, d.C), k);
+        check(b200wkv::wkv4_fwd(stream_of(k), dtype_code(k), d.B, d.T, d.C, true, in(c[2]), in(c[3]), in(c[5]), in(c[0]), in(c[1]), in(c[4]),
+                                (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), out(s_out), out(y),
+                                residual ? out(*residual) : nullptr));
+        return {s_out, y};
+    }
+    // saved: k v w u s r length new_starts residual (r may be undefined)
+    static variable_list gradients(const variable_list& saved, const variable_list& grads) {
+        const Tensor &k = saved[0], &r = saved[5];
+        const bool with_r = r.defined() && r.numel() > 0;
+        const c10::cuda::CUDAGuard guard(k.device());
+        const Dims d(k);
+        const Flags f(saved[6], saved[7], d.lead, d.T, k);
+        const Tensor gs = cotangent(grads[0], k), gy = cotangent(grads[1], k), rc = with_r ? r.contiguous() : Tensor();
+        Tensor c[4], g[6];
+        for (int i = 0; i < 4; ++i) c[i] = saved[i].contiguous();
+        for (int i = 0; i < 5; ++i) g[i] = fresh_like(saved[i]);
+        if (with_r) g[5] = fresh_like(r);
+        const Tensor sums = fresh({2, d.B, d.C}, at::kFloat, k);
+        float* gw = (float*)out(sums);
+        float* gu = gw + (size_t)d.B * d.C;
+        check(b200wkv::wkv4_bwd(stream_of(k), dtype_code(k), d.B, d.T, d.C, true, in(c[2]), in(c[3]), in(rc), in(c[0]), in(c[1]), in(gy),
+                                (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), in(gs), in(saved[8]), gw, gu, out(g[5]),
+                                out(g[0]), out(g[1]), out(g[4])));
+        check(b200wkv::wkv4_parameter_grads(stream_of(k), dtype_code(k), d.B, d.C, in(c[2]), gw, gu, out(g[2]), out(g[3])));
+        return {g[0], g[1], g[2], g[3], g[4], g[5]};
+    }
+};
+struct Wkv4Node : public torch::autograd::Function<Wkv4Node> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u,
+                                 const Tensor& s, const Tensor& r, const Tensor& length, const Tensor& starts) {
+        const Tensor t[] = {k, v, w, u, s, r};
+        Tensor residual;
+        auto [s_out, y] = Wkv4::forward(t, length, starts, &residual);
+        ctx->save_for_backward({k, v, w, u, s, r.defined() ? r : fresh({0}, k.scalar_type(), k), length, starts, residual});
+        ctx->set_materialize_grads(false);
+        return {s_out, y};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        variable_list g = gradients_of<Wkv4>(ctx, grads);
+        g.resize(8);
+        return g;
+    }
+};
+
 // ------------------------------------------------------------------------------------------------- decoding
 // One token on layer `layer` of the packed state (B, L, 2 + N, H N), in place.  An undefined tensor when it does not fit.
 Tensor step_packed(const Tensor* t /* r w k v a b */, const Tensor& state, int64_t layer, const Tensor& starts, const Tensor& length) {
@@ -365,6 +438,26 @@ PyObject* py_wkv6(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (per_to
     END_HANDLE_TH_ERRORS
 }
 
+PyObject* py_wkv4(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (r or None, k, v, w, u, s, length, new_starts)
+    HANDLE_TH_ERRORS
+    Tensor t[8], s_out, y;   // k v w u s r length new_starts
+    if (n != 8 || !take(args + 1, 5, t) || !take(args + 6, 2, t + 6)) Py_RETURN_NONE;
+    if (args[0] != Py_None && !take(args, 1, t + 5)) Py_RETURN_NONE;
+    const bool with_r = t[5].defined();
+    if (!Wkv4::fits(t, with_r)) Py_RETURN_NONE;
+    {
+        pybind11::gil_scoped_release no_gil;
+        if (any_grad(t, with_r ? 6 : 5)) {
+            variable_list o = Wkv4Node::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7]);
+            s_out = o[0]; y = o[1];
+        } else {
+            std::tie(s_out, y) = Wkv4::forward(t, t[6], t[7], nullptr);
+        }
+    }
+    return pair(s_out, y);
+    END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_step_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (r, w, k, v, a, b, state, layer, new_starts, length)
     HANDLE_TH_ERRORS
     Tensor t[7], starts, length, y;
@@ -391,6 +484,7 @@ PyObject* py_set_error_class(PyObject*, PyObject* cls) {
 PyMethodDef kMethods[] = {
     {"wkv7", (PyCFunction)(void (*)(void))py_wkv7, METH_FASTCALL, nullptr},
     {"wkv6", (PyCFunction)(void (*)(void))py_wkv6, METH_FASTCALL, nullptr},
+    {"wkv4", (PyCFunction)(void (*)(void))py_wkv4, METH_FASTCALL, nullptr},
     {"step_packed", (PyCFunction)(void (*)(void))py_step_packed, METH_FASTCALL, nullptr},
     {"set_error_class", py_set_error_class, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -139,7 +139,16 @@ class _WKV4(torch.autograd.Function):
         return (new_s, out, residual), (0, 0, None)
 
 
+def _native(r, k, v, w, time_first, s, length, new_starts):
+    """The native host path, with the product by ``r`` inside the kernels unless ``r`` is None.  None where it does not
+    apply: a transform such as vmap, or arguments that need a closer look."""
+    return _lib.host().wkv4(r, k, v, w, time_first, s, length, new_starts) if k.is_cuda else None
+
+
 def wkv4_cuda(k, v, w, time_first, s, length, new_starts):
+    native = _native(None, k, v, w, time_first, s, length, new_starts)
+    if native is not None:
+        return native
     new_s, out, _ = _WKV4.apply(k, v, w, time_first, s, length, new_starts)
     return new_s, out
 
@@ -154,5 +163,8 @@ class CudaRWKV:
     @classmethod
     def inner_loop(cls, r, k, v, w, time_first, s, length, new_starts):
         cls.get_kernels()
+        native = _native(r, k, v, w, time_first, s, length, new_starts)
+        if native is not None:
+            return native
         s, out = wkv4_cuda(k, v, w, time_first, s, length, new_starts)
         return s, r * out
