@@ -55,7 +55,7 @@ def build_host_ext():
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     cmd += [x for d in inc for x in ("-isystem", d)] + ["-o", EXT_OUT, EXT_SRC, "-L", LIBDIR, "-lb200wkv", "-Wl,-rpath,$ORIGIN"]
-    cmd += [x for d in libs for x in ("-L", d)] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    cmd += [x for d in libs for x in ("-L", d)] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcublasLt"]
     print(" ".join(cmd), file=sys.stderr)
     subprocess.check_call(cmd)
 

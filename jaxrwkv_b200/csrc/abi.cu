@@ -58,21 +58,11 @@ int wkv7_mix_partial_rows(int rows, int C);
 int wkv7_mix_pre_fwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al,
                      const void* v, const void* vf, const void* vl, const void* w0, const void* a0, const void* v0,
                      const void* k_k, const void* k_a, void* w, void* kp, void* vp, void* ai, void* bi);
-int wkv7_mix_pre_bwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al,
-                     const void* v, const void* vf, const void* vl, const void* w0, const void* a0, const void* v0,
-                     const void* k_k, const void* k_a, const void* gw, const void* gkp, const void* gvp, const void* gai,
-                     const void* gbi, void* dk, void* dwl, void* dal, void* dv, void* dvf, void* dvl, float* partial);
 int wkv7_mix_post_fwd(cudaStream_t st, int dtype, int rows, int C, float eps, const void* y, const void* r, const void* kp,
                       const void* vp, const void* g, const void* ln_w, const void* ln_b, const void* r_k, void* x);
 int wkv7_mix_post_bwd(cudaStream_t st, int dtype, int rows, int C, float eps, const void* y, const void* r, const void* kp,
                       const void* vp, const void* g, const void* ln_w, const void* ln_b, const void* r_k, const void* gx, void* dy,
                       void* dr, void* dkp, void* dvp, void* dg, float* partial);
-int token_shift_fwd(cudaStream_t st, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
-                    const void* mix, const uint32_t* length, const uint8_t* ns, void* out, void* state_out);
-int token_shift_bwd(cudaStream_t st, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
-                    const void* mix, const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate,
-                    void* gx, void* gprev, void* gmix);
-
 // The bf16 forward normally runs the chunked tensor-core kernel; a decay outside that kernel's range makes
 // the token-sequential kernel behind it redo the call.  The last bytes of the residual tell the backward
 // which of the two wrote it.
@@ -343,7 +333,7 @@ int b200wkv7_mix_pre_bwd(void* stream, int dtype, long long rows, int H, int N, 
                     dvl, partial}))
         return B200WKV_EUNSUPPORTED;
     return wkv7_mix_pre_bwd((cudaStream_t)stream, dtype, (int)rows, H * N, use_vmix ? 1 : 0, k, wl, al, v, v_first, vl, w0, a0,
-                            v0, k_k, k_a, gw, gk_out, gv_out, ga_i, gb_i, dk, dwl, dal, dv, dv_first, dvl, partial);
+                            v0, k_k, k_a, gw, gk_out, gv_out, ga_i, gb_i, dk, dwl, dal, dv, dv_first, dvl, partial, MixPreExtra{});
 }
 
 int b200wkv7_mix_post_fwd(void* stream, int dtype, long long rows, int H, int N, float eps, const void* y, const void* r,
@@ -396,13 +386,23 @@ static int check_shift(int dtype, int B, int T, int D, int M) {
     return B200WKV_OK;
 }
 
+namespace {
+struct MixRows {   // the rows of a dense (M, D) array
+    const void* p[8];
+    MixRows(const void* mix, int dtype, int D, int M) {
+        for (int m = 0; m < 8; ++m) p[m] = static_cast<const char*>(mix) + (size_t)(m < M ? m : 0) * D * (dtype == B200WKV_F32 ? 4 : 2);
+    }
+};
+}  // namespace
+
 int b200wkv_token_shift_fwd(void* stream, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
                             const void* mix, const uint32_t* length, const uint8_t* new_starts, void* out,
                             void* state_out) {
     int st = check_shift(dtype, B, T, D, M);
     if (st != B200WKV_OK) return st;
     if (!x || !prev || !mix || !length || !new_starts || !out || !state_out) return B200WKV_ENULL;
-    return token_shift_fwd((cudaStream_t)stream, dtype, B, T, D, M, x, prev, mix, length, new_starts, out, state_out);
+    const MixRows rows(mix, dtype, D, M);
+    return token_shift_fwd((cudaStream_t)stream, dtype, B, T, D, M, x, prev, rows.p, length, new_starts, out, state_out);
 }
 
 int b200wkv_token_shift_bwd(void* stream, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
@@ -411,7 +411,8 @@ int b200wkv_token_shift_bwd(void* stream, int dtype, int B, int T, int D, int M,
     int st = check_shift(dtype, B, T, D, M);
     if (st != B200WKV_OK) return st;
     if (!x || !prev || !mix || !length || !new_starts || !gout || !gx || !gprev || !gmix) return B200WKV_ENULL;
-    return token_shift_bwd((cudaStream_t)stream, dtype, B, T, D, M, x, prev, mix, length, new_starts, gout, gstate, gx,
+    const MixRows rows(mix, dtype, D, M);
+    return token_shift_bwd((cudaStream_t)stream, dtype, B, T, D, M, x, prev, rows.p, length, new_starts, gout, gstate, gx,
                            gprev, gmix);
 }
 

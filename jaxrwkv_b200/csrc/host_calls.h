@@ -16,4 +16,28 @@ int wkv4_bwd(cudaStream_t st, int dtype, int B, int T, int C, bool raw_w, const 
 // dw = -exp(w) * sum_b gw, du = sum_b gu, in the element type
 int wkv4_parameter_grads(cudaStream_t st, int dtype, int B, int C, const void* w, const float* gw, const float* gu, void* dw, void* du);
 
+
+// The token shift with the M rows of mix coefficients where the model keeps them (M <= 8).
+int token_shift_fwd(cudaStream_t st, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
+                    const void* const* mix, const uint32_t* length, const uint8_t* ns, void* out, void* state_out);
+int token_shift_bwd(cudaStream_t st, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
+                    const void* const* mix, const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate,
+                    void* gx, void* gprev, void* gmix);
+// The backward of the stage in front of the operator with what else meets there: more cotangents of k' and v' (gkp2, gvp2) and
+// of the first layer's v (gv_out), and r's second share (gr += dr).  NULL: none.
+struct MixPreExtra {
+    const void *gkp2, *gvp2, *gv_out, *dr;
+    void* gr;
+};
+int wkv7_mix_pre_bwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al,
+                     const void* v, const void* vf, const void* vl, const void* w0, const void* a0, const void* v0,
+                     const void* k_k, const void* k_a, const void* gw, const void* gkp, const void* gvp, const void* gai,
+                     const void* gbi, void* dk, void* dwl, void* dal, void* dv, void* dvf, void* dvl, float* partial,
+                     const MixPreExtra& extra);
+// y == NULL: x = act(x) in place; else x *= act'(.) in terms of y = act(.)
+enum { kTanh = 1, kSigmoid = 2 };
+int activation(cudaStream_t st, int dtype, int act, long long n, void* x, const void* y);
+// out[c] = sum over rows of partial[row][c], in the element type
+int column_sums(cudaStream_t st, int dtype, long long rows, long long cols, const float* partial, void* out);
+
 }  // namespace b200wkv

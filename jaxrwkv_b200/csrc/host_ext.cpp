@@ -7,12 +7,20 @@
 // (arguments that are no plain tensors, a functorch transform or a dispatch mode in force, shapes or types that do
 // not fit); the Python functions that call them then take their own path, which handles vmap and raises the errors.
 #include <torch/csrc/python_headers.h>
+
+#include <array>
+#include <functional>
+#include <memory>
+#include <unordered_map>
+
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/object_ptr.h>
 
 #include <ATen/ATen.h>
+#include <ATen/autocast_mode.h>
+#include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -40,6 +48,10 @@ PyObject* g_error_class = nullptr;   // jaxrwkv_b200._lib.B200WKVError
 void check(int status) {
     if (status != B200WKV_OK)
         raise(std::string("b200wkv: ") + b200wkv_strerror(status) + " (status " + std::to_string(status) + ")");
+}
+
+void cuda_check(cudaError_t e) {
+    if (e != cudaSuccess) raise(std::string("b200wkv: ") + cudaGetErrorString(e));
 }
 
 const void* in(const Tensor& t) { return t.defined() ? t.const_data_ptr() : nullptr; }
@@ -73,6 +85,11 @@ bool any_grad(const Tensor* t, int n) {
         if (t[i].requires_grad()) return true;
     return false;
 }
+bool any_grad_defined(const Tensor* t, int n) {
+    for (int i = 0; i < n; ++i)
+        if (t[i].defined() && any_grad(t + i, 1)) return true;
+    return false;
+}
 bool sizes_are(const Tensor& t, at::IntArrayRef lead, std::initializer_list<int64_t> tail) {
     if (t.dim() != (int64_t)(lead.size() + tail.size())) return false;
     size_t i = 0;
@@ -102,30 +119,34 @@ struct Flags {
     }
 };
 
-// A cotangent as the kernels read it; an absent one (undefined, or the empty stand-in of gradients_of) is undefined: the
-// kernels take NULL for zero.
+// A cotangent as the kernels read it; an undefined one stays undefined (the kernels take NULL for zero).
 Tensor cotangent(const Tensor& g, const Tensor& like) {
-    return !g.defined() || g.numel() == 0 ? Tensor() : (g.scalar_type() == like.scalar_type() ? g : g.to(like.scalar_type())).contiguous();
+    return !g.defined() ? g : (g.scalar_type() == like.scalar_type() ? g : g.to(like.scalar_type())).contiguous();
 }
 
 // Gradients asked for with create_graph=True: the values are right, differentiating them again is an error.
-template <class Op>
-struct NoSecondOrder : public torch::autograd::Function<NoSecondOrder<Op>> {
-    static variable_list forward(AutogradContext*, at::TensorList saved, at::TensorList grads) {
-        return Op::gradients(variable_list(saved.begin(), saved.end()), variable_list(grads.begin(), grads.end()));
+struct Refuse : public torch::autograd::Function<Refuse> {
+    static variable_list forward(AutogradContext* ctx, at::TensorList from, const std::function<variable_list()>& compute, std::string name) {
+        ctx->saved_data["name"] = name;
+        return compute();
     }
-    static variable_list backward(AutogradContext*, variable_list) {
-        raise(std::string(Op::kName) + ": second-order differentiation is not supported");
+    static variable_list backward(AutogradContext* ctx, variable_list) {
+        raise(ctx->saved_data["name"].toStringRef() + ": second-order differentiation is not supported");
     }
 };
+variable_list once_differentiable(const char* name, const variable_list& saved, const variable_list& grads,
+                                  const std::function<variable_list()>& compute) {
+    if (!at::GradMode::is_enabled()) return compute();
+    variable_list from;                           // a node's inputs have to be defined
+    for (const variable_list* l : {&saved, &grads})
+        for (const Tensor& t : *l)
+            if (t.defined()) from.push_back(t);
+    return Refuse::apply(at::TensorList(from), compute, std::string(name));
+}
 template <class Op>
 variable_list gradients_of(AutogradContext* ctx, const variable_list& grads) {
     const variable_list saved = ctx->get_saved_variables();
-    if (!at::GradMode::is_enabled()) return Op::gradients(saved, grads);
-    variable_list given = grads;                  // a node's inputs have to be defined
-    for (Tensor& g : given)
-        if (!g.defined()) g = fresh({0}, saved[0].scalar_type(), saved[0]);
-    return NoSecondOrder<Op>::apply(at::TensorList(saved), at::TensorList(given));
+    return once_differentiable(Op::kName, saved, grads, [&]() { return Op::gradients(saved, grads); });
 }
 
 // ------------------------------------------------------------------------------------------------- RWKV-7
@@ -383,6 +404,388 @@ Tensor step_packed(const Tensor* t /* r w k v a b */, const Tensor& state, int64
     return y;
 }
 
+// ------------------------------------------------------------------------------------------------- matrix products
+// The framework's GEMM library with the choice of its kernel made once per shape: at::mm makes it anew on every call, 10 us
+// of host time each, and a layer has 36 products.  Row-major operands; every pointer on a 16-byte boundary.
+class Gemm {
+    static constexpr size_t kWorkspace = 32 << 20;
+    static constexpr size_t kPlans = 512;             // per host thread; then the table starts over
+    struct Plan {
+        cublasLtMatmulDesc_t op = nullptr;
+        cublasLtMatrixLayout_t a = nullptr, b = nullptr, c = nullptr;
+        cublasLtMatmulAlgo_t algo;
+        ~Plan() {
+            if (a) cublasLtMatrixLayoutDestroy(a);
+            if (b) cublasLtMatrixLayoutDestroy(b);
+            if (c) cublasLtMatrixLayoutDestroy(c);
+            if (op) cublasLtMatmulDescDestroy(op);
+        }
+    };
+    typedef std::array<int64_t, 6> Key;               // device, m, n, k, form, type
+    struct Hash {
+        size_t operator()(const Key& k) const {
+            size_t h = 0;
+            for (int64_t x : k) h = h * 1000003 + (size_t)x;
+            return h;
+        }
+    };
+    Tensor workspace_;
+    cudaStream_t stream_;
+    cublasLtHandle_t handle_;
+    bool bf16_, tf32_;
+    int64_t device_;
+
+    static cublasLtHandle_t handle(int device) {
+        thread_local int current = -1;                // an autograd thread may not have made the device's context current yet
+        if (current != device) {
+            cuda_check(cudaSetDevice(device));
+            current = device;
+        }
+        return at::cuda::getCurrentCUDABlasLtHandle();
+    }
+    static void ok(cublasStatus_t s) {
+        if (s != CUBLAS_STATUS_SUCCESS) raise("b200wkv: matrix product failed (cublasLt status " + std::to_string((int)s) + ")");
+    }
+    std::shared_ptr<Plan> make(int64_t m, int64_t n, int64_t k, bool ta, bool tb) const {
+        auto p = std::make_shared<Plan>();
+        const cudaDataType_t type = bf16_ ? CUDA_R_16BF : CUDA_R_32F;
+        ok(cublasLtMatmulDescCreate(&p->op, tf32_ ? CUBLAS_COMPUTE_32F_FAST_TF32 : CUBLAS_COMPUTE_32F, CUDA_R_32F));
+        // the library is column-major: C^T = B^T A^T, so its first operand is B and its second A
+        const cublasOperation_t first = tb ? CUBLAS_OP_T : CUBLAS_OP_N, second = ta ? CUBLAS_OP_T : CUBLAS_OP_N;
+        ok(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSA, &first, sizeof(first)));
+        ok(cublasLtMatmulDescSetAttribute(p->op, CUBLASLT_MATMUL_DESC_TRANSB, &second, sizeof(second)));
+        ok(cublasLtMatrixLayoutCreate(&p->a, type, tb ? k : n, tb ? n : k, tb ? k : n));
+        ok(cublasLtMatrixLayoutCreate(&p->b, type, ta ? m : k, ta ? k : m, ta ? m : k));
+        ok(cublasLtMatrixLayoutCreate(&p->c, type, n, m, n));
+        cublasLtMatmulPreference_t pref;
+        ok(cublasLtMatmulPreferenceCreate(&pref));
+        const size_t ws = kWorkspace;
+        const uint32_t align = 16;
+        cublasLtMatmulPreferenceSetAttribute(pref, CUBLASLT_MATMUL_PREF_MAX_WORKSPACE_BYTES, &ws, sizeof(ws));
+        for (auto a : {CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_A_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_B_BYTES,
+                       CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_C_BYTES, CUBLASLT_MATMUL_PREF_MIN_ALIGNMENT_D_BYTES})
+            cublasLtMatmulPreferenceSetAttribute(pref, a, &align, sizeof(align));
+        cublasLtMatmulHeuristicResult_t found;
+        int n_found = 0;
+        const cublasStatus_t s = cublasLtMatmulAlgoGetHeuristic(handle_, p->op, p->a, p->b, p->c, p->c, pref, 1, &found, &n_found);
+        cublasLtMatmulPreferenceDestroy(pref);
+        ok(s);
+        if (n_found < 1) ok(CUBLAS_STATUS_NOT_SUPPORTED);
+        p->algo = found.algo;
+        return p;
+    }
+    void run(int64_t m, int64_t n, int64_t k, bool ta, bool tb, const void* A, const void* B, void* C, bool add) const {
+        thread_local std::unordered_map<Key, std::shared_ptr<Plan>, Hash> plans;
+        const Key key{device_, m, n, k, ta * 2 + tb, bf16_ * 2 + tf32_};
+        auto it = plans.find(key);
+        if (it == plans.end()) {
+            if (plans.size() >= kPlans) plans.clear();
+            it = plans.emplace(key, make(m, n, k, ta, tb)).first;
+        }
+        const Plan& p = *it->second;
+        const float alpha = 1.f, beta = add ? 1.f : 0.f;
+        ok(cublasLtMatmul(handle_, p.op, &alpha, B, p.a, A, p.b, &beta, C, p.c, C, p.c, &p.algo, out(workspace_), kWorkspace, stream_));
+    }
+
+   public:
+    Gemm(const Tensor& like, cudaStream_t st)
+        : workspace_(bytes(kWorkspace, like)), stream_(st), handle_(handle(like.device().index())),
+          bf16_(like.scalar_type() == at::kBFloat16), tf32_(!bf16_ && at::globalContext().allowTF32CuBLAS()), device_(like.device().index()) {}
+    // C (m, n) = A (m, k) B (k, n)
+    void nn(int64_t m, int64_t n, int64_t k, const void* A, const void* B, void* C) const { run(m, n, k, false, false, A, B, C, false); }
+    // C (m, n) [+]= A (m, k) B^T, B (n, k)
+    void nt(int64_t m, int64_t n, int64_t k, const void* A, const void* B, void* C, bool add = false) const { run(m, n, k, false, true, A, B, C, add); }
+    // C (m, n) = A^T B, A (k, m), B (k, n)
+    void tn(int64_t m, int64_t n, int64_t k, const void* A, const void* B, void* C) const { run(m, n, k, true, false, A, B, C, false); }
+};
+
+// ------------------------------------------------------------------------------------------------- time mixing
+// A whole RWKV-7 time-mixing layer as one node: the token shift, the projections (library GEMMs, as before), the elementwise
+// stage in front of the operator, the operator, the elementwise stage behind it.  As separate autograd functions and
+// torch ops the host needs 2.6 ms for a forward and backward whatever the size.  Here the intermediates of a pass share one
+// allocation, gradients of one tensor that meet from several places are added where a kernel reads or a GEMM
+// writes them anyway, the shift's six cotangents are written where its backward kernel reads them, and parameter
+// gradients leave one reduction kernel in their final type.
+struct Layer {
+    static constexpr const char* kName = "time_mixing_seq";
+    enum { kMix = 0, kWr = 6, kWk, kWv, kWo, kW1, kW2, kA1, kA2, kV1, kV2, kG1, kG2, kW0, kA0, kV0, kKk, kKa, kRk, kLnW, kLnB, kParams };
+    static constexpr int64_t kN = 64;
+
+    struct Dims {
+        int64_t B, T, C, H, rows;
+        bool first;                    // the first layer: no value mix
+        int64_t inner[4];              // widths of the low-rank projections w, a, v, g
+        Dims(const Tensor& x, const Tensor* p, int64_t H_, bool first_)
+            : B(x.size(0)), T(x.size(1)), C(x.size(2)), H(H_), rows(B * T), first(first_),
+              inner{p[kW1].size(1), p[kA1].size(1), first_ ? 0 : p[kV1].size(1), p[kG1].size(1)} {}
+    };
+    static constexpr float kEps = 64e-5f;
+
+    // One allocation cut into pieces of whole 256-byte lines.
+    struct Slab {
+        Tensor t;
+        int64_t esz, used = 0;
+        static int64_t padded(int64_t n, int64_t esz) { return (n * esz + 255) / 256 * 256; }
+        Slab(const Tensor& like, std::initializer_list<int64_t> pieces) : esz(like.element_size()) {
+            int64_t n = 0;
+            for (int64_t p : pieces) n += padded(p, esz);
+            t = bytes((size_t)n, like);
+        }
+        Slab(const Tensor& given, int64_t element) : t(given), esz(element) {}
+        void* take(int64_t n) {
+            void* p = (char*)out(t) + used;
+            used += padded(n, esz);
+            return p;
+        }
+    };
+    // The forward's intermediates, all in one slab: streams of (rows, C) and the low-rank hidden rows.
+    struct Inter {
+        void *mixed, *r, *k, *wl, *al, *vl, *g, *w, *kp, *vp, *ai, *bi, *y, *xo, *hidden[4];
+        static Slab make(const Tensor& x, const Dims& d) {
+            const int64_t n = d.rows * d.C;
+            return Slab(x, {6 * n, n, n, n, n, n, n, n, n, n, n, n, n, n, d.rows * d.inner[0], d.rows * d.inner[1], d.rows * d.inner[2],
+                            d.rows * d.inner[3]});
+        }
+        Inter(Slab s, const Dims& d) {
+            const int64_t n = d.rows * d.C;
+            mixed = s.take(6 * n);
+            for (void** p : {&r, &k, &wl, &al, &vl, &g, &w, &kp, &vp, &ai, &bi, &y, &xo}) *p = s.take(n);
+            for (int i = 0; i < 4; ++i) hidden[i] = s.take(d.rows * d.inner[i]);
+        }
+    };
+    static void* at(void* p, int64_t elements, const Tensor& x) { return (char*)p + elements * x.element_size(); }
+
+    // rows `first`.. of every sequence's (1 + N, C) state block as a dense array, and back (no copy where they are dense)
+    static const void* dense_rows(const Tensor& state, int64_t first, int64_t n, Tensor& room, cudaStream_t st) {
+        const int64_t C = state.size(2), e = state.element_size(), pitch = state.size(1) * C * e;
+        const char* src = (const char*)in(state) + first * C * e;
+        if (state.size(0) == 1) return src;
+        room = fresh({state.size(0), n, C}, state.scalar_type(), state);
+        cuda_check(cudaMemcpy2DAsync(out(room), n * C * e, src, pitch, n * C * e, state.size(0), cudaMemcpyDeviceToDevice, st));
+        return in(room);
+    }
+    struct Landing {                   // where a kernel writes a dense array that belongs into rows of a state
+        Tensor state, room;
+        int64_t first, n;
+        void* p;
+        Landing(const Tensor& s, int64_t first_, int64_t n_) : state(s), first(first_), n(n_) {
+            if (s.size(0) > 1) room = fresh({s.size(0), n, s.size(2)}, s.scalar_type(), s);
+            p = room.defined() ? out(room) : place();
+        }
+        void* place() const { return (char*)out(state) + first * state.size(2) * state.element_size(); }
+        void finish(cudaStream_t st) const {
+            if (!room.defined()) return;
+            const int64_t row = state.size(2) * state.element_size();
+            cuda_check(cudaMemcpy2DAsync(place(), state.size(1) * row, in(room), n * row, n * row, state.size(0), cudaMemcpyDeviceToDevice, st));
+        }
+    };
+
+    static bool fits(const Tensor& x, const Tensor& state, const Tensor& v_first, const Tensor* p, int64_t H, int64_t S, bool first) {
+        if (x.dim() != 3 || state.dim() != 3 || S != kN || H < 1 || H > 128) return false;
+        const int64_t B = x.size(0), C = x.size(2);
+        const Tensor t[] = {x, state, v_first};
+        if (C != H * S || B > 65535 || x.size(0) * x.size(1) > 2147483647 / 8 || !same_kind(t, 3) || !sizes_are(state, {}, {B, 1 + S, C}) ||
+            !v_first.sizes().equals(x.sizes()))
+            return false;
+        for (int i = 0; i < kParams; ++i) {
+            if (first && (i == kV0 || i == kV1 || i == kV2)) continue;
+            if (!p[i].defined() || p[i].scalar_type() != x.scalar_type() || p[i].device() != x.device() || !p[i].is_contiguous() ||
+                (uintptr_t)in(p[i]) % 16 != 0)
+                return false;
+            if (i >= kWr && i <= kWo) {
+                if (!sizes_are(p[i], {}, {C, C})) return false;
+            } else if (i >= kW1 && i <= kG2) {
+                if (p[i].dim() != 2 || p[i].numel() == 0) return false;
+                const bool down = (i - kW1) % 2 == 0;
+                if (p[i].size(down ? 0 : 1) != C || p[i].size(down ? 1 : 0) != p[down ? i + 1 : i - 1].size(down ? 0 : 1)) return false;
+            } else if (p[i].numel() != C) {
+                return false;
+            }
+        }
+        return true;
+    }
+
+    struct Kept {                      // what the backward needs beside the parameters
+        Tensor x, state, v_first, v, slab, length, starts, residual;
+    };
+
+    // returns (out (B, T, C), new_state)
+    static std::pair<Tensor, Tensor> forward(const Dims& d, const Tensor& x_, const Tensor& state_, const Tensor& v_first, const Tensor* p,
+                                             const Tensor& length, const Tensor& starts, bool residual, Kept& kept) {
+        const c10::cuda::CUDAGuard guard(x_.device());
+        const cudaStream_t st = stream_of(x_);
+        const int code = dtype_code(x_), B = (int)d.B, T = (int)d.T, C = (int)d.C, H = (int)d.H;
+        const Flags f(length, starts, {d.B}, d.T, x_);
+        const Tensor x = x_.contiguous(), state = state_.contiguous();
+        kept = {x, state, d.first ? Tensor() : v_first.contiguous(), fresh({d.B, d.T, d.C}, x.scalar_type(), x), Inter::make(x, d).t, f.length,
+                f.starts, Tensor()};
+        const Inter q(Slab(kept.slab, x.element_size()), d);
+        Gemm gemm(x, st);
+        Tensor room[2], new_state = fresh_like(state), o = fresh({d.B, d.T, d.C}, x.scalar_type(), x);
+        const void* prev = dense_rows(state, 0, 1, room[0], st);
+        const void* s0 = dense_rows(state, 1, kN, room[1], st);
+        const Landing shift_row(new_state, 0, 1), s_out(new_state, 1, kN);
+        const void* mix[6];
+        for (int i = 0; i < 6; ++i) mix[i] = in(p[kMix + i]);
+        check(b200wkv::token_shift_fwd(st, code, B, T, C, 6, in(x), prev, mix, (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), q.mixed,
+                                       shift_row.p));
+        shift_row.finish(st);
+        void* m[6];                    // the inputs of r, w, k, v, a, g
+        for (int i = 0; i < 6; ++i) m[i] = at(q.mixed, i * d.rows * d.C, x);
+        void* const v = out(kept.v);
+        gemm.nt(d.rows, d.C, d.C, m[0], in(p[kWr]), q.r);
+        gemm.nt(d.rows, d.C, d.C, m[2], in(p[kWk]), q.k);
+        gemm.nt(d.rows, d.C, d.C, m[3], in(p[kWv]), v);
+        const auto lora = [&](int which, int down, void* input, int act, void* to) {
+            gemm.nn(d.rows, d.inner[which], d.C, input, in(p[down]), q.hidden[which]);
+            if (act) check(b200wkv::activation(st, code, act, d.rows * d.inner[which], q.hidden[which], nullptr));
+            gemm.nn(d.rows, d.C, d.inner[which], q.hidden[which], in(p[down + 1]), to);
+        };
+        lora(0, kW1, m[1], b200wkv::kTanh, q.wl);
+        lora(1, kA1, m[4], 0, q.al);
+        if (!d.first) lora(2, kV1, m[3], 0, q.vl);
+        lora(3, kG1, m[5], b200wkv::kSigmoid, q.g);
+        check(b200wkv7_mix_pre_fwd(st, code, d.rows, H, (int)kN, !d.first, q.k, q.wl, q.al, v, in(kept.v_first), d.first ? nullptr : q.vl, in(p[kW0]),
+                                   in(p[kA0]), in(p[kV0]), in(p[kKk]), in(p[kKa]), q.w, q.kp, q.vp, q.ai, q.bi));
+        const size_t rbytes = residual ? b200wkv7_residual_bytes(code, B, T, H, (int)kN) : 0;
+        if (residual) kept.residual = bytes(rbytes, x);
+        check(b200wkv7_fwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(f.length),
+                           (const uint8_t*)in(f.starts), q.y, s_out.p, out(kept.residual), rbytes, 0));
+        s_out.finish(st);
+        check(b200wkv7_mix_post_fwd(st, code, d.rows, H, (int)kN, kEps, q.y, q.r, q.kp, q.vp, q.g, in(p[kLnW]), in(p[kLnB]), in(p[kRk]), q.xo));
+        gemm.nt(d.rows, d.C, d.C, q.xo, in(p[kWo]), out(o));
+        return {o, new_state};
+    }
+
+    // grads: of out, new_state and (first layer) v.  Returns gradients of x, state, v_first and the parameters;
+    // `wanted` says which of them anybody asked for.
+    static variable_list gradients(const Dims& d, const Kept& kept, const Tensor* p, const variable_list& grads, const std::vector<bool>& wanted) {
+        const Tensor& x = kept.x;
+        const c10::cuda::CUDAGuard guard(x.device());
+        const cudaStream_t st = stream_of(x);
+        const int code = dtype_code(x), B = (int)d.B, T = (int)d.T, C = (int)d.C, H = (int)d.H;
+        const int64_t n = d.rows * d.C, widest = std::max(std::max(d.inner[0], d.inner[1]), std::max(d.inner[2], d.inner[3]));
+        const Inter q(Slab(kept.slab, x.element_size()), d);
+        Gemm gemm(x, st);
+        variable_list g(3 + kParams);
+        const auto want = [&](int i) { return (bool)wanted[3 + i]; };
+        // d W of y = input W (or input W^T where the weight is kept transposed): a sum over the rows
+        const auto weight = [&](int i, int64_t a, int64_t b, const void* left, const void* right) {
+            if (!want(i)) return;
+            g[3 + i] = fresh({a, b}, x.scalar_type(), x);
+            gemm.tn(a, b, d.rows, left, right, out(g[3 + i]));
+        };
+        const Tensor gout = cotangent(grads[0], x), gstate = cotangent(grads[1], x);
+        Slab room(x, {6 * n, n, n, n, n, n, n, n, n, n, n, n, n, n, d.rows * widest});
+        void* const gmixed = room.take(6 * n);
+        void *gxo, *dr, *dkp, *dvp, *dg, *gr, *gw, *gk, *gv, *ga, *gb, *dvl, *dwl;
+        for (void** b : {&gxo, &dr, &dkp, &dvp, &dg, &gr, &gw, &gk, &gv, &ga, &gb, &dvl, &dwl}) *b = room.take(n);
+        void* const dh = room.take(d.rows * widest);
+        void* m[6];                    // the inputs of r, w, k, v, a, g, and their cotangents where the shift's backward reads them
+        void* gm[6];
+        for (int i = 0; i < 6; ++i) {
+            m[i] = at(q.mixed, i * n, x);
+            gm[i] = at(gmixed, i * n, x);
+        }
+        const int n_part = b200wkv7_mix_partial_rows(d.rows, H, (int)kN), tiles = (T + B200WKV_SHIFT_TILE - 1) / B200WKV_SHIFT_TILE;
+        const Tensor partial = fresh({(int64_t)n_part * 8 + d.B * tiles * 6, d.C}, at::kFloat, x);
+        float* const part_pre = (float*)out(partial);
+        float* const part_post = part_pre + (size_t)n_part * 5 * d.C;
+        float* const part_mix = part_post + (size_t)n_part * 3 * d.C;
+
+        gemm.nn(d.rows, d.C, d.C, in(gout), in(p[kWo]), gxo);
+        weight(kWo, d.C, d.C, in(gout), q.xo);
+        void* const dy = gm[0];        // gmixed is room until its parts are written, last of all
+        check(b200wkv7_mix_post_bwd(st, code, d.rows, H, (int)kN, kEps, q.y, q.r, q.kp, q.vp, q.g, in(p[kLnW]), in(p[kLnB]), in(p[kRk]), gxo, dy, dr,
+                                    dkp, dvp, dg, part_post));
+        Tensor copies[2];
+        const void* s0 = dense_rows(kept.state, 1, kN, copies[0], st);
+        const void* gs = dense_rows(gstate, 1, kN, copies[1], st);
+        if (wanted[1]) g[1] = fresh_like(kept.state);
+        const Tensor state_room = wanted[1] ? g[1] : fresh_like(kept.state);
+        const Landing gprev(state_room, 0, 1), gs0(state_room, 1, kN);
+        check(b200wkv7_bwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(kept.length),
+                           (const uint8_t*)in(kept.starts), dy, gs, out(kept.residual), (size_t)kept.residual.numel(), gw, gr, gk, gv, ga, gb, gs0.p, 0));
+        if (wanted[1]) gs0.finish(st);
+        // r, k' and v' also feed the stage behind the operator: its shares (dr, dkp, dvp) are added where the next kernel reads
+        // anyway (gr in place)
+        const Tensor gv_out = d.first ? cotangent(grads[2], x) : Tensor();
+        void *const dk = gxo, *const dal = gm[1], *const dv = gm[2];
+        if (!d.first && wanted[2]) g[2] = fresh({d.B, d.T, d.C}, x.scalar_type(), x);
+        void* const dvf = d.first ? nullptr : g[2].defined() ? out(g[2]) : gm[3];
+        check(b200wkv::wkv7_mix_pre_bwd(st, code, (int)d.rows, C, !d.first, q.k, q.wl, q.al, in(kept.v), in(kept.v_first), q.vl, in(p[kW0]), in(p[kA0]),
+                                        in(p[kV0]), in(p[kKk]), in(p[kKa]), gw, gk, gv, ga, gb, dk, dwl, dal, dv, dvf, dvl, part_pre,
+                                        {dkp, dvp, in(gv_out), dr, gr}));
+        // dal and dv lie in parts of gmixed that the products below fill: the products that read them come first
+        const auto lora = [&](int which, int down, const void* up_grad, const void* input, void* into, int act, bool add) {
+            weight(down + 1, d.inner[which], d.C, q.hidden[which], up_grad);
+            gemm.nt(d.rows, d.inner[which], d.C, up_grad, in(p[down + 1]), dh);
+            if (act) check(b200wkv::activation(st, code, act, d.rows * d.inner[which], dh, q.hidden[which]));
+            weight(down, d.C, d.inner[which], input, dh);
+            gemm.nt(d.rows, d.C, d.inner[which], dh, in(p[down]), into, add);
+        };
+        lora(1, kA1, dal, m[4], gm[4], 0, false);
+        weight(kWv, d.C, d.C, dv, m[3]);
+        gemm.nn(d.rows, d.C, d.C, dv, in(p[kWv]), gm[3]);
+        if (!d.first) lora(2, kV1, dvl, m[3], gm[3], 0, true);
+        weight(kWr, d.C, d.C, gr, m[0]);
+        gemm.nn(d.rows, d.C, d.C, gr, in(p[kWr]), gm[0]);
+        weight(kWk, d.C, d.C, dk, m[2]);
+        gemm.nn(d.rows, d.C, d.C, dk, in(p[kWk]), gm[2]);
+        lora(0, kW1, dwl, m[1], gm[1], b200wkv::kTanh, false);
+        lora(3, kG1, dg, m[5], gm[5], b200wkv::kSigmoid, false);
+
+        const Tensor gx = fresh({d.B, d.T, d.C}, x.scalar_type(), x);
+        const void* mix[6];
+        for (int i = 0; i < 6; ++i) mix[i] = in(p[kMix + i]);
+        Tensor rows0[2];
+        const void* prev = dense_rows(kept.state, 0, 1, rows0[0], st);
+        const void* gstate0 = dense_rows(gstate, 0, 1, rows0[1], st);
+        check(b200wkv::token_shift_bwd(st, code, B, T, C, 6, in(x), prev, mix, (const uint32_t*)in(kept.length), (const uint8_t*)in(kept.starts), gmixed,
+                                       gstate0, out(gx), gprev.p, part_mix));
+        if (wanted[0]) g[0] = gx;
+        if (wanted[1]) gprev.finish(st);
+        // parameter gradients: column sums of the kernels' partial rows
+        const Tensor sums = fresh({14, d.C}, x.scalar_type(), x);
+        const auto row = [&](int i) { return at(out(sums), i * d.C, x); };
+        check(b200wkv::column_sums(st, code, d.B * tiles, 6 * C, part_mix, row(0)));
+        check(b200wkv::column_sums(st, code, n_part, 5 * C, part_pre, row(6)));
+        check(b200wkv::column_sums(st, code, n_part, 3 * C, part_post, row(11)));
+        const int order[14] = {kMix, kMix + 1, kMix + 2, kMix + 3, kMix + 4, kMix + 5, kW0, kA0, kV0, kKk, kKa, kLnW, kLnB, kRk};
+        for (int i = 0; i < 14; ++i)
+            if (want(order[i]) && p[order[i]].defined()) g[3 + order[i]] = sums[i].view(p[order[i]].sizes());
+        return g;
+    }
+};
+
+struct LayerNode : public torch::autograd::Function<LayerNode> {
+    static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& state, const Tensor& v_first, at::TensorList params,
+                                 const Tensor& length, const Tensor& starts, int64_t H, bool first) {
+        const Layer::Dims d(x, params.data(), H, first);
+        Layer::Kept k;
+        auto [o, new_state] = Layer::forward(d, x, state, v_first, params.data(), length, starts, true, k);
+        variable_list keep(params.begin(), params.end());
+        for (const Tensor& t : {k.x, k.state, k.v_first, k.v, k.slab, k.length, k.starts, k.residual}) keep.push_back(t);
+        ctx->saved_data["H"] = H;
+        ctx->saved_data["first"] = first;
+        ctx->save_for_backward(keep);
+        if (first) return {o, new_state, k.v};
+        return {o, new_state};
+    }
+    static variable_list backward(AutogradContext* ctx, variable_list grads) {
+        const variable_list saved = ctx->get_saved_variables();
+        const bool first = ctx->saved_data["first"].toBool();
+        const Tensor* s = saved.data() + Layer::kParams;
+        const Layer::Kept k{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7]};
+        const Layer::Dims d(k.x, saved.data(), ctx->saved_data["H"].toInt(), first);
+        std::vector<bool> wanted(3 + Layer::kParams);
+        for (int j = 0; j < 3 + Layer::kParams; ++j) wanted[j] = ctx->needs_input_grad(j);
+        variable_list g = once_differentiable(Layer::kName, saved, grads, [&]() { return Layer::gradients(d, k, saved.data(), grads, wanted); });
+        g.resize(3 + Layer::kParams + 4);
+        return g;
+    }
+};
+
 // ------------------------------------------------------------------------------------------------- Python
 bool take(PyObject* const* args, int n, Tensor* to) {
     for (int i = 0; i < n; ++i) {
@@ -458,6 +861,53 @@ PyObject* py_wkv4(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (r or N
     END_HANDLE_TH_ERRORS
 }
 
+// (x, state, v_first, att, length, new_starts, H, S, layer_id) -> (out, new_state, v_first)
+PyObject* py_time_mixing(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    static const char* const kNames[Layer::kParams] = {"x_r", "x_w", "x_k", "x_v", "x_a", "x_g", "receptance", "key", "value", "output",
+                                                       "w1", "w2", "a1", "a2", "v1", "v2", "g1", "g2", "w0", "a0", "v0", "k_k", "k_a", "r_k",
+                                                       "ln_x", "ln_x"};
+    Tensor t[3], flags[2], p[Layer::kParams];
+    if (n != 9 || !take(args, 3, t) || !PyDict_CheckExact(args[3]) || !take(args + 4, 2, flags) || at::autocast::is_autocast_enabled(at::kCUDA))
+        Py_RETURN_NONE;
+    for (int i = 6; i < 9; ++i)
+        if (!PyLong_CheckExact(args[i])) Py_RETURN_NONE;
+    const int64_t H = PyLong_AsLongLong(args[6]), S = PyLong_AsLongLong(args[7]);
+    const bool first = PyLong_AsLongLong(args[8]) == 0;
+    for (int i = 0; i < Layer::kParams; ++i) {
+        if (first && (i == Layer::kV0 || i == Layer::kV1 || i == Layer::kV2)) continue;      // not used by the first layer
+        PyObject* item = PyDict_GetItemString(args[3], kNames[i]);
+        if (item && ((i >= Layer::kWr && i <= Layer::kWo) || i >= Layer::kLnW))
+            item = PyDict_CheckExact(item) ? PyDict_GetItemString(item, i == Layer::kLnB ? "bias" : "weight") : nullptr;
+        if (!item || !take(&item, 1, &p[i])) Py_RETURN_NONE;
+    }
+    if (!Layer::fits(t[0], t[1], t[2], p, H, S, first)) Py_RETURN_NONE;
+    Tensor o, new_state, v;
+    {
+        pybind11::gil_scoped_release no_gil;
+        const Tensor vf = first ? Tensor() : t[2];
+        if (any_grad(t, first ? 2 : 3) || any_grad_defined(p, Layer::kParams)) {
+            variable_list r = LayerNode::apply(t[0], t[1], vf, at::TensorList(p, Layer::kParams), flags[0], flags[1], H, first);
+            o = r[0]; new_state = r[1];
+            if (first) v = r[2];
+        } else {
+            const at::AutoGradMode no_grad(false);
+            const Layer::Dims d(t[0], p, H, first);
+            Layer::Kept k;
+            std::tie(o, new_state) = Layer::forward(d, t[0], t[1], vf, p, flags[0], flags[1], false, k);
+            v = k.v;
+        }
+    }
+    THPObjectPtr tuple(PyTuple_New(3));
+    if (!tuple) throw python_error();
+    PyTuple_SET_ITEM(tuple.get(), 0, THPVariable_Wrap(o));
+    PyTuple_SET_ITEM(tuple.get(), 1, THPVariable_Wrap(new_state));
+    if (!first) Py_INCREF(args[2]);
+    PyTuple_SET_ITEM(tuple.get(), 2, first ? THPVariable_Wrap(v) : args[2]);
+    return tuple.release();
+    END_HANDLE_TH_ERRORS
+}
+
 PyObject* py_step_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (r, w, k, v, a, b, state, layer, new_starts, length)
     HANDLE_TH_ERRORS
     Tensor t[7], starts, length, y;
@@ -485,6 +935,7 @@ PyMethodDef kMethods[] = {
     {"wkv7", (PyCFunction)(void (*)(void))py_wkv7, METH_FASTCALL, nullptr},
     {"wkv6", (PyCFunction)(void (*)(void))py_wkv6, METH_FASTCALL, nullptr},
     {"wkv4", (PyCFunction)(void (*)(void))py_wkv4, METH_FASTCALL, nullptr},
+    {"time_mixing", (PyCFunction)(void (*)(void))py_time_mixing, METH_FASTCALL, nullptr},
     {"step_packed", (PyCFunction)(void (*)(void))py_step_packed, METH_FASTCALL, nullptr},
     {"set_error_class", py_set_error_class, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};

@@ -7,11 +7,13 @@
 // One pass over x, M outputs: purely HBM-bound, so every thread moves V channels per access with
 // V = 16 bytes / element size when the channel count allows it (else V = 4).
 #include "common.cuh"
+#include "host_calls.h"
 
 namespace b200wkv {
 namespace {
 
 template <int V> struct Vec { float f[V]; };
+struct MixPtrs { const void* p[8]; };   // one row of D coefficients each
 
 template <int V, typename T> __device__ __forceinline__ Vec<V> loadv(const T* p);
 template <> __device__ __forceinline__ Vec<4> loadv<4, float>(const float* p) {
@@ -90,7 +92,7 @@ __device__ __forceinline__ int last_row(uint32_t length, int Tlen) {
 // grid (B*T, ceil(D / V / 128)); one token row per blockIdx.x
 template <typename T, int V>
 __global__ void token_shift_fwd_kernel(int B, int Tlen, int D, int M, const T* __restrict__ x, const T* __restrict__ prev,
-                                       const T* __restrict__ mix, const uint32_t* __restrict__ length,
+                                       const MixPtrs mix, const uint32_t* __restrict__ length,
                                        const uint8_t* __restrict__ new_starts, T* __restrict__ out,
                                        T* __restrict__ state_out) {
     const int d = (blockIdx.y * blockDim.x + threadIdx.x) * V;
@@ -103,8 +105,10 @@ __global__ void token_shift_fwd_kernel(int B, int Tlen, int D, int M, const T* _
     if (!new_starts[bt]) df = (t == 0) ? loadv<V>(prev + (size_t)bi * D + d) : loadv<V>(x + row - D);
 #pragma unroll
     for (int i = 0; i < V; ++i) df.f[i] -= xc.f[i];
-    for (int m = 0; m < M; ++m) {
-        const Vec<V> c = loadv<V>(mix + (size_t)m * D + d);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        if (m >= M) break;
+        const Vec<V> c = loadv<V>((const T*)mix.p[m] + d);
         Vec<V> o;
 #pragma unroll
         for (int i = 0; i < V; ++i) o.f[i] = fmaf(df.f[i], c.f[i], xc.f[i]);
@@ -121,7 +125,7 @@ __global__ void token_shift_fwd_kernel(int B, int Tlen, int D, int M, const T* _
 template <typename T, int V, int MM>
 __global__ void __launch_bounds__(64)
 token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T* __restrict__ prev,
-                       const T* __restrict__ mix, const uint32_t* __restrict__ length,
+                       const MixPtrs mix, const uint32_t* __restrict__ length,
                        const uint8_t* __restrict__ new_starts, const T* __restrict__ gout,
                        const T* __restrict__ gstate, T* __restrict__ gx, T* __restrict__ gprev,
                        float* __restrict__ gmix) {
@@ -136,7 +140,7 @@ token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T*
     Vec<V> acc[MM];
 #pragma unroll
     for (int m = 0; m < MM; ++m) {
-        craw[m].load(mix + (size_t)m * D + d);
+        craw[m].load((const T*)mix.p[m] + d);
         acc[m] = zerov<V>();
     }
     const size_t base = (size_t)bi * Tlen * D + d;
@@ -211,24 +215,24 @@ token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T*
 }
 
 template <typename T, int V>
-void launch_fwd(cudaStream_t st, int B, int Tlen, int D, int M, const void* x, const void* prev, const void* mix,
+void launch_fwd(cudaStream_t st, int B, int Tlen, int D, int M, const void* x, const void* prev, const MixPtrs& mix,
                 const uint32_t* length, const uint8_t* ns, void* out, void* state_out) {
     dim3 grid(B * Tlen, (D / V + 127) / 128);
-    token_shift_fwd_kernel<T, V><<<grid, 128, 0, st>>>(B, Tlen, D, M, (const T*)x, (const T*)prev, (const T*)mix, length, ns,
+    token_shift_fwd_kernel<T, V><<<grid, 128, 0, st>>>(B, Tlen, D, M, (const T*)x, (const T*)prev, mix, length, ns,
                                                        (T*)out, (T*)state_out);
 }
 
 template <typename T, int V, int MM>
-void launch_bwd_m(cudaStream_t st, int B, int Tlen, int D, const void* x, const void* prev, const void* mix,
+void launch_bwd_m(cudaStream_t st, int B, int Tlen, int D, const void* x, const void* prev, const MixPtrs& mix,
                   const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate, void* gx, void* gprev,
                   void* gmix) {
     dim3 grid((D / V + 63) / 64, (Tlen + B200WKV_SHIFT_TILE - 1) / B200WKV_SHIFT_TILE, B);
-    token_shift_bwd_kernel<T, V, MM><<<grid, 64, 0, st>>>(B, Tlen, D, (const T*)x, (const T*)prev, (const T*)mix, length, ns,
+    token_shift_bwd_kernel<T, V, MM><<<grid, 64, 0, st>>>(B, Tlen, D, (const T*)x, (const T*)prev, mix, length, ns,
                                                           (const T*)gout, (const T*)gstate, (T*)gx, (T*)gprev, (float*)gmix);
 }
 
 template <typename T, int V>
-void launch_bwd(cudaStream_t st, int B, int Tlen, int D, int M, const void* x, const void* prev, const void* mix,
+void launch_bwd(cudaStream_t st, int B, int Tlen, int D, int M, const void* x, const void* prev, const MixPtrs& mix,
                 const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate, void* gx, void* gprev,
                 void* gmix) {
 #define B200WKV_SHIFT_CASE(MM) \
@@ -242,19 +246,23 @@ void launch_bwd(cudaStream_t st, int B, int Tlen, int D, int M, const void* x, c
 }  // namespace
 
 int token_shift_fwd(cudaStream_t st, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
-                    const void* mix, const uint32_t* length, const uint8_t* ns, void* out, void* state_out) {
-    if (dtype == B200WKV_F32) launch_fwd<float, 4>(st, B, T, D, M, x, prev, mix, length, ns, out, state_out);
-    else if (D % 8 == 0) launch_fwd<__nv_bfloat16, 8>(st, B, T, D, M, x, prev, mix, length, ns, out, state_out);
-    else launch_fwd<__nv_bfloat16, 4>(st, B, T, D, M, x, prev, mix, length, ns, out, state_out);
+                    const void* const* mix, const uint32_t* length, const uint8_t* ns, void* out, void* state_out) {
+    MixPtrs rows;
+    for (int m = 0; m < 8; ++m) rows.p[m] = mix[m < M ? m : 0];
+    if (dtype == B200WKV_F32) launch_fwd<float, 4>(st, B, T, D, M, x, prev, rows, length, ns, out, state_out);
+    else if (D % 8 == 0) launch_fwd<__nv_bfloat16, 8>(st, B, T, D, M, x, prev, rows, length, ns, out, state_out);
+    else launch_fwd<__nv_bfloat16, 4>(st, B, T, D, M, x, prev, rows, length, ns, out, state_out);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 int token_shift_bwd(cudaStream_t st, int dtype, int B, int T, int D, int M, const void* x, const void* prev,
-                    const void* mix, const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate,
+                    const void* const* mix, const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate,
                     void* gx, void* gprev, void* gmix) {
-    if (dtype == B200WKV_F32) launch_bwd<float, 4>(st, B, T, D, M, x, prev, mix, length, ns, gout, gstate, gx, gprev, gmix);
-    else if (D % 8 == 0) launch_bwd<__nv_bfloat16, 8>(st, B, T, D, M, x, prev, mix, length, ns, gout, gstate, gx, gprev, gmix);
-    else launch_bwd<__nv_bfloat16, 4>(st, B, T, D, M, x, prev, mix, length, ns, gout, gstate, gx, gprev, gmix);
+    MixPtrs rows;
+    for (int m = 0; m < 8; ++m) rows.p[m] = mix[m < M ? m : 0];
+    if (dtype == B200WKV_F32) launch_bwd<float, 4>(st, B, T, D, M, x, prev, rows, length, ns, gout, gstate, gx, gprev, gmix);
+    else if (D % 8 == 0) launch_bwd<__nv_bfloat16, 8>(st, B, T, D, M, x, prev, rows, length, ns, gout, gstate, gx, gprev, gmix);
+    else launch_bwd<__nv_bfloat16, 4>(st, B, T, D, M, x, prev, rows, length, ns, gout, gstate, gx, gprev, gmix);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 

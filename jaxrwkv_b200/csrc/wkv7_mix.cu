@@ -17,6 +17,7 @@
 // per-head sums with three shuffles.  Everything is computed in fp32 whatever the element type.
 #include "common.cuh"
 #include "device_once.cuh"
+#include "host_calls.h"
 
 namespace b200wkv {
 
@@ -86,6 +87,14 @@ template <> struct Raw<__nv_bfloat16> {
         }
     }
 };
+
+template <typename T>
+__device__ __forceinline__ void add8(const Raw<T>& q, float* f) {
+    float x[8];
+    q.get(x);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] += x[e];
+}
 
 __device__ __forceinline__ float head_sum(float x) {   // over the eight lanes that hold one head of one row
     x += __shfl_xor_sync(0xffffffffu, x, 1);
@@ -187,7 +196,7 @@ mix_pre_bwd_kernel(int rows, int C, int use_vmix, const T* __restrict__ k, const
                    const T* __restrict__ k_k, const T* __restrict__ k_a, const T* __restrict__ gw, const T* __restrict__ gkp,
                    const T* __restrict__ gvp, const T* __restrict__ gai, const T* __restrict__ gbi, T* __restrict__ dk,
                    T* __restrict__ dwl, T* __restrict__ dal, T* __restrict__ dv, T* __restrict__ dvf, T* __restrict__ dvl,
-                   float* __restrict__ partial) {
+                   float* __restrict__ partial, const MixPreExtra extra) {
     const Walk wk = make_walk(C);
     if (!wk.live) return;
     float pw0[8], pa0[8], pv0[8], pkk[8], pka[8];
@@ -204,9 +213,22 @@ mix_pre_bwd_kernel(int rows, int C, int use_vmix, const T* __restrict__ k, const
         qk.load(k + off); qa.load(al + off); qgk.load(gkp + off); qgai.load(gai + off); qgbi.load(gbi + off);
         qw.load(wl + off); qgw.load(gw + off); qgv.load(gvp + off);
         if (use_vmix) { qv.load(v + off); qf.load(vf + off); ql.load(vl + off); }
+        Raw<T> qgk2, qgv2, qr, qr2, qgo;
+        if (extra.gkp2) qgk2.load((const T*)extra.gkp2 + off);
+        if (extra.gvp2) qgv2.load((const T*)extra.gvp2 + off);
+        if (extra.gr) { qr.load((const T*)extra.gr + off); qr2.load((const T*)extra.dr + off); }
+        if (extra.gv_out) qgo.load((const T*)extra.gv_out + off);
+        if (extra.gr) {
+            float a[8], b[8];
+            qr.get(a); qr2.get(b);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) a[e] += b[e];
+            if (in) store8((T*)extra.gr + off, a);
+        }
         {   // the key / a group
             float xk[8], xa[8], g_kp[8], g_ai[8], g_bi[8];
             qk.get(xk); qa.get(xa); qgk.get(g_kp); qgai.get(g_ai); qgbi.get(g_bi);
+            if (extra.gkp2) add8(qgk2, g_kp);
             float u[8], n2 = 0.f;
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
@@ -252,6 +274,8 @@ mix_pre_bwd_kernel(int rows, int C, int use_vmix, const T* __restrict__ k, const
         {   // the value
             float g_vp[8];
             qgv.get(g_vp);
+            if (extra.gvp2) add8(qgv2, g_vp);
+            if (!use_vmix && extra.gv_out) add8(qgo, g_vp);
             if (use_vmix) {
                 float xv[8], xf[8], xl[8], o_dv[8], o_dvf[8], o_dvl[8];
                 qv.get(xv); qf.get(xf); ql.get(xl);
@@ -385,26 +409,79 @@ mix_post_bwd_kernel(int rows, int C, float eps, const T* __restrict__ y, const T
         else KERNEL<T, 1024><<<g.grid, g.block, 0, st>>>(__VA_ARGS__);                    \
     } while (0)
 
+// Column sums of fp32 partial rows: a block owns 32 columns, its eight warps every eighth row, added in a fixed order.
+template <typename T>
+__global__ void __launch_bounds__(256) column_sums_kernel(int rows, int cols, const float* __restrict__ partial, T* __restrict__ out) {
+    __shared__ float part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    if (c < cols)
+        for (int r = warp; r < rows; r += 32)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (r + 8 * j < rows) s[j] += partial[(size_t)(r + 8 * j) * cols + c];
+    part[warp][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    if (warp == 0 && c < cols) {
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) t += part[w][lane];
+        out[c] = from_f32<T>(t);
+    }
+}
+
+// The activations between the two products of a low-rank projection (few, narrow rows).
+template <typename T>
+__global__ void __launch_bounds__(256) activation_kernel(int act, long long n, T* __restrict__ x, const T* __restrict__ y) {
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const float a = to_f32(x[i]);
+    float o;
+    if (y == nullptr) o = act == kTanh ? tanhf(a) : 1.f / (1.f + expf(-a));
+    else {
+        const float h = to_f32(y[i]);
+        o = a * (act == kTanh ? 1.f - h * h : h * (1.f - h));
+    }
+    x[i] = from_f32<T>(o);
+}
+
 struct Geometry {
     int block, slots, grid;
 };
 // Threads per row = C / 8; a block holds as many rows side by side as fit ~256 threads; the grid is what is
-// resident at once (the walk is grid-strided), capped by the number of row groups.
-Geometry geometry(int rows, int C) {
+// resident at once (the walk is grid-strided), capped by the number of row groups.  The backward kernels are compiled for
+// MIX_THREADS_PER_SM resident threads, and every block of theirs leaves a partial row of parameter gradients: more blocks
+// than fit would not run sooner, only write and read more partial rows (at 4096 rows of 2048 channels, 1184 blocks of which
+// 296 fit left 77 MB of them beside 450 MB of streams).
+Geometry geometry(int rows, int C, int threads_per_sm) {
     Geometry g;
     const int per_row = C / kOct;
     g.slots = per_row >= 256 ? 1 : 256 / per_row;
     g.block = per_row * g.slots;
     const long long groups = ((long long)rows + g.slots - 1) / g.slots;
-    const long long resident = (long long)sm_count_of_current_device() * (2048 / g.block > 0 ? 2048 / g.block : 1);
+    const long long resident = (long long)sm_count_of_current_device() * (threads_per_sm / g.block > 0 ? threads_per_sm / g.block : 1);
     g.grid = (int)(groups < resident ? groups : resident);
     return g;
 }
 
 }  // namespace
 
+int column_sums(cudaStream_t st, int dtype, long long rows, long long cols, const float* partial, void* out) {
+    const int grid = (int)((cols + 31) / 32);
+    if (dtype == B200WKV_F32) column_sums_kernel<float><<<grid, 256, 0, st>>>((int)rows, (int)cols, partial, (float*)out);
+    else column_sums_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((int)rows, (int)cols, partial, (__nv_bfloat16*)out);
+    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+}
+
+int activation(cudaStream_t st, int dtype, int act, long long n, void* x, const void* y) {
+    const int grid = (int)((n + 255) / 256);
+    if (dtype == B200WKV_F32) activation_kernel<float><<<grid, 256, 0, st>>>(act, n, (float*)x, (const float*)y);
+    else activation_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(act, n, (__nv_bfloat16*)x, (const __nv_bfloat16*)y);
+    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+}
+
 int wkv7_mix_partial_rows(int rows, int C) {
-    const Geometry g = geometry(rows, C);
+    const Geometry g = geometry(rows, C, MIX_THREADS_PER_SM);
     return g.grid * g.slots;
 }
 
@@ -412,7 +489,7 @@ template <typename T>
 int mix_pre_fwd_t(cudaStream_t st, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al, const void* v,
                   const void* vf, const void* vl, const void* w0, const void* a0, const void* v0, const void* k_k,
                   const void* k_a, void* w, void* kp, void* vp, void* ai, void* bi) {
-    const Geometry g = geometry(rows, C);
+    const Geometry g = geometry(rows, C, 2048);
     B200WKV_MIX_LAUNCH(mix_pre_fwd_kernel, rows, C, use_vmix, (const T*)k, (const T*)wl, (const T*)al, (const T*)v,
                                                       (const T*)vf, (const T*)vl, (const T*)w0, (const T*)a0, (const T*)v0,
                                                       (const T*)k_k, (const T*)k_a, (T*)w, (T*)kp, (T*)vp, (T*)ai, (T*)bi);
@@ -422,17 +499,17 @@ template <typename T>
 int mix_pre_bwd_t(cudaStream_t st, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al, const void* v,
                   const void* vf, const void* vl, const void* w0, const void* a0, const void* v0, const void* k_k,
                   const void* k_a, const void* gw, const void* gkp, const void* gvp, const void* gai, const void* gbi,
-                  void* dk, void* dwl, void* dal, void* dv, void* dvf, void* dvl, float* partial) {
-    const Geometry g = geometry(rows, C);
+                  void* dk, void* dwl, void* dal, void* dv, void* dvf, void* dvl, float* partial, const MixPreExtra& extra) {
+    const Geometry g = geometry(rows, C, MIX_THREADS_PER_SM);
     B200WKV_MIX_LAUNCH(mix_pre_bwd_kernel, rows, C, use_vmix, (const T*)k, (const T*)wl, (const T*)al, (const T*)v, (const T*)vf, (const T*)vl, (const T*)w0,
         (const T*)a0, (const T*)v0, (const T*)k_k, (const T*)k_a, (const T*)gw, (const T*)gkp, (const T*)gvp, (const T*)gai,
-        (const T*)gbi, (T*)dk, (T*)dwl, (T*)dal, (T*)dv, (T*)dvf, (T*)dvl, partial);
+        (const T*)gbi, (T*)dk, (T*)dwl, (T*)dal, (T*)dv, (T*)dvf, (T*)dvl, partial, extra);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 template <typename T>
 int mix_post_fwd_t(cudaStream_t st, int rows, int C, float eps, const void* y, const void* r, const void* kp, const void* vp,
                    const void* g_, const void* ln_w, const void* ln_b, const void* r_k, void* x) {
-    const Geometry g = geometry(rows, C);
+    const Geometry g = geometry(rows, C, 2048);
     B200WKV_MIX_LAUNCH(mix_post_fwd_kernel, rows, C, eps, (const T*)y, (const T*)r, (const T*)kp, (const T*)vp,
                                                        (const T*)g_, (const T*)ln_w, (const T*)ln_b, (const T*)r_k, (T*)x);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
@@ -441,7 +518,7 @@ template <typename T>
 int mix_post_bwd_t(cudaStream_t st, int rows, int C, float eps, const void* y, const void* r, const void* kp, const void* vp,
                    const void* g_, const void* ln_w, const void* ln_b, const void* r_k, const void* gx, void* dy, void* dr,
                    void* dkp, void* dvp, void* dg, float* partial) {
-    const Geometry g = geometry(rows, C);
+    const Geometry g = geometry(rows, C, MIX_THREADS_PER_SM);
     B200WKV_MIX_LAUNCH(mix_post_bwd_kernel, rows, C, eps, (const T*)y, (const T*)r, (const T*)kp, (const T*)vp,
                                                        (const T*)g_, (const T*)ln_w, (const T*)ln_b, (const T*)r_k,
                                                        (const T*)gx, (T*)dy, (T*)dr, (T*)dkp, (T*)dvp, (T*)dg, partial);
@@ -457,10 +534,10 @@ int wkv7_mix_pre_fwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, 
 int wkv7_mix_pre_bwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, const void* k, const void* wl, const void* al,
                      const void* v, const void* vf, const void* vl, const void* w0, const void* a0, const void* v0,
                      const void* k_k, const void* k_a, const void* gw, const void* gkp, const void* gvp, const void* gai,
-                     const void* gbi, void* dk, void* dwl, void* dal, void* dv, void* dvf, void* dvl, float* partial) {
+                     const void* gbi, void* dk, void* dwl, void* dal, void* dv, void* dvf, void* dvl, float* partial, const MixPreExtra& extra) {
     return dtype == B200WKV_F32
-               ? mix_pre_bwd_t<float>(st, rows, C, use_vmix, k, wl, al, v, vf, vl, w0, a0, v0, k_k, k_a, gw, gkp, gvp, gai, gbi, dk, dwl, dal, dv, dvf, dvl, partial)
-               : mix_pre_bwd_t<__nv_bfloat16>(st, rows, C, use_vmix, k, wl, al, v, vf, vl, w0, a0, v0, k_k, k_a, gw, gkp, gvp, gai, gbi, dk, dwl, dal, dv, dvf, dvl, partial);
+               ? mix_pre_bwd_t<float>(st, rows, C, use_vmix, k, wl, al, v, vf, vl, w0, a0, v0, k_k, k_a, gw, gkp, gvp, gai, gbi, dk, dwl, dal, dv, dvf, dvl, partial, extra)
+               : mix_pre_bwd_t<__nv_bfloat16>(st, rows, C, use_vmix, k, wl, al, v, vf, vl, w0, a0, v0, k_k, k_a, gw, gkp, gvp, gai, gbi, dk, dwl, dal, dv, dvf, dvl, partial, extra);
 }
 int wkv7_mix_post_fwd(cudaStream_t st, int dtype, int rows, int C, float eps, const void* y, const void* r, const void* kp,
                       const void* vp, const void* g, const void* ln_w, const void* ln_b, const void* r_k, void* x) {

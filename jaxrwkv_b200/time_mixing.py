@@ -155,6 +155,10 @@ def time_mixing_seq(x, state, v_first, att, length, new_starts, H, S, layer_id):
     (rwkv7.py:254-255); ``v_first`` (B, T, C); ``att`` the layer's parameter dict with the reference's keys;
     ``length`` (B,), ``new_starts`` (B, T).  Returns ``(out (B, T, C), new_state, v_first)``.
     """
+    if x.is_cuda:
+        native = _lib.host().time_mixing(x, state, v_first, att, length, new_starts, H, S, layer_id)
+        if native is not None:                   # None: a transform such as vmap, or arguments that need a closer look
+            return native
     B, T, C = x.shape
     mix = torch.stack([att[n].reshape(C) for n in ("x_r", "x_w", "x_k", "x_v", "x_a", "x_g")]).to(x.dtype)
     mixed, shift_row = token_shift(x, state[:, 0], mix, length, new_starts)
