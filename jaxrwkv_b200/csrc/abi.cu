@@ -13,7 +13,7 @@ int wkv7_seq_fwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w,
                  int* residual_mark);
 int wkv7_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w, const void* r, const void* k,
                  const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
-                 const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* dw, void* dr,
+                 const uint8_t* ns, const void* dy, const void* ds_out, void* residual, size_t residual_bytes, void* dw, void* dr,
                  void* dk, void* dv, void* da, void* db, void* ds0, const int* run_if);
 
 int wkv7_step(cudaStream_t st, int dtype, int B, int H, const void* w, const void* r, const void* k, const void* v,
@@ -71,6 +71,10 @@ static int* residual_mark_of(void* residual, size_t bytes) {
     return residual ? reinterpret_cast<int*>(static_cast<char*>(residual) + bytes - kResidualMarkBytes) : nullptr;
 }
 
+size_t wkv7_residual_min_bytes(int dtype, int B, int T, int H) {
+    return dtype == B200WKV_F32 ? wkv7_seq_residual_bytes(B, T, H) : b200wkv7_residual_bytes(dtype, B, T, H, kN);
+}
+
 static int check_dims(int dtype, int B, int T, int H, int N) {
     if (dtype != B200WKV_F32 && dtype != B200WKV_BF16) return B200WKV_EDTYPE;
     if (B < 1 || T < 1 || H < 1 || N != kN) return B200WKV_ESHAPE;
@@ -107,8 +111,9 @@ size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N) {
     if (check_dims(dtype, B, T, H, N) != B200WKV_OK) return 0;
     // fp32 uses the sequential kernels (a state every 16 tokens); bf16 uses the chunked tensor-core
     // kernels (a state every 64 tokens) unless B200WKV_FLAG_SEQUENTIAL asks otherwise, so size for both
+    // (fp32: and as much again for the state gradients that the backward leaves between the chunks it walks side by side)
     const size_t seq = wkv7_seq_residual_bytes(B, T, H);
-    if (dtype == B200WKV_F32) return seq;
+    if (dtype == B200WKV_F32) return 2 * seq;
     const size_t chk = wkv7_chunk_residual_bytes(B, T, H);
     // + one word at the end that says which of the two formats the forward left (see residual_mark_of)
     return (seq > chk ? seq : chk) + kResidualMarkBytes;
@@ -121,7 +126,7 @@ int b200wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void
     int st = check_dims(dtype, B, T, H, N);
     if (st != B200WKV_OK) return st;
     if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
-    if (residual != nullptr && residual_bytes < b200wkv7_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
+    if (residual != nullptr && residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
     // one token and no residual wanted (recurrent decoding): a single pass over the state
     if (T == 1 && residual == nullptr)
         return wkv7_step((cudaStream_t)stream, dtype, B, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out);
@@ -149,7 +154,7 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
     if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !residual || !dw || !dr || !dk || !dv ||
         !da || !db || !ds0)
         return B200WKV_ENULL;
-    if (residual_bytes < b200wkv7_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
+    if (residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
     // must match the kernel family that filled the residual in b200wkv7_fwd (same dtype and flags)
     if (dtype == B200WKV_BF16 && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
         const int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
@@ -168,10 +173,10 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
                             fast, dw, dr, dk, dv, da, db, ds0);
         if (st != B200WKV_OK) return st;
         return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
-                            residual, dw, dr, dk, dv, da, db, ds0, mark);
+                            residual, b200wkv7_residual_bytes(dtype, B, T, H, N) - kResidualMarkBytes, dw, dr, dk, dv, da, db, ds0, mark);
     }
     return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
-                        residual, dw, dr, dk, dv, da, db, ds0, nullptr);
+                        residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, nullptr);
 }
 
 size_t b200wkv6_residual_bytes(int dtype, int B, int T, int H, int N) {

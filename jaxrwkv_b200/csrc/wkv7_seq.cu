@@ -1,165 +1,28 @@
-// RWKV-7 WKV recurrence, token-sequential CUDA-core kernels (fp32 arithmetic).
+// RWKV-7 gradients on CUDA cores (fp32 arithmetic), and the single-token step for unaligned operands.
 //
-// These are the exact-arithmetic kernels: one CTA per (batch, head) walks the
-// sequence token by token with the 64x64 state held in registers.  They serve the
-// fp32 element type (whose 1e-4 tolerance rules out bf16 tensor-core products) and
-// are the in-library cross-check for the chunked tensor-core kernels.
+// With the forward and the state-gradient carry of wkv7_chain.cu these are the exact-arithmetic kernels: they serve
+// the fp32 element type (whose 1e-4 tolerance rules out bf16 tensor-core products) and are the in-library cross-check
+// for the chunked tensor-core kernels.
 //
-// Semantics: BaseRWKV.inner_loop of jaxrwkv (src/jaxrwkv/rwkv7.py:199-220); the
-// backward is the reverse-time recurrence of the same loop.
+// Semantics: the reverse-time recurrence of BaseRWKV.inner_loop of jaxrwkv (src/jaxrwkv/rwkv7.py:199-220).
 #include "common.cuh"
 #include "device_once.cuh"
+#include "wkv7_exact.cuh"
 
 namespace b200wkv {
 
-constexpr int kCk = 16;  // tokens per staged chunk == spacing of the saved state checkpoints
-
-// ------------------------------------------------------------------ forward ---------
-// 128 threads per (batch, head).  Warps 0-1 compute: thread i owns the whole row i of S in
-// registers, so S.a and S.r are in-thread dot products and every shared-memory read of the
-// token vectors is a warp-uniform (broadcast) address.  Warps 2-3 stream: they convert the next
-// 16-token chunk into the other shared buffer and write the previous chunk's outputs, so the
-// compute warps' instruction stream is only LDS + FMA.
-struct FwdSmem {
-    float in[2][6][kCk][kN];  // decay, r, k, v, a, b
-    float y[2][kCk][kN];
-    uint8_t ns[2][kCk];
-};
-
-template <typename T>
-__global__ void __launch_bounds__(128)
-wkv7_seq_fwd_kernel(int Tlen, int H, const T* __restrict__ w, const T* __restrict__ r,
-                    const T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ a,
-                    const T* __restrict__ b, const T* __restrict__ s0,
-                    const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts,
-                    T* __restrict__ y, T* __restrict__ s_out, float* __restrict__ ckpt,
-                    const int* __restrict__ run_if, int run_ticket, int* __restrict__ residual_mark) {
-    // As the fallback behind the chunked kernel: run only when that kernel left its ticket in *run_if,
-    // and mark the residual as being in this kernel's format.
-    if (run_if != nullptr && *run_if != run_ticket) return;
-    if (residual_mark != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *residual_mark = 1;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    FwdSmem& sm = *reinterpret_cast<FwdSmem*>(smem_raw);
-    const int bh = blockIdx.x, bi = bh / H, h = bh % H;
-    const int tid = threadIdx.x;
-    const bool streamer = tid >= 64;
-    const int i = tid & 63;
-    const size_t seq_base = (size_t)bi * Tlen * H * kN + (size_t)h * kN;
-    const size_t tok_stride = (size_t)H * kN;
-    const T* src[6] = {w, r, k, v, a, b};
-    const int L = min((int)length[bi], Tlen);
-    const size_t row_base = ((size_t)bh * kN + i) * kN;
-    const int nC = (Tlen + kCk - 1) / kCk;
-
-    // streamer: 64 threads move one chunk = 6 streams x 16 tokens x 16 groups of 4 elements
-    auto stage = [&](int c, int buf) {
-        const int t0 = c * kCk;
-#pragma unroll
-        for (int m = 0; m < 6; ++m) {
-            float4 x[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int g = i + 64 * u, lt = g >> 4, lc = (g & 15) * 4;
-                x[u] = (t0 + lt < Tlen) ? load4(src[m] + seq_base + (size_t)(t0 + lt) * tok_stride + lc)
-                                        : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int g = i + 64 * u, lt = g >> 4, lc = (g & 15) * 4;
-                if (m == 0) x[u] = make_float4(expf(-expf(x[u].x)), expf(-expf(x[u].y)), expf(-expf(x[u].z)), expf(-expf(x[u].w)));
-                *reinterpret_cast<float4*>(&sm.in[buf][m][lt][lc]) = x[u];
-            }
-        }
-        if (i < kCk) sm.ns[buf][i] = (t0 + i < Tlen) ? new_starts[(size_t)bi * Tlen + t0 + i] : 0;
-    };
-    auto flush_y = [&](int c, int buf) {
-        const int t0 = c * kCk;
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int g = i + 64 * u, lt = g >> 4, lc = (g & 15) * 4;
-            if (t0 + lt < Tlen)
-                store4(y + seq_base + (size_t)(t0 + lt) * tok_stride + lc, *reinterpret_cast<const float4*>(&sm.y[buf][lt][lc]));
-        }
-    };
-
-    float S[kN];
-    if (!streamer) {
-#pragma unroll
-        for (int g = 0; g < 16; ++g) {
-            float4 x = load4(s0 + row_base + g * 4);
-            S[g * 4 + 0] = x.x; S[g * 4 + 1] = x.y; S[g * 4 + 2] = x.z; S[g * 4 + 3] = x.w;
-        }
-        if (L == 0) {
-#pragma unroll
-            for (int g = 0; g < 16; ++g)
-                store4(s_out + row_base + g * 4, make_float4(S[g * 4], S[g * 4 + 1], S[g * 4 + 2], S[g * 4 + 3]));
-        }
-    } else {
-        stage(0, 0);
-    }
-    __syncthreads();
-
-    for (int c = 0; c < nC; ++c) {
-        const int buf = c & 1, t0 = c * kCk;
-        if (streamer) {
-            if (c > 0) flush_y(c - 1, buf ^ 1);
-            if (c + 1 < nC) stage(c + 1, buf ^ 1);
-        } else {
-            if (ckpt != nullptr) {
-                float* dst = ckpt + (((size_t)bh * nC + c) * kN + i) * kN;
-#pragma unroll
-                for (int g = 0; g < 16; ++g)
-                    *reinterpret_cast<float4*>(dst + g * 4) = make_float4(S[g * 4], S[g * 4 + 1], S[g * 4 + 2], S[g * 4 + 3]);
-            }
-            const int nt = min(kCk, Tlen - t0);
-            for (int tt = 0; tt < nt; ++tt) {
-                if (sm.ns[buf][tt]) {
-#pragma unroll
-                    for (int j = 0; j < kN; ++j) S[j] = 0.f;
-                }
-                float sa0 = 0.f, sa1 = 0.f, sa2 = 0.f, sa3 = 0.f;
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                    const float4 av = *reinterpret_cast<const float4*>(&sm.in[buf][4][tt][g * 4]);
-                    sa0 = fmaf(S[g * 4 + 0], av.x, sa0); sa1 = fmaf(S[g * 4 + 1], av.y, sa1);
-                    sa2 = fmaf(S[g * 4 + 2], av.z, sa2); sa3 = fmaf(S[g * 4 + 3], av.w, sa3);
-                }
-                const float sa = (sa0 + sa1) + (sa2 + sa3);
-                const float vi = sm.in[buf][3][tt][i];
-                float y0 = 0.f, y1 = 0.f, y2 = 0.f, y3 = 0.f;
-#pragma unroll
-                for (int g = 0; g < 16; ++g) {
-                    const float4 wv = *reinterpret_cast<const float4*>(&sm.in[buf][0][tt][g * 4]);
-                    const float4 kv = *reinterpret_cast<const float4*>(&sm.in[buf][2][tt][g * 4]);
-                    const float4 bv = *reinterpret_cast<const float4*>(&sm.in[buf][5][tt][g * 4]);
-                    const float4 rv = *reinterpret_cast<const float4*>(&sm.in[buf][1][tt][g * 4]);
-                    float* s4 = &S[g * 4];
-                    s4[0] = fmaf(s4[0], wv.x, fmaf(vi, kv.x, sa * bv.x));
-                    s4[1] = fmaf(s4[1], wv.y, fmaf(vi, kv.y, sa * bv.y));
-                    s4[2] = fmaf(s4[2], wv.z, fmaf(vi, kv.z, sa * bv.z));
-                    s4[3] = fmaf(s4[3], wv.w, fmaf(vi, kv.w, sa * bv.w));
-                    y0 = fmaf(s4[0], rv.x, y0); y1 = fmaf(s4[1], rv.y, y1);
-                    y2 = fmaf(s4[2], rv.z, y2); y3 = fmaf(s4[3], rv.w, y3);
-                }
-                sm.y[buf][tt][i] = (y0 + y1) + (y2 + y3);
-                if (t0 + tt == L - 1) {
-#pragma unroll
-                    for (int g = 0; g < 16; ++g)
-                        store4(s_out + row_base + g * 4, make_float4(S[g * 4], S[g * 4 + 1], S[g * 4 + 2], S[g * 4 + 3]));
-                }
-            }
-        }
-        __syncthreads();
-    }
-    if (streamer) flush_y(nC - 1, (nC - 1) & 1);
-}
+constexpr int kCk = kExactChunk;
+int wkv7_chain_bwd(cudaStream_t st, int dtype, int B, int T, int H, int run, const void* w, const void* r, const void* a, const void* b,
+                   const void* dy, const void* ds_out, const uint32_t* length, const uint8_t* ns, void* ds0, float* carry, const int* run_if);
 
 // ------------------------------------------------------------------ backward --------
 // 256 threads: thread (ti, tj) owns the 4x4 tile rows 4ti.., cols 4tj.. of S and dS, with
 // tj = lane%16 and ti = 2*warp + lane/16, so sums over columns stay inside a half-warp and
 // sums over rows need one shuffle plus an ordered 8-way add through shared memory.
 // Each 16-token chunk is replayed from its checkpoint in two halves of 8 tokens whose
-// entering states are kept in registers for the reverse sweep.
+// entering states are kept in registers for the reverse sweep.  A CTA does one run of `run` chunks of one (sequence,
+// head), starting from the state gradient that the carry left behind it, so that the runs of a sequence are walked side
+// by side (one CTA per sequence for all of it: 1.25 us per token, 643 us at T = 512 with 24 of the 148 SMs in use).
 struct BwdSmem {
     float in[8][kCk][kN];      // decay, r, k, v, a, b, dy, dwfac (= -exp(w) * decay)
     float sa[kCk][kN];
@@ -175,20 +38,20 @@ wkv7_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ w, const T* __restric
                     const T* __restrict__ b, const T* __restrict__ s0,
                     const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts,
                     const T* __restrict__ dy, const T* __restrict__ ds_out,
-                    const float* __restrict__ ckpt,
+                    const float* __restrict__ ckpt, const float* __restrict__ carry, int run,
                     T* __restrict__ dw, T* __restrict__ dr, T* __restrict__ dk, T* __restrict__ dv,
                     T* __restrict__ da, T* __restrict__ db, T* __restrict__ ds0, const int* __restrict__ run_if) {
     // as the fallback behind the chunked backward: run only when the forward marked the residual as this kernel's
     if (run_if != nullptr && *run_if == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
-    const int bh = blockIdx.x, bi = bh / H, h = bh % H;
+    const int nC = (Tlen + kCk - 1) / kCk, runs = (nC + run - 1) / run;
+    const int bh = blockIdx.x / runs, run_at = blockIdx.x % runs, bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int tj = lane & 15, ti = warp * 2 + (lane >> 4);
     const size_t seq_base = (size_t)bi * Tlen * H * kN + (size_t)h * kN;
     const size_t tok_stride = (size_t)H * kN;
     const int L = min((int)length[bi], Tlen);
-    const int nC = (Tlen + kCk - 1) / kCk;
     const int lt = tid >> 4, lc = (tid & 15) * 4;
     const T* src[7] = {w, r, k, v, a, b, dy};
     T* dst[6] = {dw, dr, dk, dv, da, db};
@@ -199,9 +62,17 @@ wkv7_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ w, const T* __restric
     for (int ii = 0; ii < 4; ++ii)
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) dS[ii][jj] = 0.f;
+    if (run_at + 1 < runs) {
+        const float* g = carry + (((size_t)bh * (runs - 1) + run_at) * kN + 4 * ti) * kN + 4 * tj;
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii) {
+            const float4 x = *reinterpret_cast<const float4*>(g + ii * kN);
+            dS[ii][0] = x.x; dS[ii][1] = x.y; dS[ii][2] = x.z; dS[ii][3] = x.w;
+        }
+    }
 
     int step = 0;  // parity counter for the partial-sum double buffer
-    for (int c = nC - 1; c >= 0; --c) {
+    for (int c = min(nC, (run_at + 1) * run) - 1; c >= run_at * run; --c) {
         const int t0 = c * kCk;
         __syncthreads();
         {   // stage the chunk's inputs
@@ -402,6 +273,7 @@ wkv7_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ w, const T* __restric
                        *reinterpret_cast<const float4*>(&sm.out[m][lt][lc]));
         }
     }
+    if (runs > 1) return;   // the carry goes on to the initial state
     // gradient with respect to the initial state
     if (L == 0 && ds_out != nullptr) {
 #pragma unroll
@@ -503,34 +375,37 @@ size_t wkv7_seq_residual_bytes(int B, int T, int H) {
     return (size_t)B * H * ((T + kCk - 1) / kCk) * kN * kN * sizeof(float);
 }
 
-template <typename T>
-static int launch_fwd(cudaStream_t st, int B, int Tlen, int H, const void* w, const void* r, const void* k,
-                      const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
-                      const uint8_t* ns, void* y, void* s_out, void* residual, const int* run_if, int run_ticket,
-                      int* residual_mark) {
-    auto kern = wkv7_seq_fwd_kernel<T>;
-    static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
-    if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem)); }))
-        return B200WKV_ELAUNCH;
-    kern<<<B * H, 128, sizeof(FwdSmem), st>>>(Tlen, H, (const T*)w, (const T*)r, (const T*)k, (const T*)v,
-                                              (const T*)a, (const T*)b, (const T*)s0, length, ns, (T*)y,
-                                              (T*)s_out, (float*)residual, run_if, run_ticket, residual_mark);
-    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+// Chunks per run: as few as the room behind the checkpoints has places for (one state gradient between two runs), and all
+// of them, without a carry, where there is none.
+static int run_length(int B, int T, int H, size_t room) {
+    const int nC = (T + kCk - 1) / kCk;
+    const size_t one = (size_t)B * H * kN * kN * sizeof(float);
+    int run = 1;
+    while (run < nC && (size_t)((nC - 1) / run) * one > room) run *= 2;
+    return run < nC ? run : nC;
 }
 
 template <typename T>
 static int launch_bwd(cudaStream_t st, int B, int Tlen, int H, const void* w, const void* r, const void* k,
                       const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
-                      const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* dw,
+                      const uint8_t* ns, const void* dy, const void* ds_out, void* residual, size_t residual_bytes, void* dw,
                       void* dr, void* dk, void* dv, void* da, void* db, void* ds0, const int* run_if) {
     auto kern = wkv7_seq_bwd_kernel<T>;
     static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
     if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem)); }))
         return B200WKV_ELAUNCH;
-    kern<<<B * H, 256, sizeof(BwdSmem), st>>>(Tlen, H, (const T*)w, (const T*)r, (const T*)k, (const T*)v,
-                                              (const T*)a, (const T*)b, (const T*)s0, length, ns, (const T*)dy,
-                                              (const T*)ds_out, (const float*)residual, (T*)dw, (T*)dr, (T*)dk,
-                                              (T*)dv, (T*)da, (T*)db, (T*)ds0, run_if);
+    const size_t used = wkv7_seq_residual_bytes(B, Tlen, H);
+    const int nC = (Tlen + kCk - 1) / kCk, run = run_length(B, Tlen, H, residual_bytes - used), runs = (nC + run - 1) / run;
+    float* const carry = reinterpret_cast<float*>(static_cast<char*>(residual) + used);
+    if (runs > 1) {
+        const int code = sizeof(T) == 4 ? B200WKV_F32 : B200WKV_BF16;
+        const int s = wkv7_chain_bwd(st, code, B, Tlen, H, run, w, r, a, b, dy, ds_out, length, ns, ds0, carry, run_if);
+        if (s != B200WKV_OK) return s;
+    }
+    kern<<<B * H * runs, 256, sizeof(BwdSmem), st>>>(Tlen, H, (const T*)w, (const T*)r, (const T*)k, (const T*)v,
+                                                     (const T*)a, (const T*)b, (const T*)s0, length, ns, (const T*)dy,
+                                                     (const T*)ds_out, (const float*)residual, carry, run, (T*)dw, (T*)dr, (T*)dk,
+                                                     (T*)dv, (T*)da, (T*)db, (T*)ds0, run_if);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
@@ -561,23 +436,14 @@ int wkv7_step(cudaStream_t st, int dtype, int B, int H, const void* w, const voi
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
-// run_if / run_ticket / residual_mark: see the kernels; all NULL / 0 for an unconditional call
-int wkv7_seq_fwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w, const void* r, const void* k,
-                 const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
-                 const uint8_t* ns, void* y, void* s_out, void* residual, const int* run_if, int run_ticket,
-                 int* residual_mark) {
-    if (dtype == B200WKV_F32)
-        return launch_fwd<float>(st, B, T, H, w, r, k, v, a, b, s0, length, ns, y, s_out, residual, run_if, run_ticket, residual_mark);
-    return launch_fwd<__nv_bfloat16>(st, B, T, H, w, r, k, v, a, b, s0, length, ns, y, s_out, residual, run_if, run_ticket, residual_mark);
-}
-
+// run_if: see the kernels; NULL for an unconditional call.  `residual_bytes` is what of the residual the two may use: the
+// forward's checkpoints and, behind them, room for the carry.
 int wkv7_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w, const void* r, const void* k,
                  const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
-                 const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* dw, void* dr,
+                 const uint8_t* ns, const void* dy, const void* ds_out, void* residual, size_t residual_bytes, void* dw, void* dr,
                  void* dk, void* dv, void* da, void* db, void* ds0, const int* run_if) {
-    if (dtype == B200WKV_F32)
-        return launch_bwd<float>(st, B, T, H, w, r, k, v, a, b, s0, length, ns, dy, ds_out, residual, dw, dr, dk, dv, da, db, ds0, run_if);
-    return launch_bwd<__nv_bfloat16>(st, B, T, H, w, r, k, v, a, b, s0, length, ns, dy, ds_out, residual, dw, dr, dk, dv, da, db, ds0, run_if);
+    return (dtype == B200WKV_F32 ? launch_bwd<float> : launch_bwd<__nv_bfloat16>)(st, B, T, H, w, r, k, v, a, b, s0, length, ns, dy, ds_out,
+                                                                                  residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, run_if);
 }
 
 }  // namespace b200wkv
