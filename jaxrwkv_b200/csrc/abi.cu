@@ -41,11 +41,18 @@ size_t wkv6_seq_residual_bytes(int B, int T, int H);
 int wkv6_seq_fwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r, const void* k, const void* v,
                  const void* w, int per_token, const void* u, const void* s0, const uint32_t* length,
                  const uint8_t* ns, void* y, void* s_out, void* residual, const int* run_if, int run_ticket,
-                 int* residual_mark);
+                 int* residual_mark, bool rest_only = false);
 int wkv6_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r, const void* k, const void* v,
                  const void* w, int per_token, const void* u, const uint32_t* length, const uint8_t* ns,
                  const void* dy, const void* ds_out, const void* residual, void* dr, void* dk, void* dv, void* dw,
-                 void* du, void* ds0, const int* run_if);
+                 void* du, void* ds0, const int* run_if, bool rest_only = false);
+// A constant decay (versions 5, 5.2): fp32-accurate, run-parallel; `rest_only` above: what of the call these two left out
+size_t wkv5_exact_partial_bytes(int B, int T, int H);
+int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
+                   const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark);
+int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
+                   const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* partial,
+                   void* dr, void* dk, void* dv, void* dw, void* du, void* ds0);
 size_t wkv6_chunk_residual_bytes(int B, int T, int H);
 int wkv6_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w,
                    int per_token, const void* u, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
@@ -184,9 +191,10 @@ size_t b200wkv6_residual_bytes(int dtype, int B, int T, int H, int N) {
     // fp32 uses the sequential kernels (an fp32 state every 16 tokens); bf16 uses the chunked tensor-core kernels (a
     // bf16 state every 16 tokens) with the sequential ones as their fallback, so size for both, plus one word at
     // the end that says which of the two formats the forward left
-    const size_t seq = wkv6_seq_residual_bytes(B, T, H);
+    size_t seq = wkv6_seq_residual_bytes(B, T, H);
     if (dtype == B200WKV_F32) return seq;
     const size_t chk = wkv6_chunk_residual_bytes(B, T, H);
+    seq += wkv5_exact_partial_bytes(B, T, H);      // behind the checkpoints: the runs' shares of a constant decay's gradients
     return (seq > chk ? seq : chk) + kResidualMarkBytes;
 }
 
@@ -203,9 +211,16 @@ int b200wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int 
         int* mark = residual_mark_of(residual, b200wkv6_residual_bytes(dtype, B, T, H, N));
         // With a constant decay (versions 5, 5.2) the decay's gradient is a sum over ALL tokens of per-token terms that
         // largely cancel; taken from bf16 tensor-core products it is only good to a few percent (10 % on short
-        // sequences), so training calls of those versions keep the fp32-arithmetic sequential kernels.  Their
-        // inference calls, and everything of version 6, take the chunked kernels.
-        if ((flags & B200WKV_FLAG_SEQUENTIAL) || (version != 6 && residual != nullptr))
+        // sequences), so training calls of those versions take the fp32-accurate kernels of wkv5_exact.cu, with the
+        // token-sequential ones for heads outside their domain (same checkpoints, marked as such).  Their inference
+        // calls, and everything of version 6, take the chunked kernels.
+        if (version != 6 && residual != nullptr && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
+            st = wkv5_exact_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, s0, length, new_starts, y, s_out, residual, mark);
+            if (st != B200WKV_OK) return st;
+            return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, s0, length, new_starts, y, s_out, residual, nullptr, 0,
+                                mark, true);
+        }
+        if (flags & B200WKV_FLAG_SEQUENTIAL)
             return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
                                 s_out, residual, nullptr, 0, mark);
         // the chunked tensor-core kernel, and behind it the sequential kernel, which runs only if the chunked one met
@@ -232,14 +247,23 @@ int b200wkv6_bwd(void* stream, int dtype, int version, int B, int T, int H, int 
     if (!r || !k || !v || !w || !u || !s0 || !length || !new_starts || !residual || !dr || !dk || !dv || !dw || !du || !ds0)
         return B200WKV_ENULL;
     if (residual_bytes < b200wkv6_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
-    (void)flags;
+    if (dtype == B200WKV_BF16 && version != 6) {
+        const bool sequential = (flags & B200WKV_FLAG_SEQUENTIAL) != 0;
+        if (!sequential) {
+            st = wkv5_exact_bwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, length, new_starts, dy, ds_out, residual,
+                                static_cast<char*>(residual) + wkv6_seq_residual_bytes(B, T, H), dr, dk, dv, dw, du, ds0);
+            if (st != B200WKV_OK) return st;
+        }
+        return wkv6_seq_bwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, length, new_starts, dy, ds_out, residual, dr, dk, dv, dw, du,
+                            ds0, nullptr, !sequential);
+    }
     if (dtype == B200WKV_BF16) {
         // the forward's mark decides on the device which of the two runs; the other returns at once
         const int* mark = residual_mark_of(residual, b200wkv6_residual_bytes(dtype, B, T, H, N));
-        st = wkv6_chunk_bwd((cudaStream_t)stream, B, T, H, r, k, v, w, version == 6, u, length, new_starts, dy, ds_out,
+        st = wkv6_chunk_bwd((cudaStream_t)stream, B, T, H, r, k, v, w, 1, u, length, new_starts, dy, ds_out,
                             residual, mark, dr, dk, dv, dw, du, ds0);
         if (st != B200WKV_OK) return st;
-        return wkv6_seq_bwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, length, new_starts, dy, ds_out,
+        return wkv6_seq_bwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 1, u, length, new_starts, dy, ds_out,
                             residual, dr, dk, dv, dw, du, ds0, mark);
     }
     return wkv6_seq_bwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, length, new_starts, dy,
