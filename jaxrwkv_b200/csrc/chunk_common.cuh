@@ -15,60 +15,60 @@ constexpr float kCumFloor = -86.56f;   // floor of the in-chunk cumulative log2-
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
-// Residual written by the chunked forward for the chunked backward (all fp32):
-//   [B*H][ceil(T/64)][64][64]  state entering every 64-token block (before a start flag is applied)
-//   [B*H][64][64]              state at position `length` (what the forward returns as s_out)
-//   [kHandoffSlots][64*64 + 64] carries passed between CTAs that share one (batch, head) sequence
-//   [kHandoffSlots]             their ready flags (int)
-// The last two are scratch of whichever kernel runs: a sequence may be cut at 64-token block
-// boundaries into runs owned by neighbouring CTAs, so that B*H sequences spread evenly over the SMs.
+// Residual written by the chunked forward for the chunked backward.  Its unit is the slot: one per 64-token block of every
+// (batch, head) sequence, and one more for the second part of the block that `length` cuts in two (nBlk + 1 in all).
+//   s_at_len [B*H][64][64]        fp32  state at position `length` (what the forward returns as s_out)
+//   saved    [B*H][slots][6 tiles] bf16 the operands T = (I - A_ab)^-1, A_ak, P_rb, P_rk, sa and the entering state S0
+//                                       exactly as the forward used them, so the backward loads them instead of
+//                                       recomputing them.  A tile is 8 column blocks of [64 rows][16 bytes] (the
+//                                       operand slab layout without the shared-memory padding), 8 KB.
+//   mprime   [B*H][slots] tile          M' = W~^T B^: S_C = S0 diag(L_C) + S0 M' + (terms without S0)
+//   rbar     [B*T][H*64]           bf16 R- = R~ + P_rb W~ (token rows, laid out like the streams): y_t = R-_t S0^T + ...
+//   lam      [B*H][slots][64]      fp32 L_C, the decay over the whole slot; 0 where a start flag cuts it
+//   dstate   [B*H][slots] tile          scratch of the backward: the state gradient leaving every slot
+//   fscr     [kGradCtas][4 tiles]       scratch of the gradient kernel, one set per CTA: the decay factors 1/L_t, L_t,
+//                                       L_{t-1} and the log-decay of the block in hand (written when the operands are
+//                                       scaled, read back by the last epilogue; it lives in L2)
 constexpr int kHandoffSlots = 512;
-constexpr int kHandoffFloats = kN * kN + kN;
-inline size_t chunk_states_floats(int B, int T, int H) {
-    return (size_t)B * H * ((size_t)((T + kC - 1) / kC) + 1) * kN * kN;
-}
-//   [B*H][ceil(T/64)][6 tiles]  for every 64-token block that the forward walked as ONE chunk: the bf16
-//                               operands T = (I - A_ab)^-1, A_ak, P_rb, P_rk, sa and the entering state S0
-//                               exactly as the forward used them, so the backward loads them instead of
-//                               recomputing them.  A tile is 8 column blocks of [64 rows][16 bytes] (the
-//                               operand slab layout without the shared-memory padding), 8 KB.
-constexpr int kSavedSlabs = 6;   // order: T, A_ak, P_rb, P_rk, sa, S0
 constexpr int SAVED_T = 0, SAVED_AAK = 1, SAVED_PRB = 2, SAVED_PRK = 3, SAVED_SA = 4, SAVED_S0 = 5;
 constexpr int GCB = kC * 16;          // column-block pitch of a tile in global memory (1024)
 constexpr int GTILE = 8 * GCB;        // 8192
-constexpr size_t kSavedBytes = (size_t)kSavedSlabs * GTILE;
-inline size_t chunk_saved_offset_floats(int B, int T, int H) {
-    return chunk_states_floats(B, T, H) + (size_t)kHandoffSlots * (kHandoffFloats + 1);
-}
-// What the carry / gradient split of the backward adds behind the saved tiles (see wkv7_carry.cu, wkv7_grad.cu):
-//   [B*H][ceil(T/64)][64][64] bf16  M' = W~^T B^ of every saved block: S_C = S0 diag(L_C) + S0 M' + (terms without S0)
-//                                   (8 column blocks of [64 rows][16 bytes], like the saved tiles)
-//   [B*T][H*64]               bf16  R- = R~ + P_rb W~ (token rows, laid out like the streams): y_t = R-_t S0^T + ...
-//   [B*H][ceil(T/64)][64]     fp32  L_C, the decay over the whole block
-//   [B*H][ceil(T/64)][64][64] bf16  scratch of the backward: the state gradient leaving every block (column blocks, as M')
-//   [B*H]                     int   1 if the forward walked the whole sequence as full, saved blocks
-//   [kGradCtas][4][64][64]    bf16  scratch of the gradient kernel, one set per CTA: the decay factors 1/L_t, L_t,
-//                                   L_{t-1} and the log-decay of the block in hand (written when the operands are
-//                                   scaled, read back by the last epilogue; it lives in L2)
+constexpr size_t kSavedBytes = (size_t)6 * GTILE;
 constexpr int kGradCtas = 512;
-struct CarryLayout {
-    size_t mprime, rbar, lam, dstate, fast, fscr, end;   // byte offsets from the start of the residual
+__host__ __device__ __forceinline__ int block_slots(int T) { return (T + kC - 1) / kC + 1; }
+struct ResidualLayout {
+    size_t s_at_len, saved, mprime, rbar, lam, dstate, fscr, end;   // byte offsets from the start of the residual
 };
-inline CarryLayout carry_layout(int B, int T, int H) {
-    const size_t nBlk = (size_t)((T + kC - 1) / kC), BH = (size_t)B * H;
-    CarryLayout l;
-    l.mprime = (chunk_saved_offset_floats(B, T, H)) * sizeof(float) + BH * nBlk * kSavedBytes;
-    l.rbar = l.mprime + BH * nBlk * GTILE;
+inline ResidualLayout residual_layout(int B, int T, int H) {
+    const size_t BH = (size_t)B * H, slots = BH * block_slots(T), nBlk = (size_t)((T + kC - 1) / kC);
+    ResidualLayout l;
+    l.s_at_len = 0;
+    l.saved = BH * kN * kN * sizeof(float);
+    l.mprime = l.saved + slots * kSavedBytes;
+    l.rbar = l.mprime + slots * GTILE;
     l.lam = l.rbar + (size_t)B * nBlk * kC * H * kN * 2;      // token rows padded to whole blocks
-    l.dstate = l.lam + BH * nBlk * kN * sizeof(float);
-    l.fast = l.dstate + BH * nBlk * GTILE;
-    l.fscr = (l.fast + BH * sizeof(int) + 255) / 256 * 256;
-    const size_t ctas = BH * nBlk < (size_t)kGradCtas ? BH * nBlk : (size_t)kGradCtas;
-    l.end = l.fscr + ctas * 4 * GTILE;
+    l.dstate = l.lam + slots * kN * sizeof(float);
+    l.fscr = l.dstate + slots * GTILE;
+    l.end = l.fscr + (slots < (size_t)kGradCtas ? slots : (size_t)kGradCtas) * 4 * GTILE;
     return l;
 }
-inline size_t chunk_residual_floats(int B, int T, int H) { return carry_layout(B, T, H).end / sizeof(float); }
+// A slot's tokens: p .. p + n - 1 (n = 0: the slot is not used)
+struct Slot { int p, n; };
+__host__ __device__ __forceinline__ Slot slot_tokens(int slot, int T, int L) {
+    const int cut = L < T && (L & (kC - 1)) != 0 ? L : -1, bl = L / kC;    // `length` inside a block
+    const int last = block_slots(T) - 1;
+    if (slot == last) {
+        if (cut < 0) return Slot{0, 0};
+        const int end = (bl + 1) * kC < T ? (bl + 1) * kC : T;
+        return Slot{cut, end - cut};
+    }
+    const int p = slot * kC;
+    int end = p + kC < T ? p + kC : T;
+    if (cut >= 0 && slot == bl) end = cut;
+    return Slot{p, end - p};
+}
 
+// What the schedule queries of b200wkv_debug.h answer: how sequences could be cut into runs of blocks over fewer CTAs.
 // Host side of the split: grid size and segments per sequence for `chains` sequences of `n_blk`
 // blocks with `per_sm` resident CTAs per SM on a device of `sm_count` SMs (the launchers pass the
 // count of the device that is current, looked up once per device).

@@ -1,6 +1,6 @@
 // RWKV-7 WKV backward, part 1 of 2: the state-gradient carry.
 //
-// The forward leaves, for every 64-token block it walked as one chunk, what makes the block an affine
+// The forward leaves, for every 64-token block (and both parts of a block that `length` cuts), what makes the block an affine
 // map of the state that enters it (S0, row = value index i, column = key index j):
 //     S_C = S0 diag(L_C) + S0 M' + (terms without S0)          M' = W~^T B^      (64 x 64)
 //     y_t = R-_t S0^T    + (terms without S0)                   R- = R~ + P_rb W~ (64 tokens x 64)
@@ -14,9 +14,7 @@
 // leaving every block goes to global memory in bf16; the second part (wkv7_grad.cu) turns it, block by
 // block and in parallel over all blocks, into the gradients of the six streams.
 //
-// Handles the sequences the forward marked as walked in full saved blocks (T a multiple of 64, start
-// flags only at multiples of 64, length 0, a multiple of 64, or >= T); the others are left to the
-// one-kernel backward (wkv7_chunk_bwd.cu).
+// Start flags need nothing here: a block with one has L_C = 0, M' = 0 and R- zero from the first flag on.
 //
 // Semantics: reverse-mode derivative of BaseRWKV.inner_loop of jaxrwkv (src/jaxrwkv/rwkv7.py:199-220).
 #include "common.cuh"
@@ -40,8 +38,9 @@ struct CarryStage {
 template <int kStages>
 constexpr int carry_smem() { return kStages * (int)sizeof(CarryStage); }
 
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src) : "memory");
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, bool valid) {   // zeros where not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -66,36 +65,42 @@ __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uin
 
 template <int kStages>
 __global__ void __launch_bounds__(128)
-wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts,
+wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length,
                       const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ ds_out,
                       const __nv_bfloat16* __restrict__ mprime, const __nv_bfloat16* __restrict__ rbar,
-                      const float* __restrict__ lam, const int* __restrict__ fast, const int* __restrict__ residual_mark,
+                      const float* __restrict__ lam, const int* __restrict__ residual_mark,
                       __nv_bfloat16* __restrict__ dstate, __nv_bfloat16* __restrict__ ds0) {
     if (*residual_mark != 0) return;            // the forward fell back to the sequential kernels
     const int bh = blockIdx.x;
-    if (fast[bh] == 0) return;                  // left to the one-kernel backward
     extern __shared__ __align__(128) unsigned char smem[];
     CarryStage* stages = reinterpret_cast<CarryStage*>(smem);
     const int bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
     const int i0 = warp * 16;                   // this warp's rows of the state gradient
     const int L = min((int)length[bi], Tlen);
-    const int nBlk = Tlen / kC;
+    const int nSlot = block_slots(Tlen), bl = L / kC;
+    const bool cut = slot_tokens(nSlot - 1, Tlen, L).n > 0;
+    const int steps = cut ? nSlot : nSlot - 1;  // slots of this sequence, walked from the last to the first
+    auto slot_of = [&](int m) { return !cut || m <= bl ? m : m == bl + 1 ? nSlot - 1 : m - 1; };   // in order of time
     const size_t tok_stride = (size_t)H * kN;
     const size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
     const size_t st_base = (size_t)bh * kN * kN;
 
-    auto issue = [&](int blk) {
-        if (blk >= 0) {
-            CarryStage& s = stages[blk % kStages];
-            const size_t slot = (size_t)bh * nBlk + blk;
+    auto issue = [&](int m) {
+        if (m >= 0) {
+            CarryStage& s = stages[m % kStages];
+            const int sl = slot_of(m);
+            const Slot tok = slot_tokens(sl, Tlen, L);
+            const size_t slot = (size_t)bh * nSlot + sl;
             for (int c = tid; c < 512; c += 128) {
                 const int rr = c >> 3, c8 = (c & 7) * 8;
-                cp_async16(&s.m[c >> 6][c & 63][0], mprime + slot * (kN * kN) + (size_t)c * 8);
-                cp_async16(&s.rb[rr][c8], rbar + seq_base + (size_t)(blk * kC + rr) * tok_stride + c8);
-                if (dy != nullptr) cp_async16(&s.dy[rr][c8], dy + seq_base + (size_t)(blk * kC + rr) * tok_stride + c8);
+                const bool in = rr < tok.n;     // rows behind the slot's tokens: zeros
+                const size_t off = seq_base + (size_t)(tok.p + (in ? rr : 0)) * tok_stride + c8;
+                cp_async16(&s.m[c >> 6][c & 63][0], mprime + slot * (kN * kN) + (size_t)c * 8, true);
+                cp_async16(&s.rb[rr][c8], rbar + off, in);
+                if (dy != nullptr) cp_async16(&s.dy[rr][c8], dy + off, in);
             }
-            if (tid < 16) cp_async16(&s.lam[tid * 4], lam + slot * kN + tid * 4);
+            if (tid < 16) cp_async16(&s.lam[tid * 4], lam + slot * kN + tid * 4, true);
         }
         cp_async_commit();                      // an empty group keeps the group count in step
     };
@@ -117,22 +122,22 @@ wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length, cons
     };
 
 #pragma unroll
-    for (int i = 1; i < kStages; ++i) issue(nBlk - i);
-    uint8_t flag_here = new_starts[(size_t)bi * Tlen + (size_t)(nBlk - 1) * kC];   // start flag of the block's first token
-    for (int blk = nBlk - 1; blk >= 0; --blk) {
-        cp_async_wait<kStages - 2>();           // the copies of block blk have landed (younger groups may be in flight)
+    for (int i = 1; i < kStages; ++i) issue(steps - i);
+    for (int m = steps - 1; m >= 0; --m) {
+        cp_async_wait<kStages - 2>();           // the copies of this slot have landed (younger groups may be in flight)
         __syncthreads();                        // ... for every thread; and everyone is done with the stage refilled next
-        issue(blk - (kStages - 1));
-        const uint8_t flag_next = (blk > 0) ? new_starts[(size_t)bi * Tlen + (size_t)(blk - 1) * kC] : 0;   // asked for a block ahead
-        const CarryStage& s = stages[blk % kStages];
-        const int p1 = (blk + 1) * kC;
+        issue(m - (kStages - 1));
+        const CarryStage& s = stages[m % kStages];
+        const int sl = slot_of(m);
+        const Slot tok = slot_tokens(sl, Tlen, L);
+        const int p1 = tok.p + tok.n;
         // cotangent of the returned state enters behind token length - 1
         if (p1 == L && ds_out != nullptr) add_ds_out();
         // the gradient leaving this block, in bf16: to global memory for the gradient kernel, and as the left
         // operand of the next product
         uint32_t afrag[4][4];
         {
-            __nv_bfloat16* out = dstate + ((size_t)bh * nBlk + blk) * kN * kN;
+            __nv_bfloat16* out = dstate + ((size_t)bh * nSlot + sl) * kN * kN;
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
                 const uint32_t lo = pack2(acc[nt][0], acc[nt][1]), hi = pack2(acc[nt][2], acc[nt][3]);
@@ -176,14 +181,6 @@ wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length, cons
                 }
             }
         }
-        // a start flag on the block's first token cuts the dependency on everything before it
-        if (flag_here != 0) {
-#pragma unroll
-            for (int nt = 0; nt < 8; ++nt)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[nt][e] = 0.f;
-        }
-        flag_here = flag_next;
     }
     if (L == 0 && ds_out != nullptr) add_ds_out();   // the returned state IS the input state
 #pragma unroll
@@ -195,7 +192,7 @@ wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length, cons
 
 }  // namespace
 
-int wkv7_carry_bwd(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* dy,
+int wkv7_carry_bwd(cudaStream_t st, int B, int T, int H, const uint32_t* length, const void* dy,
                    const void* ds_out, void* residual, const int* residual_mark, void* ds0) {
     typedef __nv_bfloat16 bf;
     static DeviceOnce smem_attr;
@@ -205,13 +202,13 @@ int wkv7_carry_bwd(cudaStream_t st, int B, int T, int H, const uint32_t* length,
             return cudaFuncSetAttribute(wkv7_carry_bwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, carry_smem<2>());
         }))
         return B200WKV_ELAUNCH;
-    const CarryLayout lay = carry_layout(B, T, H);
+    const ResidualLayout lay = residual_layout(B, T, H);
     char* base = static_cast<char*>(residual);
     const bool deep = (long long)B * H <= 2LL * sm_count_of_current_device();
     auto launch = deep ? wkv7_carry_bwd_kernel<3> : wkv7_carry_bwd_kernel<2>;
-    launch<<<B * H, 128, deep ? carry_smem<3>() : carry_smem<2>(), st>>>(T, H, length, ns, (const bf*)dy, (const bf*)ds_out, (const bf*)(base + lay.mprime),
+    launch<<<B * H, 128, deep ? carry_smem<3>() : carry_smem<2>(), st>>>(T, H, length, (const bf*)dy, (const bf*)ds_out, (const bf*)(base + lay.mprime),
                                                                          (const bf*)(base + lay.rbar), (const float*)(base + lay.lam),
-                                                                         (const int*)(base + lay.fast), residual_mark, (bf*)(base + lay.dstate), (bf*)ds0);
+                                                                         residual_mark, (bf*)(base + lay.dstate), (bf*)ds0);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 

@@ -13,15 +13,21 @@
 //   S_C = S0 diag(L_C) + sa^T B^ + V^T K^
 // All products are tcgen05.mma (M=128, bf16 operands from shared memory, fp32 accumulators in
 // TMEM); the unit-triangular inverse is an fp32 forward substitution on CUDA cores; the state
-// stays in TMEM in fp32 for the whole sequence.  Start flags and `length` never need masks:
-// a chunk simply ends early in front of a start position and at `length`, and the rows of a
-// short chunk are zero-filled.
+// stays in TMEM in fp32 for the whole sequence.
+//
+// A start flag on a token of the chunk cuts every dependence of the tokens from it on, on what came before: the pairwise
+// products lose the columns in front of the row's last flag, the S0 products the rows from the first flag on, B^ and K^
+// the rows in front of the last flag, and the decayed entering state is dropped.  (Ending the chunk in front of every
+// flag instead, as an earlier form did, costs a whole chunk's time per flag, and a backward that can follow it: forward and
+// backward at B=6, T=2043, H=32 with a flag every 512 tokens took 970-990 us so, and take 676 us with the masks, while
+// sequences without flags, B=8, T=4096, H=32, take 1.44 ms either way.)  The
+// cumulative decay is not restarted: only ratios inside a segment survive the masks.  A chunk ends early only where the
+// state is wanted, at `length`, and at the end of the sequence; the rows behind its end are zero.
 //
 // Data movement: the raw rows of the next chunk arrive in shared memory by tiled bulk copies
-// (cp.async.bulk.tensor) while the current chunk finishes.  When a residual is requested, every block
-// walked as one full chunk leaves bf16 operand slabs for the backward (T, A_ak, P_rb, P_rk, sa, S0; most
-// of them by bulk stores out of shared memory) so that the backward need not recompute them; the fp32
-// state entering a block is written only when the block's first chunk is short.
+// (cp.async.bulk.tensor) while the current chunk finishes.  When a residual is requested, every chunk
+// leaves bf16 operand slabs for the backward (T, A_ak, P_rb, P_rk, sa, S0; most of them by bulk stores out of shared
+// memory) so that the backward need not recompute them.
 //
 // Semantics: BaseRWKV.inner_loop of jaxrwkv (src/jaxrwkv/rwkv7.py:199-220).
 #include "common.cuh"
@@ -95,12 +101,11 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                       const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                       const __nv_bfloat16* __restrict__ s0, const uint32_t* __restrict__ length,
                       const uint8_t* __restrict__ new_starts, __nv_bfloat16* __restrict__ y,
-                      __nv_bfloat16* __restrict__ s_out, float* __restrict__ ckpt, float* __restrict__ s_at_len,
+                      __nv_bfloat16* __restrict__ s_out, float* __restrict__ s_at_len,
                       const __grid_constant__ StreamMaps maps, const __grid_constant__ CUtensorMap y_map, const __grid_constant__ CUtensorMap rbar_map,
                       unsigned char* __restrict__ saved,
                       int* __restrict__ range_flag, int range_ticket, int* __restrict__ residual_mark,
-                      __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out,
-                      int* __restrict__ fast_flag, int pieces) {
+                      __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces) {
     extern __shared__ __align__(1024) unsigned char smem[];   // (the swizzle of the output tile is a function of the address)
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     // (all first pieces come first in the grid: where no cut exists the other pieces' CTAs return at once, and the
@@ -144,7 +149,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
     const size_t tok_stride = (size_t)H * kN;
     const size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
     const size_t st_row = ((size_t)bh * kN + (row & 63)) * kN + hsel * 32;  // this thread's 32 state elements
-    const int nBlk = (Tlen + kC - 1) / kC;
+    const int nSlot = block_slots(Tlen);
 
     if (tid == 0) {
 #pragma unroll
@@ -193,10 +198,9 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
 
     constexpr int kIssuer2 = 96;   // a thread of the warp with the least epilogue work
     int p = t_begin;
-    bool all_saved = (saved != nullptr);   // every chunk so far was a full block with its operands saved
     uint32_t par = 0, spar = 0;   // phase parities of the product barriers and of the staging barrier
     // result tiles of the chunk just finished, waiting in shared memory for the next CTA barrier
-    bool pend_y = false, pend_m = false;
+    bool pend_y = false, pend_m = false, pend_r = false;
     int pend_p = 0;
     size_t pend_slot = 0;
     auto send_tiles = [&]() {   // behind a CTA barrier that follows the epilogue's stores
@@ -205,11 +209,11 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             if (pend_m) {
                 tc::bulk_store(mprime + pend_slot * (kN * kN), smem + OFF_MT, GTILE);
                 // R- = R~ + P_rb W~: added in bf16 onto the R~ rows that went to global memory when the operands were scaled
-                tc::tensor_reduce_add_2d(&rbar_map, h * kN, bi * Tlen + pend_p, smem + OFF_RT);
+                if (pend_r) tc::tensor_reduce_add_2d(&rbar_map, h * kN, bi * Tlen + pend_p, smem + OFF_RT);
             }
             tc::bulk_commit();
         }
-        pend_y = pend_m = false;
+        pend_y = pend_m = pend_r = false;
     };
     uint8_t flag_ahead = (tid < 64 && t_begin + tid < Tlen) ? new_starts[(size_t)bi * Tlen + t_begin + tid] : 0;
     // the 64 token rows from cp on of w, r, k, v, a, b into the staging tiles (thread 0; one tiled copy
@@ -240,36 +244,25 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         }
         if (p >= t_end) break;
         // ================= extent of this chunk =================
-        const int be = min(((p >> 6) + 1) << 6, t_end);
+        // (with a residual the chunks are the 64-token blocks of the sequence, so that the backward can number them)
+        const int be = min(saved != nullptr ? ((p >> 6) + 1) << 6 : p + kC, t_end);
+        const int p1 = L > p && L < be ? L : be, n = p1 - p;
         if (tid < 64) {
             // the flag byte of position p + tid was requested while the previous chunk's products ran
-            const bool f = (p + tid < be) && (flag_ahead != 0);
+            const bool f = tid < n && flag_ahead != 0;
             const uint32_t m = __ballot_sync(0xffffffffu, f);
             if (lane == 0) sm.nsm[warp] = m;
         }
         __syncthreads();   // nsm visible; previous chunk's shared-memory readers are done
         send_tiles();
         const uint64_t mask = (uint64_t)sm.nsm[0] | ((uint64_t)sm.nsm[1] << 32);
-        const bool reset_here = (mask & 1ull) != 0;
-        int p1 = be;
-        if ((mask >> 1) != 0) p1 = p + __ffsll((long long)(mask >> 1));
-        if (L > p && L < p1) p1 = L;
-        const int n = p1 - p;
-        // a block walked as one full chunk leaves its operand slabs T, A_ak, P_rb, P_rk, sa for the backward
-        unsigned char* const keep = (saved != nullptr && n == kC && (p & (kC - 1)) == 0)
-                                        ? saved + ((size_t)bh * nBlk + (p >> 6)) * kSavedBytes : nullptr;
-        all_saved = all_saved && (keep != nullptr);
-        const size_t blk_slot = (size_t)bh * nBlk + (p >> 6);
-        // the fp32 state entering a block is only needed by a backward that recomputes the block's first chunk,
-        // i.e. when that chunk is short; a full chunk passes its bf16 entering state with the saved slabs
-        if (quad < 2 && ckpt != nullptr && (p & (kC - 1)) == 0 && n < kC) {
-            float s[32];
-            tc::tmem_ld32(lane_addr + DS + hsel * 32, s);
-            tc::tmem_wait_ld();
-            float* dst = ckpt + (((size_t)bh * nBlk + p / kC) * kN + row) * kN + hsel * 32;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) *reinterpret_cast<float4*>(dst + c * 4) = make_float4(s[c * 4], s[c * 4 + 1], s[c * 4 + 2], s[c * 4 + 3]);
-        }
+        const bool reset_here = (mask & 1ull) != 0, inner = (mask >> 1) != 0;   // a flag on the first token; on others
+        auto in_first = [&](int t) { return (mask & ((2ull << t) - 1ull)) == 0; };   // no flag at or before token t of the chunk
+        auto in_last = [&](int t) { return ((mask >> t) >> 1) == 0; };               // none behind it
+        // the chunk leaves its operand slabs T, A_ak, P_rb, P_rk, sa, S0 for the backward: slot p / 64, and the last slot for
+        // the second part of a block that `length` cuts (the only chunk that starts inside a block)
+        const size_t blk_slot = (size_t)bh * nSlot + ((p & (kC - 1)) == 0 ? p >> 6 : nSlot - 1);
+        unsigned char* const keep = saved != nullptr ? saved + blk_slot * kSavedBytes : nullptr;
         // ================= stage inputs (registers), log-decay into the scan buffer =================
         uint4 raw[2][5];   // r, k, v, a, b
         float lw[2][8];    // log2 of the decay: -exp(w) * log2(e)
@@ -355,7 +348,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                     // a second copy of A~ waits in the sa slab, which is idle until sa itself is stored; R~ goes
                     // to the R- rows in global memory, where P_rb W~ is added at the end of the chunk
                     slab_store(smem + OFF_SA, CB64, t, jb, a_t);
-                    *reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + jb * 8) = r_t;
+                    if (t < n) *reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + jb * 8) = r_t;
                     tc::fence_async_global();   // a bulk copy adds onto these rows at the end of the chunk
                 }
                 slab_store(smem + OFF_BK, CB128, t, jb, scale8(raw[q][4], eI));
@@ -363,6 +356,22 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 slab_store(smem + OFF_BH, CB64, t, jb, scale8(raw[q][4], eE));
                 slab_store(smem + OFF_KH, CB64, t, jb, scale8(raw[q][1], eE));
                 slab_store(smem + OFF_V, CB64, t, jb, raw[q][2]);
+            }
+            if (mask != 0) {   // the rare chunk with start flags: the masked rows are written over
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int t = q * 32 + tsub;
+                    const uint4 none = make_uint4(0, 0, 0, 0);
+                    if (keep != nullptr && !in_first(t)) {   // what carries the dependence on S0: nothing from the first flag on
+                        slab_store(smem + OFF_SA, CB64, t, jb, none);
+                        if (t < n) *reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + jb * 8) = none;
+                        tc::fence_async_global();
+                    }
+                    if (!in_last(t)) {                       // what reaches S_C: nothing in front of the last flag
+                        slab_store(smem + OFF_BH, CB64, t, jb, none);
+                        slab_store(smem + OFF_KH, CB64, t, jb, none);
+                    }
+                }
             }
         }
         // ================= entering state: bf16 copy for the products, decayed fp32 copy back to TMEM =====
@@ -382,6 +391,10 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 const float4 l4 = *reinterpret_cast<const float4*>(&sm.lam[hsel * 32 + c * 4]);
                 s[c * 4] *= l4.x; s[c * 4 + 1] *= l4.y; s[c * 4 + 2] *= l4.z; s[c * 4 + 3] *= l4.w;
             }
+            if (mask != 0) {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) s[c] = 0.f;
+            }
             tc::tmem_st32(lane_addr + DS + hsel * 32, s);
             tc::tmem_wait_st();
         }
@@ -399,7 +412,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             tc::bulk_store(keep + (size_t)SAVED_S0 * GTILE + lane * GCB, smem + OFF_S0 + lane * CB64, 64 * 16);
             tc::bulk_commit();
         }
-        if (keep != nullptr && tid < 64) lam_out[blk_slot * kN + tid] = sm.lam[tid];
+        if (keep != nullptr && tid < 64) lam_out[blk_slot * kN + tid] = mask != 0 ? 0.f : sm.lam[tid];
         if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
         tc::fence_after_sync();
         // ================= E1: triangular masks, operands of the next products =================
@@ -409,6 +422,12 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             tc::tmem_ld32(lane_addr + D1 + hsel * 64, d);
             tc::tmem_ld32(lane_addr + D1 + hsel * 64 + 32, d + 32);
             tc::tmem_wait_ld();
+            if (inner) {                          // nothing from in front of the row's last start flag
+                const uint64_t upto = mask & ((2ull << t) - 1ull);
+                const int from = upto != 0 ? 63 - __clzll((long long)upto) : 0;
+#pragma unroll
+                for (int s = 0; s < 64; ++s) d[s] = s >= from ? d[s] : 0.f;
+            }
             if (row < 64 && hsel == 0) {          // A_ab, strictly lower, fp32 for the inverse
 #pragma unroll
                 for (int c = 0; c < 16; ++c)
@@ -424,6 +443,16 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
 #pragma unroll
                 for (int c = 0; c < 8; ++c) slab_store(dst, CB128, row, c, pack8(&d[c * 8]));
             }
+        }
+        if (inner) {                              // A~ S0^T and R~ S0^T: nothing from the first flag on
+            float g[32];
+            tc::tmem_ld32(lane_addr + D2 + hsel * 32, g);
+            tc::tmem_wait_ld();
+            const bool first = in_first(row & 63);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) g[c] = first ? g[c] : 0.f;
+            tc::tmem_st32(lane_addr + D2 + hsel * 32, g);
+            tc::tmem_wait_st();
         }
         if (warp == 7) tc::bulk_wait_read<0>();   // the S0 slab has been read: the inverse writes over part of it next
         tc::fence_async_smem();
@@ -536,6 +565,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         pend_y = (n == kC);
         pend_p = p;
         pend_m = (keep != nullptr);
+        pend_r = pend_m && n == kC;
         pend_slot = blk_slot;
         if (keep != nullptr) {
             float m[32];
@@ -548,9 +578,21 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 const int t = row - 64;
                 tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, m);
                 tc::tmem_wait_ld();
+                if (n == kC) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    *reinterpret_cast<uint4*>(smem + OFF_RT + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&m[c * 8]);
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<uint4*>(smem + OFF_RT + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&m[c * 8]);
+                } else if (t < n) {   // a short chunk's rows one by one: a tiled copy would go over the next sequence's
+                    uint4* to = reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + hsel * 32);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        float x[8];
+                        unpack8(to[c], x);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) x[e] += m[c * 8 + e];
+                        to[c] = pack8(x);
+                    }
+                }
             }
         }
         tc::fence_async_smem();   // the result tiles are read by bulk copies
@@ -561,7 +603,6 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
     }
     __syncthreads();
     send_tiles();   // of the last chunk
-    if (fast_flag != nullptr && tid == 0) fast_flag[bh] = all_saved ? 1 : 0;
     if (warp == 7) tc::bulk_wait_all<0>();   // every copy to the residual has landed before the CTA retires
     if (failed) atomicExch(&g_status, 1);
     tc::fence_before_sync();
@@ -571,7 +612,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
 
 }  // namespace
 
-size_t wkv7_chunk_residual_bytes(int B, int T, int H) { return chunk_residual_floats(B, T, H) * sizeof(float); }
+size_t wkv7_chunk_residual_bytes(int B, int T, int H) { return residual_layout(B, T, H).end; }
 
 // A forward call that meets a decay outside the chunked kernels' range tells the fallback launched behind
 // it through one int of device memory.  Calls may be in flight on several streams, so each call takes the
@@ -612,7 +653,8 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
         return B200WKV_ELAUNCH;
     *range_flag = wkv_call_flag(range_ticket);
     if (*range_flag == nullptr) return B200WKV_ELAUNCH;
-    const CarryLayout lay = carry_layout(B, T, H);
+    const ResidualLayout lay = residual_layout(B, T, H);
+    char* const base = static_cast<char*>(residual);
     StreamMaps maps;
     const void* bases[6] = {w, r, k, v, a, b};   // maps[m]: the six streams as [B*T tokens][H*64 channels]
     if (!make_stream_maps(&maps, bases, 6, B, T, H)) return B200WKV_ELAUNCH;
@@ -632,15 +674,13 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
     }
     wkv7_chunk_fwd_kernel<<<B * H * pieces, 256, SMEM_BYTES, st>>>(T, H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v,
                                                           (const bf*)a, (const bf*)b, (const bf*)s0, length, ns,
-                                                          (bf*)y, (bf*)s_out, (float*)residual,
-                                                          residual ? (float*)residual + (size_t)B * H * ((T + kC - 1) / kC) * kN * kN : nullptr,
+                                                          (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : nullptr,
                                                           maps, out_maps.m[0], out_maps.m[1],
-                                                          residual ? (unsigned char*)((float*)residual + chunk_saved_offset_floats(B, T, H)) : nullptr,
+                                                          residual ? (unsigned char*)(base + lay.saved) : nullptr,
                                                           *range_flag, *range_ticket, residual_mark,
-                                                          residual ? (bf*)((char*)residual + lay.mprime) : nullptr,
-                                                          residual ? (bf*)((char*)residual + lay.rbar) : nullptr,
-                                                          residual ? (float*)((char*)residual + lay.lam) : nullptr,
-                                                          residual ? (int*)((char*)residual + lay.fast) : nullptr, pieces);
+                                                          residual ? (bf*)(base + lay.mprime) : nullptr,
+                                                          residual ? (bf*)(base + lay.rbar) : nullptr,
+                                                          residual ? (float*)(base + lay.lam) : nullptr, pieces);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 

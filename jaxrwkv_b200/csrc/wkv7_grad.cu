@@ -17,6 +17,14 @@
 // D_{t-1} = D_t + u_t holds and d(log decay)_t = D_{t-1} - a_t da_t; D at the block end comes exactly from dS
 // and the state leaving the block (the next block's saved S0, or the state at `length`).
 //
+// A start flag inside the block (wkv7_chunk.cu): the saved tiles carry its masks already; here W keeps pairs of one
+// segment only, the dS products keep the rows behind the last flag, the S0 products those in front of the first, and the
+// decay-gradient scan restarts at each flag; these products go to accumulators of their own.  A block need not be full: the
+// last one of a sequence, and the two parts of the block that `length` cuts, have zero rows behind their end and leave row by
+// row.  (As a second instantiation and launch these blocks, few and of uneven distance in the list, took 128 us instead of 40
+// at B=6, T=2043, H=32.  What describes a block - its tokens, its flags - is kept in shared memory and read where it is
+// needed: at the 128 registers that two CTAs per SM leave, holding it in registers cost every block 2 %.)
+//
 // Shared memory holds every operand as an unpadded slab (8 column blocks of [rows][16 bytes]); the thread
 // that scales a token's operands owns one token and two column blocks, so that its 16-byte stores and the
 // 128-byte-swizzled staging rows it reads are both free of bank conflicts.  The raw rows of the next block
@@ -59,10 +67,15 @@ constexpr int OFF_UB = OFF_X1;              // last epilogue: fp32 a da - b db (
 // the block the decay gradient, use the 8 KB that only the last epilogue's fp32 buffer shares.
 constexpr int OFF_TK = OFF_VSA, OFF_TB = OFF_VSA + T64, OFF_TR = OFF_DD, OFF_TA = OFF_DD + T64;
 constexpr int OFF_TV = OFF_X2;
+struct Item {            // a slot of the work list; id >= the length of the list: none is left
+    int id, slot, bi, h, p, n, L;      // slot: its number among all slots
+};
 struct Small {
     uint64_t bar[8];     // 0..3 product rounds, 4 staging, 5 P_rb|P_rk|sa, 6 T|A_ak, 7 S0
     uint32_t tmem;
-    uint32_t pad[3];
+    uint32_t pad;
+    uint32_t starts[2][2];   // start flags of the block's tokens, of this block and the next in turn
+    Item item[2];            // this block and the next in turn, looked up by one thread (divisions and dependent loads)
     float lam[kN];       // 2^(block total)
     float d_end[kN];     // D at the block end
     float seg_tail[kN];  // with lam and d_end (both dead by then): per-16-token totals of the decay-gradient scan, [3][64]
@@ -114,7 +127,7 @@ __device__ __forceinline__ uint4 mul8(uint4 a, uint4 b) {
 __global__ void __launch_bounds__(256, 2)
 wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts,
                      const __nv_bfloat16* __restrict__ ds_state, const float* __restrict__ s_at_len,
-                     const unsigned char* __restrict__ saved, const int* __restrict__ fast, const int* __restrict__ residual_mark,
+                     const unsigned char* __restrict__ saved, const int* __restrict__ residual_mark,
                      __nv_bfloat16* __restrict__ dw, __nv_bfloat16* __restrict__ dr, __nv_bfloat16* __restrict__ dk,
                      __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ da, __nv_bfloat16* __restrict__ db,
                      int* __restrict__ status, int has_dy, unsigned char* __restrict__ fscr_all,
@@ -125,21 +138,31 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, hsel = warp >> 2;     // TMEM lane quadrant / column half handled by this warp
     const int row = quad * 32 + lane;                // TMEM lane == tile row
-    const int nBlk = Tlen / kC;
-    const int n_items = BH * nBlk;   // (the launcher refuses shapes whose block count overflows an int)
+    const int nSlot = block_slots(Tlen), nBlk = nSlot - 1;
+    const int n_items = BH * nSlot;   // (the launcher refuses shapes whose slot count overflows an int)
     unsigned char* const fscr = fscr_all + (size_t)blockIdx.x * 4 * GTILE;
     // the 128-byte swizzle of the staging tiles is a function of the shared-memory address
     if ((tc::smem_u32(smem) & 1023u) != 0) {
         if (tid == 0 && status != nullptr) atomicExch(status, 4);
         return;
     }
-    // next item of the flat (sequence, block) list that belongs to a sequence this kernel handles
-    auto next_item = [&](int it) {
-        while (it < n_items && fast[it / nBlk] == 0) it += (int)gridDim.x;
-        return it;
+    // the list: the blocks of all sequences, then the sequences' last slots, which most do not use (see slot_tokens())
+    constexpr int kFindThread = 160;
+    auto find_item = [&](int id, Item* to) {
+        for (; id < n_items; id += (int)gridDim.x) {
+            const int bh = id < BH * nBlk ? id / nBlk : id - BH * nBlk, sl = id < BH * nBlk ? id - bh * nBlk : nBlk;
+            const int bi = bh / H, L = min((int)length[bi], Tlen);
+            const Slot t = slot_tokens(sl, Tlen, L);
+            if (t.n > 0) {
+                *to = Item{id, bh * nSlot + sl, bi, bh - bi * H, t.p, t.n, L};
+                return;
+            }
+        }
+        to->id = n_items;
     };
-    int item = next_item((int)blockIdx.x);
-    if (item >= n_items) return;
+    if (tid == kFindThread) find_item((int)blockIdx.x, &sm.item[0]);
+    __syncthreads();
+    if (sm.item[0].id >= n_items) return;
 
     if (tid == 0) {
 #pragma unroll
@@ -182,32 +205,34 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
 
     const int n_streams = has_dy ? 7 : 6;
     // raw tiles m_from..m_to-1 of block `it` (thread kStageThread; the first call of a block announces all of them)
-    auto issue_stage = [&](int it, int m_from, int m_to) {
+    auto issue_stage = [&](const Item& it, int m_from, int m_to) {
         if (tid == kStageThread) {
-            const int bh_ = it / nBlk, blk_ = it % nBlk;
             if (m_from == 0) tc::mbar_expect_tx(&sm.bar[4], (uint32_t)(n_streams * T64));
-            const int x = (bh_ % H) * kN, y = (bh_ / H) * Tlen + blk_ * kC;
+            const int x = it.h * kN, y = it.bi * Tlen + it.p;
 #pragma unroll
             for (int m = 0; m < 7; ++m)
                 if (m >= m_from && m < m_to && m < n_streams) tc::tensor_load_2d(smem + OFF_STG + m * T64, &maps.m[m], x, y, &sm.bar[4]);
         }
     };
     tc::fence_async_smem();
-    issue_stage(item, 0, 7);
+    issue_stage(sm.item[0], 0, 7);
     bool pend_dw = false;    // the decay-gradient tile of the previous block waits for a CTA barrier
     int pend_x = 0, pend_y = 0;
-    // what the loop needs to know about a block before it touches it, fetched one block ahead
-    int meta_L = min((int)length[(item / nBlk) / H], Tlen);
-    bool meta_reset = new_starts[(size_t)((item / nBlk) / H) * Tlen + (item % nBlk) * kC] != 0;
+    // the start flags of a block's tokens, fetched one block ahead
+    auto flag_at = [&](const Item& it) -> uint8_t { return tid < it.n && tid < kC ? new_starts[(size_t)it.bi * Tlen + it.p + tid] : (uint8_t)0; };
+    uint8_t meta_flag = flag_at(sm.item[0]);
 
-    while (item < n_items) {
-        const int bh = item / nBlk, blk = item % nBlk, bi = bh / H;
-        const int L = meta_L;
-        const bool reset_here = meta_reset;
-        const int p = blk * kC, p1 = p + kC;
-        const size_t st_base = (size_t)bh * kN * kN;
-        const unsigned char* tiles = saved + ((size_t)bh * nBlk + blk) * kSavedBytes;
-        const __nv_bfloat16* dsg = ds_state + ((size_t)bh * nBlk + blk) * kN * kN;
+    while (true) {
+        // (volatile: read anew where they are used)
+        const volatile Item& it = sm.item[par];
+        const volatile uint32_t* const starts = sm.starts[par];
+        auto mask_of = [&]() { return (uint64_t)starts[0] | ((uint64_t)starts[1] << 32); };
+        auto inner = [&]() { return ((starts[0] & ~1u) | starts[1]) != 0; };                       // a flag behind the first token
+        auto in_first = [&](int t) { return (mask_of() & ((2ull << t) - 1ull)) == 0; };            // no flag at or before token t
+        auto in_last = [&](int t) { return ((mask_of() >> t) >> 1) == 0; };                        // none behind it
+        const int item = it.slot;
+        const unsigned char* tiles = saved + (size_t)item * kSavedBytes;
+        const __nv_bfloat16* dsg = ds_state + (size_t)item * kN * kN;
 
         // the state gradient leaving this block (global memory) is asked for before anything waits
         const uint4 ds_raw0 = *reinterpret_cast<const uint4*>(dsg + sc * (kN * 8) + si * 8);         // column block sc, row si
@@ -221,6 +246,15 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             for (int h2 = 0; h2 < 2; ++h2)
                 raw[m][h2] = (m < n_streams) ? *reinterpret_cast<const uint4*>(smem + OFF_STG + m * T64 + st_t * 128 + (((st_jb + h2) ^ (st_t & 7)) << 4))
                                              : make_uint4(0, 0, 0, 0);
+        const bool behind_end = st_t >= it.n;      // rows behind the block's tokens: zeros, and no decay
+        if (behind_end) {
+#pragma unroll
+            for (int m = 0; m < 7; ++m) raw[m][0] = raw[m][1] = make_uint4(0, 0, 0, 0);
+        }
+        if (tid < 64) {
+            const uint32_t m = __ballot_sync(0xffffffffu, meta_flag != 0);
+            if (lane == 0) sm.starts[par][warp] = m;
+        }
         tc::fence_async_smem();
         __syncthreads();   // the staging tiles are empty; the previous block's last epilogue has finished everywhere
         if (issuer_b && pend_dw) {
@@ -247,6 +281,10 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             unpack8(raw[0][h2], wf);
 #pragma unroll
             for (int e = 0; e < 8; ++e) lw[h2 * 8 + e] = -kLog2e * __expf(wf[e]);
+        }
+        if (behind_end) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) lw[e] = 0.f;
         }
 #pragma unroll
         for (int c4 = 0; c4 < 4; ++c4)
@@ -326,9 +364,9 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         // ================= R2: [Gd ; dVpart] = [B~;K~] dSL^T + [P_rb|P_rk]^T dY =================
         if (issuer_a) {
             tc::fence_after_sync();
-            mma_k64(tbase + T_GD, kmaj128u(sBK), kmaj64u(sDSL), ID_KK, false);
+            mma_k64(tbase + (inner() ? T_W : T_GD), kmaj128u(sBK), kmaj64u(sDSL), ID_KK, false);
             if (!tc::mbar_wait(&sm.bar[5], par)) failed = true;   // P_rb | P_rk (and sa) have landed
-            mma_k64(tbase + T_GD, mnmaj64u(sPRB), mnmaj128u(sDD), ID_MM, true);
+            mma_k64(tbase + T_GD, mnmaj64u(sPRB), mnmaj128u(sDD), ID_MM, !inner());
             tc::commit(&sm.bar[0]);
         }
         if (quad >= 2) {
@@ -342,10 +380,11 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             float acc[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) acc[e] = 0.f;
-            if (p1 == L || blk + 1 < nBlk) {
+            const int p1 = it.p + it.n, L = it.L, bh = it.bi * H + it.h;
+            if (p1 == L || p1 < Tlen) {
                 const bool at_len = (p1 == L);
-                const float* sf = s_at_len + st_base + cbk * 8;
-                const unsigned char* sb = tiles + kSavedBytes + SAVED_S0 * GTILE + cbk * GCB;
+                const float* sf = s_at_len + (size_t)bh * kN * kN + cbk * 8;
+                const unsigned char* sb = saved + ((size_t)bh * nSlot + (p1 >> 6)) * kSavedBytes + SAVED_S0 * GTILE + cbk * GCB;
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {
                     const int i = ig + 16 * m;
@@ -372,6 +411,19 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
 #pragma unroll
                 for (int e = 0; e < 8; ++e) sm.d_end[cbk * 8 + e] = acc[e] / sm.lam[cbk * 8 + e];
             }
+            if (inner()) {   // dV: the dS share of the rows behind the last flag joins the rest
+                if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
+                tc::fence_after_sync();
+                float x[32], y[32];
+                tc::tmem_ld32(lane_addr + T_GD + hsel * 32, x);
+                tc::tmem_ld32(lane_addr + T_W + hsel * 32, y);
+                tc::tmem_wait_ld();
+                const bool last = in_last(row - 64);
+#pragma unroll
+                for (int c = 0; c < 32; ++c) x[c] += last ? y[c] : 0.f;
+                tc::tmem_st32(lane_addr + T_GD + hsel * 32, x);
+                tc::tmem_wait_st();
+            }
         }
         if (quad < 2) {
             if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
@@ -379,6 +431,14 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             float gd[32];
             tc::tmem_ld32(lane_addr + T_GD + hsel * 32, gd);
             tc::tmem_wait_ld();
+            if (inner()) {
+                float y[32];
+                tc::tmem_ld32(lane_addr + T_W + hsel * 32, y);
+                tc::tmem_wait_ld();
+                const bool last = in_last(row);
+#pragma unroll
+                for (int c = 0; c < 32; ++c) gd[c] += last ? y[c] : 0.f;
+            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) slab_store(smem + OFF_X1, P64, row, hsel * 4 + c, pack8(&gd[c * 8]));   // over P_rk, which is read
         }
@@ -420,19 +480,18 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             mma_k64(tbase + T_KB, kmaj128u(sVSA), mnmaj64u(sDSL), ID_KM, false);
             tc::commit(&sm.bar[2]);
         }
-        // the next block of this CTA, and what the loop needs to know about it
-        const int item_next = next_item(item + (int)gridDim.x);
-        if (item_next < n_items) {
-            const int bi_n = (item_next / nBlk) / H;
-            meta_L = min((int)length[bi_n], Tlen);
-            meta_reset = new_starts[(size_t)bi_n * Tlen + (item_next % nBlk) * kC] != 0;
-        }
+        if (tid == kFindThread) find_item(it.id + (int)gridDim.x, &sm.item[par ^ 1]);   // the next block of this CTA
         if (!tc::mbar_wait(&sm.bar[2], par)) failed = true;
         tc::fence_after_sync();
         {
             // keep s >= t for the dY blocks, s > t for the dG blocks.  Rows t < 32 keep all of columns 32..63;
             // rows t >= 32 keep nothing of columns 0..31 (zeros are stored without reading the accumulator).
+            // With start flags in the block, s stays in front of the first one behind t.
             const int t = row & 63, lo = t + hsel;
+            auto first_behind = [&]() {
+                const uint64_t behind = (mask_of() >> t) >> 1;
+                return behind != 0 ? t + __ffsll((long long)behind) : kC;
+            };
             unsigned char* dst = smem + (hsel == 0 ? OFF_WY : OFF_WSA);   // over T, A_ak, dSL, P_rb: all read by now
             float d[32];
             if ((quad & 1) == 0) {
@@ -440,10 +499,20 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                 tc::tmem_wait_ld();
 #pragma unroll
                 for (int s = 0; s < 32; ++s) d[s] = (s >= lo) ? d[s] : 0.f;
+                if (inner()) {
+                    const int hi = first_behind();
+#pragma unroll
+                    for (int s = 0; s < 32; ++s) d[s] = s < hi ? d[s] : 0.f;
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) slab_store(dst, P128, row, c, pack8(&d[c * 8]));
                 tc::tmem_ld32(lane_addr + T_W + hsel * 64 + 32, d);
                 tc::tmem_wait_ld();
+                if (inner()) {
+                    const int hi = first_behind();
+#pragma unroll
+                    for (int s = 0; s < 32; ++s) d[s] = s + 32 < hi ? d[s] : 0.f;
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) slab_store(dst, P128, row, 4 + c, pack8(&d[c * 8]));
             } else {
@@ -453,15 +522,35 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                 tc::tmem_wait_ld();
 #pragma unroll
                 for (int s = 0; s < 32; ++s) d[s] = (s + 32 >= lo) ? d[s] : 0.f;
+                if (inner()) {
+                    const int hi = first_behind();
+#pragma unroll
+                    for (int s = 0; s < 32; ++s) d[s] = s + 32 < hi ? d[s] : 0.f;
+                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) slab_store(dst, P128, row, 4 + c, pack8(&d[c * 8]));
             }
+        }
+        if (inner()) {   // [V;sa] dSL: only the rows behind the last flag
+            float x[32];
+            tc::tmem_ld32(lane_addr + T_KB + hsel * 32, x);
+            tc::tmem_wait_ld();
+            const bool last = in_last(row & 63);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) x[c] = last ? x[c] : 0.f;
+            tc::tmem_st32(lane_addr + T_KB + hsel * 32, x);
+            tc::tmem_wait_st();
         }
         if (quad >= 2) {   // dV rows
             const int t = row - 64;
             float x[32];
             tc::tmem_ld32(lane_addr + T_GD + hsel * 32, x);
             tc::tmem_wait_ld();
+            if (it.n < kC && t < it.n) {
+                uint4* const to = reinterpret_cast<uint4*>(dv + ((size_t)(it.bi * (size_t)Tlen + it.p + t) * H + it.h) * kN + hsel * 32);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) to[c] = pack8(&x[c * 8]);
+            }
 #pragma unroll
             for (int c = 0; c < 4; ++c)
                 *reinterpret_cast<uint4*>(smem + OFF_TV + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&x[c * 8]);
@@ -469,6 +558,9 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         tc::fence_async_smem();
         tc::fence_before_sync();
         __syncthreads();
+        const Item& next = sm.item[par ^ 1];
+        const bool more = next.id < n_items;
+        if (more) meta_flag = flag_at(next);
         // ================= R5: [dK~';dB~'] += W . [A~;R~] ; [dR~';dA~'] = [dY;dG] S0 + W^T . [B~;K~] =================
         if (issuer_a) {
             tc::fence_after_sync();
@@ -477,12 +569,14 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             tc::commit(&sm.bar[3]);
         } else if (issuer_b) {
             tc::fence_after_sync();
-            tc::tensor_store_2d(&out_maps.m[OUT_V], (bh % H) * kN, bi * Tlen + p, smem + OFF_TV);
-            tc::bulk_commit();
+            if (it.n == kC) {
+                tc::tensor_store_2d(&out_maps.m[OUT_V], it.h * kN, it.bi * Tlen + it.p, smem + OFF_TV);
+                tc::bulk_commit();
+            }
             mma_k64(tbase + T_RA, mnmaj128u(sWY + HALF), mnmaj128u(sBK), ID_MM, false);
             mma_k64(tbase + T_RA, mnmaj128u(sWY), mnmaj128u(sBK + HALF), ID_MM, true);
             if (!tc::mbar_wait(&sm.bar[7], par)) failed = true;   // S0 has landed
-            mma_k64(tbase + T_RA, kmaj128u(sDD), mnmaj64u(sX1), ID_KM, true);
+            mma_k64(tbase + (inner() ? T_GD : T_RA), kmaj128u(sDD), mnmaj64u(sX1), ID_KM, !inner());
             tc::bulk_wait_read<0>();   // the dV tile has left before this round is reported done: the last epilogue writes over it
             tc::commit(&sm.bar[3]);
         }
@@ -507,6 +601,14 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             tc::tmem_ld16(lane_addr + T_KB + hsel * 32 + hh * 16, x);
             tc::tmem_ld16(lane_addr + T_RA + hsel * 32 + hh * 16, z);
             tc::tmem_wait_ld();
+            if (inner()) {   // [dY;dG] S0: only the rows in front of the first flag
+                float y[16];
+                tc::tmem_ld16(lane_addr + T_GD + hsel * 32 + hh * 16, y);
+                tc::tmem_wait_ld();
+                const bool first = in_first(t);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) z[e] += first ? y[e] : 0.f;
+            }
 #pragma unroll
             for (int h2 = 0; h2 < 2; ++h2) {
                 const int c = hh * 2 + h2, cb = hsel * 4 + c;
@@ -539,30 +641,55 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         tc::fence_async_smem();   // the gradient tiles are read by bulk copies
         tc::fence_before_sync();
         __syncthreads();   // every operand slab has been read for the last time: the next block's rows may arrive
-        if (tid == kStageThread) {
-            const int x = (bh % H) * kN, y = bi * Tlen + p;
+        if (it.n < kC) {   // a tiled copy would go over the rows behind the block: row by row
+            const struct { __nv_bfloat16* to; int tile; } out4[4] = {{dk, OFF_TK}, {db, OFF_TB}, {dr, OFF_TR}, {da, OFF_TA}};
+#pragma unroll
+            for (int o = 0; o < 4; ++o)
+                for (int idx = tid; idx < it.n * 8; idx += 256) {
+                    const int tt = idx >> 3, piece = idx & 7;
+                    *reinterpret_cast<uint4*>(out4[o].to + ((size_t)(it.bi * (size_t)Tlen + it.p + tt) * H + it.h) * kN + piece * 8) =
+                        *reinterpret_cast<const uint4*>(smem + out4[o].tile + tt * 128 + ((piece ^ (tt & 7)) << 4));
+                }
+            __syncthreads();   // the tiles are read: staging tiles 4..6 may land on them
+        } else if (tid == kStageThread) {
+            const int x = it.h * kN, y = it.bi * Tlen + it.p;
             tc::tensor_store_2d(&out_maps.m[OUT_K], x, y, smem + OFF_TK);
             tc::tensor_store_2d(&out_maps.m[OUT_B], x, y, smem + OFF_TB);
             tc::tensor_store_2d(&out_maps.m[OUT_R], x, y, smem + OFF_TR);
             tc::tensor_store_2d(&out_maps.m[OUT_A], x, y, smem + OFF_TA);
             tc::bulk_commit();
         }
-        if (item_next < n_items) issue_stage(item_next, 0, 4);   // tiles 0..3 land on [A~;R~], [B~;K~]
+        if (more) issue_stage(next, 0, 4);   // tiles 0..3 land on [A~;R~], [B~;K~]
         if (tid == kStageThread) tc::bulk_wait_read<0>();        // tiles 4..6 on the gradient tiles, once those are read
-        if (item_next < n_items) issue_stage(item_next, 4, 7);
+        if (more) issue_stage(next, 4, 7);
         {   // D_{t-1} = D_t + u_t from D at the block end: suffix sums over 4 segments of 16 tokens, all loads first
             const int c = tid & 63, sg = tid >> 6;
             float vv[16];
 #pragma unroll
             for (int tt = 0; tt < 16; ++tt) vv[tt] = lf[swz1(sg * 16 + tt, c)] + ubuf[swz1(sg * 16 + tt, c)];
+            const uint32_t cuts = (starts[sg >> 1] >> ((sg & 1) * 16)) & 0xffffu;   // a flag: nothing passes to the tokens in front of it
+            if (cuts == 0) {
 #pragma unroll
-            for (int tt = 14; tt >= 0; --tt) vv[tt] += vv[tt + 1];
-            if (sg > 0) seg[(sg - 1) * 64 + c] = vv[0];
+                for (int tt = 14; tt >= 0; --tt) vv[tt] += vv[tt + 1];
+            } else {
+#pragma unroll
+                for (int tt = 14; tt >= 0; --tt) vv[tt] += (cuts >> (tt + 1)) & 1u ? 0.f : vv[tt + 1];
+            }
+            if (sg > 0) seg[(sg - 1) * 64 + c] = (cuts & 1u) ? 0.f : vv[0];
             __syncthreads();
             float off = d_end_c;
-            for (int s2 = 3; s2 > sg; --s2) off += seg[(s2 - 1) * 64 + c];
+            const bool any = (starts[0] | starts[1]) != 0;
+            for (int s2 = 3; s2 > sg; --s2) {
+                if (any && ((starts[s2 >> 1] >> ((s2 & 1) * 16)) & 0xffffu)) off = 0.f;
+                off += seg[(s2 - 1) * 64 + c];
+            }
+            if (cuts == 0) {
 #pragma unroll
-            for (int tt = 0; tt < 16; ++tt) lf[swz1(sg * 16 + tt, c)] = vv[tt] + off;
+                for (int tt = 0; tt < 16; ++tt) lf[swz1(sg * 16 + tt, c)] = vv[tt] + off;
+            } else {
+#pragma unroll
+                for (int tt = 0; tt < 16; ++tt) lf[swz1(sg * 16 + tt, c)] = vv[tt] + ((cuts >> tt) >> 1 ? 0.f : off);
+            }
         }
         __syncthreads();
         if (row >= 64) {
@@ -579,21 +706,27 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                 o[c * 8 + 4] = (d1.x - q1.x) * lg[4]; o[c * 8 + 5] = (d1.y - q1.y) * lg[5];
                 o[c * 8 + 6] = (d1.z - q1.z) * lg[6]; o[c * 8 + 7] = (d1.w - q1.w) * lg[7];
             }
-            if (reset_here && t == 0) {   // the state entering a start token is zero: no decay gradient
+            if ((starts[t >> 5] >> (t & 31)) & 1u) {   // the state entering a start token is zero: no decay gradient
 #pragma unroll
                 for (int e = 0; e < 32; ++e) o[e] = 0.f;
             }
+            if (it.n == kC) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                *reinterpret_cast<uint4*>(smem + OFF_TV + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&o[c * 8]);
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(smem + OFF_TV + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&o[c * 8]);
+            } else if (t < it.n) {
+                uint4* const to = reinterpret_cast<uint4*>(dw + ((size_t)(it.bi * (size_t)Tlen + it.p + t) * H + it.h) * kN + hsel * 32);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) to[c] = pack8(&o[c * 8]);
+            }
         }
-        pend_dw = true;
-        pend_x = (bh % H) * kN;
-        pend_y = bi * Tlen + p;
+        pend_dw = it.n == kC;
+        pend_x = it.h * kN;
+        pend_y = it.bi * Tlen + it.p;
         tc::fence_async_smem();   // the scan buffers are rewritten by bulk copies early in the next block; the tile is read by one
         tc::fence_before_sync();
         par ^= 1u;
-        item = item_next;
+        if (!more) break;
     }
     if (failed && status != nullptr) atomicExch(status, 2);
     tc::fence_before_sync();
@@ -620,24 +753,24 @@ int wkv7_grad_bwd(cudaStream_t st, int B, int T, int H, const void* w, const voi
     static DeviceOnce smem_attr;
     if (!smem_attr.ok([]() { return cudaFuncSetAttribute(wkv7_grad_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); }))
         return B200WKV_ELAUNCH;
-    const CarryLayout lay = carry_layout(B, T, H);
+    const ResidualLayout lay = residual_layout(B, T, H);
     char* base = static_cast<char*>(residual);
-    const int nBlk = T / kC, BH = B * H;
-    const float* s_at_len = (const float*)residual + (size_t)BH * nBlk * kN * kN;
-    const unsigned char* saved = reinterpret_cast<const unsigned char*>((const float*)residual + chunk_saved_offset_floats(B, T, H));
+    const int BH = B * H;
+    const float* s_at_len = (const float*)(base + lay.s_at_len);
+    const unsigned char* saved = (const unsigned char*)(base + lay.saved);
     StreamMaps maps;
     const void* bases[7] = {w, r, k, v, a, b, dy};
     if (!make_stream_maps(&maps, bases, dy != nullptr ? 7 : 6, B, T, H, /*swizzle128=*/true)) return B200WKV_ELAUNCH;
     StreamMaps out_maps;
     const void* out_bases[6] = {dw, dr, dk, dv, da, db};
     if (!make_stream_maps(&out_maps, out_bases, 6, B, T, H, /*swizzle128=*/true)) return B200WKV_ELAUNCH;
-    const long long items = (long long)BH * nBlk;
+    const long long items = (long long)BH * block_slots(T);
     if (items > 2147483647LL) return B200WKV_ESHAPE;
     long long slots = 2LL * sm_count_of_current_device();
     if (slots > kGradCtas) slots = kGradCtas;        // every CTA owns a set of factor tiles in the residual
     const int grid = (int)(items < slots ? items : slots);
     wkv7_grad_bwd_kernel<<<grid, 256, SMEM_BYTES, st>>>(T, H, BH, length, ns, (const bf*)(base + lay.dstate), s_at_len, saved,
-                                                        (const int*)(base + lay.fast), residual_mark, (bf*)dw, (bf*)dr, (bf*)dk,
+                                                        residual_mark, (bf*)dw, (bf*)dr, (bf*)dk,
                                                         (bf*)dv, (bf*)da, (bf*)db, wkv7_chunk_status_word(), dy != nullptr ? 1 : 0,
                                                         (unsigned char*)(base + lay.fscr), maps, out_maps);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;

@@ -395,7 +395,9 @@ static int launch_bwd(cudaStream_t st, int B, int Tlen, int H, const void* w, co
     if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem)); }))
         return B200WKV_ELAUNCH;
     const size_t used = wkv7_seq_residual_bytes(B, Tlen, H);
-    const int nC = (Tlen + kCk - 1) / kCk, run = run_length(B, Tlen, H, residual_bytes - used), runs = (nC + run - 1) / run;
+    const int nC = (Tlen + kCk - 1) / kCk;
+    // (behind the chunked kernels the launch nearly always finds nothing to do: one CTA per sequence, no carry)
+    const int run = run_if != nullptr ? nC : run_length(B, Tlen, H, residual_bytes - used), runs = (nC + run - 1) / run;
     float* const carry = reinterpret_cast<float*>(static_cast<char*>(residual) + used);
     if (runs > 1) {
         const int code = sizeof(T) == 4 ? B200WKV_F32 : B200WKV_BF16;
