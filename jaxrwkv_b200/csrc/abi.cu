@@ -54,7 +54,7 @@ int wkv6_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
                    int per_token, const void* u, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
                    void* s_out, void* residual, int* residual_mark, int** flag, int* ticket);
 int wkv6_chunk_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w,
-                   int per_token, const void* u, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out,
+                   const void* u, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out,
                    void* residual, const int* residual_mark, void* dr, void* dk, void* dv, void* dw, void* du, void* ds0);
 size_t wkv4_residual_bytes(int B, int T, int C);
 int wkv7_mix_partial_rows(int rows, int C);
@@ -248,7 +248,7 @@ int b200wkv6_bwd(void* stream, int dtype, int version, int B, int T, int H, int 
     if (dtype == B200WKV_BF16) {
         // the forward's mark decides on the device which of the two runs; the other returns at once
         const int* mark = residual_mark_of(residual, b200wkv6_residual_bytes(dtype, B, T, H, N));
-        st = wkv6_chunk_bwd((cudaStream_t)stream, B, T, H, r, k, v, w, 1, u, length, new_starts, dy, ds_out,
+        st = wkv6_chunk_bwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, length, new_starts, dy, ds_out,
                             residual, mark, dr, dk, dv, dw, du, ds0);
         if (st != B200WKV_OK) return st;
         return wkv6_seq_bwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 1, u, length, new_starts, dy, ds_out,

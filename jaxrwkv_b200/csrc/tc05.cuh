@@ -117,6 +117,20 @@ __device__ __forceinline__ void tensor_store_2d(const void* tmap, int x, int y, 
                  "r"(x), "r"(y), "r"(smem_u32(src_smem))
                  : "memory");
 }
+// 3-D maps, same rules
+__device__ __forceinline__ void tensor_load_3d(void* dst_smem, const void* tmap, int x, int y, int z, uint64_t* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+            smem_u32(dst_smem)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
+__device__ __forceinline__ void tensor_store_3d(const void* tmap, int x, int y, int z, const void* src_smem) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
+                     reinterpret_cast<uint64_t>(tmap)),
+                 "r"(x), "r"(y), "r"(z), "r"(smem_u32(src_smem))
+                 : "memory");
+}
 // The same with an element-wise add onto what global memory holds (the element type is the tensor map's).
 __device__ __forceinline__ void tensor_reduce_add_2d(const void* tmap, int x, int y, const void* src_smem) {
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(

@@ -80,4 +80,48 @@ inline bool make_stream_maps(StreamMaps* out, const void* const* bases, int coun
     return true;
 }
 
+// The same streams as [B sequences][T tokens][H*64 channels], boxes of `box` tokens of one head and one sequence, 128-byte
+// swizzle: rows behind a sequence's end arrive as zeros and are not stored.  Up to nine streams.
+constexpr int kSeqMaps = 9;
+struct SeqMaps {
+    CUtensorMap m[kSeqMaps];
+};
+inline bool make_seq_maps(SeqMaps* out, const void* const* bases, int count, int B, int T, int H, int box) {
+    constexpr int kSlots = 8;
+    struct Key { const void* base[kSeqMaps]; int count, B, T, H, box, pad; };
+    struct Slot { Key key; SeqMaps maps; bool used; };
+    thread_local Slot cache[kSlots];
+    thread_local int next = 0;
+    Key key;
+    memset(&key, 0, sizeof(key));
+    for (int m = 0; m < kSeqMaps; ++m) key.base[m] = bases[m < count && bases[m] != nullptr ? m : 0];
+    key.count = count; key.B = B; key.T = T; key.H = H; key.box = box;
+    for (int i = 0; i < kSlots; ++i)
+        if (cache[i].used && memcmp(&cache[i].key, &key, sizeof(key)) == 0) {
+            *out = cache[i].maps;
+            return true;
+        }
+    EncodeTiledFn enc = tmap_encoder();
+    if (enc == nullptr) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)H * 64, (cuuint64_t)T, (cuuint64_t)B};
+    const cuuint64_t strides[2] = {(cuuint64_t)H * 128, (cuuint64_t)T * H * 128};
+    const cuuint32_t boxes[3] = {64, (cuuint32_t)box, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    for (int m = 0; m < kSeqMaps; ++m) {
+        if (key.base[m] == nullptr || (reinterpret_cast<uintptr_t>(key.base[m]) & 15u) != 0) return false;
+        if (m >= count && m > 0) {
+            out->m[m] = out->m[0];
+            continue;
+        }
+        if (enc(&out->m[m], CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(key.base[m]), dims, strides, boxes, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+    }
+    Slot& s = cache[next];
+    next = (next + 1) % kSlots;
+    s.key = key; s.maps = *out; s.used = true;
+    return true;
+}
+
 }  // namespace b200wkv

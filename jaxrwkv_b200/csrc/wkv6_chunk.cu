@@ -23,9 +23,12 @@
 
 #include "common.cuh"
 #include "device_once.cuh"
+#include "tc05.cuh"
+#include "tmap.cuh"
 
 namespace b200wkv {
 
+int* wkv7_chunk_status_word();      // wkv7_chunk.cu: where a kernel leaves the code of a bounded wait that ran out
 int* wkv_call_flag(int* ticket);   // wkv7_chunk.cu: a slot of the per-device flag ring and a fresh ticket
 
 namespace {
@@ -34,12 +37,7 @@ typedef __nv_bfloat16 bf;
 constexpr int kC6 = 16;          // tokens per chunk
 constexpr int kRunLen6 = 16;    // chunks per run of the run-parallel backward
 constexpr int PITCH = 72;        // bf16 per shared-memory row (144 bytes): 4-byte fragment reads and ldmatrix rows hit 32 banks
-constexpr int kStages6 = 3;
 constexpr float kMaxHalfDecay = 80.f;   // |sum of lw over half a chunk| the scaling can represent
-
-struct RawStage {
-    bf r[kC6][PITCH], k[kC6][PITCH], v[kC6][PITCH], w[kC6][PITCH];
-};
 
 __device__ __forceinline__ void cp_async16_zfill(void* dst_smem, const void* src, bool valid) {
     const int n = valid ? 16 : 0;
@@ -66,12 +64,6 @@ __device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t
 struct Frag {
     uint32_t f[4];
 };
-__device__ __forceinline__ Frag load_frag(const bf (*tile)[72], int ks, int lane) {
-    Frag x;
-    const int mi = lane >> 3, r8 = lane & 7;
-    ldmatrix_x4(x.f[0], x.f[1], x.f[2], x.f[3], &tile[(mi & 1) * 8 + r8][16 * ks + (mi >> 1) * 8]);
-    return x;
-}
 __device__ __forceinline__ void mma_ab(float* d, const Frag& a, const Frag& b, int nt) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -88,64 +80,112 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Sums each of eight per-lane values over the warp with nine shuffles: three halving steps leave one value per lane,
-// two butterflies finish.  Returns the total of v[which] with which = 4 bit4(lane) + 2 bit3(lane) + bit2(lane).
-__device__ __forceinline__ float warp_sum8(const float* v, int lane, int* which) {
-    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-    float a[4], b[2], c;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) a[j] = (b4 ? v[j + 4] : v[j]) + __shfl_xor_sync(0xffffffffu, b4 ? v[j] : v[j + 4], 16);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) b[j] = (b3 ? a[j + 2] : a[j]) + __shfl_xor_sync(0xffffffffu, b3 ? a[j] : a[j + 2], 8);
-    c = (b2 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, b2 ? b[0] : b[1], 4);
-    c += __shfl_xor_sync(0xffffffffu, c, 1);
-    c += __shfl_xor_sync(0xffffffffu, c, 2);
-    *which = (b4 ? 4 : 0) + (b3 ? 2 : 0) + (b2 ? 1 : 0);
-    return c;
-}
-
-// The same for four values with six shuffles: which = 2 bit4(lane) + bit3(lane); every lane ends with the total.
-__device__ __forceinline__ float warp_sum4(const float* v, int lane, int* which) {
-    const bool b4 = lane & 16, b3 = lane & 8;
-    float a[2], c;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) a[j] = (b4 ? v[j + 2] : v[j]) + __shfl_xor_sync(0xffffffffu, b4 ? v[j] : v[j + 2], 16);
-    c = (b3 ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, b3 ? a[0] : a[1], 8);
-    c += __shfl_xor_sync(0xffffffffu, c, 4);
-    c += __shfl_xor_sync(0xffffffffu, c, 2);
-    c += __shfl_xor_sync(0xffffffffu, c, 1);
-    *which = (b4 ? 2 : 0) + (b3 ? 1 : 0);
-    return c;
+// exp in two instructions (results below the smallest normal number are zero; __expf spends three more on them)
+__device__ __forceinline__ float exp_fast(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.4426950408889634f));
+    return y;
 }
 
 // ------------------------------------------------------------------ forward ---------
+// What bounds it is the instructions of the operands' preparation (512 sequences of 256 chunks on 592 CTA slots: every
+// chunk's instructions lie in one chain per CTA, four CTAs deep on an SM).  So a warp prepares the 16 channels that it also
+// owns as value columns, for all 16 tokens, in the layout of the tensor cores' tiles: the cumulative log-decay, referenced to
+// the chunk's middle, is a product of constant triangles of -1, 0, 1 with the raw log-decay rows (exact products, fp32 sums),
+// so that it needs neither a scan nor another warp; its result lies where r and k of the same (token, channel) pairs can be
+// read as words; and what leaves for shared memory are whole fragments (stmatrix).  One barrier per chunk.
+// At B=16, T=4096, H=32: 0.55 ms with the residual (0.81 ms with the sums a scan over quarters of the
+// chunk, 4-byte operand stores, and raw rows fetched by every thread).
+constexpr int kRing6 = 3;        // raw rows of r, k, w: read before a chunk's barrier only
+constexpr int kRingV6 = 4;       // raw rows of v: read behind it
+constexpr int kTile6 = kC6 * kN * 2;     // bytes of a chunk's rows of one stream, as the tiled copies move them (rows of 128 bytes, swizzled)
 struct Fwd6cSmem {
-    RawStage raw[kStages6];
-    bf rt[kC6][PITCH], kt[kC6][PITCH], r0[kC6][PITCH], kh[kC6][PITCH];   // R~, K~, R0, K^
-    bf ys[kC6][PITCH];                                                   // the chunk's outputs, token-major
-    float tot[4][kN];        // sum of lw over each quarter of the chunk
-    float wc[kN];            // exp(c_C), or 0 when a start flag lies in the chunk
-    float dpart[2][kC6];     // sum_i r u k per token, one partial per 32 channels
-    int seg[kC6];            // number of start flags at or before the token, inside the chunk
-    unsigned startmask;      // bit t: start flag on token t of the chunk
-    uint8_t ns[kStages6][kC6];
+    unsigned char r[kRing6][kTile6], k[kRing6][kTile6], w[kRing6][kTile6], v[kRingV6][kTile6];
+    unsigned char ys[2][kTile6];         // a chunk's outputs
+    bf ops[2][4][kC6][PITCH];            // R~, K~, R0, K^ of this chunk and the next in turn
+    uint64_t full[kRingV6];              // a chunk's raw rows have landed
+    float wc[2][kN];                     // exp(c_C), or 0 when a start flag lies in the chunk
+    float dpart[2][kC6][4];              // sum_i r u k per token over each warp's 16 channels
 };
+static_assert(4 * (sizeof(Fwd6cSmem) + 1024) <= 228 * 1024, "four CTAs per SM");
 
-// One CTA of 128 threads per (batch, head).  ckpt: the state entering every chunk, bf16 S^T[value j][key i] in 8 column blocks of [64 j][8 i], for
-// the backward (may be NULL).  The kernel gives up (flag := ticket, see the file header) on a decay above 1 and on a
-// half-chunk decay beyond exp(-80).
+// Constant left operands (rows = token t, columns = token s; the two off-diagonal 8x8 blocks are zero) of the products with
+// the log-decay rows that give, for every token and channel,
+//   c_t - c_m (upto), c_{t-1} - c_m (before), and c_m | c_C - c_m (rows 0-7 | 8-15 of halves).
+struct DecaySums {
+    uint32_t upto_lo, upto_hi, before_lo, before_hi;
+    __device__ __forceinline__ explicit DecaySums(int g, int q) {
+        const int s = 2 * q;
+        upto_lo = pack2(g < s ? -1.f : 0.f, g < s + 1 ? -1.f : 0.f);
+        upto_hi = pack2(s <= g ? 1.f : 0.f, s + 1 <= g ? 1.f : 0.f);
+        before_lo = pack2(g <= s ? -1.f : 0.f, g <= s + 1 ? -1.f : 0.f);
+        before_hi = pack2(s < g ? 1.f : 0.f, s + 1 < g ? 1.f : 0.f);
+    }
+};
+// Log-decay sums of a warp's 16 channels c0 .. c0 + 15: thread (g, q) gets, in x[nt][2 hh + e], the value of token g + 8 hh
+// and channel c0 + 8 nt + 2 q + e.  wb: the raw rows as right operands (tokens 0-7 | 8-15 of channels 0-7, then 8-15).
+__device__ __forceinline__ void decay_sums(const DecaySums& d, const uint32_t* wb, float (*upto)[4], float (*before)[4], float (*halves)[4]) {
+    constexpr uint32_t kOnes = 0x3f803f80u;
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) upto[nt][e] = before[nt][e] = halves[nt][e] = 0.f;
+        mma_bf16(upto[nt], d.upto_lo, 0u, 0u, d.upto_hi, wb[2 * nt], wb[2 * nt + 1]);
+        mma_bf16(before[nt], d.before_lo, 0u, 0u, d.before_hi, wb[2 * nt], wb[2 * nt + 1]);
+        mma_bf16(halves[nt], kOnes, 0u, 0u, kOnes, wb[2 * nt], wb[2 * nt + 1]);
+    }
+}
+// The same for a decay that is constant over the tokens: token x of the chunk counts if lo <= x < n.
+__device__ __forceinline__ void decay_sums_const(const float* lw, int g, int lo, int n, float (*upto)[4], float (*before)[4], float (*halves)[4]) {
+    auto count = [&](int t) { return min(max(t + 1 - lo, 0), max(n - lo, 0)); };     // tokens that count, up to t
+    const int half = count(kC6 / 2 - 1), all = count(kC6 - 1);
+#pragma unroll
+    for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int t = g + 8 * (e >> 1);
+            const float l = lw[2 * nt + (e & 1)];
+            upto[nt][e] = l * (float)(count(t) - half);
+            before[nt][e] = l * (float)(count(t - 1) - half);
+            halves[nt][e] = l * (float)(e < 2 ? half : all - half);
+        }
+}
+// both halves of a pair of bf16 at most zero (false for NaN)
+__device__ __forceinline__ bool none_positive(uint32_t x) {
+    return __hble2(*reinterpret_cast<const __nv_bfloat162*>(&x), __float2bfloat162_rn(0.f));
+}
+__device__ __forceinline__ float2 unpack2(uint32_t x) { return make_float2(__uint_as_float(x << 16), __uint_as_float(x & 0xffff0000u)); }
+__device__ __forceinline__ void stmatrix_x4(void* row, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"((uint32_t)__cvta_generic_to_shared(row)),
+                 "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+                 : "memory");
+}
+// an 8x8 tile, one pair of columns per lane, transposed inside the warp
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t a) {
+    uint32_t d;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+    return d;
+}
+
+// start flags of a chunk as bits; no start in (s, t]
+__device__ __forceinline__ bool same_segment(unsigned starts, int s, int t) { return ((starts & ((2u << t) - 1u)) >> (s + 1)) == 0; }
+
+// One CTA of 128 threads per (batch, head).  ckpt: the state entering every chunk, bf16 S^T[value j][key i] in 8 column blocks
+// of [64 j][8 i], and scores: every chunk's A^T as the left operand's words, lane by lane, for the backward (both NULL without one).  The kernel gives up (flag := ticket, see the file header) on a decay above 1
+// and on a half-chunk decay beyond exp(-80).
 __global__ void __launch_bounds__(128, 4)
 wkv6_chunk_fwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
                       const bf* __restrict__ w, int w_per_token, const bf* __restrict__ u, const bf* __restrict__ s0,
                       const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts, bf* __restrict__ y,
-                      bf* __restrict__ s_out, bf* __restrict__ ckpt, int* __restrict__ flag, int ticket,
-                      int* __restrict__ residual_mark) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+                      bf* __restrict__ s_out, bf* __restrict__ ckpt, uint4* __restrict__ scores, int* __restrict__ flag, int ticket,
+                      int* __restrict__ residual_mark, const __grid_constant__ SeqMaps maps) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];   // (the swizzle is a function of the address)
     Fwd6cSmem& sm = *reinterpret_cast<Fwd6cSmem*>(smem_raw);
     const int bh = blockIdx.x, bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, q = lane & 3;
-    const int j0 = warp * 16;                                    // this warp's value rows of S^T
+    const int j0 = warp * 16;                                    // this warp's value rows of S^T, and the channels it prepares
+    const int frow = (lane & 15), fcol = (lane >> 4) * 8;        // a lane's row of a 16x16 block's four 8x8 tiles (ldmatrix, stmatrix)
     const size_t tok_stride = (size_t)H * kN;
     const size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
     const size_t st_base = (size_t)bh * kN * kN;
@@ -174,266 +214,302 @@ wkv6_chunk_fwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
     };
     if (L == 0) write_state(s_out);
 
-    const int srow = tid >> 3, spiece = (tid & 7) * 8;            // staging: one 16-byte piece of one token row per stream
+    // raw rows by tiled copies, three chunks ahead (rows behind the sequence's end arrive as zeros)
     auto issue = [&](int c) {
-        if (c < nC) {
-            RawStage& st = sm.raw[c % kStages6];
-            const int t = c * kC6 + srow;
-            const bool ok = t < Tlen;
-            const size_t off = seq_base + (size_t)(ok ? t : 0) * tok_stride + spiece;
-            cp_async16_zfill(&st.r[srow][spiece], r + off, ok);
-            cp_async16_zfill(&st.k[srow][spiece], k + off, ok);
-            cp_async16_zfill(&st.v[srow][spiece], v + off, ok);
-            if (w_per_token) cp_async16_zfill(&st.w[srow][spiece], w + off, ok);
+        if (tid == 0 && c < nC) {
+            uint64_t* bar = &sm.full[c % kRingV6];
+            tc::mbar_expect_tx(bar, (w_per_token ? 4 : 3) * kTile6);
+            tc::tensor_load_3d(sm.r[c % kRing6], &maps.m[0], h * kN, c * kC6, bi, bar);
+            tc::tensor_load_3d(sm.k[c % kRing6], &maps.m[1], h * kN, c * kC6, bi, bar);
+            tc::tensor_load_3d(sm.v[c % kRingV6], &maps.m[2], h * kN, c * kC6, bi, bar);
+            if (w_per_token) tc::tensor_load_3d(sm.w[c % kRing6], &maps.m[3], h * kN, c * kC6, bi, bar);
         }
-        cp_async_commit();
     };
-    auto load_ns = [&](int c) -> uint8_t {
-        const int t = c * kC6 + tid;
-        return (tid < kC6 && c < nC && t < Tlen) ? new_starts[(size_t)bi * Tlen + t] : (uint8_t)0;
-    };
+    if (tid == 0) {
+#pragma unroll
+        for (int i = 0; i < kRingV6; ++i) tc::mbar_init(&sm.full[i], 1);
+        tc::mbar_init_fence();
+    }
+    __syncthreads();
+    // this thread's places in a swizzled tile: its row of the warp's 16x16 block (matrix loads and stores), and the word of
+    // channels j0 + 2 q, + 1 of token g (those of j0 + 8 + 2 q, + 1: XOR 16; token g + 8: + 1024)
+    const int tile_row = frow * 128 + (((2 * warp + (lane >> 4)) ^ (frow & 7)) << 4);
+    const int tile_word = g * 128 + (((2 * warp) ^ g) << 4) + 4 * q;
+    // start flags: every warp fetches a chunk's sixteen for itself, two chunks ahead
+    const uint8_t* const ns_row = new_starts + (size_t)bi * Tlen;
+    auto load_ns = [&](int c) -> unsigned { return ns_row[min(c * kC6 + (lane & 15), Tlen - 1)]; };
     issue(0);
     issue(1);
-    if (tid < kC6) {
-        sm.ns[0][tid] = load_ns(0);
-        sm.ns[1 % kStages6][tid] = load_ns(1);
-    }
-    uint8_t ns_ahead = load_ns(2);
+    issue(2);
+    unsigned ns_now = load_ns(0), ns_next = load_ns(1);
 
-    // phase A ownership: the channel pair cp, cp + 1 and the four tokens of quarter qt (= the warp, which so holds all 64
-    // channels of its tokens)
-    const int cp = (tid & 31) * 2, qt = warp;
-    const float2 uu = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(u + (size_t)h * kN + cp));
-    float2 lw_const = make_float2(0.f, 0.f);
-    if (!w_per_token) {
-        const float2 wv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(w + (size_t)h * kN + cp));
-        lw_const = make_float2(__logf(wv.x), __logf(wv.y));
+    float uu[4], lw_const[4];                                     // of channels j0 + 2 q, + 1, + 8, + 9
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const size_t at = (size_t)h * kN + j0 + 8 * (e >> 1) + 2 * q + (e & 1);
+        uu[e] = __bfloat162float(u[at]);
+        lw_const[e] = w_per_token ? 0.f : __logf(__bfloat162float(w[at]));
     }
-    bool bad = false;
+    const DecaySums sums(g, q);
+    bool good = true;
 
+    // the chunk whose outputs wait in a tile: from token out_t on; a whole one leaves by a tiled copy, the parts of a split one
+    // by rows out_lo .. out_hi - 1
+    int out_t = -1, out_lo = 0, out_hi = kC6;
+    auto send_outputs = [&](int buf) {
+        if (out_t < 0) return;
+        if (out_lo == 0 && out_hi == kC6) {
+            if (tid == 0) {
+                tc::tensor_store_3d(&maps.m[4], h * kN, out_t, bi, sm.ys[buf]);
+                tc::bulk_commit();
+            }
+        } else {
+            const int row = tid >> 3, piece = tid & 7;
+            if (row >= out_lo && row < out_hi && out_t + row < Tlen)
+                *reinterpret_cast<uint4*>(y + seq_base + (size_t)(out_t + row) * tok_stride + piece * 8) =
+                    *reinterpret_cast<const uint4*>(sm.ys[buf] + row * 128 + ((piece ^ (row & 7)) << 4));
+        }
+    };
     // One chunk, or one part of the split chunk.  The two cases are separate instantiations: in the common one the
     // bounds of the part are the constants 0 and 16 and every test against them folds away.
-    auto walk = [&](auto split_tag, const int c, const int part_arg) {
+    auto walk = [&](auto split_tag, const int c, const int buf, const int part_arg) {
         constexpr bool kSplitHere = decltype(split_tag)::value;
         const int part = kSplitHere ? part_arg : 0;
         const int lo = (kSplitHere && part == 1) ? p_out + 1 : 0, hi = (kSplitHere && part == 0) ? p_out + 1 : kC6;
-        const RawStage& st = sm.raw[c % kStages6];
-        const int t0 = c * kC6;
-        if (part == 0) {
-            cp_async_wait<1>();
-            __syncthreads();          // chunk c has landed for everyone; the tiles of chunk c - 1 are no longer read
-            issue(c + 2);
-            if (tid < kC6) sm.ns[(c + 2) % kStages6][tid] = ns_ahead;
-            ns_ahead = load_ns(c + 3);
-            // ---- outputs of the previous chunk to global memory
-            if (c > 0 && t0 - kC6 + srow < Tlen)
-                *reinterpret_cast<uint4*>(y + seq_base + (size_t)(t0 - kC6 + srow) * tok_stride + spiece) =
-                    *reinterpret_cast<const uint4*>(&sm.ys[srow][spiece]);
-        } else {
-            __syncthreads();          // the first part's products have read the operand tiles
-        }
-        // ---- the entering state for the backward (of the second part of a split chunk: slot nC)
-        if (ckpt != nullptr) {
-            bf* dst = ckpt + ((size_t)bh * (nC + 1) + (part == 0 ? c : nC)) * kN * kN;
-#pragma unroll
-            for (int ni = 0; ni < 8; ++ni) {
-                // (8 column blocks of [64 rows j][8 keys i]: the eight row groups of a warp write one 128-byte line)
-                *reinterpret_cast<uint32_t*>(dst + ni * (kN * 8) + (j0 + g) * 8 + 2 * q) = pack2(acc[ni][0], acc[ni][1]);
-                *reinterpret_cast<uint32_t*>(dst + ni * (kN * 8) + (j0 + g + 8) * 8 + 2 * q) = pack2(acc[ni][2], acc[ni][3]);
-            }
-        }
-        // ---- phase A: cumulative log-decay and scaled operands
-        if (warp == 0) {
-            const unsigned m = __ballot_sync(0xffffffffu, lane < kC6 && sm.ns[c % kStages6][lane] != 0);
-            if (lane == 0) sm.startmask = m;
-        }
-        float2 lw[4], cl[4];
-        float2 run = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int tt = 0; tt < 4; ++tt) {
-            const int t = 4 * qt + tt;
-            const bool ok = t0 + t < Tlen && t >= lo && t < hi;
-            lw[tt] = !ok ? make_float2(0.f, 0.f)
-                         : (w_per_token ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.w[t][cp])) : lw_const);
-            if (!(lw[tt].x <= 0.f) || !(lw[tt].y <= 0.f)) bad = true;      // a decay above 1 (or NaN) is outside what the scaling covers
-            run.x += lw[tt].x;
-            run.y += lw[tt].y;
-            cl[tt] = run;
-        }
-        *reinterpret_cast<float2*>(&sm.tot[qt][cp]) = run;
-        // the operands need the other quarters' totals: a barrier of the whole CTA
-        __syncthreads();
-        // segments: seg(t) = number of start flags at or before token t
-        const unsigned starts = sm.startmask;
-        auto seg_of = [&](int t) { return __popc(starts & ((2u << t) - 1u)); };
-        const int seg_last = seg_of(hi - 1), seg_base = lo > 0 ? seg_of(lo - 1) : 0;   // of the part's last token; of the state entering it
-        if (tid < kC6) sm.seg[tid] = seg_of(tid);
-        const float2 tq0 = *reinterpret_cast<const float2*>(&sm.tot[0][cp]), tq1 = *reinterpret_cast<const float2*>(&sm.tot[1][cp]);
-        const float2 tq2 = *reinterpret_cast<const float2*>(&sm.tot[2][cp]), tq3 = *reinterpret_cast<const float2*>(&sm.tot[3][cp]);
-        const float2 tot0 = make_float2(tq0.x + tq1.x, tq0.y + tq1.y), tot1 = make_float2(tq2.x + tq3.x, tq2.y + tq3.y);
-        if (fabsf(tot0.x) > kMaxHalfDecay || fabsf(tot1.x) > kMaxHalfDecay || fabsf(tot0.y) > kMaxHalfDecay || fabsf(tot1.y) > kMaxHalfDecay) bad = true;
-        const float2 c_m = make_float2(fmaxf(tot0.x, -kMaxHalfDecay), fmaxf(tot0.y, -kMaxHalfDecay));
-        const float2 c_C = make_float2(c_m.x + fmaxf(tot1.x, -kMaxHalfDecay), c_m.y + fmaxf(tot1.y, -kMaxHalfDecay));
-        // cumulative log-decay in front of this quarter (the second half counts from the clamped middle, as c_C does)
-        const float2 base = qt == 0 ? make_float2(0.f, 0.f) : (qt == 1 ? tq0 : (qt == 2 ? c_m : make_float2(c_m.x + tq2.x, c_m.y + tq2.y)));
-        if (qt == 3)
-            *reinterpret_cast<float2*>(&sm.wc[cp]) = seg_last == seg_base ? make_float2(__expf(c_C.x), __expf(c_C.y)) : make_float2(0.f, 0.f);
-        float dsum[4];
-#pragma unroll
-        for (int tt = 0; tt < 4; ++tt) {
-            const int t = 4 * qt + tt;
-            const bool in_part = t >= lo && t < hi;
-            const int seg_t = seg_of(t);
-            const float2 c_t = make_float2(base.x + cl[tt].x, base.y + cl[tt].y), c_prev = make_float2(c_t.x - lw[tt].x, c_t.y - lw[tt].y);
-            const float2 zero2 = make_float2(0.f, 0.f);
-            const float2 rv = in_part ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.r[t][cp])) : zero2;
-            const float2 kv = in_part ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.k[t][cp])) : zero2;
-            *reinterpret_cast<uint32_t*>(&sm.rt[t][cp]) = pack2(rv.x * __expf(fminf(c_prev.x - c_m.x, kMaxHalfDecay)), rv.y * __expf(fminf(c_prev.y - c_m.y, kMaxHalfDecay)));
-            *reinterpret_cast<uint32_t*>(&sm.kt[t][cp]) = pack2(kv.x * __expf(fminf(c_m.x - c_t.x, kMaxHalfDecay)), kv.y * __expf(fminf(c_m.y - c_t.y, kMaxHalfDecay)));
-            const bool first = seg_t == seg_base, last = seg_t == seg_last;
-            *reinterpret_cast<uint32_t*>(&sm.r0[t][cp]) = pack2(first ? rv.x * __expf(c_prev.x) : 0.f, first ? rv.y * __expf(c_prev.y) : 0.f);
-            *reinterpret_cast<uint32_t*>(&sm.kh[t][cp]) = pack2(last ? kv.x * __expf(c_C.x - c_t.x) : 0.f, last ? kv.y * __expf(c_C.y - c_t.y) : 0.f);
-            dsum[tt] = fmaf(rv.x * uu.x, kv.x, rv.y * uu.y * kv.y);
-        }
+        const int t0 = c * kC6, sl = c % kRing6;
+        unsigned starts = __ballot_sync(0xffffffffu, ns_now != 0) & (0xffffu >> max(t0 + kC6 - Tlen, 0));
+        if (kSplitHere) starts &= ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+        // ---- phase A: the scaled operands of this warp's channels
+        if (!tc::mbar_wait(&sm.full[c % kRingV6], (c / kRingV6) & 1)) good = false;
         {
-            int which;
-            const float total = warp_sum4(dsum, lane, &which);      // over all 64 channels: the warp holds them all
-            if ((lane & 7) == 0) {
-                sm.dpart[0][4 * qt + which] = total;
-                sm.dpart[1][4 * qt + which] = 0.f;
-            }
-        }
-        __syncthreads();
-
-        // ---- phase B: the products
-        uint32_t va[4];            // V^T of this warp: A fragments (M = value row, K = token)
-        {
-            const int mi = lane >> 3, r8 = lane & 7;
-            ldmatrix_x4_trans(va[0], va[1], va[2], va[3], &st.v[(mi >> 1) * 8 + r8][j0 + (mi & 1) * 8]);
-        }
-        float yacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};    // Y^T: rows value j, columns token t
-        float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};    // A: rows token t, columns token s
+            float upto[2][4], before[2][4], halves[2][4];
+            if (w_per_token) {
+                uint32_t wb[4];
+                ldmatrix_x4_trans(wb[0], wb[1], wb[2], wb[3], sm.w[sl] + tile_row);
+                if (kSplitHere) {
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            const uint32_t s_a0 = pack2(acc[2 * ks][0], acc[2 * ks][1]), s_a1 = pack2(acc[2 * ks][2], acc[2 * ks][3]);
-            const uint32_t s_a2 = pack2(acc[2 * ks + 1][0], acc[2 * ks + 1][1]), s_a3 = pack2(acc[2 * ks + 1][2], acc[2 * ks + 1][3]);
-            const Frag fr = load_frag(sm.rt, ks, lane), f0 = load_frag(sm.r0, ks, lane), fk = load_frag(sm.kt, ks, lane);
+                    for (int i = 0; i < 4; ++i) {
+                        const int s = 8 * (i & 1) + 2 * q;
+                        wb[i] &= (s >= lo && s < hi ? 0xffffu : 0u) | (s + 1 >= lo && s + 1 < hi ? 0xffff0000u : 0u);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) good = good && none_positive(wb[i]);   // a decay above 1 (or NaN) is outside what the scaling covers
+                decay_sums(sums, wb, upto, before, halves);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) good = good && lw_const[i] <= 0.f;
+                decay_sums_const(lw_const, g, lo, min(hi, Tlen - t0), upto, before, halves);
+            }
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) good = good && halves[nt][e] >= -kMaxHalfDecay;
+            uint32_t rt[4], kt[4], r0[4], kh[4];                  // fragments, in the order (hh, nt) = 00, 10, 01, 11
+            float dsum[2] = {0.f, 0.f};
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                mma_bf16(yacc[nt], s_a0, s_a1, s_a2, s_a3, f0.f[nt], f0.f[nt + 2]);
-                mma_ab(sacc[nt], fr, fk, nt);
+                const float2 em = make_float2(exp_fast(halves[nt][0]), exp_fast(halves[nt][1]));
+                const float2 ecm = make_float2(exp_fast(halves[nt][2]), exp_fast(halves[nt][3]));
+                if (g == 0)
+                    *reinterpret_cast<float2*>(&sm.wc[buf][j0 + 8 * nt + 2 * q]) = starts == 0 ? make_float2(em.x * ecm.x, em.y * ecm.y) : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int t = g + 8 * hh;
+                    uint32_t rw = *reinterpret_cast<const uint32_t*>(sm.r[sl] + (tile_word ^ (16 * nt)) + 1024 * hh);
+                    uint32_t kw = *reinterpret_cast<const uint32_t*>(sm.k[sl] + (tile_word ^ (16 * nt)) + 1024 * hh);
+                    if (kSplitHere && !(t >= lo && t < hi)) rw = kw = 0;
+                    const float2 rv = unpack2(rw), kv = unpack2(kw);
+                    const float2 f2 = make_float2(exp_fast(before[nt][2 * hh]), exp_fast(before[nt][2 * hh + 1]));
+                    const float2 f3 = make_float2(exp_fast(-upto[nt][2 * hh]), exp_fast(-upto[nt][2 * hh + 1]));
+                    const int at = 2 * nt + hh;
+                    rt[at] = pack2(rv.x * f2.x, rv.y * f2.y);
+                    kt[at] = pack2(kv.x * f3.x, kv.y * f3.y);
+                    r0[at] = pack2(rv.x * (f2.x * em.x), rv.y * (f2.y * em.y));
+                    kh[at] = pack2(kv.x * (f3.x * ecm.x), kv.y * (f3.y * ecm.y));
+                    dsum[hh] = fmaf(rv.x * uu[2 * nt], kv.x, fmaf(rv.y * uu[2 * nt + 1], kv.y, dsum[hh]));
+                }
+            }
+            if (starts != 0) {     // tokens behind the first flag do not see S0, those in front of the last one do not reach S_C
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int t = g + 8 * hh;
+                    const bool first = (starts & ((2u << t) - 1u)) == 0, last = (starts >> (t + 1)) == 0;
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) {
+                        r0[2 * nt + hh] = first ? r0[2 * nt + hh] : 0u;
+                        kh[2 * nt + hh] = last ? kh[2 * nt + hh] : 0u;
+                    }
+                }
+            }
+            stmatrix_x4(&sm.ops[buf][0][frow][j0 + fcol], rt[0], rt[1], rt[2], rt[3]);
+            stmatrix_x4(&sm.ops[buf][1][frow][j0 + fcol], kt[0], kt[1], kt[2], kt[3]);
+            stmatrix_x4(&sm.ops[buf][2][frow][j0 + fcol], r0[0], r0[1], r0[2], r0[3]);
+            stmatrix_x4(&sm.ops[buf][3][frow][j0 + fcol], kh[0], kh[1], kh[2], kh[3]);
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                dsum[hh] += __shfl_xor_sync(0xffffffffu, dsum[hh], 1);
+                dsum[hh] += __shfl_xor_sync(0xffffffffu, dsum[hh], 2);
+                if (q == 0) sm.dpart[buf][g + 8 * hh][warp] = dsum[hh];
             }
         }
-        // masks: strictly earlier tokens of the same segment; the diagonal is the u term
+        if (tid == 0) tc::bulk_wait_read<0>();      // the outputs sent a chunk ago have left the tile that this chunk's go to
+        tc::fence_async_smem();                     // (the previous chunk's outputs, for the copy that takes them)
+        // the chunk's operands are complete; what the chunk before this one read behind its barrier (its v rows, the other
+        // operand tiles) is free, and so are this chunk's r, k, w rows
+        __syncthreads();
+        if (!kSplitHere || part == 1) {
+            issue(c + 3);
+            ns_now = ns_next;
+            ns_next = load_ns(c + 2);
+        }
+        send_outputs(buf ^ 1);
+        out_t = t0;
+        out_lo = lo;
+        out_hi = hi;
+
+        // ---- phase B: the products
+        float yacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};    // Y: rows token t, columns value j
+        float sacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};    // A: rows token t, columns token s
+        bf* const dst = ckpt + ((size_t)bh * (nC + 1) + (part == 0 ? c : nC)) * kN * kN + (j0 + g) * 8 + 2 * q;
 #pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int t = g + 8 * (e >> 1), s = 8 * nt + 2 * q + (e & 1);
-                const bool keep = s < t && sm.seg[s] == sm.seg[t];      // (rows and columns outside the part are zero operands)
-                sacc[nt][e] = keep ? sacc[nt][e] : (s == t ? sm.dpart[0][t] + sm.dpart[1][t] : 0.f);
+        for (int ks = 0; ks < 4; ++ks) {
+            Frag fr, f0, fk;
+            ldmatrix_x4(fr.f[0], fr.f[1], fr.f[2], fr.f[3], &sm.ops[buf][0][frow][16 * ks + fcol]);
+            ldmatrix_x4(fk.f[0], fk.f[1], fk.f[2], fk.f[3], &sm.ops[buf][1][frow][16 * ks + fcol]);
+            ldmatrix_x4(f0.f[0], f0.f[1], f0.f[2], f0.f[3], &sm.ops[buf][2][frow][16 * ks + fcol]);
+            // S^T tiles are right operands as they are: K = key channel (their columns), n = value row
+            const uint32_t s00 = pack2(acc[2 * ks][0], acc[2 * ks][1]), s01 = pack2(acc[2 * ks + 1][0], acc[2 * ks + 1][1]);
+            const uint32_t s10 = pack2(acc[2 * ks][2], acc[2 * ks][3]), s11 = pack2(acc[2 * ks + 1][2], acc[2 * ks + 1][3]);
+            mma_bf16(yacc[0], f0.f[0], f0.f[1], f0.f[2], f0.f[3], s00, s01);
+            mma_bf16(yacc[1], f0.f[0], f0.f[1], f0.f[2], f0.f[3], s10, s11);
+            mma_ab(sacc[0], fr, fk, 0);
+            mma_ab(sacc[1], fr, fk, 1);
+            // the entering state for the backward (of the second part of a split chunk: slot nC), in 8 column blocks of
+            // [64 rows j][8 keys i]: the eight row groups of a warp write one 128-byte line
+            if (ckpt != nullptr) {
+                *reinterpret_cast<uint32_t*>(dst + (2 * ks) * (kN * 8)) = s00;
+                *reinterpret_cast<uint32_t*>(dst + (2 * ks) * (kN * 8) + 64) = s10;
+                *reinterpret_cast<uint32_t*>(dst + (2 * ks + 1) * (kN * 8)) = s01;
+                *reinterpret_cast<uint32_t*>(dst + (2 * ks + 1) * (kN * 8) + 64) = s11;
             }
-        // Y^T += V^T A^T: the score tiles are the right operand as they are
-        mma_bf16(yacc[0], va[0], va[1], va[2], va[3], pack2(sacc[0][0], sacc[0][1]), pack2(sacc[1][0], sacc[1][1]));
-        mma_bf16(yacc[1], va[0], va[1], va[2], va[3], pack2(sacc[0][2], sacc[0][3]), pack2(sacc[1][2], sacc[1][3]));
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int t = 8 * nt + 2 * q + (e & 1);
-                if (t >= lo && t < hi) sm.ys[t][j0 + g + 8 * (e >> 1)] = __float2bfloat16_rn(yacc[nt][e]);
-            }
-        // S^T <- S^T diag(exp(c_C)) [no start in the chunk] + V^T K^
+        }
+        uint32_t va[4];            // V^T of this warp: A fragments (M = value row, K = token), and V as right operands
+        ldmatrix_x4_trans(va[0], va[2], va[1], va[3], sm.v[c % kRingV6] + tile_row);
+        // strictly earlier tokens of the same segment; the diagonal is the u term.  (Rows and columns outside the part are zero
+        // operands; the block of rows 0-7 and columns 8-15 is not used.)
         {
-            const int mi = lane >> 3, r8 = lane & 7;
+            const float4 d0 = *reinterpret_cast<const float4*>(&sm.dpart[buf][g][0]), d1 = *reinterpret_cast<const float4*>(&sm.dpart[buf][g + 8][0]);
+            const float dg0 = (d0.x + d0.y) + (d0.z + d0.w), dg1 = (d1.x + d1.y) + (d1.z + d1.w);
 #pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                const float2 w0 = *reinterpret_cast<const float2*>(&sm.wc[16 * np + 2 * q]);
-                const float2 w1 = *reinterpret_cast<const float2*>(&sm.wc[16 * np + 8 + 2 * q]);
-                acc[2 * np][0] *= w0.x; acc[2 * np][1] *= w0.y; acc[2 * np][2] *= w0.x; acc[2 * np][3] *= w0.y;
-                acc[2 * np + 1][0] *= w1.x; acc[2 * np + 1][1] *= w1.y; acc[2 * np + 1][2] *= w1.x; acc[2 * np + 1][3] *= w1.y;
-                uint32_t b0, b1, b2, b3;        // key tiles 2 np (b0, b1) and 2 np + 1 (b2, b3)
-                ldmatrix_x4_trans(b0, b1, b2, b3, &sm.kh[(mi & 1) * 8 + r8][(2 * np + (mi >> 1)) * 8]);
-                mma_bf16(acc[2 * np], va[0], va[1], va[2], va[3], b0, b1);
-                mma_bf16(acc[2 * np + 1], va[0], va[1], va[2], va[3], b2, b3);
+            for (int e = 0; e < 2; ++e) {
+                const int s = 2 * q + e;
+                sacc[0][e] = s < g ? sacc[0][e] : (s == g ? dg0 : 0.f);
+                sacc[1][2 + e] = s < g ? sacc[1][2 + e] : (s == g ? dg1 : 0.f);
             }
+            if (starts != 0) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int s = 2 * q + e;
+                    if (s < g && !same_segment(starts, s, g)) sacc[0][e] = 0.f;
+                    if (!same_segment(starts, s, g + 8)) sacc[0][2 + e] = 0.f;
+                    if (s < g && !same_segment(starts, s + 8, g + 8)) sacc[1][2 + e] = 0.f;
+                }
+            }
+        }
+        const uint32_t a0 = pack2(sacc[0][0], sacc[0][1]), a1 = pack2(sacc[0][2], sacc[0][3]), a3 = pack2(sacc[1][2], sacc[1][3]);
+        if (scores != nullptr && warp == (c & 3))
+            scores[((size_t)bh * (nC + 1) + (part == 0 ? c : nC)) * 32 + lane] = make_uint4(transpose8x8(a0), 0u, transpose8x8(a1), transpose8x8(a3));
+        mma_bf16(yacc[0], a0, a1, 0u, a3, va[0], va[2]);
+        mma_bf16(yacc[1], a0, a1, 0u, a3, va[1], va[3]);
+        stmatrix_x4(sm.ys[buf] + tile_row, pack2(yacc[0][0], yacc[0][1]), pack2(yacc[0][2], yacc[0][3]), pack2(yacc[1][0], yacc[1][1]),
+                    pack2(yacc[1][2], yacc[1][3]));
+        // S^T <- S^T diag(exp(c_C)) [no start in the chunk] + V^T K^
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+            const float2 w0 = *reinterpret_cast<const float2*>(&sm.wc[buf][16 * np + 2 * q]);
+            const float2 w1 = *reinterpret_cast<const float2*>(&sm.wc[buf][16 * np + 8 + 2 * q]);
+            acc[2 * np][0] *= w0.x; acc[2 * np][1] *= w0.y; acc[2 * np][2] *= w0.x; acc[2 * np][3] *= w0.y;
+            acc[2 * np + 1][0] *= w1.x; acc[2 * np + 1][1] *= w1.y; acc[2 * np + 1][2] *= w1.x; acc[2 * np + 1][3] *= w1.y;
+            uint32_t b0, b1, b2, b3;        // key tiles 2 np (b0, b1) and 2 np + 1 (b2, b3)
+            ldmatrix_x4_trans(b0, b1, b2, b3, &sm.ops[buf][3][frow][16 * np + fcol]);
+            mma_bf16(acc[2 * np], va[0], va[1], va[2], va[3], b0, b1);
+            mma_bf16(acc[2 * np + 1], va[0], va[1], va[2], va[3], b2, b3);
         }
         if (c == c_out && part == 0) write_state(s_out);
     };
+    int buf = 0;
     for (int c = 0; c < nC; ++c) {
         if (split && c == c_out) {
 #pragma unroll 1
-            for (int part = 0; part < 2; ++part) walk(std::true_type{}, c, part);
+            for (int part = 0; part < 2; ++part, buf ^= 1) walk(std::true_type{}, c, buf, part);
         } else {
-            walk(std::false_type{}, c, 0);
+            walk(std::false_type{}, c, buf, 0);
+            buf ^= 1;
         }
     }
+    tc::fence_async_smem();
     __syncthreads();
-    {
-        const int t = (nC - 1) * kC6 + srow;
-        if (t < Tlen) *reinterpret_cast<uint4*>(y + seq_base + (size_t)t * tok_stride + spiece) = *reinterpret_cast<const uint4*>(&sm.ys[srow][spiece]);
-    }
-    if (bad) atomicExch(flag, ticket);
+    send_outputs(buf ^ 1);
+    if (tid == 0) tc::bulk_wait_read<0>();
+    if (!good) atomicExch(flag, ticket);
 }
 
 
 // ------------------------------------------------------------------ backward --------
 // Chunks in reverse order with the gradient of the state, dS^T[j][i], in accumulator tiles.  Per chunk, with the
-// forward's operands rebuilt from the raw rows and the entering state S0 read from the forward's checkpoint:
+// forward's operands rebuilt from the raw rows, and the entering state S0 and the scores A as the forward left them:
 //     dA = mask(dY V^T)                                   dd_t = dy_t . v_t  (its diagonal, the u term)
 //     dV  = A^T dY + K^ dS_C
-//     dR0 = dY S0^T        dR~ = dA K~        dK~ = dA^T R~        dK^ = V dS_C^T
-//     dr = dR0 exp(c_{t-1}) + dR~ exp(c_{t-1} - c_m) + dd u k        dk = dK~ exp(c_m - c_s) + dK^ exp(c_C - c_s) + dd u r
+//     dR~ = dY S0^T exp(c_m) + dA K~                      dK~ = V dS_C^T exp(c_C - c_m) + dA^T R~
+//     dr = dR~ exp(c_{t-1} - c_m) + dd u k                dk = dK~ exp(c_m - c_s) + dd u r
 //     dS0^T = dS_C^T diag(exp(c_C)) + dY^T R0
 // and the gradient of the log-decay from the positions at which each factor depends on the cumulative sum:
 //     dlw_tau = sum_{x >= tau} [ (r dr')_{x+1} - (k dk')_x ] + sum_s k dK^ exp(c_C - c_s) + exp(c_C) sum_j dS_C S0
-// (dr', dk' without the u terms; the two references to the middle cancel).  Every warp owns 16 channels of the
-// token-by-channel results and 16 value rows of dS^T, and computes the 16x16 score blocks for itself.
+// (dr', dk' without the u terms; dK^ = V dS_C^T; the two references to the middle cancel).
+//
+// Bound by instructions, as the forward, and split as it is: a warp prepares its 16 channels for all 16 tokens in fragment
+// layout, and since that is also the layout of the gradients of those channels, the rows of r and k and the decay factors
+// stay in its registers from the preparation to the results: nothing but operands and finished results passes through shared
+// memory, the suffix sums over the tokens run over the lanes, and the sum over j of dS_C S0 is the diagonal of a product whose
+// operands the other products load anyway (with dS_C as a high and a low bf16 part: the decay's gradient starts from this sum,
+// and rounding dS_C once made it 4 % less accurate).  dA is computed by every warp for itself.  Two barriers per chunk.  At
+// B=16, T=4096, H=32: 0.93 ms (1.56 ms with the factors, rows and sums exchanged through shared memory and four more score
+// products per warp, which the forward now leaves).
 struct BwdStage {
-    bf r[kC6][PITCH], k[kC6][PITCH], v[kC6][PITCH], w[kC6][PITCH], dy[kC6][PITCH];
-    // S0^T[j][i] as it lies in the residual: 8 column blocks of [64 rows j][8 keys i] (a linear copy; the eight rows of an
-    // ldmatrix tile are 128 contiguous bytes); once the products have read it, r dr' and k dk' per token and channel
-    // (fp32, two tiles of [16][EPITCH], which need the tail)
-    bf s0[8][kN][8];
-    bf s0_tail[kN * PITCH - 8 * kN * 8];
+    unsigned char r[kTile6], k[kTile6], v[kTile6], w[kTile6], dy[kTile6];
+    uint4 scores[32];          // A^T: the words of the left operand, lane by lane
+    unsigned char pad[512];
+    bf s0[8][kN][8];           // S0^T[j][i] as it lies in the residual: 8 column blocks of [64 rows j][8 keys i]
 };
-// fp32 [token][channel] tiles that the epilogue's threads address as (row g, column pair 2 q): with 72 floats per row the
-// sixteen lanes of a 64-bit access (four rows, four column pairs) fall into 32 different banks
-constexpr int EPITCH = 72;
-static_assert(sizeof(bf) * kN * PITCH >= 2 * sizeof(float) * kC6 * EPITCH, "the two fp32 tiles must fit over the state tile and its tail");
 struct Bwd6cSmem {
     BwdStage st[2];
-    bf ops[4][kC6][PITCH];     // R~, K~, R0, K^ while the products run; then dr, dk, dv, dw on their way out
-    bf ds[kN][PITCH];          // dS_C^T[j][i] in bf16, for the one product that contracts over j
-    float e2[kC6][EPITCH], e3[kC6][EPITCH];   // exp(c_{t-1} - c_m) and exp(c_m - c_t): what turns dR~, dK~ into dr, dk
-    float em[kN], ecm[kN];     // exp(c_m) and exp(c_C - c_m): the same for dR0 and dK^
-    float tot[4][kN];          // sum of lw over each quarter of the chunk
+    unsigned char res[4][kTile6];   // dr, dk, dv, dw on their way out
+    bf ops[4][kC6][PITCH];     // R~, K~ (each warp's own channels only), R0, K^
+    bf ds[kN][PITCH];          // dS_C^T[j][i] in bf16, for the products that contract over j
+    bf ds_low[kN][PITCH];      // and what that rounds off, for the sum that the decay's gradient starts from
     float wc[kN];              // exp(c_C), or 0 when a start flag lies in the chunk
-    float lump[kN];            // what every token of the chunk receives: the K^ references and the carried state
-    float gw[4][kN];           // sum_j dS_C S0 over each warp's value rows
-    float dpart[2][kC6];
-    int seg[kC6];
-    unsigned startmask;
-    uint8_t ns[2][kC6];
+    uint64_t full[2];
 };
+static_assert(sizeof(BwdStage) % 1024 == 0, "the swizzle is a function of the address");
+static_assert(3 * (sizeof(Bwd6cSmem) + 1024) <= 228 * 1024, "three CTAs per SM");
 
 __global__ void __launch_bounds__(128, 3)
-wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
-                      const bf* __restrict__ w, int w_per_token, const bf* __restrict__ u,
-                      const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts,
-                      const bf* __restrict__ dy, const bf* __restrict__ ds_out, const bf* __restrict__ ckpt,
+wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ u, const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts, int has_dy, const bf* __restrict__ ds_out, const bf* __restrict__ ckpt, const uint4* __restrict__ scores,
                       const int* __restrict__ residual_mark, bf* __restrict__ dr, bf* __restrict__ dk, bf* __restrict__ dv,
-                      bf* __restrict__ dw_tok, float* __restrict__ dw_head, float* __restrict__ du_head, bf* __restrict__ ds0,
-                      int n_runs, int run_len, const bf* __restrict__ dsck, float* __restrict__ partial) {
+                      bf* __restrict__ dw, float* __restrict__ du_head, bf* __restrict__ ds0,
+                      int n_runs, int run_len, const bf* __restrict__ dsck, float* __restrict__ partial, int* __restrict__ status,
+                      const __grid_constant__ SeqMaps maps) {
     if (*residual_mark != 0) return;          // the forward fell back to the sequential kernels
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
     Bwd6cSmem& sm = *reinterpret_cast<Bwd6cSmem*>(smem_raw);
     // n_runs > 1: a sequence is walked by n_runs CTAs, run rho = chunks [rho run_len, (rho + 1) run_len), each starting
     // from the state gradient that the carry kernel (wkv6_carry_bwd_kernel) left for the end of its run
     const int bh = blockIdx.x / n_runs, run = blockIdx.x % n_runs, bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, q = lane & 3, mi = lane >> 3, r8 = lane & 7;
-    const int j0 = warp * 16;                 // value rows of dS^T, and key channels of the token-by-channel results
+    const int g = lane >> 2, q = lane & 3;
+    const int frow = (lane & 15), fcol = (lane >> 4) * 8;
+    const int j0 = warp * 16;                 // value rows of dS^T, and channels of the token-by-channel results
     const size_t tok_stride = (size_t)H * kN;
     const size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
     const size_t st_base = (size_t)bh * kN * kN;
@@ -443,6 +519,34 @@ wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
     const bool split = L > 0 && L < Tlen && p_out != kC6 - 1;      // see the forward: that chunk is walked in two parts
     const int c_lo = run * run_len, c_hi = min(nC, c_lo + run_len);
     if (c_lo >= c_hi) return;
+
+    auto issue = [&](int c, int stage) {
+        if (tid == 0 && c >= c_lo) {
+            BwdStage& st = sm.st[stage];
+            uint64_t* bar = &sm.full[stage];
+            tc::mbar_expect_tx(bar, (4 + has_dy) * kTile6 + sizeof(st.s0) + sizeof(st.scores));
+            tc::tensor_load_3d(st.r, &maps.m[0], h * kN, c * kC6, bi, bar);
+            tc::tensor_load_3d(st.k, &maps.m[1], h * kN, c * kC6, bi, bar);
+            tc::tensor_load_3d(st.v, &maps.m[2], h * kN, c * kC6, bi, bar);
+            tc::tensor_load_3d(st.w, &maps.m[3], h * kN, c * kC6, bi, bar);
+            if (has_dy) tc::tensor_load_3d(st.dy, &maps.m[4], h * kN, c * kC6, bi, bar);
+            tc::bulk_load(st.s0, ckpt + ((size_t)bh * (nC + 1) + c) * kN * kN, sizeof(st.s0), bar);
+            tc::bulk_load(st.scores, scores + ((size_t)bh * (nC + 1) + c) * 32, sizeof(st.scores), bar);
+        }
+    };
+    if (tid == 0) {
+        tc::mbar_init(&sm.full[0], 1);
+        tc::mbar_init(&sm.full[1], 1);
+        tc::mbar_init_fence();
+    }
+    if (!has_dy)
+#pragma unroll
+        for (int stg = 0; stg < 2; ++stg) *reinterpret_cast<uint4*>(sm.st[stg].dy + tid * 16) = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    issue(c_hi - 1, 0);
+    const uint8_t* const ns_row = new_starts + (size_t)bi * Tlen;
+    auto load_ns = [&](int c) -> unsigned { return ns_row[min(max(c, 0) * kC6 + (lane & 15), Tlen - 1)]; };
+    unsigned ns_now = load_ns(c_hi - 1), ns_next = load_ns(c_hi - 2);
 
     float acc[8][4];
     if (run == n_runs - 1 || c_hi >= nC) {
@@ -467,339 +571,318 @@ wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
             for (int e = 0; e < 4; ++e)
                 acc[ni][e] += __bfloat162float(ds_out[st_base + (size_t)(8 * ni + 2 * q + (e & 1)) * kN + j0 + g + 8 * (e >> 1)]);
     };
-
-    const int srow = tid >> 3, spiece = (tid & 7) * 8;
-    auto issue = [&](int c, int stage) {
-        if (c >= c_lo) {
-            BwdStage& st = sm.st[stage];
-            const int t = c * kC6 + srow;
-            const bool ok = t < Tlen;
-            const size_t off = seq_base + (size_t)(ok ? t : 0) * tok_stride + spiece;
-            cp_async16_zfill(&st.r[srow][spiece], r + off, ok);
-            cp_async16_zfill(&st.k[srow][spiece], k + off, ok);
-            cp_async16_zfill(&st.v[srow][spiece], v + off, ok);
-            if (w_per_token) cp_async16_zfill(&st.w[srow][spiece], w + off, ok);
-            cp_async16_zfill(&st.dy[srow][spiece], dy != nullptr ? dy + off : r + off, ok && dy != nullptr);
-            const bf* src = ckpt + ((size_t)bh * (nC + 1) + c) * kN * kN;
-#pragma unroll
-            for (int rr = 0; rr < 4; ++rr) {   // piece tid + 128 rr of the tile: row = piece mod 64 of column block piece / 64
-                const int pc = tid + 128 * rr;
-                cp_async16_zfill(&st.s0[pc >> 6][pc & 63][0], src + (size_t)pc * 8, true);
-            }
-        }
-        cp_async_commit();
-    };
-    // the state entering a part of the split chunk, fetched on the spot (once or twice per sequence)
+    // the state entering a part of the split chunk and the part's scores, fetched on the spot (once or twice per sequence)
     auto fetch_state = [&](int slot, int stage) {
-        const bf* src = ckpt + ((size_t)bh * (nC + 1) + slot) * kN * kN;
+        const uint4* src = reinterpret_cast<const uint4*>(ckpt + ((size_t)bh * (nC + 1) + slot) * kN * kN);
+        uint4* dst = reinterpret_cast<uint4*>(&sm.st[stage].s0[0][0][0]);
+        __syncthreads();
 #pragma unroll
-        for (int rr = 0; rr < 4; ++rr)
-            cp_async16_zfill(&sm.st[stage].s0[(tid + 128 * rr) >> 6][(tid + 128 * rr) & 63][0], src + (size_t)(tid + 128 * rr) * 8, true);
-        cp_async_commit();
-        cp_async_wait<0>();
+        for (int rr = 0; rr < 4; ++rr) dst[tid + 128 * rr] = src[tid + 128 * rr];
+        if (warp == 0) sm.st[stage].scores[lane] = scores[((size_t)bh * (nC + 1) + slot) * 32 + lane];
         __syncthreads();
     };
-    auto load_ns = [&](int c) -> uint8_t {
-        const int t = c * kC6 + tid;
-        return (tid < kC6 && c >= 0 && t < Tlen) ? new_starts[(size_t)bi * Tlen + t] : (uint8_t)0;
-    };
-    issue(c_hi - 1, 0);
-    if (tid < kC6) sm.ns[0][tid] = load_ns(c_hi - 1);
-    uint8_t ns_ahead = load_ns(c_hi - 2);
 
-    // phase A ownership as in the forward: the channel pair cp, cp + 1 and the four tokens of quarter qt (= the warp)
-    const int cp = (tid & 31) * 2, qt = warp;
-    const float2 uu_a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(u + (size_t)h * kN + cp));
-    float2 lw_const = make_float2(0.f, 0.f);
-    if (!w_per_token) {
-        const float2 wv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(w + (size_t)h * kN + cp));
-        lw_const = make_float2(__logf(wv.x), __logf(wv.y));
-    }
-    float u_col[2][2];                         // u of this thread's four result columns
+    float uu[4];                                                  // of channels j0 + 2 q, + 1, + 8, + 9
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) u_col[nt][e] = __bfloat162float(u[(size_t)h * kN + j0 + 8 * nt + 2 * q + e]);
-    float du_acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-    float dw_acc = 0.f;                        // constant decay: sum over tokens of the log-decay gradient (thread ch < 64)
+    for (int e = 0; e < 4; ++e) uu[e] = __bfloat162float(u[(size_t)h * kN + j0 + 8 * (e >> 1) + 2 * q + (e & 1)]);
+    const DecaySums sums(g, q);
+    const int tile_row = frow * 128 + (((2 * warp + (lane >> 4)) ^ (frow & 7)) << 4);      // as in the forward
+    const int tile_word = g * 128 + (((2 * warp) ^ g) << 4) + 4 * q;
+    float du_acc[4] = {0.f, 0.f, 0.f, 0.f};    // this thread's tokens of those channels
+    bool waited = true;
 
-    int out_t0 = -1, out_lo = 0, out_hi = 0;     // the chunk (part) whose results wait in the result tiles
-    auto flush_results = [&]() {
-        const int t = out_t0 + srow;
-        if (out_t0 >= 0 && t < Tlen && srow >= out_lo && srow < out_hi) {
-            const size_t off = seq_base + (size_t)t * tok_stride + spiece;
-            *reinterpret_cast<uint4*>(dr + off) = *reinterpret_cast<const uint4*>(&sm.ops[0][srow][spiece]);
-            *reinterpret_cast<uint4*>(dk + off) = *reinterpret_cast<const uint4*>(&sm.ops[1][srow][spiece]);
-            *reinterpret_cast<uint4*>(dv + off) = *reinterpret_cast<const uint4*>(&sm.ops[2][srow][spiece]);
-            if (w_per_token) *reinterpret_cast<uint4*>(dw_tok + off) = *reinterpret_cast<const uint4*>(&sm.ops[3][srow][spiece]);
+    // the chunk whose results wait in the result tiles (see send_outputs of the forward)
+    int out_t = -1, out_lo = 0, out_hi = kC6;
+    auto send_results = [&]() {
+        if (out_t < 0) return;
+        if (out_lo == 0 && out_hi == kC6) {
+            if (tid == 0) {
+                tc::tensor_store_3d(&maps.m[5], h * kN, out_t, bi, sm.res[0]);
+                tc::tensor_store_3d(&maps.m[6], h * kN, out_t, bi, sm.res[1]);
+                tc::tensor_store_3d(&maps.m[7], h * kN, out_t, bi, sm.res[2]);
+                tc::tensor_store_3d(&maps.m[8], h * kN, out_t, bi, sm.res[3]);
+                tc::bulk_commit();
+            }
+        } else {
+            const int row = tid >> 3, piece = tid & 7;
+            if (row >= out_lo && row < out_hi && out_t + row < Tlen) {
+                const size_t off = seq_base + (size_t)(out_t + row) * tok_stride + piece * 8;
+                const int at = row * 128 + ((piece ^ (row & 7)) << 4);
+                *reinterpret_cast<uint4*>(dr + off) = *reinterpret_cast<const uint4*>(sm.res[0] + at);
+                *reinterpret_cast<uint4*>(dk + off) = *reinterpret_cast<const uint4*>(sm.res[1] + at);
+                *reinterpret_cast<uint4*>(dv + off) = *reinterpret_cast<const uint4*>(sm.res[2] + at);
+                *reinterpret_cast<uint4*>(dw + off) = *reinterpret_cast<const uint4*>(sm.res[3] + at);
+            }
         }
     };
     auto walk = [&](auto split_tag, const int c, const int it, const int part_arg) {
         constexpr bool kSplitHere = decltype(split_tag)::value;
-        const bool split_here = kSplitHere;
         const int part = kSplitHere ? part_arg : 0;
         const int stage = it & 1;
+        BwdStage& st = sm.st[stage];
         const int lo = (kSplitHere && part == 1) ? p_out + 1 : 0, hi = (kSplitHere && part == 0) ? p_out + 1 : kC6;
-        if (!split_here || part == 1) {                               // first visit of the chunk
-            cp_async_wait<0>();
-            __syncthreads();                                          // S1
-            issue(c - 1, stage ^ 1);
-            if (tid < kC6) sm.ns[stage ^ 1][tid] = ns_ahead;
-            ns_ahead = load_ns(c - 2);
-            if (split_here) fetch_state(nC, stage);                   // the state behind token p_out
-        } else {
-            __syncthreads();                                          // the first visit's suffix sums have read the tile refilled here
-            fetch_state(c, stage);
-        }
-        flush_results();                                              // of the walk before this one; phase A rewrites the tiles behind S2
-        const BwdStage& st = sm.st[stage];
         const int t0 = c * kC6;
+        const bool first_visit = !kSplitHere || part == 1;
+        if (first_visit) issue(c - 1, stage ^ 1);
+        unsigned starts = __ballot_sync(0xffffffffu, ns_now != 0) & (0xffffu >> max(t0 + kC6 - Tlen, 0));
+        if (kSplitHere) starts &= ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+        if (!kSplitHere || part == 0) {
+            ns_now = ns_next;
+            ns_next = load_ns(c - 2);
+        }
+        if (!tc::mbar_wait(&sm.full[stage], (it >> 1) & 1)) waited = false;
+        if (kSplitHere) fetch_state(part == 1 ? nC : c, stage);       // (slot nC: the state behind token p_out)
         if (c == c_out && part == 0) add_ds_out();
-        // dS_C^T in bf16 for the product that contracts over value rows
+
+        // ---- phase A: dS_C^T in bf16; the scaled operands of this warp's channels, as in the forward
+        uint32_t dsp[8][2];                   // [ni][value rows g | g + 8]
 #pragma unroll
         for (int ni = 0; ni < 8; ++ni) {
-            *reinterpret_cast<uint32_t*>(&sm.ds[j0 + g][8 * ni + 2 * q]) = pack2(acc[ni][0], acc[ni][1]);
-            *reinterpret_cast<uint32_t*>(&sm.ds[j0 + g + 8][8 * ni + 2 * q]) = pack2(acc[ni][2], acc[ni][3]);
+            dsp[ni][0] = pack2(acc[ni][0], acc[ni][1]);
+            dsp[ni][1] = pack2(acc[ni][2], acc[ni][3]);
         }
-        // ---- phase A: as in the forward
-        if (warp == 0) {
-            const unsigned m = __ballot_sync(0xffffffffu, lane < kC6 && sm.ns[stage][lane] != 0);
-            if (lane == 0) sm.startmask = m;
-        }
-        float2 lw[4], cl[4];
-        float2 run = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int tt = 0; tt < 4; ++tt) {
-            const int t = 4 * qt + tt;
-            const bool ok = t0 + t < Tlen && t >= lo && t < hi;
-            lw[tt] = !ok ? make_float2(0.f, 0.f)
-                         : (w_per_token ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.w[t][cp])) : lw_const);
-            run.x += lw[tt].x;
-            run.y += lw[tt].y;
-            cl[tt] = run;
+        for (int np = 0; np < 4; ++np) stmatrix_x4(&sm.ds[j0 + frow][16 * np + fcol], dsp[2 * np][0], dsp[2 * np][1], dsp[2 * np + 1][0], dsp[2 * np + 1][1]);
+#pragma unroll
+        for (int np = 0; np < 4; ++np) {
+            uint32_t low[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int ni = 2 * np + (i >> 1), half = i & 1;
+                const float2 high = unpack2(dsp[ni][half]);
+                low[i] = pack2(acc[ni][2 * half] - high.x, acc[ni][2 * half + 1] - high.y);
+            }
+            stmatrix_x4(&sm.ds_low[j0 + frow][16 * np + fcol], low[0], low[1], low[2], low[3]);
         }
-        *reinterpret_cast<float2*>(&sm.tot[qt][cp]) = run;
-        __syncthreads();                                              // S2
+        uint32_t rw[4], kw[4];                // raw rows, [2 nt + hh]
+        float2 f2[4], f3[4], em[2], ecm[2];   // what turns dR~, dK~ into dr, dk; and dR0, dK^ into dR~, dK~
         {
-            const unsigned starts = sm.startmask;
-            auto seg_of = [&](int t) { return __popc(starts & ((2u << t) - 1u)); };
-            const int seg_last = seg_of(hi - 1), seg_base = lo > 0 ? seg_of(lo - 1) : 0;
-            if (tid < kC6) sm.seg[tid] = seg_of(tid);
-            const float2 tq0 = *reinterpret_cast<const float2*>(&sm.tot[0][cp]), tq1 = *reinterpret_cast<const float2*>(&sm.tot[1][cp]);
-            const float2 tq2 = *reinterpret_cast<const float2*>(&sm.tot[2][cp]), tq3 = *reinterpret_cast<const float2*>(&sm.tot[3][cp]);
-            const float2 c_m = make_float2(fmaxf(tq0.x + tq1.x, -kMaxHalfDecay), fmaxf(tq0.y + tq1.y, -kMaxHalfDecay));
-            const float2 c_C = make_float2(c_m.x + fmaxf(tq2.x + tq3.x, -kMaxHalfDecay), c_m.y + fmaxf(tq2.y + tq3.y, -kMaxHalfDecay));
-            const float2 base = qt == 0 ? make_float2(0.f, 0.f) : (qt == 1 ? tq0 : (qt == 2 ? c_m : make_float2(c_m.x + tq2.x, c_m.y + tq2.y)));
-            if (qt == 3) {
-                const bool carried = seg_last == seg_base;
-                *reinterpret_cast<float2*>(&sm.wc[cp]) = carried ? make_float2(__expf(c_C.x), __expf(c_C.y)) : make_float2(0.f, 0.f);
-                *reinterpret_cast<float2*>(&sm.em[cp]) = make_float2(__expf(c_m.x), __expf(c_m.y));
-                *reinterpret_cast<float2*>(&sm.ecm[cp]) = make_float2(__expf(c_C.x - c_m.x), __expf(c_C.y - c_m.y));
-            }
-            float dsum[4];
+            float upto[2][4], before[2][4], halves[2][4];
+            uint32_t wb[4];
+            ldmatrix_x4_trans(wb[0], wb[1], wb[2], wb[3], st.w + tile_row);
+            if (kSplitHere) {
 #pragma unroll
-            for (int tt = 0; tt < 4; ++tt) {
-                const int t = 4 * qt + tt;
-                const int seg_t = seg_of(t);
-                const float2 c_t = make_float2(base.x + cl[tt].x, base.y + cl[tt].y), c_prev = make_float2(c_t.x - lw[tt].x, c_t.y - lw[tt].y);
-                const bool in_part = t >= lo && t < hi;
-                const float2 zero2 = make_float2(0.f, 0.f);
-                const float2 rv = in_part ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.r[t][cp])) : zero2;
-                const float2 kv = in_part ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.k[t][cp])) : zero2;
-                const float2 f2 = make_float2(__expf(fminf(c_prev.x - c_m.x, kMaxHalfDecay)), __expf(fminf(c_prev.y - c_m.y, kMaxHalfDecay)));
-                const float2 f3 = make_float2(__expf(fminf(c_m.x - c_t.x, kMaxHalfDecay)), __expf(fminf(c_m.y - c_t.y, kMaxHalfDecay)));
-                *reinterpret_cast<float2*>(&sm.e2[t][cp]) = f2;
-                *reinterpret_cast<float2*>(&sm.e3[t][cp]) = f3;
-                const bool first = seg_t == seg_base, last = seg_t == seg_last;
-                *reinterpret_cast<uint32_t*>(&sm.ops[0][t][cp]) = pack2(rv.x * f2.x, rv.y * f2.y);
-                *reinterpret_cast<uint32_t*>(&sm.ops[1][t][cp]) = pack2(kv.x * f3.x, kv.y * f3.y);
-                *reinterpret_cast<uint32_t*>(&sm.ops[2][t][cp]) = pack2(first ? rv.x * __expf(c_prev.x) : 0.f, first ? rv.y * __expf(c_prev.y) : 0.f);
-                *reinterpret_cast<uint32_t*>(&sm.ops[3][t][cp]) = pack2(last ? kv.x * __expf(c_C.x - c_t.x) : 0.f, last ? kv.y * __expf(c_C.y - c_t.y) : 0.f);
-                dsum[tt] = fmaf(rv.x * uu_a.x, kv.x, rv.y * uu_a.y * kv.y);
+                for (int i = 0; i < 4; ++i) {
+                    const int s = 8 * (i & 1) + 2 * q;
+                    wb[i] &= (s >= lo && s < hi ? 0xffffu : 0u) | (s + 1 >= lo && s + 1 < hi ? 0xffff0000u : 0u);
+                }
             }
-            int which;
-            const float total = warp_sum4(dsum, lane, &which);       // over all 64 channels: the warp holds them all
-            if ((lane & 7) == 0) {
-                sm.dpart[0][4 * qt + which] = total;
-                sm.dpart[1][4 * qt + which] = 0.f;
-            }
-        }
-        __syncthreads();                                              // S3
-        const bf (*Rt)[PITCH] = sm.ops[0];
-        const bf (*Kt)[PITCH] = sm.ops[1];
-        const bf (*R0)[PITCH] = sm.ops[2];
-        const bf (*Kh)[PITCH] = sm.ops[3];
-
-        // ---- the 16x16 blocks: dA (t x s), dA^T (s x t), A^T (s x t)
-        float dA[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, dAT[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        float AT[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        Frag fdy[4], fv[4];                   // dY and V, all four K steps (left and right operands alike)
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-            fdy[ks] = load_frag(st.dy, ks, lane);
-            fv[ks] = load_frag(st.v, ks, lane);
-            const Frag fk = load_frag(Kt, ks, lane), fr = load_frag(Rt, ks, lane);
+            decay_sums(sums, wb, upto, before, halves);
+            uint32_t rt[4], kt[4], r0[4], kh[4];
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt) {
-                mma_ab(dA[nt], fdy[ks], fv[ks], nt);
-                mma_ab(dAT[nt], fv[ks], fdy[ks], nt);
-                mma_ab(AT[nt], fk, fr, nt);
+                em[nt] = make_float2(exp_fast(halves[nt][0]), exp_fast(halves[nt][1]));
+                ecm[nt] = make_float2(exp_fast(halves[nt][2]), exp_fast(halves[nt][3]));
+                if (g == 0)
+                    *reinterpret_cast<float2*>(&sm.wc[j0 + 8 * nt + 2 * q]) = starts == 0 ? make_float2(em[nt].x * ecm[nt].x, em[nt].y * ecm[nt].y) : make_float2(0.f, 0.f);
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int at = 2 * nt + hh, t = g + 8 * hh;
+                    rw[at] = *reinterpret_cast<const uint32_t*>(st.r + (tile_word ^ (16 * nt)) + 1024 * hh);
+                    kw[at] = *reinterpret_cast<const uint32_t*>(st.k + (tile_word ^ (16 * nt)) + 1024 * hh);
+                    if (kSplitHere && !(t >= lo && t < hi)) rw[at] = kw[at] = 0;
+                    const float2 rv = unpack2(rw[at]), kv = unpack2(kw[at]);
+                    f2[at] = make_float2(exp_fast(before[nt][2 * hh]), exp_fast(before[nt][2 * hh + 1]));
+                    f3[at] = make_float2(exp_fast(-upto[nt][2 * hh]), exp_fast(-upto[nt][2 * hh + 1]));
+                    rt[at] = pack2(rv.x * f2[at].x, rv.y * f2[at].y);
+                    kt[at] = pack2(kv.x * f3[at].x, kv.y * f3[at].y);
+                    r0[at] = pack2(rv.x * (f2[at].x * em[nt].x), rv.y * (f2[at].y * em[nt].y));
+                    kh[at] = pack2(kv.x * (f3[at].x * ecm[nt].x), kv.y * (f3[at].y * ecm[nt].y));
+                }
             }
+            if (starts != 0) {
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int t = g + 8 * hh;
+                    const bool first = (starts & ((2u << t) - 1u)) == 0, last = (starts >> (t + 1)) == 0;
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) {
+                        r0[2 * nt + hh] = first ? r0[2 * nt + hh] : 0u;
+                        kh[2 * nt + hh] = last ? kh[2 * nt + hh] : 0u;
+                    }
+                }
+            }
+            stmatrix_x4(&sm.ops[0][frow][j0 + fcol], rt[0], rt[1], rt[2], rt[3]);
+            stmatrix_x4(&sm.ops[1][frow][j0 + fcol], kt[0], kt[1], kt[2], kt[3]);
+            stmatrix_x4(&sm.ops[2][frow][j0 + fcol], r0[0], r0[1], r0[2], r0[3]);
+            stmatrix_x4(&sm.ops[3][frow][j0 + fcol], kh[0], kh[1], kh[2], kh[3]);
         }
-        // dd of this thread's two token rows: the diagonal of dA sits in lane 4 g + g / 2
-        float dd_lo, dd_hi;
-        {
-            const float cand_lo = (g & 1) ? dA[0][1] : dA[0][0], cand_hi = (g & 1) ? dA[1][3] : dA[1][2];
-            const int src = (lane & ~3) | (g >> 1);
-            dd_lo = __shfl_sync(0xffffffffu, cand_lo, src);
-            dd_hi = __shfl_sync(0xffffffffu, cand_hi, src);
-        }
-        int seg_r[2] = {sm.seg[g], sm.seg[g + 8]};
-        const int seg_end = sm.seg[hi - 1], seg_in = lo > 0 ? sm.seg[lo - 1] : 0;     // as seg_last / seg_base of phase A
-        const bool row_in[2] = {g >= lo && g < hi, g + 8 >= lo && g + 8 < hi};
+        tc::fence_async_smem();               // (the previous chunk's results, for the copies that take them)
+        __syncthreads();                      // the operands are complete
+        send_results();
+
+        // ---- phase B: the products
+        float dA[2][4];                       // t x s
+        float dR[2][4], dK[2][4], dV[2][4];   // token x this warp's 16 channels (dV: its value columns)
+        float dot[2][4];                      // its diagonals: sum_j dS_C S0 of channels j0 + g (tile 0) and j0 + 8 + g (tile 1)
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int row = g + 8 * (e >> 1), col = 8 * nt + 2 * q + (e & 1);
-                const bool same = sm.seg[col] == seg_r[e >> 1] && row_in[e >> 1] && col >= lo && col < hi;
-                dA[nt][e] = (col < row && same) ? dA[nt][e] : 0.f;                       // rows t, columns s < t
-                dAT[nt][e] = (row < col && same) ? dAT[nt][e] : 0.f;                     // rows s, columns t > s
-                AT[nt][e] = (row < col && same) ? AT[nt][e] : (row == col ? sm.dpart[0][row] + sm.dpart[1][row] : 0.f);
-            }
-        // ---- dV (s x j of this warp) = A^T dY + K^ dS_C
-        float dV[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(b0, b1, b2, b3, &st.dy[(mi & 1) * 8 + r8][j0 + (mi >> 1) * 8]);
-            const uint32_t a0 = pack2(AT[0][0], AT[0][1]), a1 = pack2(AT[0][2], AT[0][3]);
-            const uint32_t a2 = pack2(AT[1][0], AT[1][1]), a3 = pack2(AT[1][2], AT[1][3]);
-            mma_bf16(dV[0], a0, a1, a2, a3, b0, b1);
-            mma_bf16(dV[1], a0, a1, a2, a3, b2, b3);
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-                const Frag fh = load_frag(Kh, ks, lane);
-                const uint32_t h0 = fh.f[0], h1 = fh.f[1], h2 = fh.f[2], h3 = fh.f[3];
-                // dS_C^T tiles as right operand: K = key channel (their columns), n = value row (their rows)
-                mma_bf16(dV[0], h0, h1, h2, h3, pack2(acc[2 * ks][0], acc[2 * ks][1]), pack2(acc[2 * ks + 1][0], acc[2 * ks + 1][1]));
-                mma_bf16(dV[1], h0, h1, h2, h3, pack2(acc[2 * ks][2], acc[2 * ks][3]), pack2(acc[2 * ks + 1][2], acc[2 * ks + 1][3]));
-            }
-        }
-        // ---- the token x channel results for this warp's 16 key channels
-        float dR0[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, dRt[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-        float dKt[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, dKh[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+            for (int e = 0; e < 4; ++e) dA[nt][e] = dR[nt][e] = dK[nt][e] = dV[nt][e] = dot[nt][e] = 0.f;
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(b0, b1, b2, b3, &st.s0[j0 / 8 + (mi >> 1)][16 * ks + (mi & 1) * 8 + r8][0]);
-            mma_bf16(dR0[0], fdy[ks].f[0], fdy[ks].f[1], fdy[ks].f[2], fdy[ks].f[3], b0, b1);
-            mma_bf16(dR0[1], fdy[ks].f[0], fdy[ks].f[1], fdy[ks].f[2], fdy[ks].f[3], b2, b3);
-            ldmatrix_x4_trans(b0, b1, b2, b3, &sm.ds[16 * ks + (mi & 1) * 8 + r8][j0 + (mi >> 1) * 8]);
-            mma_bf16(dKh[0], fv[ks].f[0], fv[ks].f[1], fv[ks].f[2], fv[ks].f[3], b0, b1);
-            mma_bf16(dKh[1], fv[ks].f[0], fv[ks].f[1], fv[ks].f[2], fv[ks].f[3], b2, b3);
+            Frag fdy, fv, fh, fs, fd, fl;
+            const int row_at = frow * 128 + (((2 * ks + (lane >> 4)) ^ (frow & 7)) << 4);
+            ldmatrix_x4(fdy.f[0], fdy.f[1], fdy.f[2], fdy.f[3], st.dy + row_at);
+            ldmatrix_x4(fv.f[0], fv.f[1], fv.f[2], fv.f[3], st.v + row_at);
+            ldmatrix_x4(fh.f[0], fh.f[1], fh.f[2], fh.f[3], &sm.ops[3][frow][16 * ks + fcol]);
+            // [value j][channel i] tiles as right operands (K = j); as left operands their transposes are the same words
+            ldmatrix_x4_trans(fs.f[0], fs.f[1], fs.f[2], fs.f[3], &st.s0[j0 / 8 + (lane >> 4)][16 * ks + frow][0]);
+            ldmatrix_x4_trans(fd.f[0], fd.f[1], fd.f[2], fd.f[3], &sm.ds[16 * ks + frow][j0 + fcol]);
+            ldmatrix_x4_trans(fl.f[0], fl.f[1], fl.f[2], fl.f[3], &sm.ds_low[16 * ks + frow][j0 + fcol]);
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                mma_ab(dA[nt], fdy, fv, nt);
+                mma_bf16(dR[nt], fdy.f[0], fdy.f[1], fdy.f[2], fdy.f[3], fs.f[2 * nt], fs.f[2 * nt + 1]);
+                mma_bf16(dK[nt], fv.f[0], fv.f[1], fv.f[2], fv.f[3], fd.f[2 * nt], fd.f[2 * nt + 1]);
+                // dS_C^T tiles as right operand: K = key channel (their columns), n = value row (their rows)
+                mma_bf16(dV[nt], fh.f[0], fh.f[1], fh.f[2], fh.f[3], dsp[2 * ks][nt], dsp[2 * ks + 1][nt]);
+                mma_bf16(dot[nt], fs.f[0], fs.f[2], fs.f[1], fs.f[3], fd.f[2 * nt], fd.f[2 * nt + 1]);
+                mma_bf16(dot[nt], fs.f[0], fs.f[2], fs.f[1], fs.f[3], fl.f[2 * nt], fl.f[2 * nt + 1]);
+            }
         }
+        // dd of this thread's two token rows: the diagonal of dA sits in lane 4 g + g / 2
+        float dd[2];
         {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(b0, b1, b2, b3, &Kt[(mi & 1) * 8 + r8][j0 + (mi >> 1) * 8]);
-            uint32_t a0 = pack2(dA[0][0], dA[0][1]), a1 = pack2(dA[0][2], dA[0][3]), a2 = pack2(dA[1][0], dA[1][1]), a3 = pack2(dA[1][2], dA[1][3]);
-            mma_bf16(dRt[0], a0, a1, a2, a3, b0, b1);
-            mma_bf16(dRt[1], a0, a1, a2, a3, b2, b3);
-            ldmatrix_x4_trans(b0, b1, b2, b3, &Rt[(mi & 1) * 8 + r8][j0 + (mi >> 1) * 8]);
-            a0 = pack2(dAT[0][0], dAT[0][1]); a1 = pack2(dAT[0][2], dAT[0][3]); a2 = pack2(dAT[1][0], dAT[1][1]); a3 = pack2(dAT[1][2], dAT[1][3]);
-            mma_bf16(dKt[0], a0, a1, a2, a3, b0, b1);
-            mma_bf16(dKt[1], a0, a1, a2, a3, b2, b3);
+            const int src = (lane & ~3) | (g >> 1);
+            dd[0] = __shfl_sync(0xffffffffu, (g & 1) ? dA[0][1] : dA[0][0], src);
+            dd[1] = __shfl_sync(0xffffffffu, (g & 1) ? dA[1][3] : dA[1][2], src);
         }
-        // ---- sum_j dS_C[i][j] S0[i][j] over this warp's value rows
+        // masks: pairs s < t of one segment (the block t < 8 <= s is not used)
         {
 #pragma unroll
-            for (int ni = 0; ni < 8; ++ni) {
-                const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.s0[ni][j0 + g][2 * q]));
-                const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.s0[ni][j0 + g + 8][2 * q]));
-                float p0 = acc[ni][0] * lo.x + acc[ni][2] * hi.x, p1 = acc[ni][1] * lo.y + acc[ni][3] * hi.y;
+            for (int e = 0; e < 2; ++e) {
+                const int col = 2 * q + e;
+                dA[0][e] = col < g ? dA[0][e] : 0.f;
+                dA[1][2 + e] = col < g ? dA[1][2 + e] : 0.f;
+            }
+            if (starts != 0) {
 #pragma unroll
-                for (int m = 4; m < 32; m <<= 1) {
-                    p0 += __shfl_xor_sync(0xffffffffu, p0, m);
-                    p1 += __shfl_xor_sync(0xffffffffu, p1, m);
+                for (int e = 0; e < 2; ++e) {
+                    const int col = 2 * q + e;
+                    if (col < g && !same_segment(starts, col, g)) dA[0][e] = 0.f;
+                    if (!same_segment(starts, col, g + 8)) dA[0][2 + e] = 0.f;
+                    if (col < g && !same_segment(starts, col + 8, g + 8)) dA[1][2 + e] = 0.f;
                 }
-                if (g == 0) *reinterpret_cast<float2*>(&sm.gw[warp][8 * ni + 2 * q]) = make_float2(p0, p1);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {          // S0 reaches the tokens in front of the first flag, S_C holds those from the last one on
+                    const int t = g + 8 * (e >> 1);
+                    const bool first = (starts & ((2u << t) - 1u)) == 0, last = (starts >> (t + 1)) == 0;
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) {
+                        dR[nt][e] = first ? dR[nt][e] : 0.f;
+                        dK[nt][e] = last ? dK[nt][e] : 0.f;
+                    }
+                }
+            }
+        }
+        uint32_t yf[4];                       // dY of this warp's value columns, transposed: (tokens 0-7 | 8-15) of columns 0-7, then 8-15
+        ldmatrix_x4_trans(yf[0], yf[1], yf[2], yf[3], st.dy + tile_row);
+        {   // dV += A^T dY
+            const uint4 at = st.scores[lane];
+            mma_bf16(dV[0], at.x, 0u, at.z, at.w, yf[0], yf[1]);
+            mma_bf16(dV[1], at.x, 0u, at.z, at.w, yf[2], yf[3]);
+        }
+        float lump[4];                        // per channel: sum_s k dK^ exp(c_C - c_s) over this thread's tokens
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float m = e ? em[nt].y : em[nt].x, mc = e ? ecm[nt].y : ecm[nt].x;
+                float sum = 0.f;
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int at = 2 * nt + hh;
+                    dR[nt][2 * hh + e] *= m;
+                    dK[nt][2 * hh + e] *= mc;
+                    const float kv = e ? unpack2(kw[at]).y : unpack2(kw[at]).x;
+                    sum = fmaf(kv * (e ? f3[at].y : f3[at].x), dK[nt][2 * hh + e], sum);
+                }
+                lump[2 * nt + e] = sum;
+            }
+        }
+        {   // dR~ += dA K~, dK~ += dA^T R~
+            const uint32_t a0 = pack2(dA[0][0], dA[0][1]), a1 = pack2(dA[0][2], dA[0][3]), a3 = pack2(dA[1][2], dA[1][3]);
+            uint32_t b0, b1, b2, b3;
+            ldmatrix_x4_trans(b0, b1, b2, b3, &sm.ops[1][frow][j0 + fcol]);
+            mma_bf16(dR[0], a0, a1, 0u, a3, b0, b1);
+            mma_bf16(dR[1], a0, a1, 0u, a3, b2, b3);
+            ldmatrix_x4_trans(b0, b1, b2, b3, &sm.ops[0][frow][j0 + fcol]);
+            const uint32_t t0_ = transpose8x8(a0), t2 = transpose8x8(a1), t3 = transpose8x8(a3);
+            mma_bf16(dK[0], t0_, 0u, t2, t3, b0, b1);
+            mma_bf16(dK[1], t0_, 0u, t2, t3, b2, b3);
+        }
+        // + exp(c_C) sum_j dS_C S0, from the lanes that hold the diagonals (as one of the sum's eight summands, below)
+        {
+            const float d0 = __shfl_sync(0xffffffffu, dot[0][0], 9 * q), d1 = __shfl_sync(0xffffffffu, dot[0][1], 9 * q + 4);
+            const float d2 = __shfl_sync(0xffffffffu, dot[1][2], 9 * q), d3 = __shfl_sync(0xffffffffu, dot[1][3], 9 * q + 4);
+            if (g == 0) {
+                const float2 w0 = *reinterpret_cast<const float2*>(&sm.wc[j0 + 2 * q]), w1 = *reinterpret_cast<const float2*>(&sm.wc[j0 + 8 + 2 * q]);
+                lump[0] = fmaf(d0, w0.x, lump[0]);
+                lump[1] = fmaf(d1, w0.y, lump[1]);
+                lump[2] = fmaf(d2, w1.x, lump[2]);
+                lump[3] = fmaf(d3, w1.y, lump[3]);
             }
         }
         // ---- dS0^T = dS_C^T diag(exp(c_C)) [no start in the chunk] + dY^T R0
-        {
-            uint32_t ya[4];
-            ldmatrix_x4_trans(ya[0], ya[1], ya[2], ya[3], &st.dy[(mi >> 1) * 8 + r8][j0 + (mi & 1) * 8]);
 #pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                const float2 w0 = *reinterpret_cast<const float2*>(&sm.wc[16 * np + 2 * q]);
-                const float2 w1 = *reinterpret_cast<const float2*>(&sm.wc[16 * np + 8 + 2 * q]);
-                acc[2 * np][0] *= w0.x; acc[2 * np][1] *= w0.y; acc[2 * np][2] *= w0.x; acc[2 * np][3] *= w0.y;
-                acc[2 * np + 1][0] *= w1.x; acc[2 * np + 1][1] *= w1.y; acc[2 * np + 1][2] *= w1.x; acc[2 * np + 1][3] *= w1.y;
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(b0, b1, b2, b3, &R0[(mi & 1) * 8 + r8][(2 * np + (mi >> 1)) * 8]);
-                mma_bf16(acc[2 * np], ya[0], ya[1], ya[2], ya[3], b0, b1);
-                mma_bf16(acc[2 * np + 1], ya[0], ya[1], ya[2], ya[3], b2, b3);
+        for (int np = 0; np < 4; ++np) {
+            const float2 w0 = *reinterpret_cast<const float2*>(&sm.wc[16 * np + 2 * q]);
+            const float2 w1 = *reinterpret_cast<const float2*>(&sm.wc[16 * np + 8 + 2 * q]);
+            acc[2 * np][0] *= w0.x; acc[2 * np][1] *= w0.y; acc[2 * np][2] *= w0.x; acc[2 * np][3] *= w0.y;
+            acc[2 * np + 1][0] *= w1.x; acc[2 * np + 1][1] *= w1.y; acc[2 * np + 1][2] *= w1.x; acc[2 * np + 1][3] *= w1.y;
+            uint32_t b0, b1, b2, b3;
+            ldmatrix_x4_trans(b0, b1, b2, b3, &sm.ops[2][frow][16 * np + fcol]);
+            mma_bf16(acc[2 * np], yf[0], yf[2], yf[1], yf[3], b0, b1);
+            mma_bf16(acc[2 * np + 1], yf[0], yf[2], yf[1], yf[3], b2, b3);
+        }
+        if (tid == 0) tc::bulk_wait_read<0>();      // the previous chunk's results have left the result tiles
+        __syncthreads();                            // nobody reads this chunk's tiles any more
+        // ---- epilogue
+        uint32_t rdr[4], rdk[4], rdw[4];
+        float dlw[2][4];
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+            float ea[2][2], z[2][2];                // [hh][column]: r dr', and r dr' - k dk'
+#pragma unroll
+            for (int hh = 0; hh < 2; ++hh) {
+                const int at = 2 * nt + hh, e0 = 2 * hh;
+                const float2 rv = unpack2(rw[at]), kv = unpack2(kw[at]);
+                const float drx = dR[nt][e0] * f2[at].x, dry = dR[nt][e0 + 1] * f2[at].y;
+                const float dkx = dK[nt][e0] * f3[at].x, dky = dK[nt][e0 + 1] * f3[at].y;
+                const float dux = dd[hh] * uu[2 * nt], duy = dd[hh] * uu[2 * nt + 1];
+                rdr[at] = pack2(fmaf(dux, kv.x, drx), fmaf(duy, kv.y, dry));
+                rdk[at] = pack2(fmaf(dux, rv.x, dkx), fmaf(duy, rv.y, dky));
+                ea[hh][0] = rv.x * drx;
+                ea[hh][1] = rv.y * dry;
+                z[hh][0] = ea[hh][0] - kv.x * dkx;
+                z[hh][1] = ea[hh][1] - kv.y * dky;
+                du_acc[2 * nt] = fmaf(dd[hh] * rv.x, kv.x, du_acc[2 * nt]);
+                du_acc[2 * nt + 1] = fmaf(dd[hh] * rv.y, kv.y, du_acc[2 * nt + 1]);
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                // sums over the tokens from each on (lanes g, g + 1, ..., 7 of both halves), and of `lump` over all lanes
+                float s0_ = z[0][e], s1 = z[1][e], l = lump[2 * nt + e];
+#pragma unroll
+                for (int d = 1; d < 8; d <<= 1) {
+                    const float a = __shfl_down_sync(0xffffffffu, s0_, 4 * d), b = __shfl_down_sync(0xffffffffu, s1, 4 * d);
+                    s0_ += g + d < 8 ? a : 0.f;
+                    s1 += g + d < 8 ? b : 0.f;
+                    l += __shfl_xor_sync(0xffffffffu, l, 4 * d);
+                }
+                s0_ += __shfl_sync(0xffffffffu, s1, q);        // the second half's total
+                dlw[nt][e] = s0_ - ea[0][e] + l;
+                dlw[nt][2 + e] = s1 - ea[1][e] + l;
             }
         }
-        __syncthreads();                                              // S4: nobody reads the operand tiles any more
-        // ---- epilogue: rows t = g, g + 8; column pairs i = j0 + 8 nt + 2 q, + 1
-        float (*ea)[EPITCH] = reinterpret_cast<float (*)[EPITCH]>(&sm.st[stage].s0[0][0][0]);
-        float (*eb)[EPITCH] = ea + kC6;
-        {
+        stmatrix_x4(sm.res[0] + tile_row, rdr[0], rdr[1], rdr[2], rdr[3]);
+        stmatrix_x4(sm.res[1] + tile_row, rdk[0], rdk[1], rdk[2], rdk[3]);
+        stmatrix_x4(sm.res[2] + tile_row, pack2(dV[0][0], dV[0][1]), pack2(dV[0][2], dV[0][3]), pack2(dV[1][0], dV[1][1]), pack2(dV[1][2], dV[1][3]));
 #pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                const int i = j0 + 8 * nt + 2 * q;
-                const float2 em2 = *reinterpret_cast<const float2*>(&sm.em[i]), ecm2 = *reinterpret_cast<const float2*>(&sm.ecm[i]);
-                float lump0 = 0.f, lump1 = 0.f;
-#pragma unroll
-                for (int hh = 0; hh < 2; ++hh) {       // the two token rows
-                    const int t = g + 8 * hh, e0 = 2 * hh;
-                    const float2 f2 = *reinterpret_cast<const float2*>(&sm.e2[t][i]), f3 = *reinterpret_cast<const float2*>(&sm.e3[t][i]);
-                    const float2 rv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.r[t][i]));
-                    const float2 kv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.k[t][i]));
-                    const float dd = hh ? dd_hi : dd_lo;
-                    const int sg = seg_r[hh];
-                    const float live = row_in[hh] ? 1.f : 0.f;
-                    const float m0 = sg == seg_in ? live : 0.f, mE = sg == seg_end ? live : 0.f;
-                    // x: column i, y: column i + 1
-                    const float drp_x = (m0 * dR0[nt][e0] * em2.x + dRt[nt][e0]) * f2.x, drp_y = (m0 * dR0[nt][e0 + 1] * em2.y + dRt[nt][e0 + 1]) * f2.y;
-                    const float khp_x = mE * dKh[nt][e0] * ecm2.x * f3.x, khp_y = mE * dKh[nt][e0 + 1] * ecm2.y * f3.y;
-                    const float dkp_x = fmaf(dKt[nt][e0], f3.x, khp_x), dkp_y = fmaf(dKt[nt][e0 + 1], f3.y, khp_y);
-                    *reinterpret_cast<uint32_t*>(&sm.ops[0][t][i]) = pack2(fmaf(dd * u_col[nt][0], kv.x, drp_x), fmaf(dd * u_col[nt][1], kv.y, drp_y));
-                    *reinterpret_cast<uint32_t*>(&sm.ops[1][t][i]) = pack2(fmaf(dd * u_col[nt][0], rv.x, dkp_x), fmaf(dd * u_col[nt][1], rv.y, dkp_y));
-                    *reinterpret_cast<uint32_t*>(&sm.ops[2][t][i]) = pack2(dV[nt][e0], dV[nt][e0 + 1]);   // dV: rows s = t, columns j = i
-                    *reinterpret_cast<float2*>(&ea[t][i]) = make_float2(rv.x * drp_x, rv.y * drp_y);
-                    *reinterpret_cast<float2*>(&eb[t][i]) = make_float2(kv.x * dkp_x, kv.y * dkp_y);
-                    lump0 = fmaf(kv.x, khp_x, lump0);
-                    lump1 = fmaf(kv.y, khp_y, lump1);
-                    du_acc[nt][0] = fmaf(live * dd * rv.x, kv.x, du_acc[nt][0]);
-                    du_acc[nt][1] = fmaf(live * dd * rv.y, kv.y, du_acc[nt][1]);
-                }
-#pragma unroll
-                for (int m = 4; m < 32; m <<= 1) {
-                    lump0 += __shfl_xor_sync(0xffffffffu, lump0, m);
-                    lump1 += __shfl_xor_sync(0xffffffffu, lump1, m);
-                }
-                if (g == 0) {
-                    const float2 wc2 = *reinterpret_cast<const float2*>(&sm.wc[i]);
-                    const float gx = sm.gw[0][i] + sm.gw[1][i] + sm.gw[2][i] + sm.gw[3][i];
-                    const float gy = sm.gw[0][i + 1] + sm.gw[1][i + 1] + sm.gw[2][i + 1] + sm.gw[3][i + 1];
-                    *reinterpret_cast<float2*>(&sm.lump[i]) = make_float2(fmaf(gx, wc2.x, lump0), fmaf(gy, wc2.y, lump1));
-                }
-            }
-        }
-        __syncthreads();                                              // S5
-        if (tid < kN) {
-            // suffix sums over the chunk's 16 positions: the log-decay of token tau acts on every cumulative sum c_x, x >= tau
-            float run2 = sm.lump[tid];
-#pragma unroll
-            for (int x = kC6 - 1; x >= 0; --x) {
-                run2 += (x + 1 < kC6 ? ea[x + 1][tid] : 0.f) - eb[x][tid];
-                if (w_per_token) sm.ops[3][x][tid] = __float2bfloat16_rn(run2);
-                else if (t0 + x < Tlen && x >= lo && x < hi) dw_acc += run2;
-            }
-        }
-        // the four result tiles leave after the next barrier (the top of the next walk, or the one behind the loop)
-        out_t0 = t0;
+        for (int at = 0; at < 4; ++at) rdw[at] = pack2(dlw[at >> 1][2 * (at & 1)], dlw[at >> 1][2 * (at & 1) + 1]);
+        stmatrix_x4(sm.res[3] + tile_row, rdw[0], rdw[1], rdw[2], rdw[3]);
+        out_t = t0;
         out_lo = lo;
         out_hi = hi;
     };
@@ -811,8 +894,10 @@ wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
             walk(std::false_type{}, c, it, 0);
         }
     }
+    tc::fence_async_smem();
     __syncthreads();
-    flush_results();
+    send_results();
+    if (tid == 0) tc::bulk_wait_read<0>();
     if (run == 0) {
         if (L == 0) add_ds_out();
 #pragma unroll
@@ -821,20 +906,17 @@ wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
             for (int e = 0; e < 4; ++e)
                 ds0[st_base + (size_t)(8 * ni + 2 * q + (e & 1)) * kN + j0 + g + 8 * (e >> 1)] = __float2bfloat16_rn(acc[ni][e]);
     }
-    // per-(batch, head) sums over tokens: directly, or this run's share for the reduction behind the kernel
-    float* const du_dst = n_runs == 1 ? du_head + (size_t)bh * kN : partial + ((size_t)bh * n_runs + run) * 2 * kN;
-    float* const dw_dst = n_runs == 1 ? (dw_head != nullptr ? dw_head + (size_t)bh * kN : nullptr) : du_dst + kN;
-    // du: sum over this thread's token rows, then over the eight row groups of the warp
+    // du of the (batch, head), or this run's share for the reduction behind the kernel: the sum over this thread's token rows,
+    // then over the eight row groups of the warp
+    float* const du_dst = n_runs == 1 ? du_head + (size_t)bh * kN : partial + ((size_t)bh * n_runs + run) * kN;
 #pragma unroll
-    for (int nt = 0; nt < 2; ++nt)
+    for (int e = 0; e < 4; ++e) {
+        float p = du_acc[e];
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            float p = du_acc[nt][e];
-#pragma unroll
-            for (int m = 4; m < 32; m <<= 1) p += __shfl_xor_sync(0xffffffffu, p, m);
-            if (g == 0) du_dst[j0 + 8 * nt + 2 * q + e] = p;
-        }
-    if (!w_per_token && tid < kN && dw_dst != nullptr) dw_dst[tid] = dw_acc / __bfloat162float(w[(size_t)h * kN + tid]);
+        for (int m = 4; m < 32; m <<= 1) p += __shfl_xor_sync(0xffffffffu, p, m);
+        if (g == 0) du_dst[j0 + 8 * (e >> 1) + 2 * q + (e & 1)] = p;
+    }
+    if (!waited && status != nullptr) atomicExch(status, 5);
 }
 
 // ------------------------------------------------------------------ the state-gradient carry
@@ -861,7 +943,7 @@ struct Carry6Smem {
 static_assert(4 * (sizeof(Carry6Smem) + 1024) <= 228 * 1024, "four CTAs per SM");
 
 __global__ void __launch_bounds__(128, 4)
-wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __restrict__ w, int w_per_token,
+wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __restrict__ w,
                       const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts, const bf* __restrict__ dy,
                       const bf* __restrict__ ds_out, const int* __restrict__ residual_mark, int n_runs, int run_len,
                       bf* __restrict__ dsck) {
@@ -897,7 +979,7 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
                 const bool ok = t < Tlen;
                 const size_t off = seq_base + (size_t)(ok ? t : 0) * tok_stride + piece;
                 cp_async16_zfill(&st.r[row][piece], r + off, ok);
-                if (w_per_token) cp_async16_zfill(&st.w[row][piece], w + off, ok);
+                cp_async16_zfill(&st.w[row][piece], w + off, ok);
                 cp_async16_zfill(&st.dy[row][piece], dy != nullptr ? dy + off : r + off, ok && dy != nullptr);
             }
         }
@@ -915,11 +997,6 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
     uint8_t ns_ahead = load_ns(nB - kCarryStages);
     // phase A ownership: the channel pair cp, cp + 1 and the kQT tokens of quarter qt
     const int cp = (tid & 31) * 2, qt = tid >> 5;
-    float2 lw_const = make_float2(0.f, 0.f);
-    if (!w_per_token) {
-        const float2 wv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(w + (size_t)h * kN + cp));
-        lw_const = make_float2(__logf(wv.x), __logf(wv.y));
-    }
 
     auto walk = [&](auto split_tag, const int c, const int part_arg) {
         constexpr bool kSplitHere = decltype(split_tag)::value;
@@ -961,8 +1038,7 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
         auto lw_of = [&](int tt) -> float2 {
             const int t = kQT * qt + tt;
             const bool ok = t0 + t < Tlen && t >= lo && t < hi;
-            return !ok ? make_float2(0.f, 0.f)
-                       : (w_per_token ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.w[t][cp])) : lw_const);
+            return ok ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.w[t][cp])) : make_float2(0.f, 0.f);
         };
         float2 run = make_float2(0.f, 0.f);
 #pragma unroll
@@ -1045,20 +1121,16 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
     cp_async_wait<0>();
 }
 
-// du (and the gradient of a constant decay) of a (batch, head): the runs' shares added in a fixed order
+// du of a (batch, head): the runs' shares added in a fixed order
 __global__ void wkv6_reduce_runs_kernel(int BH, int n_runs, const float* __restrict__ partial, const int* __restrict__ residual_mark,
-                                        float* __restrict__ du_head, float* __restrict__ dw_head) {
+                                        float* __restrict__ du_head) {
     if (*residual_mark != 0) return;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= BH * kN) return;
     const int bh = idx / kN, i = idx % kN;
-    float su = 0.f, sw = 0.f;
-    for (int rho = 0; rho < n_runs; ++rho) {
-        su += partial[((size_t)bh * n_runs + rho) * 2 * kN + i];
-        if (dw_head != nullptr) sw += partial[((size_t)bh * n_runs + rho) * 2 * kN + kN + i];
-    }
-    du_head[idx] = su;
-    if (dw_head != nullptr) dw_head[idx] = sw;
+    float sum = 0.f;
+    for (int rho = 0; rho < n_runs; ++rho) sum += partial[((size_t)bh * n_runs + rho) * kN + i];
+    du_head[idx] = sum;
 }
 
 }  // namespace
@@ -1070,15 +1142,16 @@ static int runs_of(int T) {
     return nC >= 2 * kRunLen ? (nC + kRunLen - 1) / kRunLen : 1;
 }
 struct Layout6 {
-    size_t states, dsck, partial, end;
+    size_t states, scores, dsck, partial, end;
 };
 static Layout6 layout6(int B, int T, int H) {
     const size_t nC = (size_t)(T + kC6 - 1) / kC6, runs = (size_t)runs_of(T), tile = (size_t)kN * kN * sizeof(bf);
     Layout6 l;
     l.states = 0;                                              // every chunk's entering state, and the second part of a split one
-    l.dsck = l.states + (size_t)B * H * (nC + 1) * tile;       // the state gradient at the end of every run (written by the backward)
-    l.partial = l.dsck + (size_t)B * H * runs * tile;          // the runs' shares of du and of a constant decay's gradient (fp32)
-    l.end = l.partial + (size_t)B * H * runs * 2 * kN * sizeof(float);
+    l.scores = l.states + (size_t)B * H * (nC + 1) * tile;     // its score block A^T (512 bytes)
+    l.dsck = l.scores + (size_t)B * H * (nC + 1) * 32 * sizeof(uint4);   // the state gradient at the end of every run (written by the backward)
+    l.partial = l.dsck + (size_t)B * H * runs * tile;          // the runs' shares of du (fp32)
+    l.end = l.partial + (size_t)B * H * runs * kN * sizeof(float);
     return l;
 }
 
@@ -1092,14 +1165,18 @@ int wkv6_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
         return B200WKV_ELAUNCH;
     *flag = wkv_call_flag(ticket);
     if (*flag == nullptr) return B200WKV_ELAUNCH;
+    const void* streams[5] = {r, k, v, per_token ? w : nullptr, y};
+    SeqMaps maps;
+    if (!make_seq_maps(&maps, streams, 5, B, T, H, kC6)) return B200WKV_ELAUNCH;
     wkv6_chunk_fwd_kernel<<<B * H, 128, sizeof(Fwd6cSmem), st>>>(T, H, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, per_token,
                                                                 (const bf*)u, (const bf*)s0, length, ns, (bf*)y, (bf*)s_out,
-                                                                (bf*)residual, *flag, *ticket, residual_mark);
+                                                                (bf*)residual,
+                                                                residual != nullptr ? reinterpret_cast<uint4*>(static_cast<char*>(residual) + layout6(B, T, H).scores) : nullptr, *flag, *ticket, residual_mark, maps);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 int wkv6_chunk_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w,
-                   int per_token, const void* u, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out,
+                   const void* u, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out,
                    void* residual, const int* residual_mark, void* dr, void* dk, void* dv, void* dw, void* du, void* ds0) {
     static DeviceOnce smem_attr;
     if (!smem_attr.ok([]() {
@@ -1113,20 +1190,20 @@ int wkv6_chunk_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
     const int n_runs = runs_of(T);
     bf* dsck = reinterpret_cast<bf*>(base + lay.dsck);
     float* partial = reinterpret_cast<float*>(base + lay.partial);
-    float* dw_head = per_token ? nullptr : (float*)dw;
     if (n_runs > 1) {
-        wkv6_carry_bwd_kernel<<<B * H, 128, sizeof(Carry6Smem), st>>>(T, H, (const bf*)r, (const bf*)w, per_token, length, ns, (const bf*)dy,
+        wkv6_carry_bwd_kernel<<<B * H, 128, sizeof(Carry6Smem), st>>>(T, H, (const bf*)r, (const bf*)w, length, ns, (const bf*)dy,
                                                                      (const bf*)ds_out, residual_mark, n_runs, kRunLen, dsck);
         if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
     }
+    const void* streams[9] = {r, k, v, w, dy, dr, dk, dv, dw};
+    SeqMaps maps;
+    if (!make_seq_maps(&maps, streams, 9, B, T, H, kC6)) return B200WKV_ELAUNCH;
     wkv6_chunk_bwd_kernel<<<B * H * n_runs, 128, sizeof(Bwd6cSmem), st>>>(
-        T, H, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, per_token, (const bf*)u, length, ns, (const bf*)dy,
-        (const bf*)ds_out, (const bf*)(base + lay.states), residual_mark, (bf*)dr, (bf*)dk, (bf*)dv, per_token ? (bf*)dw : nullptr,
-        dw_head, (float*)du, (bf*)ds0, n_runs, n_runs > 1 ? kRunLen : (T + kC6 - 1) / kC6, dsck, partial);
+        T, H, (const bf*)u, length, ns, dy != nullptr ? 1 : 0, (const bf*)ds_out, (const bf*)(base + lay.states), (const uint4*)(base + lay.scores), residual_mark, (bf*)dr, (bf*)dk, (bf*)dv, (bf*)dw, (float*)du, (bf*)ds0, n_runs, n_runs > 1 ? kRunLen : (T + kC6 - 1) / kC6, dsck, partial, wkv7_chunk_status_word(), maps);
     if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
     if (n_runs > 1) {
         const int total = B * H * kN;
-        wkv6_reduce_runs_kernel<<<(total + 255) / 256, 256, 0, st>>>(B * H, n_runs, partial, residual_mark, (float*)du, dw_head);
+        wkv6_reduce_runs_kernel<<<(total + 255) / 256, 256, 0, st>>>(B * H, n_runs, partial, residual_mark, (float*)du);
         if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
     }
     return B200WKV_OK;
