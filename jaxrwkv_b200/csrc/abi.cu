@@ -25,7 +25,7 @@ int wkv7_step_stream(cudaStream_t st, int dtype, int B, int H, const void* w, co
 size_t wkv7_chunk_residual_bytes(int B, int T, int H);
 int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v,
                    const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
-                   void* s_out, void* residual, int* residual_mark, int** range_flag, int* range_ticket);
+                   void* s_out, void* residual, void* workspace, int* residual_mark, int** range_flag, int* range_ticket);
 int wkv7_carry_bwd(cudaStream_t st, int B, int T, int H, const uint32_t* length, const void* dy,
                    const void* ds_out, void* residual, const int* residual_mark, void* ds0);
 int wkv7_grad_bwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v,
@@ -85,6 +85,30 @@ static int check_dims(int dtype, int B, int T, int H, int N) {
     if ((long long)B * H > 2147483647LL || (long long)B * T > 2147483647LL) return B200WKV_ESHAPE;   // token rows index tensor maps
     return B200WKV_OK;
 }
+
+int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k, const void* v,
+             const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
+             void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace) {
+    int st = check_dims(dtype, B, T, H, N);
+    if (st != B200WKV_OK) return st;
+    if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
+    if (residual != nullptr && residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
+    // one token and no residual wanted (recurrent decoding): a single pass over the state
+    if (T == 1 && residual == nullptr)
+        return wkv7_step((cudaStream_t)stream, dtype, B, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out);
+    if (dtype == B200WKV_BF16 && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
+        int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
+        int *range_flag = nullptr, ticket = 0;
+        st = wkv7_chunk_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, workspace, mark,
+                            &range_flag, &ticket);
+        if (st != B200WKV_OK) return st;
+        // does nothing unless the kernel above met a decay outside its range and left its ticket
+        return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual,
+                            range_flag, ticket, mark);
+    }
+    return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out,
+                        residual, nullptr, 0, nullptr);
+}
 }  // namespace b200wkv
 
 using namespace b200wkv;
@@ -126,25 +150,7 @@ int b200wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void
                  const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
                  const uint8_t* new_starts, void* y, void* s_out, void* residual, size_t residual_bytes,
                  unsigned flags) {
-    int st = check_dims(dtype, B, T, H, N);
-    if (st != B200WKV_OK) return st;
-    if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
-    if (residual != nullptr && residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
-    // one token and no residual wanted (recurrent decoding): a single pass over the state
-    if (T == 1 && residual == nullptr)
-        return wkv7_step((cudaStream_t)stream, dtype, B, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out);
-    if (dtype == B200WKV_BF16 && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
-        int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
-        int *range_flag = nullptr, ticket = 0;
-        st = wkv7_chunk_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, mark,
-                            &range_flag, &ticket);
-        if (st != B200WKV_OK) return st;
-        // does nothing unless the kernel above met a decay outside its range and left its ticket
-        return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual,
-                            range_flag, ticket, mark);
-    }
-    return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out,
-                        residual, nullptr, 0, nullptr);
+    return b200wkv::wkv7_fwd(stream, dtype, B, T, H, N, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, residual_bytes, flags, nullptr);
 }
 
 int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k,

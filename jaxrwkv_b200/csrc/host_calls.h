@@ -6,6 +6,12 @@
 
 namespace b200wkv {
 
+// b200wkv7_fwd with a workspace of wkv7_blocks_bytes() (0: the call wants none, workspace NULL).
+size_t wkv7_blocks_bytes(int B, int T, int H, bool residual);
+int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k, const void* v,
+             const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
+             void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace);
+
 // RWKV-4 with the receptance product inside (y = r * wkv; r NULL: without) and, with `raw_w`, the decay parameter w
 // before -exp().  The backward writes dr when r is given, and per-sequence sums of dw' and du (B, C).
 int wkv4_fwd(cudaStream_t st, int dtype, int B, int T, int C, bool raw_w, const void* w, const void* u, const void* r, const void* k,

@@ -151,6 +151,15 @@ variable_list gradients_of(AutogradContext* ctx, const variable_list& grads) {
 
 // ------------------------------------------------------------------------------------------------- RWKV-7
 // Streams (lead, T, H, N), state (lead, H, N, N), any number of leading batch axes.
+// the workspace of a forward call over few sequences (NULL: it wants none); `scratch` keeps it until the call is enqueued
+static void* wkv7_workspace(Tensor& scratch, const Tensor& like, int B, int T, int H, int N, bool residual) {
+    if (like.scalar_type() != at::kBFloat16 || N != 64 || B < 1 || T < 2 || H < 1) return nullptr;
+    const size_t n = b200wkv::wkv7_blocks_bytes(B, T, H, residual);
+    if (n == 0) return nullptr;
+    scratch = bytes(n, like);
+    return out(scratch);
+}
+
 struct Wkv7 {
     static constexpr const char* kName = "wkv7";
     static constexpr int kIn = 7;                 // r w k v a b s
@@ -173,9 +182,11 @@ struct Wkv7 {
         Tensor y = fresh_like(k), s_out = fresh_like(t[6]);
         const size_t rbytes = residual ? b200wkv7_residual_bytes(dtype_code(k), B, T, H, N) : 0;
         if (residual) *residual = bytes(rbytes, k);
-        check(b200wkv7_fwd(stream_of(k), dtype_code(k), B, T, H, N, in(c[1]), in(c[0]), in(c[2]), in(c[3]), in(c[4]), in(c[5]),
+        Tensor scratch;
+        void* const ws = wkv7_workspace(scratch, k, B, T, H, N, residual != nullptr);
+        check(b200wkv::wkv7_fwd(stream_of(k), dtype_code(k), B, T, H, N, in(c[1]), in(c[0]), in(c[2]), in(c[3]), in(c[4]), in(c[5]),
                            in(c[6]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), out(y), out(s_out),
-                           residual ? out(*residual) : nullptr, rbytes, 0));
+                           residual ? out(*residual) : nullptr, rbytes, 0, ws));
         return {s_out, y};
     }
     // saved: the seven operands, length, new_starts, residual; grads: of the returned state and of the output
@@ -649,8 +660,10 @@ struct Layer {
                                    in(p[kA0]), in(p[kV0]), in(p[kKk]), in(p[kKa]), q.w, q.kp, q.vp, q.ai, q.bi));
         const size_t rbytes = residual ? b200wkv7_residual_bytes(code, B, T, H, (int)kN) : 0;
         if (residual) kept.residual = bytes(rbytes, x);
-        check(b200wkv7_fwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(f.length),
-                           (const uint8_t*)in(f.starts), q.y, s_out.p, out(kept.residual), rbytes, 0));
+        Tensor scratch;
+        void* const ws = wkv7_workspace(scratch, x, B, T, H, (int)kN, residual);
+        check(b200wkv::wkv7_fwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(f.length),
+                           (const uint8_t*)in(f.starts), q.y, s_out.p, out(kept.residual), rbytes, 0, ws));
         s_out.finish(st);
         check(b200wkv7_mix_post_fwd(st, code, d.rows, H, (int)kN, kEps, q.y, q.r, q.kp, q.vp, q.g, in(p[kLnW]), in(p[kLnB]), in(p[kRk]), q.xo));
         gemm.nt(d.rows, d.C, d.C, q.xo, in(p[kWo]), out(o));

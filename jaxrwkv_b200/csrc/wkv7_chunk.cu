@@ -34,6 +34,7 @@
 #include "tc05.cuh"
 #include "chunk_common.cuh"
 #include "tmap.cuh"
+#include "wkv7_blocks.h"
 
 #include <atomic>
 
@@ -93,10 +94,20 @@ __device__ __forceinline__ void mma_k64(uint32_t d, Op a, Op b, uint32_t idesc, 
 __device__ int g_status;  // last device-side error (0 = none); see wkv7_chunk_status()
 
 
+// 32 columns of one row of an fp32 tile [16 column pieces][64 rows] (of four columns): a warp's rows are contiguous
+__device__ __forceinline__ void store_part(float4* tiles, size_t slot, int hsel, int row, const float* x) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) tiles[slot * 1024 + (hsel * 8 + c) * 64 + row] = make_float4(x[c * 4], x[c * 4 + 1], x[c * 4 + 2], x[c * 4 + 3]);
+}
+
+// kBlocks: the blocks of all sequences as one list, each from a zero state; a CTA walks consecutive ones, and what depends on
+// the entering state is left to the kernels of wkv7_blocks.cu.  Otherwise a CTA walks one sequence (or piece of one).
+//
 // 256 threads: warp = (quad, hsel); quad selects the 32 TMEM lanes (tile rows) the warp may access,
 // hsel the column half it works on, so every accumulator tile is shared by two warps per row group.
+template <bool kBlocks>
 __global__ void __launch_bounds__(256, 2)
-wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ r,
+wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ r,
                       const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
                       const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
                       const __nv_bfloat16* __restrict__ s0, const uint32_t* __restrict__ length,
@@ -105,23 +116,31 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                       const __grid_constant__ StreamMaps maps, const __grid_constant__ CUtensorMap y_map, const __grid_constant__ CUtensorMap rbar_map,
                       unsigned char* __restrict__ saved,
                       int* __restrict__ range_flag, int range_ticket, int* __restrict__ residual_mark,
-                      __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces) {
+                      __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces,
+                      const BlockParts parts) {
     extern __shared__ __align__(1024) unsigned char smem[];   // (the swizzle of the output tile is a function of the address)
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     // (all first pieces come first in the grid: where no cut exists the other pieces' CTAs return at once, and the
     // CTAs that do the work are then spread over the SMs before any SM takes a second one)
-    const int n_seq = (int)gridDim.x / pieces;
-    const int bh = blockIdx.x % n_seq, piece = blockIdx.x / n_seq, bi = bh / H, h = bh % H;
+    const int nSlot = block_slots(Tlen);
+    // blocks [unit, unit_end) of the list are this CTA's
+    const int units = kBlocks ? n_seq * (nSlot - 1) : 0;
+    int unit = kBlocks ? (int)((long long)units * blockIdx.x / gridDim.x) : 0;
+    const int unit_end = kBlocks ? (int)((long long)units * (blockIdx.x + 1) / gridDim.x) : 0;
+    int bh = kBlocks ? unit / (nSlot - 1) : blockIdx.x % n_seq;
+    const int piece = kBlocks ? 0 : blockIdx.x / n_seq;
+    int bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, hsel = warp >> 2;
     const int row = quad * 32 + lane;
-    const int L = min((int)length[bi], Tlen);
+    int L = min((int)length[bi], Tlen);
     // ---- sequence-parallel mode (pieces > 1, calls without a residual): a start flag cuts every dependence, so a
     // sequence may be walked as independent pieces whose first token carries a start flag.  Cut k, k = 1..pieces-1,
     // is the start flag nearest to k T / pieces within half a piece of it, if there is one; every CTA of the
     // sequence finds the same cuts by itself, a CTA whose own cut does not exist has nothing to do.
     int t_begin = 0, t_end = Tlen;
-    if (pieces > 1) {
+    if (kBlocks) t_begin = (unit - bh * (nSlot - 1)) * kC;
+    if (!kBlocks && pieces > 1) {
         const uint8_t* ns_row = new_starts + (size_t)bi * Tlen;
         const int half = Tlen / (2 * pieces);
         auto find_cut = [&](int k) -> int {       // position of cut k, or -1; all threads of the CTA take part
@@ -147,15 +166,14 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         __syncthreads();
     }
     const size_t tok_stride = (size_t)H * kN;
-    const size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
+    size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
     const size_t st_row = ((size_t)bh * kN + (row & 63)) * kN + hsel * 32;  // this thread's 32 state elements
-    const int nSlot = block_slots(Tlen);
 
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < 5; ++i) tc::mbar_init(&sm.bar[i], (i == 2 || i == 3) ? 2 : 1);   // M3, M4: two issuing threads
         tc::mbar_init_fence();
-        if (bh == 0 && residual_mark != nullptr) *residual_mark = 0;   // this residual is in the chunked format (so far)
+        if (blockIdx.x == 0 && residual_mark != nullptr) *residual_mark = 0;   // this residual is in the chunked format (so far)
     }
     if (warp == 0) tc::tmem_alloc(&sm.tmem, 256);
     tc::fence_before_sync();
@@ -167,7 +185,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
     bool failed = false;
 
     // ---- state into TMEM (rows 0..63 = S0 in fp32, rows 64..127 are never read) --------------
-    {
+    if (!kBlocks) {
         float s[32];
         if (row < 64 && t_begin == 0) {
 #pragma unroll
@@ -218,18 +236,18 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
     uint8_t flag_ahead = (tid < 64 && t_begin + tid < Tlen) ? new_starts[(size_t)bi * Tlen + t_begin + tid] : 0;
     // the 64 token rows from cp on of w, r, k, v, a, b into the staging tiles (thread 0; one tiled copy
     // per stream).  Rows past the chunk arrive too and are ignored.
-    auto issue_stage = [&](int cp) {
+    auto issue_stage = [&](int cbi, int ch, int cp) {
         if (tid == 0) {
             tc::mbar_expect_tx(&sm.bar[4], (uint32_t)(6 * STG_TILE));
 #pragma unroll
-            for (int m = 0; m < 6; ++m) tc::tensor_load_2d(smem + stage_off(m), &maps.m[m], h * kN, bi * Tlen + cp, &sm.bar[4]);
+            for (int m = 0; m < 6; ++m) tc::tensor_load_2d(smem + stage_off(m), &maps.m[m], ch * kN, cbi * Tlen + cp, &sm.bar[4]);
         }
     };
-    issue_stage(t_begin);
+    issue_stage(bi, h, t_begin);
     while (true) {
         // ================= boundary at position p: TMEM holds the state after token p-1 =================
         // (of the pieces of a sequence, the one that has walked token L - 1 holds it; L == 0: the first)
-        const bool want_out = (p == L) && (p > t_begin || t_begin == 0);
+        const bool want_out = !kBlocks && (p == L) && (p > t_begin || t_begin == 0);
         if (quad < 2 && want_out) {
             float s[32];
             tc::tmem_ld32(lane_addr + DS + hsel * 32, s);
@@ -242,11 +260,15 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                     *reinterpret_cast<float4*>(s_at_len + st_row + c * 4) = make_float4(s[c * 4], s[c * 4 + 1], s[c * 4 + 2], s[c * 4 + 3]);
             }
         }
-        if (p >= t_end) break;
+        if (kBlocks ? unit >= unit_end : p >= t_end) break;
         // ================= extent of this chunk =================
         // (with a residual the chunks are the 64-token blocks of the sequence, so that the backward can number them)
-        const int be = min(saved != nullptr ? ((p >> 6) + 1) << 6 : p + kC, t_end);
+        const int be = min(kBlocks || saved != nullptr ? ((p >> 6) + 1) << 6 : p + kC, t_end);
         const int p1 = L > p && L < be ? L : be, n = p1 - p;
+        // what is walked next: the second part of this block, the next block, or the first of the next sequence
+        const bool next_seq = kBlocks && p1 == Tlen;
+        const bool more = kBlocks ? p1 < be || unit + 1 < unit_end : p1 < t_end;
+        const int np = next_seq ? 0 : p1, nh = next_seq ? (h + 1 == H ? 0 : h + 1) : h, nbi = next_seq && h + 1 == H ? bi + 1 : bi;
         if (tid < 64) {
             // the flag byte of position p + tid was requested while the previous chunk's products ran
             const bool f = tid < n && flag_ahead != 0;
@@ -263,6 +285,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         // the second part of a block that `length` cuts (the only chunk that starts inside a block)
         const size_t blk_slot = (size_t)bh * nSlot + ((p & (kC - 1)) == 0 ? p >> 6 : nSlot - 1);
         unsigned char* const keep = saved != nullptr ? saved + blk_slot * kSavedBytes : nullptr;
+        const bool affine = kBlocks || keep != nullptr;   // M', R- and L_C are wanted
         // ================= stage inputs (registers), log-decay into the scan buffer =================
         uint4 raw[2][5];   // r, k, v, a, b
         float lw[2][8];    // log2 of the decay: -exp(w) * log2(e)
@@ -343,7 +366,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 const uint4 a_t = scale8(raw[q][3], eP), r_t = scale8(raw[q][0], eL);
                 slab_store(smem + OFF_AR, CB128, t, jb, a_t);
                 slab_store(smem + OFF_AR, CB128, 64 + t, jb, r_t);
-                if (keep != nullptr) {
+                if (affine) {
                     // W~ = T A~ is formed after the inverse, when the [A~ ; R~] slab has long been written over:
                     // a second copy of A~ waits in the sa slab, which is idle until sa itself is stored; R~ goes
                     // to the R- rows in global memory, where P_rb W~ is added at the end of the chunk
@@ -362,7 +385,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 for (int q = 0; q < 2; ++q) {
                     const int t = q * 32 + tsub;
                     const uint4 none = make_uint4(0, 0, 0, 0);
-                    if (keep != nullptr && !in_first(t)) {   // what carries the dependence on S0: nothing from the first flag on
+                    if (affine && !in_first(t)) {   // what carries the dependence on S0: nothing from the first flag on
                         slab_store(smem + OFF_SA, CB64, t, jb, none);
                         if (t < n) *reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + jb * 8) = none;
                         tc::fence_async_global();
@@ -375,7 +398,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             }
         }
         // ================= entering state: bf16 copy for the products, decayed fp32 copy back to TMEM =====
-        if (quad < 2) {
+        if (!kBlocks && quad < 2) {
             float s[32];
             if (reset_here) {
 #pragma unroll
@@ -405,14 +428,14 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         if (tid == 0) {
             tc::fence_after_sync();
             mma_k64(tbase + D1, kmaj128(sAR), kmaj128(sBK), ID_128x128_KK, false);
-            mma_k64(tbase + D2, kmaj128(sAR), kmaj64(sS0), ID_128x64_KK, false);
+            if (!kBlocks) mma_k64(tbase + D2, kmaj128(sAR), kmaj64(sS0), ID_128x64_KK, false);
             tc::commit(&sm.bar[0]);
         }
-        if (keep != nullptr && warp == 7 && lane < 8) {   // the bf16 entering state goes to the residual as it is
+        if (!kBlocks && keep != nullptr && warp == 7 && lane < 8) {   // the bf16 entering state goes to the residual as it is
             tc::bulk_store(keep + (size_t)SAVED_S0 * GTILE + lane * GCB, smem + OFF_S0 + lane * CB64, 64 * 16);
             tc::bulk_commit();
         }
-        if (keep != nullptr && tid < 64) lam_out[blk_slot * kN + tid] = mask != 0 ? 0.f : sm.lam[tid];
+        if (affine && tid < 64) lam_out[blk_slot * kN + tid] = mask != 0 ? 0.f : sm.lam[tid];
         if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
         tc::fence_after_sync();
         // ================= E1: triangular masks, operands of the next products =================
@@ -444,7 +467,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 for (int c = 0; c < 8; ++c) slab_store(dst, CB128, row, c, pack8(&d[c * 8]));
             }
         }
-        if (inner) {                              // A~ S0^T and R~ S0^T: nothing from the first flag on
+        if (!kBlocks && inner) {                  // A~ S0^T and R~ S0^T: nothing from the first flag on
             float g[32];
             tc::tmem_ld32(lane_addr + D2 + hsel * 32, g);
             tc::tmem_wait_ld();
@@ -461,7 +484,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         // ================= M2: G += A_ak V, Ypart += P_rk V ; meanwhile the triangular inverse =================
         if (tid == 0) {
             tc::fence_after_sync();
-            mma_k64(tbase + D2, kmaj128(sM2A), mnmaj64(sV), ID_128x64_KM, true);
+            mma_k64(tbase + D2, kmaj128(sM2A), mnmaj64(sV), ID_128x64_KM, !kBlocks);
             tc::commit(&sm.bar[1]);
         }
         // A_ak, P_rk and P_rb leave for the residual as bulk copies out of their slabs (one 64-row column
@@ -499,12 +522,13 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             tc::commit(&sm.bar[2]);
         } else if (tid == kIssuer2) {   // what only the backward's carry needs is issued by a second thread
             tc::fence_after_sync();
-            if (keep != nullptr) mma_k64(tbase + D1 + 64, kmaj128(sTP), mnmaj64(sSA), ID_128x64_KM, false);   // W~ = Tinv A~
+            if (affine) mma_k64(tbase + D1 + 64, kmaj128(sTP), mnmaj64(sSA), ID_128x64_KM, false);   // W~ = Tinv A~
             tc::commit(&sm.bar[2]);
         }
         // the rows of the next chunk start travelling: their tiles lie over buffers that are idle from
         // here to the next chunk's operand stores (the inverse and the A_ak / P_rk product are done)
-        if (p1 < t_end) issue_stage(p1);
+        if (more) issue_stage(nbi, nh, np);
+        const int nL = next_seq && more ? min((int)length[nbi], Tlen) : L;
         if (quad < 2) {
             if (!tc::mbar_wait(&sm.bar[2], par)) failed = true;
             tc::fence_after_sync();
@@ -513,17 +537,22 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             tc::tmem_wait_ld();
 #pragma unroll
             for (int c = 0; c < 4; ++c) slab_store(smem + OFF_SA, CB64, row, hsel * 4 + c, pack8(&sa[c * 8]));
-            if (keep != nullptr) {
+            if (kBlocks && keep != nullptr) store_part(parts.sa, blk_slot, hsel, row, sa);
+            if (affine) {
                 tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, sa);
                 tc::tmem_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 4; ++c) slab_store(smem + OFF_G, CB64, row, hsel * 4 + c, pack8(&sa[c * 8]));
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 w16 = pack8(&sa[c * 8]);
+                    slab_store(smem + OFF_G, CB64, row, hsel * 4 + c, w16);
+                    if (kBlocks && keep != nullptr) parts.w_tilde[blk_slot * 512 + (hsel * 4 + c) * 64 + row] = w16;
+                }
             }
         }
         tc::fence_async_smem();
         tc::fence_before_sync();
         __syncthreads();
-        if (keep != nullptr && warp == 7 && lane < 8) {   // sa
+        if (!kBlocks && keep != nullptr && warp == 7 && lane < 8) {   // sa
             tc::bulk_store(keep + (size_t)SAVED_SA * GTILE + lane * GCB, smem + OFF_SA + lane * CB64, 64 * 16);
             tc::bulk_commit();
         }
@@ -531,12 +560,12 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
         if (tid == 0) {
             tc::fence_after_sync();
             mma_k64(tbase + D2, kmaj128(sTP), mnmaj64(sSA), ID_128x64_KM, true);
-            mma_k64(tbase + DS, mnmaj64(sSA), mnmaj64(sBH), ID_128x64_MM, true);
+            mma_k64(tbase + DS, mnmaj64(sSA), mnmaj64(sBH), ID_128x64_MM, !kBlocks);
             mma_k64(tbase + DS, mnmaj64(sV), mnmaj64(sKH), ID_128x64_MM, true);
             tc::commit(&sm.bar[3]);
         } else if (tid == kIssuer2) {
             tc::fence_after_sync();
-            if (keep != nullptr) {
+            if (affine) {
                 // the transition's off-diagonal part M' = W~^T B^ (rows 0..63 of the accumulator are used) and
                 // the state-dependent part of the outputs, P_rb W~ (rows 64..127)
                 mma_k64(tbase + D1, mnmaj64(sG), mnmaj64(sBH), ID_128x64_MM, false);
@@ -544,9 +573,49 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
             }
             tc::commit(&sm.bar[3]);
         }
-        if (tid < 64) flag_ahead = (p1 + tid < Tlen) ? new_starts[(size_t)bi * Tlen + p1 + tid] : 0;   // next chunk's start flags
+        if (tid < 64) flag_ahead = (more && np + tid < Tlen) ? new_starts[(size_t)nbi * Tlen + np + tid] : 0;   // next chunk's start flags
         if (!tc::mbar_wait(&sm.bar[3], par)) failed = true;
         tc::fence_after_sync();
+        if constexpr (kBlocks) {
+            float x[32];
+            if (quad < 2) {
+                tc::tmem_ld32(lane_addr + DS + hsel * 32, x);
+                tc::tmem_wait_ld();
+                store_part(parts.state, blk_slot, hsel, row, x);
+                tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);          // M'[j][j'], row j = this thread's lane, as high + low parts
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 high = pack8(&x[c * 8]);
+                    float hf[8];
+                    unpack8(high, hf);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) hf[e] = x[c * 8 + e] - hf[e];
+                    const size_t at = blk_slot * 512 + (hsel * 4 + c) * 64 + row;
+                    reinterpret_cast<uint4*>(mprime)[at] = high;
+                    parts.m_low[at] = pack8(hf);
+                }
+            } else {
+                const int t = row - 64;
+                uint4* const to = reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + min(t, n - 1)) * tok_stride + hsel * 32);
+                uint4 rt[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) rt[c] = to[c];             // R~, stored when the operands were scaled
+                tc::tmem_ld32(lane_addr + D2 + hsel * 32, x);
+                tc::tmem_wait_ld();
+                store_part(parts.out, blk_slot, hsel, t, x);
+                tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, x);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float rf[8];
+                    unpack8(rt[c], rf);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) rf[e] += x[c * 8 + e];
+                    if (t < n) to[c] = pack8(rf);
+                }
+            }
+        } else {
         if (quad >= 2) {
             const int t = row - 64;
             float yv[32];
@@ -595,10 +664,21 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, const __nv_bfloat16* __restrict__ w, cons
                 }
             }
         }
+        }
         tc::fence_async_smem();   // the result tiles are read by bulk copies
         tc::fence_before_sync();
         if (warp == 7) tc::bulk_wait_read<0>();   // the slabs copied out may be rewritten after the next barrier
-        p = p1;
+        p = np;
+        if (kBlocks) {
+            if (p1 == be) ++unit;
+            if (next_seq) {
+                ++bh;
+                bi = nbi;
+                h = nh;
+                L = nL;
+                seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
+            }
+        }
         par ^= 1u;
     }
     __syncthreads();
@@ -644,12 +724,34 @@ int* wkv_call_flag(int* ticket) {
     return ring + (t & 63u);
 }
 
+// The rule between the two forms, as the bytes of workspace that the block-parallel one wants (0: the sequential walk).
+// Walking a sequence takes 6.6 us per block whatever else runs, up to one sequence per SM; side by side, a block costs 0.04 us
+// of the device and a step of the chain 1.2-1.5 us, and two more launches and the workspace some 10 us of host time.  Measured
+// (us, walk / side by side, forward of BH sequences without start flags): T=256: 37 / 36 at BH=40, 39 / 48 at 96; T=1024:
+// 118 / 75 at 40, 119 / 92 at 64, 123 / 116 at 96; T=4096: 435 / 208 at 40, 437 / 265 at 64.  So: from four blocks on, up to
+// half a sequence per SM.  With a residual up to two thirds of one in long sequences (BH=96: 243 / 227 at T=2048, 464 / 409
+// at 4096).  Without one, the walk is cut at start flags where there are any, and then wins where there are many blocks
+// (a flag every 256 tokens: 156 / 138 at BH=64, T=2048; 163 / 164 at 40, 181 / 227 at 64, T=4096): up to nine blocks per CTA
+// slot.  The last limit bounds the workspace, 2 GiB.
+size_t wkv7_blocks_bytes(int B, int T, int H, bool residual) {
+    const long long sms = sm_count_of_current_device(), seqs = (long long)B * H, blocks = block_slots(T) - 1;
+    if (blocks < 4 || blocks >= 65536) return 0;
+    if (2 * seqs > sms && !(residual && blocks >= 24 && 3 * seqs <= 2 * sms)) return 0;
+    if (!residual && seqs * blocks > 9 * 2 * sms) return 0;
+    const size_t bytes = blocks_layout(B, T, H, residual).end;
+    return bytes <= ((size_t)2 << 30) ? bytes : 0;
+}
+
 int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v,
                    const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
-                   void* s_out, void* residual, int* residual_mark, int** range_flag, int* range_ticket) {
+                   void* s_out, void* residual, void* workspace, int* residual_mark, int** range_flag, int* range_ticket) {
     typedef __nv_bfloat16 bf;
     static DeviceOnce smem_attr;   // the opt-in to large dynamic shared memory is a per-device function attribute
-    if (!smem_attr.ok([]() { return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES); }))
+    if (!smem_attr.ok([]() {
+            const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+            if (e != cudaSuccess) return e;
+            return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        }))
         return B200WKV_ELAUNCH;
     *range_flag = wkv_call_flag(range_ticket);
     if (*range_flag == nullptr) return B200WKV_ELAUNCH;
@@ -661,6 +763,25 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
     StreamMaps out_maps;                         // m[0]: the outputs, with the 128-byte swizzle of the kernel's output tile
     const void* out_bases[2] = {y, residual ? (const void*)((char*)residual + lay.rbar) : y};   // m[1]: the R- rows
     if (!make_stream_maps(&out_maps, out_bases, 2, B, T, H, /*swizzle128=*/true)) return B200WKV_ELAUNCH;
+    if (workspace != nullptr) {   // the blocks side by side (see wkv7_blocks_bytes)
+        const BlocksLayout bl = blocks_layout(B, T, H, residual != nullptr);
+        char* const ws = static_cast<char*>(workspace);
+        BlocksCall c;
+        c.parts = BlockParts{(float4*)(ws + bl.state), (float4*)(ws + bl.out), (float4*)(ws + bl.sa), (uint4*)(ws + bl.m_low), (uint4*)(ws + bl.w_tilde)};
+        c.saved = residual ? (unsigned char*)(base + lay.saved) : nullptr;
+        c.mprime = residual ? (bf*)(base + lay.mprime) : (bf*)(ws + bl.mprime);
+        c.rbar = residual ? (bf*)(base + lay.rbar) : (bf*)(ws + bl.rbar);
+        c.lam = residual ? (float*)(base + lay.lam) : (float*)(ws + bl.lam);
+        c.s0_tiles = residual ? c.saved + (size_t)SAVED_S0 * GTILE : (unsigned char*)(ws + bl.s0);
+        c.s0_stride = residual ? kSavedBytes : (size_t)GTILE;
+        const long long units = (long long)B * H * (block_slots(T) - 1), slots = 2LL * sm_count_of_current_device();
+        wkv7_chunk_fwd_kernel<true><<<(int)(units < slots ? units : slots), 256, SMEM_BYTES, st>>>(
+            T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a, (const bf*)b, (const bf*)s0, length, ns, (bf*)y,
+            (bf*)s_out, nullptr, maps, out_maps.m[0], out_maps.m[1], c.saved, *range_flag, *range_ticket, residual_mark, c.mprime, c.rbar, c.lam, 1,
+            c.parts);
+        if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
+        return wkv7_blocks_finish(st, B, T, H, length, ns, s0, c, y, s_out, residual ? (float*)(base + lay.s_at_len) : nullptr);
+    }
     // Without a residual (inference) and with fewer sequences than CTA slots, every sequence is offered to several
     // CTAs, which cut it at start flags where there are any (see the kernel): at most 8 pieces of at least 128 tokens.
     int pieces = 1;
@@ -672,7 +793,7 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
         if (pieces > T / 128) pieces = T / 128;
         if (pieces < 1 || T / pieces >= 32768) pieces = 1;
     }
-    wkv7_chunk_fwd_kernel<<<B * H * pieces, 256, SMEM_BYTES, st>>>(T, H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v,
+    wkv7_chunk_fwd_kernel<false><<<B * H * pieces, 256, SMEM_BYTES, st>>>(T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v,
                                                           (const bf*)a, (const bf*)b, (const bf*)s0, length, ns,
                                                           (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : nullptr,
                                                           maps, out_maps.m[0], out_maps.m[1],
@@ -680,7 +801,7 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
                                                           *range_flag, *range_ticket, residual_mark,
                                                           residual ? (bf*)(base + lay.mprime) : nullptr,
                                                           residual ? (bf*)(base + lay.rbar) : nullptr,
-                                                          residual ? (float*)(base + lay.lam) : nullptr, pieces);
+                                                          residual ? (float*)(base + lay.lam) : nullptr, pieces, BlockParts{});
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
