@@ -44,4 +44,31 @@ struct DeviceOnce {
     }
 };
 
+// A chain of kernels with the gaps between them closed: each but the first is launched with programmatic stream serialization
+// (launch_behind), so that its CTAs are set up while the one in front of it finishes, and starts with word_behind(), which
+// waits until that one has completed and then reads the word that decides whether there is anything to do.  The read is
+// volatile and everything else comes behind the caller's branch on it, so that no load can be moved in front of the wait.
+// A kernel that others are launched behind lets them in with let_next_in().
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ int word_behind(const int* word) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return *static_cast<const volatile int*>(word);
+}
+__device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 }  // namespace b200wkv

@@ -70,7 +70,11 @@ __global__ void __launch_bounds__(160)
 wkv7_chain_blocks_kernel(int Tlen, int H, int n_seq, int pieces, const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts,
                          const bf* __restrict__ s0, const bf* __restrict__ mprime, const uint4* __restrict__ m_low,
                          const float4* __restrict__ u, const float* __restrict__ lam, unsigned char* __restrict__ s0_tiles,
-                         size_t s0_stride, bf* __restrict__ s_out, float* __restrict__ s_at_len, int* __restrict__ status) {
+                         size_t s0_stride, bf* __restrict__ s_out, float* __restrict__ s_at_len, int* __restrict__ status,
+                         const int* __restrict__ range_flag, int range_ticket) {
+    let_next_in();
+    if (word_behind(range_flag) == range_ticket) return;       // a decay outside the range: the call is redone
+
     extern __shared__ __align__(128) unsigned char smem[];
     ChainSmem& sm = *reinterpret_cast<ChainSmem*>(smem);
     const int bh = blockIdx.x % n_seq, piece = blockIdx.x / n_seq, bi = bh / H;
@@ -232,7 +236,10 @@ __device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, bool
 // residual), most of which the chain has just left in L2.
 __global__ void __launch_bounds__(128)
 wkv7_block_outputs_kernel(int Tlen, int H, int n_blk_slots, const uint32_t* __restrict__ length, const unsigned char* __restrict__ s0_tiles, size_t s0_stride,
-                          const bf* __restrict__ rbar, BlockParts parts, unsigned char* __restrict__ saved, bf* __restrict__ y) {
+                          const bf* __restrict__ rbar, BlockParts parts, unsigned char* __restrict__ saved, bf* __restrict__ y,
+                          const int* __restrict__ range_flag, int range_ticket) {
+    let_next_in();
+    if (word_behind(range_flag) == range_ticket) return;
     __shared__ OutSmem sm;
     const int bh = blockIdx.x / n_blk_slots, sl = blockIdx.x % n_blk_slots, bi = bh / H, h = bh % H;
     const int L = min((int)length[bi], Tlen);
@@ -307,19 +314,21 @@ wkv7_block_outputs_kernel(int Tlen, int H, int n_blk_slots, const uint32_t* __re
 
 }  // namespace
 
-int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, const BlocksCall& c, void* y,
+int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, const int* range_flag, int range_ticket,
+                       const BlocksCall& c, void* y,
                        void* s_out, float* s_at_len) {
     static DeviceOnce smem_attr;
     if (!smem_attr.ok([]() { return cudaFuncSetAttribute(wkv7_chain_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChainSmem)); }))
         return B200WKV_ELAUNCH;
     // pieces: up to 8 of at least four steps
     const int quarter = block_slots(T) / 4, pieces = quarter < 1 ? 1 : quarter > 8 ? 8 : quarter;   // (steps fit 16 bits, see wkv7_blocks_bytes)
-    wkv7_chain_blocks_kernel<<<B * H * pieces, 160, sizeof(ChainSmem), st>>>(T, H, B * H, pieces, length, ns, (const bf*)s0, c.mprime, c.parts.m_low,
+    if (launch_behind(wkv7_chain_blocks_kernel, B * H * pieces, 160, sizeof(ChainSmem), st, T, H, B * H, pieces, length, ns, (const bf*)s0, c.mprime, c.parts.m_low,
                                                                              c.parts.state, c.lam, c.s0_tiles, c.s0_stride, (bf*)s_out, s_at_len,
-                                                                             wkv7_chunk_status_word());
+                      wkv7_chunk_status_word(), range_flag, range_ticket) != cudaSuccess)
+        return B200WKV_ELAUNCH;
     const int nSlot = block_slots(T);
-    wkv7_block_outputs_kernel<<<B * H * nSlot, 128, 0, st>>>(T, H, nSlot, length, c.s0_tiles, c.s0_stride, c.rbar, c.parts, c.saved, (bf*)y);
-    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+    return launch_behind(wkv7_block_outputs_kernel, B * H * nSlot, 128, 0, st, T, H, nSlot, length, c.s0_tiles, c.s0_stride, c.rbar, c.parts, c.saved,
+                         (bf*)y, range_flag, range_ticket) == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 }  // namespace b200wkv

@@ -132,7 +132,10 @@ wkv7_chain_kernel(int Tlen, int H, int run, const T* __restrict__ w, const T* __
                   int* __restrict__ residual_mark) {
     // Behind the chunked kernels: run only when the forward met something outside their domain (it left its ticket), and
     // backward only when the residual is marked as these kernels'.
-    if (run_if != nullptr && (kForward ? *run_if != run_ticket : *run_if == 0)) return;
+    if (run_if != nullptr) {
+        const int word = word_behind(run_if);
+        if (kForward ? word != run_ticket : word == 0) return;
+    }
     if (kForward && residual_mark != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *residual_mark = 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     ChainSmem<R>& sm = *reinterpret_cast<ChainSmem<R>*>(smem_raw);
@@ -341,6 +344,11 @@ int launch_rows(cudaStream_t st, int B, int Tlen, int H, int run, const void* w,
     static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
     if (!smem_attr.ok([kern, smem]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); }))
         return B200WKV_ELAUNCH;
+    if (run_if != nullptr)
+        return launch_behind(kern, B * H * (8 / R), kThreads, smem, st, Tlen, H, run, (const T*)w, (const T*)r, (const T*)k, (const T*)v, (const T*)a,
+                             (const T*)b, (const T*)x0, length, ns, (T*)y, (T*)out, ckpt, run_if, run_ticket, residual_mark) == cudaSuccess
+                   ? B200WKV_OK
+                   : B200WKV_ELAUNCH;
     kern<<<B * H * (8 / R), kThreads, smem, st>>>(Tlen, H, run, (const T*)w, (const T*)r, (const T*)k, (const T*)v, (const T*)a, (const T*)b,
                                                   (const T*)x0, length, ns, (T*)y, (T*)out, ckpt, run_if, run_ticket, residual_mark);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;

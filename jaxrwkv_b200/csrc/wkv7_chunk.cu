@@ -118,6 +118,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                       int* __restrict__ range_flag, int range_ticket, int* __restrict__ residual_mark,
                       __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces,
                       const BlockParts parts) {
+    let_next_in();
     extern __shared__ __align__(1024) unsigned char smem[];   // (the swizzle of the output tile is a function of the address)
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     // (all first pieces come first in the grid: where no cut exists the other pieces' CTAs return at once, and the
@@ -780,7 +781,7 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
             (bf*)s_out, nullptr, maps, out_maps.m[0], out_maps.m[1], c.saved, *range_flag, *range_ticket, residual_mark, c.mprime, c.rbar, c.lam, 1,
             c.parts);
         if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
-        return wkv7_blocks_finish(st, B, T, H, length, ns, s0, c, y, s_out, residual ? (float*)(base + lay.s_at_len) : nullptr);
+        return wkv7_blocks_finish(st, B, T, H, length, ns, s0, *range_flag, *range_ticket, c, y, s_out, residual ? (float*)(base + lay.s_at_len) : nullptr);
     }
     // Without a residual (inference) and with fewer sequences than CTA slots, every sequence is offered to several
     // CTAs, which cut it at start flags where there are any (see the kernel): at most 8 pieces of at least 128 tokens.

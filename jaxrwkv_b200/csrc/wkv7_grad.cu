@@ -132,7 +132,8 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                      __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ da, __nv_bfloat16* __restrict__ db,
                      int* __restrict__ status, int has_dy, unsigned char* __restrict__ fscr_all,
                      const __grid_constant__ StreamMaps maps, const __grid_constant__ StreamMaps out_maps) {
-    if (*residual_mark != 0) return;            // the forward fell back to the sequential kernels
+    let_next_in();
+    if (word_behind(residual_mark) != 0) return;   // the forward fell back to the sequential kernels
     extern __shared__ __align__(1024) unsigned char smem[];
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -369,6 +370,19 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             mma_k64(tbase + T_GD, mnmaj64u(sPRB), mnmaj128u(sDD), ID_MM, !inner());
             tc::commit(&sm.bar[0]);
         }
+        if (inner()) {   // the dS share: only the rows behind the last flag
+            if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
+            tc::fence_after_sync();
+            float x[32], y[32];
+            tc::tmem_ld32(lane_addr + T_GD + hsel * 32, x);
+            tc::tmem_ld32(lane_addr + T_W + hsel * 32, y);
+            tc::tmem_wait_ld();
+            const bool last = in_last(row & 63);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) x[c] += last ? y[c] : 0.f;
+            tc::tmem_st32(lane_addr + T_GD + hsel * 32, x);
+            tc::tmem_wait_st();
+        }
         if (quad >= 2) {
             // D at the block end, by the four warps that have no part in the next two epilogues:
             //   D_end[c] = sum_i dS[i][c] S_end[i][c] = (sum_i dSL[i][c] S_end[i][c]) / L_C[c]
@@ -411,19 +425,6 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
 #pragma unroll
                 for (int e = 0; e < 8; ++e) sm.d_end[cbk * 8 + e] = acc[e] / sm.lam[cbk * 8 + e];
             }
-            if (inner()) {   // dV: the dS share of the rows behind the last flag joins the rest
-                if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
-                tc::fence_after_sync();
-                float x[32], y[32];
-                tc::tmem_ld32(lane_addr + T_GD + hsel * 32, x);
-                tc::tmem_ld32(lane_addr + T_W + hsel * 32, y);
-                tc::tmem_wait_ld();
-                const bool last = in_last(row - 64);
-#pragma unroll
-                for (int c = 0; c < 32; ++c) x[c] += last ? y[c] : 0.f;
-                tc::tmem_st32(lane_addr + T_GD + hsel * 32, x);
-                tc::tmem_wait_st();
-            }
         }
         if (quad < 2) {
             if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
@@ -431,14 +432,6 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             float gd[32];
             tc::tmem_ld32(lane_addr + T_GD + hsel * 32, gd);
             tc::tmem_wait_ld();
-            if (inner()) {
-                float y[32];
-                tc::tmem_ld32(lane_addr + T_W + hsel * 32, y);
-                tc::tmem_wait_ld();
-                const bool last = in_last(row);
-#pragma unroll
-                for (int c = 0; c < 32; ++c) gd[c] += last ? y[c] : 0.f;
-            }
 #pragma unroll
             for (int c = 0; c < 4; ++c) slab_store(smem + OFF_X1, P64, row, hsel * 4 + c, pack8(&gd[c * 8]));   // over P_rk, which is read
         }
@@ -483,15 +476,32 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         if (tid == kFindThread) find_item(it.id + (int)gridDim.x, &sm.item[par ^ 1]);   // the next block of this CTA
         if (!tc::mbar_wait(&sm.bar[2], par)) failed = true;
         tc::fence_after_sync();
+        if (inner()) {   // W: s stays in front of the first flag behind t; [V;sa] dSL: only the rows behind the last flag
+            const int t = row & 63;
+            const uint64_t behind = (mask_of() >> t) >> 1;
+            const int hi = behind != 0 ? t + __ffsll((long long)behind) : kC;
+            float x[32];
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                const uint32_t at = lane_addr + T_W + hsel * 64 + part * 32;
+                tc::tmem_ld32(at, x);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int s = 0; s < 32; ++s) x[s] = s + part * 32 < hi ? x[s] : 0.f;
+                tc::tmem_st32(at, x);
+            }
+            tc::tmem_ld32(lane_addr + T_KB + hsel * 32, x);
+            tc::tmem_wait_ld();
+            const bool last = in_last(t);
+#pragma unroll
+            for (int c = 0; c < 32; ++c) x[c] = last ? x[c] : 0.f;
+            tc::tmem_st32(lane_addr + T_KB + hsel * 32, x);
+            tc::tmem_wait_st();
+        }
         {
             // keep s >= t for the dY blocks, s > t for the dG blocks.  Rows t < 32 keep all of columns 32..63;
             // rows t >= 32 keep nothing of columns 0..31 (zeros are stored without reading the accumulator).
-            // With start flags in the block, s stays in front of the first one behind t.
             const int t = row & 63, lo = t + hsel;
-            auto first_behind = [&]() {
-                const uint64_t behind = (mask_of() >> t) >> 1;
-                return behind != 0 ? t + __ffsll((long long)behind) : kC;
-            };
             unsigned char* dst = smem + (hsel == 0 ? OFF_WY : OFF_WSA);   // over T, A_ak, dSL, P_rb: all read by now
             float d[32];
             if ((quad & 1) == 0) {
@@ -499,20 +509,10 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                 tc::tmem_wait_ld();
 #pragma unroll
                 for (int s = 0; s < 32; ++s) d[s] = (s >= lo) ? d[s] : 0.f;
-                if (inner()) {
-                    const int hi = first_behind();
-#pragma unroll
-                    for (int s = 0; s < 32; ++s) d[s] = s < hi ? d[s] : 0.f;
-                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) slab_store(dst, P128, row, c, pack8(&d[c * 8]));
                 tc::tmem_ld32(lane_addr + T_W + hsel * 64 + 32, d);
                 tc::tmem_wait_ld();
-                if (inner()) {
-                    const int hi = first_behind();
-#pragma unroll
-                    for (int s = 0; s < 32; ++s) d[s] = s + 32 < hi ? d[s] : 0.f;
-                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) slab_store(dst, P128, row, 4 + c, pack8(&d[c * 8]));
             } else {
@@ -522,24 +522,9 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                 tc::tmem_wait_ld();
 #pragma unroll
                 for (int s = 0; s < 32; ++s) d[s] = (s + 32 >= lo) ? d[s] : 0.f;
-                if (inner()) {
-                    const int hi = first_behind();
-#pragma unroll
-                    for (int s = 0; s < 32; ++s) d[s] = s + 32 < hi ? d[s] : 0.f;
-                }
 #pragma unroll
                 for (int c = 0; c < 4; ++c) slab_store(dst, P128, row, 4 + c, pack8(&d[c * 8]));
             }
-        }
-        if (inner()) {   // [V;sa] dSL: only the rows behind the last flag
-            float x[32];
-            tc::tmem_ld32(lane_addr + T_KB + hsel * 32, x);
-            tc::tmem_wait_ld();
-            const bool last = in_last(row & 63);
-#pragma unroll
-            for (int c = 0; c < 32; ++c) x[c] = last ? x[c] : 0.f;
-            tc::tmem_st32(lane_addr + T_KB + hsel * 32, x);
-            tc::tmem_wait_st();
         }
         if (quad >= 2) {   // dV rows
             const int t = row - 64;
@@ -591,6 +576,21 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         }
         if (!tc::mbar_wait(&sm.bar[3], par)) failed = true;
         tc::fence_after_sync();
+        if (inner()) {   // [dY;dG] S0: only the rows in front of the first flag
+            const bool first = in_first(t);
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                float z[16], y[16];
+                const uint32_t column = hsel * 32 + part * 16;
+                tc::tmem_ld16(lane_addr + T_RA + column, z);
+                tc::tmem_ld16(lane_addr + T_GD + column, y);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 16; ++e) z[e] += first ? y[e] : 0.f;
+                tc::tmem_st16(lane_addr + T_RA + column, z);
+            }
+            tc::tmem_wait_st();
+        }
         // ================= last epilogue: unscale, write dk db dr da, decay gradient =================
         unsigned char* const tile_x = smem + ((row < 64) ? OFF_TK : OFF_TB) + t * 128;   // dk | db
         unsigned char* const tile_z = smem + ((row < 64) ? OFF_TR : OFF_TA) + t * 128;   // dr | da
@@ -601,14 +601,6 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             tc::tmem_ld16(lane_addr + T_KB + hsel * 32 + hh * 16, x);
             tc::tmem_ld16(lane_addr + T_RA + hsel * 32 + hh * 16, z);
             tc::tmem_wait_ld();
-            if (inner()) {   // [dY;dG] S0: only the rows in front of the first flag
-                float y[16];
-                tc::tmem_ld16(lane_addr + T_GD + hsel * 32 + hh * 16, y);
-                tc::tmem_wait_ld();
-                const bool first = in_first(t);
-#pragma unroll
-                for (int e = 0; e < 16; ++e) z[e] += first ? y[e] : 0.f;
-            }
 #pragma unroll
             for (int h2 = 0; h2 < 2; ++h2) {
                 const int c = hh * 2 + h2, cb = hsel * 4 + c;
@@ -769,11 +761,12 @@ int wkv7_grad_bwd(cudaStream_t st, int B, int T, int H, const void* w, const voi
     long long slots = 2LL * sm_count_of_current_device();
     if (slots > kGradCtas) slots = kGradCtas;        // every CTA owns a set of factor tiles in the residual
     const int grid = (int)(items < slots ? items : slots);
-    wkv7_grad_bwd_kernel<<<grid, 256, SMEM_BYTES, st>>>(T, H, BH, length, ns, (const bf*)(base + lay.dstate), s_at_len, saved,
+    return launch_behind(wkv7_grad_bwd_kernel, grid, 256, SMEM_BYTES, st, T, H, BH, length, ns, (const bf*)(base + lay.dstate), s_at_len, saved,
                                                         residual_mark, (bf*)dw, (bf*)dr, (bf*)dk,
                                                         (bf*)dv, (bf*)da, (bf*)db, wkv7_chunk_status_word(), dy != nullptr ? 1 : 0,
-                                                        (unsigned char*)(base + lay.fscr), maps, out_maps);
-    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+                                                        (unsigned char*)(base + lay.fscr), maps, out_maps) == cudaSuccess
+               ? B200WKV_OK
+               : B200WKV_ELAUNCH;
 }
 
 }  // namespace b200wkv
