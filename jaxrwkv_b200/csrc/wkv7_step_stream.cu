@@ -33,7 +33,7 @@ constexpr int kThreads = 96;   // two computing warps and the warp of the copy t
 // chunk q ^ 1, and it reads the vectors with the matching permutation (vgroup()).
 template <typename T> struct Tile;
 template <> struct Tile<__nv_bfloat16> {
-    static constexpr int kStages = 5, kChunks = 2, kChunkElems = 8, kVecFlip = 2;
+    static constexpr int kStages = 4, kChunks = 2, kChunkElems = 8, kVecFlip = 2;
     static __device__ __forceinline__ void unpack(const uint4& raw, float* f) {
         const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
@@ -61,6 +61,9 @@ template <> struct Tile<float> {
     }
 };
 
+// Resident CTAs of one grid per SM.  Four rings of four 9 KB stages are 22 MB in flight over the chip, more than the latency
+// times the bandwidth; what they leave of the shared memory lets the first CTAs of the next grid in while this one drains.
+constexpr int kCtasPerSm = 4;
 constexpr int kFlagBatch = 64;   // the computing threads fetch the flags of this many pairs at a time
 
 template <typename T>
@@ -134,6 +137,10 @@ wkv7_step_stream_kernel(int BH, int H, const T* __restrict__ w, const T* __restr
     // writes global memory; everything below comes after the wait, i.e. after the preceding grid has
     // completed and its writes are visible.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // ... except that the states of the first ring are asked for in L2, where what the preceding grid still writes arrives as
+    // well: the first loads then find them there.
+    if (tid >= kComputeThreads && lane < kStages && lane < n_my)
+        tc::bulk_prefetch_l2(s0 + state_off(first + lane * stride), kTileBytes);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     __syncthreads();
     if (tid >= kComputeThreads) {
@@ -290,6 +297,7 @@ int launch(cudaStream_t st, int B, int H, const void* w, const void* r, const vo
             if (e != cudaSuccess) return e;
             int n = 0;
             if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kThreads, smem) != cudaSuccess || n < 1) n = 1;
+            if (n > kCtasPerSm) n = kCtasPerSm;
             per_sm_of[dev] = n;
             status_of[dev] = wkv7_chunk_status_word();
             return cudaSuccess;
