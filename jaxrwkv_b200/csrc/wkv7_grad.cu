@@ -554,12 +554,12 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             tc::commit(&sm.bar[3]);
         } else if (issuer_b) {
             tc::fence_after_sync();
+            mma_k64(tbase + T_RA, mnmaj128u(sWY + HALF), mnmaj128u(sBK), ID_MM, false);
+            mma_k64(tbase + T_RA, mnmaj128u(sWY), mnmaj128u(sBK + HALF), ID_MM, true);
             if (it.n == kC) {
                 tc::tensor_store_2d(&out_maps.m[OUT_V], it.h * kN, it.bi * Tlen + it.p, smem + OFF_TV);
                 tc::bulk_commit();
             }
-            mma_k64(tbase + T_RA, mnmaj128u(sWY + HALF), mnmaj128u(sBK), ID_MM, false);
-            mma_k64(tbase + T_RA, mnmaj128u(sWY), mnmaj128u(sBK + HALF), ID_MM, true);
             if (!tc::mbar_wait(&sm.bar[7], par)) failed = true;   // S0 has landed
             mma_k64(tbase + (inner() ? T_GD : T_RA), kmaj128u(sDD), mnmaj64u(sX1), ID_KM, !inner());
             tc::bulk_wait_read<0>();   // the dV tile has left before this round is reported done: the last epilogue writes over it
