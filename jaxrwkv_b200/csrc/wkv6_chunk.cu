@@ -39,15 +39,6 @@ constexpr int kRunLen6 = 16;    // chunks per run of the run-parallel backward
 constexpr int PITCH = 72;        // bf16 per shared-memory row (144 bytes): 4-byte fragment reads and ldmatrix rows hit 32 banks
 constexpr float kMaxHalfDecay = 80.f;   // |sum of lw over half a chunk| the scaling can represent
 
-__device__ __forceinline__ void cp_async16_zfill(void* dst_smem, const void* src, bool valid) {
-    const int n = valid ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "r"(n)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
@@ -925,34 +916,33 @@ wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ u, const uint32_t*
 // registers.  It leaves the state gradient at the end of every run of `run_len` chunks, from which the gradient kernel
 // above walks the runs in parallel.
 // Unlike the other kernels of this file it walks 64 tokens at a time: it uses no factor other than exp(cumulative
-// log-decay) <= 1, so nothing limits its chunk, and a quarter of the steps means a quarter of the barriers and waits.
+// log-decay) <= 1, so nothing limits its chunk, and a quarter of the steps means a quarter of the barriers and waits.  The
+// operands are prepared as in the forward, a warp its 16 channels, R0 in place over the r rows: two 24 KB stages, four CTAs
+// per SM, which 512 sequences need to run at once.  B=16, T=4096, H=32: 0.153 ms (0.257 ms with sums as a scan over
+// quarters of the step and rows fetched by every thread), 0.8 GB at 5.3 TB/s.
 constexpr int kCB = 64;            // tokens per step of the carry
 constexpr int kCarryStages = 2;
-constexpr int kQT = kCB / 4;       // tokens per thread in phase A
+constexpr int kTileCB = kCB * kN * 2;
 static_assert(kRunLen6 % (kCB / kC6) == 0, "runs must end at a step of the carry");
-struct CarryStage6 {
-    bf r[kCB][PITCH], w[kCB][PITCH], dy[kCB][PITCH];   // r becomes R0 in place
-};
 struct Carry6Smem {
-    CarryStage6 st[kCarryStages];
-    float tot[4][kN];              // sum of the log-decay over each quarter of the step
-    float wc[kN];
-    unsigned startmask[2];         // bit t of word t / 32: start flag on token t of the step (one word used when kCB == 32)
-    uint8_t ns[kCarryStages][kCB];
+    unsigned char r[kCarryStages][kTileCB], w[kCarryStages][kTileCB], dy[kCarryStages][kTileCB];
+    float wc[kN];                  // exp(c_C), or 0 when a start flag lies in the step
+    uint64_t full[kCarryStages];
 };
 static_assert(4 * (sizeof(Carry6Smem) + 1024) <= 228 * 1024, "four CTAs per SM");
 
 __global__ void __launch_bounds__(128, 4)
-wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __restrict__ w,
-                      const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts, const bf* __restrict__ dy,
-                      const bf* __restrict__ ds_out, const int* __restrict__ residual_mark, int n_runs, int run_len,
-                      bf* __restrict__ dsck) {
+wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const uint32_t* __restrict__ length,
+                      const uint8_t* __restrict__ new_starts, int has_dy, const bf* __restrict__ ds_out,
+                      const int* __restrict__ residual_mark, int n_runs, int run_len, bf* __restrict__ dsck, int* __restrict__ status,
+                      const __grid_constant__ SeqMaps maps) {
     if (*residual_mark != 0) return;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
     Carry6Smem& sm = *reinterpret_cast<Carry6Smem*>(smem_raw);
     const int bh = blockIdx.x, bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, q = lane & 3, mi = lane >> 3, r8 = lane & 7;
+    const int g = lane >> 2, q = lane & 3;
+    const int frow = lane & 15;
     const int j0 = warp * 16;
     const size_t tok_stride = (size_t)H * kN;
     const size_t seq_base = (size_t)bi * Tlen * tok_stride + (size_t)h * kN;
@@ -969,59 +959,62 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
     for (int ni = 0; ni < 8; ++ni)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[ni][e] = 0.f;
-    auto issue = [&](int c) {
-        if (c >= c_stop) {
-            CarryStage6& st = sm.st[c % kCarryStages];
+    if (tid == 0) {
 #pragma unroll
-            for (int rr = 0; rr < kCB / 16; ++rr) {
-                const int row = (tid >> 3) + 16 * rr, piece = (tid & 7) * 8;
-                const int t = c * kCB + row;
-                const bool ok = t < Tlen;
-                const size_t off = seq_base + (size_t)(ok ? t : 0) * tok_stride + piece;
-                cp_async16_zfill(&st.r[row][piece], r + off, ok);
-                cp_async16_zfill(&st.w[row][piece], w + off, ok);
-                cp_async16_zfill(&st.dy[row][piece], dy != nullptr ? dy + off : r + off, ok && dy != nullptr);
-            }
-        }
-        cp_async_commit();
-    };
-    auto load_ns = [&](int c) -> uint8_t {
-        const int t = c * kCB + tid;
-        return (tid < kCB && c >= 0 && t < Tlen) ? new_starts[(size_t)bi * Tlen + t] : (uint8_t)0;
-    };
-#pragma unroll
-    for (int i = 1; i < kCarryStages; ++i) {
-        issue(nB - i);
-        if (tid < kCB && nB - i >= 0) sm.ns[(nB - i) % kCarryStages][tid] = load_ns(nB - i);
+        for (int i = 0; i < kCarryStages; ++i) tc::mbar_init(&sm.full[i], 1);
+        tc::mbar_init_fence();
     }
-    uint8_t ns_ahead = load_ns(nB - kCarryStages);
-    // phase A ownership: the channel pair cp, cp + 1 and the kQT tokens of quarter qt
-    const int cp = (tid & 31) * 2, qt = tid >> 5;
+    __syncthreads();
+    auto issue = [&](int c) {          // step c, the (nB - 1 - c)th
+        if (tid == 0 && c >= c_stop) {
+            const int stage = (nB - 1 - c) % kCarryStages;
+            uint64_t* bar = &sm.full[stage];
+            tc::mbar_expect_tx(bar, (2 + has_dy) * kTileCB);
+            tc::tensor_load_3d(sm.r[stage], &maps.m[0], h * kN, c * kCB, bi, bar);
+            tc::tensor_load_3d(sm.w[stage], &maps.m[1], h * kN, c * kCB, bi, bar);
+            if (has_dy) tc::tensor_load_3d(sm.dy[stage], &maps.m[2], h * kN, c * kCB, bi, bar);
+        }
+    };
+    issue(nB - 1);
+    const uint8_t* const ns_row = new_starts + (size_t)bi * Tlen;
+    auto load_ns = [&](int c, int half) -> unsigned { return ns_row[min(max(c, 0) * kCB + 32 * half + lane, Tlen - 1)]; };
+    unsigned ns_lo = load_ns(nB - 1, 0), ns_hi = load_ns(nB - 1, 1);
+    // places in a swizzled tile, as in the forward; of a 16x16 block's rows in column piece 2 x, + 1
+    auto block_row = [&](int x) { return frow * 128 + (((2 * x + (lane >> 4)) ^ (frow & 7)) << 4); };
+    const int tile_row = block_row(warp);
+    const int tile_word = g * 128 + (((2 * warp) ^ g) << 4) + 4 * q;
+    // constant left operands: strictly earlier tokens of a 16-token block, and all of them
+    const uint32_t earlier = pack2(2 * q < g ? 1.f : 0.f, 2 * q + 1 < g ? 1.f : 0.f);
+    constexpr uint32_t kOnes = 0x3f803f80u;
+    bool waited = true;
 
     auto walk = [&](auto split_tag, const int c, const int part_arg) {
         constexpr bool kSplitHere = decltype(split_tag)::value;
         const int part = kSplitHere ? part_arg : 0;
         const int lo = (kSplitHere && part == 1) ? p_out + 1 : 0, hi = (kSplitHere && part == 0) ? p_out + 1 : kCB;
-        CarryStage6& st = sm.st[c % kCarryStages];
+        const int it = nB - 1 - c, stage = it % kCarryStages;
         const int t0 = c * kCB;
+        unsigned long long starts = (unsigned long long)__ballot_sync(0xffffffffu, ns_lo != 0) | (unsigned long long)__ballot_sync(0xffffffffu, ns_hi != 0) << 32;
+        starts &= ~0ull >> max(t0 + kCB - Tlen, 0);
+        if (kSplitHere) starts &= (hi < kCB ? (1ull << hi) - 1ull : ~0ull) & ~((1ull << lo) - 1ull);
+        tc::fence_async_smem();       // (R0 was written over the r rows that the next copy replaces)
+        __syncthreads();              // the tiles of step c + 1 are no longer read
         if (!kSplitHere || part == 1) {
-            cp_async_wait<kCarryStages - 2>();
-            __syncthreads();          // step c has landed for everyone; the tiles of step c + 1 are no longer read
-            issue(c - (kCarryStages - 1));
-            if (tid < kCB && c - (kCarryStages - 1) >= 0) sm.ns[(c - (kCarryStages - 1)) % kCarryStages][tid] = ns_ahead;
-            ns_ahead = load_ns(c - kCarryStages);
+            issue(c - 1);
+            if (!tc::mbar_wait(&sm.full[stage], (it / kCarryStages) & 1)) waited = false;
         } else {
             // the first visit turned r into R0 in place: fetch the rows again for the part in front of `length`
-            __syncthreads();
 #pragma unroll
             for (int rr = 0; rr < kCB / 16; ++rr) {
-                const int row = (tid >> 3) + 16 * rr, piece = (tid & 7) * 8;
-                const int t = t0 + row;
-                const bool ok = t < Tlen;
-                *reinterpret_cast<uint4*>(&st.r[row][piece]) =
-                    ok ? *reinterpret_cast<const uint4*>(r + seq_base + (size_t)t * tok_stride + piece) : make_uint4(0, 0, 0, 0);
+                const int row = (tid >> 3) + 16 * rr, piece = tid & 7;
+                *reinterpret_cast<uint4*>(sm.r[stage] + row * 128 + ((piece ^ (row & 7)) << 4)) =
+                    t0 + row < Tlen ? *reinterpret_cast<const uint4*>(r + seq_base + (size_t)(t0 + row) * tok_stride + piece * 8) : make_uint4(0, 0, 0, 0);
             }
             __syncthreads();
+        }
+        if (!kSplitHere || part == 0) {
+            ns_lo = load_ns(c - 1, 0);
+            ns_hi = load_ns(c - 1, 1);
         }
         if (c == c_out && part == 0 && ds_out != nullptr) {
 #pragma unroll
@@ -1030,54 +1023,53 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
                 for (int e = 0; e < 4; ++e)
                     acc[ni][e] += __bfloat162float(ds_out[st_base + (size_t)(8 * ni + 2 * q + (e & 1)) * kN + j0 + g + 8 * (e >> 1)]);
         }
-        if (warp < kCB / 32) {
-            const unsigned m = __ballot_sync(0xffffffffu, sm.ns[c % kCarryStages][32 * warp + lane] != 0);
-            if (lane == 0) sm.startmask[warp] = m;
-        }
-        // the log-decay of this thread's kQT tokens (two channels each), and its sum
-        auto lw_of = [&](int tt) -> float2 {
-            const int t = kQT * qt + tt;
-            const bool ok = t0 + t < Tlen && t >= lo && t < hi;
-            return ok ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.w[t][cp])) : make_float2(0.f, 0.f);
-        };
-        float2 run = make_float2(0.f, 0.f);
+        // ---- R0 of this warp's channels; before[nt][2 hh + e]: cumulative log-decay in front of token g + 8 hh of the block
+        float sum[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};      // of the blocks so far (every row the same)
 #pragma unroll
-        for (int tt = 0; tt < kQT; ++tt) {
-            const float2 l2 = lw_of(tt);
-            run.x += l2.x;
-            run.y += l2.y;
-        }
-        *reinterpret_cast<float2*>(&sm.tot[qt][cp]) = run;
-        __syncthreads();
-        {
-            const unsigned long long starts = (unsigned long long)sm.startmask[0] | (kCB > 32 ? (unsigned long long)sm.startmask[1] << 32 : 0ull);
-            auto seg_of = [&](int t) { return __popcll(starts & ((2ull << t) - 1ull)); };
-            const int seg_last = seg_of(hi - 1), seg_base = lo > 0 ? seg_of(lo - 1) : 0;
-            float2 c_prev = make_float2(0.f, 0.f);         // cumulative log-decay in front of the token
-            for (int qq = 0; qq < qt; ++qq) {
-                const float2 tq = *reinterpret_cast<const float2*>(&sm.tot[qq][cp]);
-                c_prev.x += tq.x;
-                c_prev.y += tq.y;
-            }
-            if (qt == 3)
-                *reinterpret_cast<float2*>(&sm.wc[cp]) = seg_last == seg_base ? make_float2(__expf(c_prev.x + run.x), __expf(c_prev.y + run.y))
-                                                                               : make_float2(0.f, 0.f);
-            int seg = qt > 0 ? seg_of(kQT * qt - 1) : 0;    // number of start flags at or before the token, kept in step
+        for (int ks = 0; ks < kCB / 16; ++ks) {
+            uint32_t wb[4];
+            ldmatrix_x4_trans(wb[0], wb[1], wb[2], wb[3], sm.w[stage] + ks * 2048 + tile_row);
+            if (kSplitHere) {
 #pragma unroll
-            for (int tt = 0; tt < kQT; ++tt) {
-                const int t = kQT * qt + tt;
-                seg += (int)((starts >> t) & 1ull);
-                const bool in_part = t >= lo && t < hi;
-                const float2 rv = in_part ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&st.r[t][cp])) : make_float2(0.f, 0.f);
-                const bool first_seg = seg == seg_base;
-                *reinterpret_cast<uint32_t*>(&st.r[t][cp]) =                                   // R0, in place
-                    pack2(first_seg ? rv.x * __expf(c_prev.x) : 0.f, first_seg ? rv.y * __expf(c_prev.y) : 0.f);
-                const float2 l2 = lw_of(tt);
-                c_prev.x += l2.x;
-                c_prev.y += l2.y;
+                for (int i = 0; i < 4; ++i) {
+                    const int s = 16 * ks + 8 * (i & 1) + 2 * q;
+                    wb[i] &= (s >= lo && s < hi ? 0xffffu : 0u) | (s + 1 >= lo && s + 1 < hi ? 0xffff0000u : 0u);
+                }
             }
+            uint32_t r0[4];           // in the order (hh, nt) = 00, 10, 01, 11
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt) {
+                float before[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) before[e] = sum[nt][e];
+                mma_bf16(before, earlier, kOnes, 0u, earlier, wb[2 * nt], wb[2 * nt + 1]);
+                mma_bf16(sum[nt], kOnes, kOnes, kOnes, kOnes, wb[2 * nt], wb[2 * nt + 1]);
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const int t = 16 * ks + g + 8 * hh;
+                    uint32_t rw = *reinterpret_cast<const uint32_t*>(sm.r[stage] + ks * 2048 + (tile_word ^ (16 * nt)) + 1024 * hh);
+                    if (kSplitHere && !(t >= lo && t < hi)) rw = 0;
+                    const float2 rv = unpack2(rw);
+                    r0[2 * nt + hh] = pack2(rv.x * exp_fast(before[2 * hh]), rv.y * exp_fast(before[2 * hh + 1]));
+                }
+            }
+            if (starts != 0) {        // nothing from the first flag on sees the entering state
+#pragma unroll
+                for (int hh = 0; hh < 2; ++hh) {
+                    const bool first = (starts & ((2ull << (16 * ks + g + 8 * hh)) - 1ull)) == 0;
+#pragma unroll
+                    for (int nt = 0; nt < 2; ++nt) r0[2 * nt + hh] = first ? r0[2 * nt + hh] : 0u;
+                }
+            }
+            __syncwarp();             // (the block's rows of this warp's channels have been read)
+            stmatrix_x4(sm.r[stage] + ks * 2048 + tile_row, r0[0], r0[1], r0[2], r0[3]);
         }
-        __syncthreads();
+        if (g == 0) {
+#pragma unroll
+            for (int nt = 0; nt < 2; ++nt)
+                *reinterpret_cast<float2*>(&sm.wc[j0 + 8 * nt + 2 * q]) = starts == 0 ? make_float2(exp_fast(sum[nt][0]), exp_fast(sum[nt][1])) : make_float2(0.f, 0.f);
+        }
+        __syncthreads();              // R0 and the step's decay are complete
         // dS0^T = dS_C^T diag(exp(c_C)) [no start in the step] + dY^T R0
 #pragma unroll
         for (int np = 0; np < 4; ++np) {
@@ -1086,16 +1078,18 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
             acc[2 * np][0] *= w0.x; acc[2 * np][1] *= w0.y; acc[2 * np][2] *= w0.x; acc[2 * np][3] *= w0.y;
             acc[2 * np + 1][0] *= w1.x; acc[2 * np + 1][1] *= w1.y; acc[2 * np + 1][2] *= w1.x; acc[2 * np + 1][3] *= w1.y;
         }
+        if (has_dy) {
 #pragma unroll
-        for (int ks = 0; ks < kCB / 16; ++ks) {
-            uint32_t ya[4];
-            ldmatrix_x4_trans(ya[0], ya[1], ya[2], ya[3], &st.dy[16 * ks + (mi >> 1) * 8 + r8][j0 + (mi & 1) * 8]);
+            for (int ks = 0; ks < kCB / 16; ++ks) {
+                uint32_t y[4];
+                ldmatrix_x4_trans(y[0], y[1], y[2], y[3], sm.dy[stage] + ks * 2048 + tile_row);
 #pragma unroll
-            for (int np = 0; np < 4; ++np) {
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(b0, b1, b2, b3, &st.r[16 * ks + (mi & 1) * 8 + r8][(2 * np + (mi >> 1)) * 8]);
-                mma_bf16(acc[2 * np], ya[0], ya[1], ya[2], ya[3], b0, b1);
-                mma_bf16(acc[2 * np + 1], ya[0], ya[1], ya[2], ya[3], b2, b3);
+                for (int np = 0; np < 4; ++np) {
+                    uint32_t b0, b1, b2, b3;
+                    ldmatrix_x4_trans(b0, b1, b2, b3, sm.r[stage] + ks * 2048 + block_row(np));
+                    mma_bf16(acc[2 * np], y[0], y[2], y[1], y[3], b0, b1);
+                    mma_bf16(acc[2 * np + 1], y[0], y[2], y[1], y[3], b2, b3);
+                }
             }
         }
     };
@@ -1118,7 +1112,7 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const bf* __res
             walk(std::false_type{}, c, 0);
         }
     }
-    cp_async_wait<0>();
+    if (!waited && status != nullptr) atomicExch(status, 5);
 }
 
 // du of a (batch, head): the runs' shares added in a fixed order
@@ -1191,8 +1185,11 @@ int wkv6_chunk_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
     bf* dsck = reinterpret_cast<bf*>(base + lay.dsck);
     float* partial = reinterpret_cast<float*>(base + lay.partial);
     if (n_runs > 1) {
-        wkv6_carry_bwd_kernel<<<B * H, 128, sizeof(Carry6Smem), st>>>(T, H, (const bf*)r, (const bf*)w, length, ns, (const bf*)dy,
-                                                                     (const bf*)ds_out, residual_mark, n_runs, kRunLen, dsck);
+        const void* streams[3] = {r, w, dy};
+        SeqMaps maps;
+        if (!make_seq_maps(&maps, streams, 3, B, T, H, kCB)) return B200WKV_ELAUNCH;
+        wkv6_carry_bwd_kernel<<<B * H, 128, sizeof(Carry6Smem), st>>>(T, H, (const bf*)r, length, ns, dy != nullptr ? 1 : 0, (const bf*)ds_out,
+                                                                     residual_mark, n_runs, kRunLen, dsck, wkv7_chunk_status_word(), maps);
         if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
     }
     const void* streams[9] = {r, k, v, w, dy, dr, dk, dv, dw};
