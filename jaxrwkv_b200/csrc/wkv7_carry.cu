@@ -70,8 +70,7 @@ wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length,
                       const __nv_bfloat16* __restrict__ mprime, const __nv_bfloat16* __restrict__ rbar,
                       const float* __restrict__ lam, const int* __restrict__ residual_mark,
                       __nv_bfloat16* __restrict__ dstate, __nv_bfloat16* __restrict__ ds0) {
-    let_next_in();
-    if (word_behind(residual_mark) != 0) return;   // the forward fell back to the sequential kernels
+    if (*residual_mark != 0) return;            // the forward fell back to the sequential kernels
     const int bh = blockIdx.x;
     extern __shared__ __align__(128) unsigned char smem[];
     CarryStage* stages = reinterpret_cast<CarryStage*>(smem);
@@ -207,11 +206,10 @@ int wkv7_carry_bwd(cudaStream_t st, int B, int T, int H, const uint32_t* length,
     char* base = static_cast<char*>(residual);
     const bool deep = (long long)B * H <= 2LL * sm_count_of_current_device();
     auto launch = deep ? wkv7_carry_bwd_kernel<3> : wkv7_carry_bwd_kernel<2>;
-    return launch_behind(launch, B * H, 128, deep ? carry_smem<3>() : carry_smem<2>(), st, T, H, length, (const bf*)dy, (const bf*)ds_out, (const bf*)(base + lay.mprime),
+    launch<<<B * H, 128, deep ? carry_smem<3>() : carry_smem<2>(), st>>>(T, H, length, (const bf*)dy, (const bf*)ds_out, (const bf*)(base + lay.mprime),
                                                                          (const bf*)(base + lay.rbar), (const float*)(base + lay.lam),
-                                                                         residual_mark, (bf*)(base + lay.dstate), (bf*)ds0) == cudaSuccess
-               ? B200WKV_OK
-               : B200WKV_ELAUNCH;
+                                                                         residual_mark, (bf*)(base + lay.dstate), (bf*)ds0);
+    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 }  // namespace b200wkv

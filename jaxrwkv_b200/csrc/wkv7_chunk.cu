@@ -118,7 +118,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                       int* __restrict__ range_flag, int range_ticket, int* __restrict__ residual_mark,
                       __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces,
                       const BlockParts parts) {
-    let_next_in();
+    if (kBlocks) let_next_in();
     extern __shared__ __align__(1024) unsigned char smem[];   // (the swizzle of the output tile is a function of the address)
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     // (all first pieces come first in the grid: where no cut exists the other pieces' CTAs return at once, and the
@@ -440,18 +440,27 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
         tc::fence_after_sync();
         // ================= E1: triangular masks, operands of the next products =================
+        if (inner) {                              // nothing from in front of the row's last start flag
+            const uint64_t upto = mask & ((2ull << (row & 63)) - 1ull);
+            const int from = upto != 0 ? 63 - __clzll((long long)upto) : 0;
+#pragma unroll
+            for (int part = 0; part < 2; ++part) {
+                float x[32];
+                const uint32_t at = lane_addr + D1 + hsel * 64 + part * 32;
+                tc::tmem_ld32(at, x);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int s = 0; s < 32; ++s) x[s] = s + part * 32 >= from ? x[s] : 0.f;
+                tc::tmem_st32(at, x);
+            }
+            tc::tmem_wait_st();
+        }
         {
             const int t = row & 63;
             float d[64];
             tc::tmem_ld32(lane_addr + D1 + hsel * 64, d);
             tc::tmem_ld32(lane_addr + D1 + hsel * 64 + 32, d + 32);
             tc::tmem_wait_ld();
-            if (inner) {                          // nothing from in front of the row's last start flag
-                const uint64_t upto = mask & ((2ull << t) - 1ull);
-                const int from = upto != 0 ? 63 - __clzll((long long)upto) : 0;
-#pragma unroll
-                for (int s = 0; s < 64; ++s) d[s] = s >= from ? d[s] : 0.f;
-            }
             if (row < 64 && hsel == 0) {          // A_ab, strictly lower, fp32 for the inverse
 #pragma unroll
                 for (int c = 0; c < 16; ++c)

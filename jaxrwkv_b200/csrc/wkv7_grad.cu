@@ -132,8 +132,7 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
                      __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ da, __nv_bfloat16* __restrict__ db,
                      int* __restrict__ status, int has_dy, unsigned char* __restrict__ fscr_all,
                      const __grid_constant__ StreamMaps maps, const __grid_constant__ StreamMaps out_maps) {
-    let_next_in();
-    if (word_behind(residual_mark) != 0) return;   // the forward fell back to the sequential kernels
+    if (*residual_mark != 0) return;            // the forward fell back to the sequential kernels
     extern __shared__ __align__(1024) unsigned char smem[];
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -258,6 +257,7 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         }
         tc::fence_async_smem();
         __syncthreads();   // the staging tiles are empty; the previous block's last epilogue has finished everywhere
+        const bool flagged = inner();
         if (issuer_b && pend_dw) {
             tc::tensor_store_2d(&out_maps.m[OUT_W], pend_x, pend_y, smem + OFF_TV);
             tc::bulk_commit();
@@ -365,12 +365,12 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         // ================= R2: [Gd ; dVpart] = [B~;K~] dSL^T + [P_rb|P_rk]^T dY =================
         if (issuer_a) {
             tc::fence_after_sync();
-            mma_k64(tbase + (inner() ? T_W : T_GD), kmaj128u(sBK), kmaj64u(sDSL), ID_KK, false);
+            mma_k64(tbase + (flagged ? T_W : T_GD), kmaj128u(sBK), kmaj64u(sDSL), ID_KK, false);
             if (!tc::mbar_wait(&sm.bar[5], par)) failed = true;   // P_rb | P_rk (and sa) have landed
-            mma_k64(tbase + T_GD, mnmaj64u(sPRB), mnmaj128u(sDD), ID_MM, !inner());
+            mma_k64(tbase + T_GD, mnmaj64u(sPRB), mnmaj128u(sDD), ID_MM, !flagged);
             tc::commit(&sm.bar[0]);
         }
-        if (inner()) {   // the dS share: only the rows behind the last flag
+        if (flagged) {   // the dS share: only the rows behind the last flag
             if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
             tc::fence_after_sync();
             float x[32], y[32];
@@ -476,7 +476,7 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         if (tid == kFindThread) find_item(it.id + (int)gridDim.x, &sm.item[par ^ 1]);   // the next block of this CTA
         if (!tc::mbar_wait(&sm.bar[2], par)) failed = true;
         tc::fence_after_sync();
-        if (inner()) {   // W: s stays in front of the first flag behind t; [V;sa] dSL: only the rows behind the last flag
+        if (flagged) {   // W: s stays in front of the first flag behind t; [V;sa] dSL: only the rows behind the last flag
             const int t = row & 63;
             const uint64_t behind = (mask_of() >> t) >> 1;
             const int hi = behind != 0 ? t + __ffsll((long long)behind) : kC;
@@ -554,14 +554,14 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
             tc::commit(&sm.bar[3]);
         } else if (issuer_b) {
             tc::fence_after_sync();
-            mma_k64(tbase + T_RA, mnmaj128u(sWY + HALF), mnmaj128u(sBK), ID_MM, false);
-            mma_k64(tbase + T_RA, mnmaj128u(sWY), mnmaj128u(sBK + HALF), ID_MM, true);
             if (it.n == kC) {
                 tc::tensor_store_2d(&out_maps.m[OUT_V], it.h * kN, it.bi * Tlen + it.p, smem + OFF_TV);
                 tc::bulk_commit();
             }
+            mma_k64(tbase + T_RA, mnmaj128u(sWY + HALF), mnmaj128u(sBK), ID_MM, false);
+            mma_k64(tbase + T_RA, mnmaj128u(sWY), mnmaj128u(sBK + HALF), ID_MM, true);
             if (!tc::mbar_wait(&sm.bar[7], par)) failed = true;   // S0 has landed
-            mma_k64(tbase + (inner() ? T_GD : T_RA), kmaj128u(sDD), mnmaj64u(sX1), ID_KM, !inner());
+            mma_k64(tbase + (flagged ? T_GD : T_RA), kmaj128u(sDD), mnmaj64u(sX1), ID_KM, !flagged);
             tc::bulk_wait_read<0>();   // the dV tile has left before this round is reported done: the last epilogue writes over it
             tc::commit(&sm.bar[3]);
         }
@@ -576,7 +576,7 @@ wkv7_grad_bwd_kernel(int Tlen, int H, int BH, const uint32_t* __restrict__ lengt
         }
         if (!tc::mbar_wait(&sm.bar[3], par)) failed = true;
         tc::fence_after_sync();
-        if (inner()) {   // [dY;dG] S0: only the rows in front of the first flag
+        if (flagged) {   // [dY;dG] S0: only the rows in front of the first flag
             const bool first = in_first(t);
 #pragma unroll
             for (int part = 0; part < 2; ++part) {
@@ -761,12 +761,11 @@ int wkv7_grad_bwd(cudaStream_t st, int B, int T, int H, const void* w, const voi
     long long slots = 2LL * sm_count_of_current_device();
     if (slots > kGradCtas) slots = kGradCtas;        // every CTA owns a set of factor tiles in the residual
     const int grid = (int)(items < slots ? items : slots);
-    return launch_behind(wkv7_grad_bwd_kernel, grid, 256, SMEM_BYTES, st, T, H, BH, length, ns, (const bf*)(base + lay.dstate), s_at_len, saved,
+    wkv7_grad_bwd_kernel<<<grid, 256, SMEM_BYTES, st>>>(T, H, BH, length, ns, (const bf*)(base + lay.dstate), s_at_len, saved,
                                                         residual_mark, (bf*)dw, (bf*)dr, (bf*)dk,
                                                         (bf*)dv, (bf*)da, (bf*)db, wkv7_chunk_status_word(), dy != nullptr ? 1 : 0,
-                                                        (unsigned char*)(base + lay.fscr), maps, out_maps) == cudaSuccess
-               ? B200WKV_OK
-               : B200WKV_ELAUNCH;
+                                                        (unsigned char*)(base + lay.fscr), maps, out_maps);
+    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 }  // namespace b200wkv

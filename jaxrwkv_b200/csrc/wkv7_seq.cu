@@ -42,7 +42,7 @@ wkv7_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ w, const T* __restric
                     T* __restrict__ dw, T* __restrict__ dr, T* __restrict__ dk, T* __restrict__ dv,
                     T* __restrict__ da, T* __restrict__ db, T* __restrict__ ds0, const int* __restrict__ run_if) {
     // as the fallback behind the chunked backward: run only when the forward marked the residual as this kernel's
-    if (run_if != nullptr && word_behind(run_if) == 0) return;
+    if (run_if != nullptr && *run_if == 0) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BwdSmem& sm = *reinterpret_cast<BwdSmem*>(smem_raw);
     const int nC = (Tlen + kCk - 1) / kCk, runs = (nC + run - 1) / run;
@@ -416,12 +416,6 @@ static int launch_bwd(cudaStream_t st, int B, int Tlen, int H, const void* w, co
         const int s = wkv7_chain_bwd(st, code, B, Tlen, H, run, w, r, a, b, dy, ds_out, length, ns, ds0, carry, run_if);
         if (s != B200WKV_OK) return s;
     }
-    if (run_if != nullptr)
-        return launch_behind(kern, B * H * runs, 256, sizeof(BwdSmem), st, Tlen, H, (const T*)w, (const T*)r, (const T*)k, (const T*)v, (const T*)a,
-                             (const T*)b, (const T*)s0, length, ns, (const T*)dy, (const T*)ds_out, (const float*)residual, carry, run, (T*)dw,
-                             (T*)dr, (T*)dk, (T*)dv, (T*)da, (T*)db, (T*)ds0, run_if) == cudaSuccess
-                   ? B200WKV_OK
-                   : B200WKV_ELAUNCH;
     kern<<<B * H * runs, 256, sizeof(BwdSmem), st>>>(Tlen, H, (const T*)w, (const T*)r, (const T*)k, (const T*)v,
                                                      (const T*)a, (const T*)b, (const T*)s0, length, ns, (const T*)dy,
                                                      (const T*)ds_out, (const float*)residual, carry, run, (T*)dw, (T*)dr, (T*)dk,
