@@ -43,7 +43,12 @@ int wkv7_mix_pre_bwd(cudaStream_t st, int dtype, int rows, int C, int use_vmix, 
 // y == NULL: x = act(x) in place; else x *= act'(.) in terms of y = act(.)
 enum { kTanh = 1, kSigmoid = 2 };
 int activation(cudaStream_t st, int dtype, int act, long long n, void* x, const void* y);
-// out[c] = sum over rows of partial[row][c], in the element type
-int column_sums(cudaStream_t st, int dtype, long long rows, long long cols, const float* partial, void* out);
+// The column sums of up to three arrays of partial rows, one behind the other into `out` in the element type (columns: a
+// multiple of 32 each).
+struct PartialRows {
+    const float* partial;
+    int rows, cols;
+};
+int column_sums(cudaStream_t st, int dtype, const PartialRows (&of)[3], void* out);
 
 }  // namespace b200wkv

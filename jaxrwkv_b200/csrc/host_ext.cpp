@@ -618,6 +618,7 @@ struct Layer {
 
     struct Kept {                      // what the backward needs beside the parameters
         Tensor x, state, v_first, v, slab, length, starts, residual;
+        Tensor rows[2];                // the state's first row and the others, where they had to be made dense
     };
 
     // returns (out (B, T, C), new_state)
@@ -629,12 +630,12 @@ struct Layer {
         const Flags f(length, starts, {d.B}, d.T, x_);
         const Tensor x = x_.contiguous(), state = state_.contiguous();
         kept = {x, state, d.first ? Tensor() : v_first.contiguous(), fresh({d.B, d.T, d.C}, x.scalar_type(), x), Inter::make(x, d).t, f.length,
-                f.starts, Tensor()};
+                f.starts, Tensor(), {}};
         const Inter q(Slab(kept.slab, x.element_size()), d);
         Gemm gemm(x, st);
-        Tensor room[2], new_state = fresh_like(state), o = fresh({d.B, d.T, d.C}, x.scalar_type(), x);
-        const void* prev = dense_rows(state, 0, 1, room[0], st);
-        const void* s0 = dense_rows(state, 1, kN, room[1], st);
+        Tensor new_state = fresh_like(state), o = fresh({d.B, d.T, d.C}, x.scalar_type(), x);
+        const void* prev = dense_rows(state, 0, 1, kept.rows[0], st);
+        const void* s0 = dense_rows(state, 1, kN, kept.rows[1], st);
         const Landing shift_row(new_state, 0, 1), s_out(new_state, 1, kN);
         const void* mix[6];
         for (int i = 0; i < 6; ++i) mix[i] = in(p[kMix + i]);
@@ -712,7 +713,8 @@ struct Layer {
         check(b200wkv7_mix_post_bwd(st, code, d.rows, H, (int)kN, kEps, q.y, q.r, q.kp, q.vp, q.g, in(p[kLnW]), in(p[kLnB]), in(p[kRk]), gxo, dy, dr,
                                     dkp, dvp, dg, part_post));
         Tensor copies[2];
-        const void* s0 = dense_rows(kept.state, 1, kN, copies[0], st);
+        const auto kept_rows = [&](int i) { return kept.rows[i].defined() ? in(kept.rows[i]) : at((void*)in(kept.state), i * d.C, x); };
+        const void *s0 = kept_rows(1), *prev = kept_rows(0);
         const void* gs = dense_rows(gstate, 1, kN, copies[1], st);
         if (wanted[1]) g[1] = fresh_like(kept.state);
         const Tensor state_room = wanted[1] ? g[1] : fresh_like(kept.state);
@@ -751,19 +753,14 @@ struct Layer {
         const Tensor gx = fresh({d.B, d.T, d.C}, x.scalar_type(), x);
         const void* mix[6];
         for (int i = 0; i < 6; ++i) mix[i] = in(p[kMix + i]);
-        Tensor rows0[2];
-        const void* prev = dense_rows(kept.state, 0, 1, rows0[0], st);
-        const void* gstate0 = dense_rows(gstate, 0, 1, rows0[1], st);
+        const void* gstate0 = dense_rows(gstate, 0, 1, copies[0], st);
         check(b200wkv::token_shift_bwd(st, code, B, T, C, 6, in(x), prev, mix, (const uint32_t*)in(kept.length), (const uint8_t*)in(kept.starts), gmixed,
                                        gstate0, out(gx), gprev.p, part_mix));
         if (wanted[0]) g[0] = gx;
         if (wanted[1]) gprev.finish(st);
         // parameter gradients: column sums of the kernels' partial rows
         const Tensor sums = fresh({14, d.C}, x.scalar_type(), x);
-        const auto row = [&](int i) { return at(out(sums), i * d.C, x); };
-        check(b200wkv::column_sums(st, code, d.B * tiles, 6 * C, part_mix, row(0)));
-        check(b200wkv::column_sums(st, code, n_part, 5 * C, part_pre, row(6)));
-        check(b200wkv::column_sums(st, code, n_part, 3 * C, part_post, row(11)));
+        check(b200wkv::column_sums(st, code, {{part_mix, B * tiles, 6 * C}, {part_pre, n_part, 5 * C}, {part_post, n_part, 3 * C}}, out(sums)));
         const int order[14] = {kMix, kMix + 1, kMix + 2, kMix + 3, kMix + 4, kMix + 5, kW0, kA0, kV0, kKk, kKa, kLnW, kLnB, kRk};
         for (int i = 0; i < 14; ++i)
             if (want(order[i]) && p[order[i]].defined()) g[3 + order[i]] = sums[i].view(p[order[i]].sizes());
@@ -778,7 +775,7 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
         Layer::Kept k;
         auto [o, new_state] = Layer::forward(d, x, state, v_first, params.data(), length, starts, true, k);
         variable_list keep(params.begin(), params.end());
-        for (const Tensor& t : {k.x, k.state, k.v_first, k.v, k.slab, k.length, k.starts, k.residual}) keep.push_back(t);
+        for (const Tensor& t : {k.x, k.state, k.v_first, k.v, k.slab, k.length, k.starts, k.residual, k.rows[0], k.rows[1]}) keep.push_back(t);
         ctx->saved_data["H"] = H;
         ctx->saved_data["first"] = first;
         ctx->save_for_backward(keep);
@@ -789,7 +786,7 @@ struct LayerNode : public torch::autograd::Function<LayerNode> {
         const variable_list saved = ctx->get_saved_variables();
         const bool first = ctx->saved_data["first"].toBool();
         const Tensor* s = saved.data() + Layer::kParams;
-        const Layer::Kept k{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7]};
+        const Layer::Kept k{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], {s[8], s[9]}};
         const Layer::Dims d(k.x, saved.data(), ctx->saved_data["H"].toInt(), first);
         std::vector<bool> wanted(3 + Layer::kParams);
         for (int j = 0; j < 3 + Layer::kParams; ++j) wanted[j] = ctx->needs_input_grad(j);
