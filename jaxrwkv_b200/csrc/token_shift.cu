@@ -7,6 +7,7 @@
 // One pass over x, M outputs: purely HBM-bound, so every thread moves V channels per access with
 // V = 16 bytes / element size when the channel count allows it (else V = 4).
 #include "common.cuh"
+#include "device_once.cuh"
 #include "host_calls.h"
 
 namespace b200wkv {
@@ -117,37 +118,43 @@ __global__ void token_shift_fwd_kernel(int B, int Tlen, int D, int M, const T* _
     if (t == last_row(length[bi], Tlen)) storev(state_out + (size_t)bi * D + d, xc);
 }
 
-// Backward.  Each thread owns V channels of one tile of B200WKV_SHIFT_TILE tokens of one batch row and
-// walks it from the last token to the first (the loads do not depend on the walk, so they pipeline).
+// Backward.  A thread owns V channels of a tile of B200WKV_SHIFT_TILE tokens of one batch row, or of one of the kParts parts
+// of it, and walks its tokens from the last to the first (the loads do not depend on the walk, so they pipeline; a part reads
+// the token behind it for itself).
 // The mix gradients leave as one fp32 partial sum per (batch row, tile): deterministic, no atomics.
 //   gx[t] = sum_m g_m[t] (1 - c_m) + [t+1 < T and not start[t+1]] sum_m g_m[t+1] c_m + [t == last] gstate
-// grid (ceil(D / V / 64), tiles, B)
-template <typename T, int V, int MM>
-__global__ void __launch_bounds__(64)
+// grid (ceil(D / V / kLanes), tiles, B)
+template <typename T, int V, int MM, int kLanes, int kParts>
+__global__ void __launch_bounds__(kLanes * kParts)
 token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T* __restrict__ prev,
                        const MixPtrs mix, const uint32_t* __restrict__ length,
                        const uint8_t* __restrict__ new_starts, const T* __restrict__ gout,
                        const T* __restrict__ gstate, T* __restrict__ gx, T* __restrict__ gprev,
                        float* __restrict__ gmix) {
-    const int d = (blockIdx.x * blockDim.x + threadIdx.x) * V;
+    const int lane = threadIdx.x % kLanes, part = threadIdx.x / kLanes;
+    const int d = (blockIdx.x * kLanes + lane) * V;
     const int tile = blockIdx.y, ntile = gridDim.y;
     const int bi = blockIdx.z;
-    if (d >= D) return;
-    const int t0 = tile * B200WKV_SHIFT_TILE;
-    const int t1 = min(Tlen, t0 + B200WKV_SHIFT_TILE);
+    if (kParts == 1 && d >= D) return;
+    // this thread's tokens (none, where the part lies behind the sequence's end or the channels behind the last)
+    const int t0 = tile * B200WKV_SHIFT_TILE + part * (B200WKV_SHIFT_TILE / kParts);
+    const int t1 = kParts == 1 || d < D ? min(Tlen, t0 + B200WKV_SHIFT_TILE / kParts) : t0;
+    const bool any = kParts == 1 || t0 < t1;
+    __shared__ float sums[kParts > 1 ? kParts - 1 : 1][MM][V][kLanes];
+    static_assert(B200WKV_SHIFT_TILE % kParts == 0, "parts of whole tokens");
     const int last = last_row(length[bi], Tlen);
     RawVec<V, T> craw[MM];   // the mix coefficients stay packed; unpacking them at each use is cheaper than the registers
     Vec<V> acc[MM];
 #pragma unroll
     for (int m = 0; m < MM; ++m) {
-        craw[m].load((const T*)mix.p[m] + d);
+        if (any) craw[m].load((const T*)mix.p[m] + d);
         acc[m] = zerov<V>();
     }
     const size_t base = (size_t)bi * Tlen * D + d;
     const size_t mstride = (size_t)B * Tlen * D;
     const uint8_t* ns = new_starts + (size_t)bi * Tlen;
     Vec<V> carry = zerov<V>();   // what token t+1 hands back to token t
-    if (t1 < Tlen && !ns[t1]) {
+    if (any && t1 < Tlen && !ns[t1]) {
 #pragma unroll
         for (int m = 0; m < MM; ++m) {
             const Vec<V> g = loadv<V>(gout + m * mstride + base + (size_t)t1 * D);
@@ -156,7 +163,8 @@ token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T*
             for (int i = 0; i < V; ++i) carry.f[i] = fmaf(g.f[i], cm.f[i], carry.f[i]);
         }
     }
-    Vec<V> xc = loadv<V>(x + base + (size_t)(t1 - 1) * D);
+    Vec<V> xc = zerov<V>();
+    if (any) xc = loadv<V>(x + base + (size_t)(t1 - 1) * D);
     // Tokens are taken four at a time: the 4 x (MM + 1) loads of a group are all issued, in packed form, before
     // the first token of the group is worked on, so a thread has ~450 bytes in flight at 255 registers.
     constexpr int G = 4;
@@ -205,7 +213,22 @@ token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T*
             xc = xp;
         }
     }
-    if (tile == 0) storev(gprev + (size_t)bi * D + d, carry);
+    if (any && t0 == 0) storev(gprev + (size_t)bi * D + d, carry);
+    // the parts' sums meet in a fixed order
+    if (part > 0) {
+#pragma unroll
+        for (int m = 0; m < MM; ++m)
+#pragma unroll
+            for (int i = 0; i < V; ++i) sums[part - 1][m][i][lane] = acc[m].f[i];
+    }
+    if (kParts > 1) __syncthreads();
+    if (kParts > 1 && (part > 0 || d >= D)) return;
+#pragma unroll
+    for (int m = 0; m < MM; ++m)
+#pragma unroll
+        for (int p = 0; p < kParts - 1; ++p)
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[m].f[i] += sums[p][m][i][lane];
 #pragma unroll
     for (int m = 0; m < MM; ++m) {
         float* dst = gmix + (((size_t)bi * ntile + tile) * MM + m) * D + d;
@@ -226,9 +249,17 @@ template <typename T, int V, int MM>
 void launch_bwd_m(cudaStream_t st, int B, int Tlen, int D, const void* x, const void* prev, const MixPtrs& mix,
                   const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate, void* gx, void* gprev,
                   void* gmix) {
-    dim3 grid((D / V + 63) / 64, (Tlen + B200WKV_SHIFT_TILE - 1) / B200WKV_SHIFT_TILE, B);
-    token_shift_bwd_kernel<T, V, MM><<<grid, 64, 0, st>>>(B, Tlen, D, (const T*)x, (const T*)prev, mix, length, ns,
-                                                          (const T*)gout, (const T*)gstate, (T*)gx, (T*)gprev, (float*)gmix);
+    const int tiles = (Tlen + B200WKV_SHIFT_TILE - 1) / B200WKV_SHIFT_TILE;
+    auto launch = [&](auto kernel, int lanes, int parts) {
+        const dim3 grid((D / V + lanes - 1) / lanes, tiles, B);
+        kernel<<<grid, lanes * parts, 0, st>>>(B, Tlen, D, (const T*)x, (const T*)prev, mix, length, ns, (const T*)gout, (const T*)gstate, (T*)gx,
+                                               (T*)gprev, (float*)gmix);
+    };
+    // Fewer blocks than SMs: four parts per tile instead, of 32 x V channels (B=1, T=512, D=768, M=6, bf16: 35 -> 13 us).  With
+    // more, whole tiles keep more of a row together (B=8, T=2048, D=768: 59 us against 70; B=8, T=4096, D=2048: 230 against 306).
+    const long long blocks = (long long)((D / V + 63) / 64) * tiles * B;
+    if (blocks <= sm_count_of_current_device()) launch(token_shift_bwd_kernel<T, V, MM, 32, 4>, 32, 4);
+    else launch(token_shift_bwd_kernel<T, V, MM, 64, 1>, 64, 1);
 }
 
 template <typename T, int V>
