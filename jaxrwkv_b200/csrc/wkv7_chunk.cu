@@ -20,7 +20,7 @@
 // the rows in front of the last flag, and the decayed entering state is dropped.  (Ending the chunk in front of every
 // flag instead, as an earlier form did, costs a whole chunk's time per flag, and a backward that can follow it: forward and
 // backward at B=6, T=2043, H=32 with a flag every 512 tokens took 970-990 us so, and take 676 us with the masks, while
-// sequences without flags, B=8, T=4096, H=32, take 1.44 ms either way.)  The
+// a forward without flags, B=8, T=4096, H=32, takes 595 us in that form and 597 with the masks.)  The
 // cumulative decay is not restarted: only ratios inside a segment survive the masks.  A chunk ends early only where the
 // state is wanted, at `length`, and at the end of the sequence; the rows behind its end are zero.
 //
@@ -84,6 +84,61 @@ struct Small {
 constexpr int SMEM_BYTES = OFF_SMALL + (int)sizeof(Small);
 static_assert(OFF_SCR + TRI_SCR_FLOATS * 4 <= OFF_BH, "inverse work space must fit over AR+BK+S0");
 static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
+
+// What only chunks with start flags and chunks of fewer than 64 tokens need is kept out of the walk's loop: the passes over TMEM
+// are functions that are not inlined, and the flags are read back from shared memory where a flagged chunk needs them.  With the
+// passes inlined and the flags' 64 bits live across the loop body, every chunk WITHOUT flags paid 1 % (forward with a residual at
+// B=8, T=4096, H=32: 603-607 -> 597 us; without a residual 543 -> 531; B=6, T=2043 with a flag every 512 tokens 321 -> 318).  A second copy of the loop body for full chunks without flags is no faster on such sequences and
+// loses where both kinds mix, the two bodies evicting each other's instructions (B=8, T=1024, H=32, a flag every 100 tokens: 200 us
+// against 178).
+__device__ __forceinline__ uint64_t start_mask(const Small& sm) {   // bit t: a flag on token t of the chunk
+    const volatile uint32_t* m = sm.nsm;
+    return (uint64_t)m[0] | ((uint64_t)m[1] << 32);
+}
+__device__ __forceinline__ bool in_first(uint64_t mask, int t) { return (mask & ((2ull << t) - 1ull)) == 0; }   // no flag at or before token t
+__device__ __forceinline__ bool in_last(uint64_t mask, int t) { return ((mask >> t) >> 1) == 0; }               // none behind it
+// 64 columns of the pairwise products in TMEM, row t: nothing from in front of the row's last flag
+__device__ __noinline__ void mask_pairs(uint32_t taddr, uint64_t mask, int t) {
+    const uint64_t upto = mask & ((2ull << t) - 1ull);
+    const int from = upto != 0 ? 63 - __clzll((long long)upto) : 0;
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+        float x[32];
+        tc::tmem_ld32(taddr + part * 32, x);
+        tc::tmem_wait_ld();
+#pragma unroll
+        for (int s = 0; s < 32; ++s) x[s] = s + part * 32 >= from ? x[s] : 0.f;
+        tc::tmem_st32(taddr + part * 32, x);
+    }
+    tc::tmem_wait_st();
+}
+// 32 columns of the S0 products, row t: nothing from the first flag on
+__device__ __noinline__ void mask_state_products(uint32_t taddr, uint64_t mask, int t) {
+    float g[32];
+    tc::tmem_ld32(taddr, g);
+    tc::tmem_wait_ld();
+    const bool first = in_first(mask, t);
+#pragma unroll
+    for (int c = 0; c < 32; ++c) g[c] = first ? g[c] : 0.f;
+    tc::tmem_st32(taddr, g);
+    tc::tmem_wait_st();
+}
+// 32 columns in TMEM added in fp32 onto a bf16 row in global memory; the whole warp calls it
+__device__ __noinline__ void add_to_row(uint32_t taddr, __nv_bfloat16* row, bool live) {
+    float m[32];
+    tc::tmem_ld32(taddr, m);
+    tc::tmem_wait_ld();
+    if (!live) return;
+    uint4* to = reinterpret_cast<uint4*>(row);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        float x[8];
+        unpack8(to[c], x);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[e] += m[c * 8 + e];
+        to[c] = pack8(x);
+    }
+}
 
 // four K=16 steps (64 deep) of D (+)= A B
 __device__ __forceinline__ void mma_k64(uint32_t d, Op a, Op b, uint32_t idesc, bool accumulate) {
@@ -279,9 +334,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         __syncthreads();   // nsm visible; previous chunk's shared-memory readers are done
         send_tiles();
         const uint64_t mask = (uint64_t)sm.nsm[0] | ((uint64_t)sm.nsm[1] << 32);
-        const bool reset_here = (mask & 1ull) != 0, inner = (mask >> 1) != 0;   // a flag on the first token; on others
-        auto in_first = [&](int t) { return (mask & ((2ull << t) - 1ull)) == 0; };   // no flag at or before token t of the chunk
-        auto in_last = [&](int t) { return ((mask >> t) >> 1) == 0; };               // none behind it
+        const bool reset_here = (mask & 1ull) != 0, inner = (mask >> 1) != 0, flagged = mask != 0;   // a flag on the first token; on others
         // the chunk leaves its operand slabs T, A_ak, P_rb, P_rk, sa, S0 for the backward: slot p / 64, and the last slot for
         // the second part of a block that `length` cuts (the only chunk that starts inside a block)
         const size_t blk_slot = (size_t)bh * nSlot + ((p & (kC - 1)) == 0 ? p >> 6 : nSlot - 1);
@@ -381,17 +434,18 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 slab_store(smem + OFF_KH, CB64, t, jb, scale8(raw[q][1], eE));
                 slab_store(smem + OFF_V, CB64, t, jb, raw[q][2]);
             }
-            if (mask != 0) {   // the rare chunk with start flags: the masked rows are written over
+            if (flagged) {   // the rare chunk with start flags: the masked rows are written over
+                const uint64_t m = start_mask(sm);
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int t = q * 32 + tsub;
                     const uint4 none = make_uint4(0, 0, 0, 0);
-                    if (affine && !in_first(t)) {   // what carries the dependence on S0: nothing from the first flag on
+                    if (affine && !in_first(m, t)) {   // what carries the dependence on S0: nothing from the first flag on
                         slab_store(smem + OFF_SA, CB64, t, jb, none);
                         if (t < n) *reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + jb * 8) = none;
                         tc::fence_async_global();
                     }
-                    if (!in_last(t)) {                       // what reaches S_C: nothing in front of the last flag
+                    if (!in_last(m, t)) {                       // what reaches S_C: nothing in front of the last flag
                         slab_store(smem + OFF_BH, CB64, t, jb, none);
                         slab_store(smem + OFF_KH, CB64, t, jb, none);
                     }
@@ -415,7 +469,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 const float4 l4 = *reinterpret_cast<const float4*>(&sm.lam[hsel * 32 + c * 4]);
                 s[c * 4] *= l4.x; s[c * 4 + 1] *= l4.y; s[c * 4 + 2] *= l4.z; s[c * 4 + 3] *= l4.w;
             }
-            if (mask != 0) {
+            if (flagged) {
 #pragma unroll
                 for (int c = 0; c < 32; ++c) s[c] = 0.f;
             }
@@ -436,25 +490,11 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             tc::bulk_store(keep + (size_t)SAVED_S0 * GTILE + lane * GCB, smem + OFF_S0 + lane * CB64, 64 * 16);
             tc::bulk_commit();
         }
-        if (affine && tid < 64) lam_out[blk_slot * kN + tid] = mask != 0 ? 0.f : sm.lam[tid];
+        if (affine && tid < 64) lam_out[blk_slot * kN + tid] = flagged ? 0.f : sm.lam[tid];
         if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
         tc::fence_after_sync();
         // ================= E1: triangular masks, operands of the next products =================
-        if (inner) {                              // nothing from in front of the row's last start flag
-            const uint64_t upto = mask & ((2ull << (row & 63)) - 1ull);
-            const int from = upto != 0 ? 63 - __clzll((long long)upto) : 0;
-#pragma unroll
-            for (int part = 0; part < 2; ++part) {
-                float x[32];
-                const uint32_t at = lane_addr + D1 + hsel * 64 + part * 32;
-                tc::tmem_ld32(at, x);
-                tc::tmem_wait_ld();
-#pragma unroll
-                for (int s = 0; s < 32; ++s) x[s] = s + part * 32 >= from ? x[s] : 0.f;
-                tc::tmem_st32(at, x);
-            }
-            tc::tmem_wait_st();
-        }
+        if (inner) mask_pairs(lane_addr + D1 + hsel * 64, start_mask(sm), row & 63);
         {
             const int t = row & 63;
             float d[64];
@@ -477,16 +517,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 for (int c = 0; c < 8; ++c) slab_store(dst, CB128, row, c, pack8(&d[c * 8]));
             }
         }
-        if (!kBlocks && inner) {                  // A~ S0^T and R~ S0^T: nothing from the first flag on
-            float g[32];
-            tc::tmem_ld32(lane_addr + D2 + hsel * 32, g);
-            tc::tmem_wait_ld();
-            const bool first = in_first(row & 63);
-#pragma unroll
-            for (int c = 0; c < 32; ++c) g[c] = first ? g[c] : 0.f;
-            tc::tmem_st32(lane_addr + D2 + hsel * 32, g);
-            tc::tmem_wait_st();
-        }
+        if (!kBlocks && inner) mask_state_products(lane_addr + D2 + hsel * 32, start_mask(sm), row & 63);
         if (warp == 7) tc::bulk_wait_read<0>();   // the S0 slab has been read: the inverse writes over part of it next
         tc::fence_async_smem();
         tc::fence_before_sync();
@@ -655,22 +686,14 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 for (int c = 0; c < 4; ++c) slab_store(smem + OFF_MT, GCB, row, hsel * 4 + c, pack8(&m[c * 8]));
             } else {              // R-_t = R~_t + (P_rb W~)_t on top of the R~ row stored at the start of the chunk
                 const int t = row - 64;
-                tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, m);
-                tc::tmem_wait_ld();
                 if (n == kC) {
+                    tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, m);
+                    tc::tmem_wait_ld();
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
                         *reinterpret_cast<uint4*>(smem + OFF_RT + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&m[c * 8]);
-                } else if (t < n) {   // a short chunk's rows one by one: a tiled copy would go over the next sequence's
-                    uint4* to = reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + t) * tok_stride + hsel * 32);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        float x[8];
-                        unpack8(to[c], x);
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) x[e] += m[c * 8 + e];
-                        to[c] = pack8(x);
-                    }
+                } else {              // a short chunk's rows one by one: a tiled copy would go over the next sequence's
+                    add_to_row(lane_addr + D1 + 64 + hsel * 32, rbar + seq_base + (size_t)(p + t) * tok_stride + hsel * 32, t < n);
                 }
             }
         }
