@@ -1,7 +1,7 @@
 /*
  * b200wkv_debug - schedule queries of libb200wkv.so that exist for its tests.  Not part of the
  * boundary a host framework binds (that is b200wkv.h); no jaxrwkv interface corresponds to them.
- * Neither call touches a GPU.
+ * No call launches anything.
  */
 #ifndef B200WKV_DEBUG_H_
 #define B200WKV_DEBUG_H_
@@ -18,6 +18,10 @@ extern "C" {
  * them); returns their number. */
 int b200wkv_debug_split_plan(int chains, int n_blk, int per_sm, int* grid, int* seg);
 int b200wkv_debug_runs(int chains, int seg, int grid, int cta, int* runs, int capacity);
+
+/* Decoding (b200wkv7_step_inplace): thread blocks that a full launch puts on an SM, and how many would fit one.  The kernel
+ * deals the work out in equal shares, so the two have to be equal.  Needs a device. */
+int b200wkv_debug_step_residency(int dtype, int* grid_per_sm, int* fit_per_sm);
 
 #ifdef __cplusplus
 }

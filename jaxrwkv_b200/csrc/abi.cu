@@ -22,6 +22,7 @@ int wkv7_step(cudaStream_t st, int dtype, int B, int H, const void* w, const voi
 int wkv7_step_stream(cudaStream_t st, int dtype, int B, int H, const void* w, const void* r, const void* k, const void* v,
                      const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
                      void* s_out, long long s_batch_stride);
+int wkv7_step_stream_residency(int dtype, int* grid_per_sm, int* fit_per_sm);
 size_t wkv7_chunk_residual_bytes(int B, int T, int H);
 int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v,
                    const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
@@ -379,6 +380,12 @@ int b200wkv7_mix_post_bwd(void* stream, int dtype, long long rows, int H, int N,
     if (!aligned16({y, r, k, v, g, ln_w, ln_b, r_k, gx, dy, dr, dk, dv, dg, partial})) return B200WKV_EUNSUPPORTED;
     return wkv7_mix_post_bwd((cudaStream_t)stream, dtype, (int)rows, H * N, eps, y, r, k, v, g, ln_w, ln_b, r_k, gx, dy, dr, dk,
                              dv, dg, partial);
+}
+
+int b200wkv_debug_step_residency(int dtype, int* grid_per_sm, int* fit_per_sm) {
+    if (dtype != B200WKV_F32 && dtype != B200WKV_BF16) return B200WKV_EDTYPE;
+    if (!grid_per_sm || !fit_per_sm) return B200WKV_ENULL;
+    return wkv7_step_stream_residency(dtype, grid_per_sm, fit_per_sm);
 }
 
 int b200wkv_debug_split_plan(int chains, int n_blk, int per_sm, int* grid, int* seg) {

@@ -61,9 +61,14 @@ template <> struct Tile<float> {
     }
 };
 
-// Resident CTAs of one grid per SM.  Four rings of four 9 KB stages are 22 MB in flight over the chip, more than the latency
-// times the bandwidth; what they leave of the shared memory lets the first CTAs of the next grid in while this one drains.
+// CTAs of one grid per SM.  The launcher asks for at least kMinSmem of shared memory, so that no more than these fit: the CTAs take
+// equal shares of the pairs, and with room for a fifth (four stages are 39 KB) the CTAs of a grid launched behind another fill
+// whichever SM drains first, which leaves some SMs with five of them and others with three.  us per layer, 40 heads, bf16, five
+// admitted / exactly four: 12.2 / 11.0 at B=64, 38.6 / 31.9 at 256 (32 layers), 71.8 / 58.8 at 512, 137.9 / 113.4 at 1024.  A grid of five
+// per SM: 11.1, 31.5 and (1024) 118.0; five stages with four per SM: 11.3, 32.4, 59.7 and 115.9.
 constexpr int kCtasPerSm = 4;
+constexpr int kSmemOfSm = 228 * 1024, kSmemPerCta = 1024;    // shared memory of an SM; what the system takes of it per CTA
+constexpr int kMinSmem = (kSmemOfSm / (kCtasPerSm + 1) - kSmemPerCta) / 1024 * 1024 + 2048;
 constexpr int kFlagBatch = 64;   // the computing threads fetch the flags of this many pairs at a time
 
 template <typename T>
@@ -80,6 +85,11 @@ struct StepSmem {
     uint64_t full[Tile<T>::kStages];   // the stage's bytes have arrived
     uint64_t done[Tile<T>::kStages];   // both computing warps have taken the stage into registers
 };
+
+template <typename T>
+constexpr int smem_bytes() { return (int)sizeof(StepSmem<T>) > kMinSmem ? (int)sizeof(StepSmem<T>) : kMinSmem; }
+static_assert(kCtasPerSm * (smem_bytes<__nv_bfloat16>() + kSmemPerCta) <= kSmemOfSm && kCtasPerSm * (smem_bytes<float>() + kSmemPerCta) <= kSmemOfSm,
+              "kCtasPerSm CTAs fit");
 
 __device__ __forceinline__ void compute_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory"); }
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -280,25 +290,28 @@ wkv7_step_stream_kernel(int BH, int H, const T* __restrict__ w, const T* __restr
 }
 
 template <typename T>
+cudaError_t resident_ctas(int* n) {      // that fit an SM at once
+    const cudaError_t e = cudaFuncSetAttribute(wkv7_step_stream_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes<T>());
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, wkv7_step_stream_kernel<T>, kThreads, smem_bytes<T>());
+}
+
+template <typename T>
 int launch(cudaStream_t st, int B, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
            const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out,
            long long s_batch_stride) {
     // facts that depend only on (kernel instance, device) are looked up once per device: the shared-memory
     // opt-in, how many CTAs of this kernel fit an SM, and the address of the device status word
     auto kern = wkv7_step_stream_kernel<T>;
-    const int smem = (int)sizeof(StepSmem<T>);
     static DeviceOnce setup;
     static int per_sm_of[kMaxDevices];
     static int* status_of[kMaxDevices];
     const int dev = current_device();
     if (dev < 0) return B200WKV_ELAUNCH;
     if (!setup.ok([&]() {
-            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-            if (e != cudaSuccess) return e;
             int n = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, kThreads, smem) != cudaSuccess || n < 1) n = 1;
-            if (n > kCtasPerSm) n = kCtasPerSm;
-            per_sm_of[dev] = n;
+            const cudaError_t e = resident_ctas<T>(&n);
+            if (e != cudaSuccess) return e;
+            per_sm_of[dev] = n < 1 ? 1 : n > kCtasPerSm ? kCtasPerSm : n;
             status_of[dev] = wkv7_chunk_status_word();
             return cudaSuccess;
         }))
@@ -315,7 +328,7 @@ int launch(cudaStream_t st, int B, int H, const void* w, const void* r, const vo
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = smem_bytes<T>();
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
@@ -326,6 +339,12 @@ int launch(cudaStream_t st, int B, int H, const void* w, const void* r, const vo
 }
 
 }  // namespace
+
+int wkv7_step_stream_residency(int dtype, int* grid_per_sm, int* fit_per_sm) {
+    *grid_per_sm = kCtasPerSm;
+    const cudaError_t e = dtype == B200WKV_F32 ? resident_ctas<float>(fit_per_sm) : resident_ctas<__nv_bfloat16>(fit_per_sm);
+    return e == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+}
 
 // Requires s0 and the six streams 16-byte aligned (bulk copies), s_out 32-byte aligned (32-byte stores)
 // and a batch stride that keeps every state so aligned; the caller checks.  s_out may be s0 (update in place): a pair's state
