@@ -7,6 +7,7 @@
 
 namespace b200wkv {
 size_t wkv7_seq_residual_bytes(int B, int T, int H);
+size_t wkv7_seq_carry_bytes(int B, int T, int H);
 int wkv7_seq_fwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w, const void* r, const void* k,
                  const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
                  const uint8_t* ns, void* y, void* s_out, void* residual, const int* run_if, int run_ticket,
@@ -139,9 +140,9 @@ size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N) {
     if (check_dims(dtype, B, T, H, N) != B200WKV_OK) return 0;
     // fp32 uses the sequential kernels (a state every 16 tokens); bf16 uses the chunked tensor-core
     // kernels (a state every 64 tokens) unless B200WKV_FLAG_SEQUENTIAL asks otherwise, so size for both
-    // (fp32: and as much again for the state gradients that the backward leaves between the chunks it walks side by side)
+    // (fp32: and for the state gradients between the chunks that the backward walks side by side, where it does)
     const size_t seq = wkv7_seq_residual_bytes(B, T, H);
-    if (dtype == B200WKV_F32) return 2 * seq;
+    if (dtype == B200WKV_F32) return seq + wkv7_seq_carry_bytes(B, T, H);
     const size_t chk = wkv7_chunk_residual_bytes(B, T, H);
     // + one word at the end that says which of the two formats the forward left (see residual_mark_of)
     return (seq > chk ? seq : chk) + kResidualMarkBytes;

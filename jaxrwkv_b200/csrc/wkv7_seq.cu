@@ -375,15 +375,43 @@ size_t wkv7_seq_residual_bytes(int B, int T, int H) {
     return (size_t)B * H * ((T + kCk - 1) / kCk) * kN * kN * sizeof(float);
 }
 
+// CTAs of the backward kernel that an SM takes (0: no device); opts in to its shared memory
+template <typename T>
+static int bwd_ctas_per_sm() {
+    static DeviceOnce once;   // one per template instance; the attribute is per device
+    static int per_sm_of[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0 || !once.ok([dev]() {
+            auto kern = wkv7_seq_bwd_kernel<T>;
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem));
+            int n = 0;
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, sizeof(BwdSmem)) != cudaSuccess || n < 1) n = 1;
+            per_sm_of[dev] = n;
+            return e;
+        }))
+        return 0;
+    return per_sm_of[dev];
+}
+
+// Whether the sequences fill their waves of CTAs by themselves.  Then runs would only add the carry, and a sequence is one run
+// (forward and backward, fp32, in runs / in one: 400 sequences of 200 tokens 1051 / 974 us, 128 of 512 tokens 858 / 813 us).
+template <typename T>
+static bool fills_waves(long long seqs) {
+    const long long slots = (long long)bwd_ctas_per_sm<T>() * sm_count_of_current_device();
+    return slots > 0 && 20 * seqs >= 17 * ((seqs + slots - 1) / slots) * slots;
+}
+
+// What the fp32 backward has use for behind the checkpoints: as much again, for the state gradients between the chunks, where it
+// walks them side by side.
+size_t wkv7_seq_carry_bytes(int B, int T, int H) { return fills_waves<float>((long long)B * H) ? 0 : wkv7_seq_residual_bytes(B, T, H); }
+
 // Chunks per run: as few as the room behind the checkpoints has places for (one state gradient between two runs), and all
-// of them, without a carry, where there is none.  One run per sequence also where the sequences fill their waves of `slots`
-// CTAs by themselves: then the runs only add the carry (forward and backward, fp32, in runs / in one: 400
-// sequences of 200 tokens 1051 / 974 us, 128 of 512 tokens 858 / 813 us).
-static int run_length(int B, int T, int H, size_t room, long long slots) {
-    const int nC = (T + kCk - 1) / kCk;
+// of them, without a carry, where there is none or the sequences fill their waves.
+template <typename T>
+static int run_length(int B, int Tlen, int H, size_t room) {
+    const int nC = (Tlen + kCk - 1) / kCk;
     const size_t one = (size_t)B * H * kN * kN * sizeof(float);
-    const long long seqs = (long long)B * H, waves = (seqs + slots - 1) / slots;
-    if (20 * seqs >= 17 * waves * slots) return nC;
+    if (fills_waves<T>((long long)B * H)) return nC;
     int run = 1;
     while (run < nC && (size_t)((nC - 1) / run) * one > room) run *= 2;
     return run < nC ? run : nC;
@@ -395,21 +423,11 @@ static int launch_bwd(cudaStream_t st, int B, int Tlen, int H, const void* w, co
                       const uint8_t* ns, const void* dy, const void* ds_out, void* residual, size_t residual_bytes, void* dw,
                       void* dr, void* dk, void* dv, void* da, void* db, void* ds0, const int* run_if) {
     auto kern = wkv7_seq_bwd_kernel<T>;
-    static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
-    static int per_sm_of[kMaxDevices];
-    const int dev = current_device();
-    if (dev < 0 || !smem_attr.ok([kern, dev]() {
-            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem));
-            int n = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, sizeof(BwdSmem)) != cudaSuccess || n < 1) n = 1;
-            per_sm_of[dev] = n;
-            return e;
-        }))
-        return B200WKV_ELAUNCH;
+    if (bwd_ctas_per_sm<T>() == 0) return B200WKV_ELAUNCH;
     const size_t used = wkv7_seq_residual_bytes(B, Tlen, H);
     const int nC = (Tlen + kCk - 1) / kCk;
     // (behind the chunked kernels the launch nearly always finds nothing to do: one CTA per sequence, no carry)
-    const int run = run_if != nullptr ? nC : run_length(B, Tlen, H, residual_bytes - used, (long long)per_sm_of[dev] * sm_count_of_current_device()), runs = (nC + run - 1) / run;
+    const int run = run_if != nullptr ? nC : run_length<T>(B, Tlen, H, residual_bytes - used), runs = (nC + run - 1) / run;
     float* const carry = reinterpret_cast<float*>(static_cast<char*>(residual) + used);
     if (runs > 1) {
         const int code = sizeof(T) == 4 ? B200WKV_F32 : B200WKV_BF16;
