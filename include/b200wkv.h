@@ -37,7 +37,9 @@ extern "C" {
 #define B200WKV_ENULL        -3   /* a required pointer is NULL                          */
 #define B200WKV_ERESIDUAL    -4   /* residual buffer smaller than *_residual_bytes()     */
 #define B200WKV_ELAUNCH      -5   /* the CUDA runtime refused the launch                 */
-#define B200WKV_EUNSUPPORTED -6   /* combination not available in this build             */
+#define B200WKV_EUNSUPPORTED -6   /* combination not available in this build, or an       */
+                                  /* operand's address does not suit the vector accesses  */
+                                  /* (four elements; 16 bytes on the tensor-core paths)   */
 #define B200WKV_ESCRATCH     -7   /* problem larger than a fixed built-in scratch area   */
 #define B200WKV_ESYMBOL      -8   /* the built-in scratch area could not be materialised  */
 

@@ -46,6 +46,7 @@ int wkv6_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r,
                  void* du, void* ds0, const int* run_if, bool rest_only = false);
 // A constant decay (versions 5, 5.2): fp32-accurate, run-parallel; `rest_only` above: what of the call these two left out
 size_t wkv5_exact_partial_bytes(int B, int T, int H);
+bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands);
 int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
                    const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark);
 int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
@@ -80,6 +81,16 @@ size_t wkv7_residual_min_bytes(int dtype, int B, int T, int H) {
     return dtype == B200WKV_F32 ? wkv7_seq_residual_bytes(B, T, H) : b200wkv7_residual_bytes(dtype, B, T, H, kN);
 }
 
+// Whether all of these lie on boundaries of `bytes` (NULL does).  The kernels read and write vectors; an address that does not
+// suit them is refused here, since a misaligned access ends the process's work on the device.
+static bool aligned(size_t bytes, std::initializer_list<const void*> ps) {
+    uintptr_t bits = 0;
+    for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
+    return bits % bytes == 0;
+}
+// four elements, what the token-sequential kernels access at a time
+static size_t vec4_bytes(int dtype) { return dtype == B200WKV_F32 ? 16 : 8; }
+
 static int check_dims(int dtype, int B, int T, int H, int N) {
     if (dtype != B200WKV_F32 && dtype != B200WKV_BF16) return B200WKV_EDTYPE;
     if (B < 1 || T < 1 || H < 1 || N != kN) return B200WKV_ESHAPE;
@@ -96,9 +107,14 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
     if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
     if (residual != nullptr && residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
     // one token and no residual wanted (recurrent decoding): a single pass over the state
-    if (T == 1 && residual == nullptr)
+    if (T == 1 && residual == nullptr) {
+        if (!aligned(vec4_bytes(dtype), {w, r, k, v, a, b}) || !aligned(16, {s0, s_out})) return B200WKV_EUNSUPPORTED;
         return wkv7_step((cudaStream_t)stream, dtype, B, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out);
-    if (dtype == B200WKV_BF16 && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
+    }
+    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
+    if (!aligned(sequential ? vec4_bytes(dtype) : 16, {w, r, k, v, a, b, s0, y, s_out}) || !aligned(16, {residual, workspace}))
+        return B200WKV_EUNSUPPORTED;
+    if (!sequential) {
         int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
         int *range_flag = nullptr, ticket = 0;
         st = wkv7_chunk_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, workspace, mark,
@@ -125,7 +141,7 @@ const char* b200wkv_strerror(int status) {
         case B200WKV_ENULL: return "a required pointer is NULL";
         case B200WKV_ERESIDUAL: return "residual buffer is smaller than the size reported by *_residual_bytes";
         case B200WKV_ELAUNCH: return "CUDA kernel launch failed";
-        case B200WKV_EUNSUPPORTED: return "combination not available in this build";
+        case B200WKV_EUNSUPPORTED: return "combination not available in this build, or an operand's address does not suit the kernels' vector accesses";
         case B200WKV_ESCRATCH: return "problem exceeds the fixed built-in scratch area";
         case B200WKV_ESYMBOL: return "the built-in scratch area could not be materialised on this device (module load failed: out of device memory?)";
         default: return "unknown status";
@@ -166,8 +182,12 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
         !da || !db || !ds0)
         return B200WKV_ENULL;
     if (residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
+    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
+    if (!aligned(sequential ? vec4_bytes(dtype) : 16, {w, r, k, v, a, b, dy, dw, dr, dk, dv, da, db}) ||
+        !aligned(vec4_bytes(dtype), {s0, ds_out, ds0}) || !aligned(16, {residual}))
+        return B200WKV_EUNSUPPORTED;
     // must match the kernel family that filled the residual in b200wkv7_fwd (same dtype and flags)
-    if (dtype == B200WKV_BF16 && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
+    if (!sequential) {
         const int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
         // the sequential state-gradient carry, then the gradients of all blocks in parallel; the sequential kernels behind
         // them return at once unless the forward fell back to them
@@ -203,20 +223,26 @@ int b200wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int 
     if (version != 5 && version != 6) return B200WKV_EUNSUPPORTED;
     if (!r || !k || !v || !w || !u || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
     if (residual != nullptr && residual_bytes < b200wkv6_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
+    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
+    const bool exact = !sequential && version != 6 && residual != nullptr;      // wkv5_exact.cu, see below
+    if (!aligned(sequential || exact ? vec4_bytes(dtype) : 16, {r, k, v, y}) || !aligned(version == 6 && !sequential ? 16 : vec4_bytes(dtype), {w}) ||
+        !aligned(16, {residual}))
+        return B200WKV_EUNSUPPORTED;
     if (dtype == B200WKV_BF16) {
         int* mark = residual_mark_of(residual, b200wkv6_residual_bytes(dtype, B, T, H, N));
         // With a constant decay (versions 5, 5.2) the decay's gradient is a sum over ALL tokens of per-token terms that
         // largely cancel; taken from bf16 tensor-core products it is only good to a few percent (10 % on short
         // sequences), so training calls of those versions take the fp32-accurate kernels of wkv5_exact.cu, with the
-        // token-sequential ones for heads outside their domain (same checkpoints, marked as such).  Their inference
+        // token-sequential ones for heads outside their domain (same checkpoints, marked as such) and for operands that the
+        // wider accesses of the former do not suit.  Their inference
         // calls, and everything of version 6, take the chunked kernels.
-        if (version != 6 && residual != nullptr && !(flags & B200WKV_FLAG_SEQUENTIAL)) {
+        if (exact && wkv5_exact_takes(T, {r, k, v, y, s0, s_out})) {
             st = wkv5_exact_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, s0, length, new_starts, y, s_out, residual, mark);
             if (st != B200WKV_OK) return st;
             return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, s0, length, new_starts, y, s_out, residual, nullptr, 0,
                                 mark, true);
         }
-        if (flags & B200WKV_FLAG_SEQUENTIAL)
+        if (sequential || exact)
             return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
                                 s_out, residual, nullptr, 0, mark);
         // the chunked tensor-core kernel, and behind it the sequential kernel, which runs only if the chunked one met
@@ -243,8 +269,13 @@ int b200wkv6_bwd(void* stream, int dtype, int version, int B, int T, int H, int 
     if (!r || !k || !v || !w || !u || !s0 || !length || !new_starts || !residual || !dr || !dk || !dv || !dw || !du || !ds0)
         return B200WKV_ENULL;
     if (residual_bytes < b200wkv6_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
+    if (!aligned(dtype == B200WKV_BF16 && version == 6 ? 16 : vec4_bytes(dtype), {r, k, v, dy, dr, dk, dv}) ||
+        !aligned(dtype == B200WKV_BF16 && version == 6 ? 16 : vec4_bytes(dtype), {w}) || !aligned(vec4_bytes(dtype), {ds_out, ds0}) ||
+        !aligned(16, {residual, dw, du}))
+        return B200WKV_EUNSUPPORTED;
     if (dtype == B200WKV_BF16 && version != 6) {
-        const bool sequential = (flags & B200WKV_FLAG_SEQUENTIAL) != 0;
+        // (either family reads the checkpoints of the other)
+        const bool sequential = (flags & B200WKV_FLAG_SEQUENTIAL) != 0 || !wkv5_exact_takes(T, {r, k, v, dy, dr, dk, dv});
         if (!sequential) {
             st = wkv5_exact_bwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, length, new_starts, dy, ds_out, residual,
                                 static_cast<char*>(residual) + wkv6_seq_residual_bytes(B, T, H), dr, dk, dv, dw, du, ds0);
@@ -318,11 +349,6 @@ int check_mix(int dtype, long long rows, int H, int N) {
     if (N != kN || H < 1 || H > 128 || rows < 1 || rows > 2147483647LL) return B200WKV_ESHAPE;
     return B200WKV_OK;
 }
-bool aligned16(std::initializer_list<const void*> ps) {
-    for (const void* p : ps)
-        if ((reinterpret_cast<uintptr_t>(p) & 15u) != 0) return false;
-    return true;
-}
 }  // namespace
 
 int b200wkv7_mix_partial_rows(long long rows, int H, int N) {
@@ -338,7 +364,7 @@ int b200wkv7_mix_pre_fwd(void* stream, int dtype, long long rows, int H, int N, 
     if (st != B200WKV_OK) return st;
     if (!k || !wl || !al || !v || !w0 || !a0 || !k_k || !k_a || !w || !k_out || !v_out || !a_i || !b_i) return B200WKV_ENULL;
     if (use_vmix && (!v_first || !vl || !v0)) return B200WKV_ENULL;
-    if (!aligned16({k, wl, al, v, v_first, vl, w0, a0, v0, k_k, k_a, w, k_out, v_out, a_i, b_i})) return B200WKV_EUNSUPPORTED;
+    if (!aligned(16, {k, wl, al, v, v_first, vl, w0, a0, v0, k_k, k_a, w, k_out, v_out, a_i, b_i})) return B200WKV_EUNSUPPORTED;
     return wkv7_mix_pre_fwd((cudaStream_t)stream, dtype, (int)rows, H * N, use_vmix ? 1 : 0, k, wl, al, v, v_first, vl, w0, a0,
                             v0, k_k, k_a, w, k_out, v_out, a_i, b_i);
 }
@@ -354,7 +380,7 @@ int b200wkv7_mix_pre_bwd(void* stream, int dtype, long long rows, int H, int N, 
         !dal || !dv || !partial)
         return B200WKV_ENULL;
     if (use_vmix && (!v_first || !vl || !v0 || !dv_first || !dvl)) return B200WKV_ENULL;
-    if (!aligned16({k, wl, al, v, v_first, vl, w0, a0, v0, k_k, k_a, gw, gk_out, gv_out, ga_i, gb_i, dk, dwl, dal, dv, dv_first,
+    if (!aligned(16, {k, wl, al, v, v_first, vl, w0, a0, v0, k_k, k_a, gw, gk_out, gv_out, ga_i, gb_i, dk, dwl, dal, dv, dv_first,
                     dvl, partial}))
         return B200WKV_EUNSUPPORTED;
     return wkv7_mix_pre_bwd((cudaStream_t)stream, dtype, (int)rows, H * N, use_vmix ? 1 : 0, k, wl, al, v, v_first, vl, w0, a0,
@@ -367,7 +393,7 @@ int b200wkv7_mix_post_fwd(void* stream, int dtype, long long rows, int H, int N,
     int st = check_mix(dtype, rows, H, N);
     if (st != B200WKV_OK) return st;
     if (!y || !r || !k || !v || !g || !ln_w || !ln_b || !r_k || !x) return B200WKV_ENULL;
-    if (!aligned16({y, r, k, v, g, ln_w, ln_b, r_k, x})) return B200WKV_EUNSUPPORTED;
+    if (!aligned(16, {y, r, k, v, g, ln_w, ln_b, r_k, x})) return B200WKV_EUNSUPPORTED;
     return wkv7_mix_post_fwd((cudaStream_t)stream, dtype, (int)rows, H * N, eps, y, r, k, v, g, ln_w, ln_b, r_k, x);
 }
 
@@ -378,7 +404,7 @@ int b200wkv7_mix_post_bwd(void* stream, int dtype, long long rows, int H, int N,
     if (st != B200WKV_OK) return st;
     if (!y || !r || !k || !v || !g || !ln_w || !ln_b || !r_k || !gx || !dy || !dr || !dk || !dv || !dg || !partial)
         return B200WKV_ENULL;
-    if (!aligned16({y, r, k, v, g, ln_w, ln_b, r_k, gx, dy, dr, dk, dv, dg, partial})) return B200WKV_EUNSUPPORTED;
+    if (!aligned(16, {y, r, k, v, g, ln_w, ln_b, r_k, gx, dy, dr, dk, dv, dg, partial})) return B200WKV_EUNSUPPORTED;
     return wkv7_mix_post_bwd((cudaStream_t)stream, dtype, (int)rows, H * N, eps, y, r, k, v, g, ln_w, ln_b, r_k, gx, dy, dr, dk,
                              dv, dg, partial);
 }
@@ -432,6 +458,7 @@ int b200wkv_token_shift_fwd(void* stream, int dtype, int B, int T, int D, int M,
     int st = check_shift(dtype, B, T, D, M);
     if (st != B200WKV_OK) return st;
     if (!x || !prev || !mix || !length || !new_starts || !out || !state_out) return B200WKV_ENULL;
+    if (!aligned(dtype == B200WKV_F32 || D % 8 == 0 ? 16 : 8, {x, prev, mix, out, state_out})) return B200WKV_EUNSUPPORTED;
     const MixRows rows(mix, dtype, D, M);
     return token_shift_fwd((cudaStream_t)stream, dtype, B, T, D, M, x, prev, rows.p, length, new_starts, out, state_out);
 }
@@ -442,6 +469,8 @@ int b200wkv_token_shift_bwd(void* stream, int dtype, int B, int T, int D, int M,
     int st = check_shift(dtype, B, T, D, M);
     if (st != B200WKV_OK) return st;
     if (!x || !prev || !mix || !length || !new_starts || !gout || !gx || !gprev || !gmix) return B200WKV_ENULL;
+    if (!aligned(dtype == B200WKV_F32 || D % 8 == 0 ? 16 : 8, {x, prev, mix, gout, gstate, gx, gprev}) || !aligned(16, {gmix}))
+        return B200WKV_EUNSUPPORTED;
     const MixRows rows(mix, dtype, D, M);
     return token_shift_bwd((cudaStream_t)stream, dtype, B, T, D, M, x, prev, rows.p, length, new_starts, gout, gstate, gx,
                            gprev, gmix);

@@ -24,6 +24,7 @@
 // Measured at B=4, T=1024, H=32: forward 515 -> 24 + 9 + 80 us, backward 1127 -> 30 + 9 + 194 + 3 us; bound by the
 // shared-memory path (61 % of its peak) and instruction issue (45 %) together, the tensor pipe at 37 %.
 // Powers of d outside d^{+-8} fp32 range: a head with a channel outside [1e-4, 1] is left to wkv6_seq.cu.
+#include <initializer_list>
 #include "common.cuh"
 #include "device_once.cuh"
 
@@ -844,6 +845,13 @@ int runs_of(int T) { return (T + kRun - 1) / kRun; }
 }  // namespace
 
 size_t wkv5_exact_partial_bytes(int B, int T, int H) { return (size_t)B * H * runs_of(T) * 2 * kN * sizeof(float); }
+
+// Rows travel in 16-byte pieces here (8 bytes in the token-sequential kernels), and the scan keeps a byte per run in shared memory.
+bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands) {
+    uintptr_t bits = 0;
+    for (const void* p : operands) bits |= reinterpret_cast<uintptr_t>(p);
+    return (bits & 15u) == 0 && runs_of(T) <= 48 * 1024;
+}
 
 int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
                    const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark) {
