@@ -124,6 +124,10 @@ Tensor cotangent(const Tensor& g, const Tensor& like) {
     return !g.defined() ? g : (g.scalar_type() == like.scalar_type() ? g : g.to(like.scalar_type())).contiguous();
 }
 
+// What stands for an optional operand that is not there: an autograd node's arguments have to be defined.
+Tensor nothing(const Tensor& like) { return fresh({0}, like.scalar_type(), like); }
+Tensor if_any(const Tensor& t) { return t.defined() && t.numel() > 0 ? t : Tensor(); }
+
 // Gradients asked for with create_graph=True: the values are right, differentiating them again is an error.
 struct Refuse : public torch::autograd::Function<Refuse> {
     static variable_list forward(AutogradContext* ctx, at::TensorList from, const std::function<variable_list()>& compute, std::string name) {
@@ -347,10 +351,10 @@ struct Wkv4 {
                                 residual ? out(*residual) : nullptr));
         return {s_out, y};
     }
-    // saved: k v w u s r length new_starts residual (r may be undefined)
+    // saved: k v w u s r length new_starts residual
     static variable_list gradients(const variable_list& saved, const variable_list& grads) {
-        const Tensor &k = saved[0], &r = saved[5];
-        const bool with_r = r.defined() && r.numel() > 0;
+        const Tensor &k = saved[0], r = if_any(saved[5]);
+        const bool with_r = r.defined();
         const c10::cuda::CUDAGuard guard(k.device());
         const Dims d(k);
         const Flags f(saved[6], saved[7], d.lead, d.T, k);
@@ -372,10 +376,10 @@ struct Wkv4 {
 struct Wkv4Node : public torch::autograd::Function<Wkv4Node> {
     static variable_list forward(AutogradContext* ctx, const Tensor& k, const Tensor& v, const Tensor& w, const Tensor& u,
                                  const Tensor& s, const Tensor& r, const Tensor& length, const Tensor& starts) {
-        const Tensor t[] = {k, v, w, u, s, r};
+        const Tensor t[] = {k, v, w, u, s, if_any(r)};
         Tensor residual;
         auto [s_out, y] = Wkv4::forward(t, length, starts, &residual);
-        ctx->save_for_backward({k, v, w, u, s, r.defined() ? r : fresh({0}, k.scalar_type(), k), length, starts, residual});
+        ctx->save_for_backward({k, v, w, u, s, r, length, starts, residual});
         ctx->set_materialize_grads(false);
         return {s_out, y};
     }
@@ -861,7 +865,7 @@ PyObject* py_wkv4(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (r or N
     {
         pybind11::gil_scoped_release no_gil;
         if (any_grad(t, with_r ? 6 : 5)) {
-            variable_list o = Wkv4Node::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7]);
+            variable_list o = Wkv4Node::apply(t[0], t[1], t[2], t[3], t[4], with_r ? t[5] : nothing(t[0]), t[6], t[7]);
             s_out = o[0]; y = o[1];
         } else {
             std::tie(s_out, y) = Wkv4::forward(t, t[6], t[7], nullptr);
@@ -897,7 +901,9 @@ PyObject* py_time_mixing(PyObject*, PyObject* const* args, Py_ssize_t n) {
         pybind11::gil_scoped_release no_gil;
         const Tensor vf = first ? Tensor() : t[2];
         if (any_grad(t, first ? 2 : 3) || any_grad_defined(p, Layer::kParams)) {
-            variable_list r = LayerNode::apply(t[0], t[1], vf, at::TensorList(p, Layer::kParams), flags[0], flags[1], H, first);
+            for (Tensor& q : p)
+                if (!q.defined()) q = nothing(t[0]);      // the first layer's v0, v1, v2
+            variable_list r = LayerNode::apply(t[0], t[1], first ? nothing(t[0]) : vf, at::TensorList(p, Layer::kParams), flags[0], flags[1], H, first);
             o = r[0]; new_state = r[1];
             if (first) v = r[2];
         } else {
