@@ -10,7 +10,7 @@ constant decay) are never batched, as under ``jax.vmap(..., in_axes=None)``.
 import torch
 
 from . import _lib
-from .rwkv7 import _ptr, _stream, _flatten_lead, _bcast_flags, _vmap_front
+from .rwkv7 import _ptr, _stream, _cotangent, _flatten_lead, _bcast_flags, _vmap_front
 
 
 def _expand_hn(x, H, N, dtype):
@@ -55,8 +55,7 @@ def batched_wkv6_bwd(version, res, grads, B):
     code = _lib.dtype_code(k.dtype)
     _, T, H, N = k.shape
     assert length.shape == (B,) and new_starts.shape == (B, T)
-    gy = None if gy is None else gy.to(k.dtype).contiguous()
-    gs_out = None if gs_out is None else gs_out.to(k.dtype).contiguous()
+    gy, gs_out = _cotangent(gy, k.dtype), _cotangent(gs_out, k.dtype)
     gr, gk, gv = (torch.empty_like(k) for _ in range(3))
     gs = torch.empty_like(s)
     gw = torch.empty_like(k) if version == "6" else torch.empty(B, H, N, dtype=torch.float32, device=k.device)

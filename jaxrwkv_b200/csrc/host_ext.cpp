@@ -119,9 +119,16 @@ struct Flags {
     }
 };
 
-// A cotangent as the kernels read it; an undefined one stays undefined (the kernels take NULL for zero).
+// Dense and where the widest accesses fit: a contiguous view may begin anywhere.
+bool on_16_bytes(const Tensor& t) { return (uintptr_t)in(t) % 16 == 0; }
+Tensor dense(const Tensor& t) {
+    const Tensor c = t.contiguous();
+    return on_16_bytes(c) ? c : c.clone(at::MemoryFormat::Contiguous);
+}
+// A cotangent as the kernels read it (autograd hands in slices of larger ones, such as a concatenation's); an undefined one stays
+// undefined (the kernels take NULL for zero).
 Tensor cotangent(const Tensor& g, const Tensor& like) {
-    return !g.defined() ? g : (g.scalar_type() == like.scalar_type() ? g : g.to(like.scalar_type())).contiguous();
+    return !g.defined() ? g : dense(g.scalar_type() == like.scalar_type() ? g : g.to(like.scalar_type()));
 }
 
 // What stands for an optional operand that is not there: an autograd node's arguments have to be defined.
@@ -602,6 +609,8 @@ struct Layer {
         if (C != H * S || B > 65535 || x.size(0) * x.size(1) > 2147483647 / 8 || !same_kind(t, 3) || !sizes_are(state, {}, {B, 1 + S, C}) ||
             !v_first.sizes().equals(x.sizes()))
             return false;
+        for (const Tensor* t : {&x, &v_first})        // (the state's rows are made dense below)
+            if (t->is_contiguous() && !on_16_bytes(*t)) return false;
         for (int i = 0; i < kParams; ++i) {
             if (first && (i == kV0 || i == kV1 || i == kV2)) continue;
             if (!p[i].defined() || p[i].scalar_type() != x.scalar_type() || p[i].device() != x.device() || !p[i].is_contiguous() ||
@@ -632,7 +641,7 @@ struct Layer {
         const cudaStream_t st = stream_of(x_);
         const int code = dtype_code(x_), B = (int)d.B, T = (int)d.T, C = (int)d.C, H = (int)d.H;
         const Flags f(length, starts, {d.B}, d.T, x_);
-        const Tensor x = x_.contiguous(), state = state_.contiguous();
+        const Tensor x = x_.contiguous(), state = dense(state_);
         kept = {x, state, d.first ? Tensor() : v_first.contiguous(), fresh({d.B, d.T, d.C}, x.scalar_type(), x), Inter::make(x, d).t, f.length,
                 f.starts, Tensor(), {}};
         const Inter q(Slab(kept.slab, x.element_size()), d);

@@ -27,6 +27,14 @@ def _stream():
     return torch.cuda.current_stream().cuda_stream
 
 
+def _cotangent(g, dtype):
+    """A cotangent as the kernels read it, or None; a slice of a larger one may begin where their accesses do not fit."""
+    if g is None:
+        return None
+    g = g.to(dtype).contiguous()
+    return g if g.data_ptr() % 16 == 0 else g.clone()
+
+
 def _check_inputs(r, w, k, v, a, b, s):
     dtype = k.dtype
     if not all(x.dtype == dtype for x in (r, w, k, v, a, b, s)):          # rwkv7.py:361
@@ -88,8 +96,7 @@ def batched_wkv7_bwd(res, grads, B, flags=0, buffers=None):
     code = _lib.dtype_code(k.dtype)
     _, T, H, N = k.shape
     assert length.shape == (B,) and new_starts.shape == (B, T)
-    gy = None if gy is None else gy.to(k.dtype).contiguous()
-    gs_out = None if gs_out is None else gs_out.to(k.dtype).contiguous()
+    gy, gs_out = _cotangent(gy, k.dtype), _cotangent(gs_out, k.dtype)
     buffers = buffers or {}
     gw, gr, gk, gv, ga, gb = (buffers[n] if n in buffers else torch.empty_like(k) for n in ("gw", "gr", "gk", "gv", "ga", "gb"))
     gs = buffers["gs"] if "gs" in buffers else torch.empty_like(s)

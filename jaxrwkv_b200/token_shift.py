@@ -9,6 +9,7 @@ reference vmaps the per-sequence function over it).
 import torch
 
 from . import _lib
+from .rwkv7 import _cotangent
 
 SHIFT_TILE = 64   # B200WKV_SHIFT_TILE of the C header
 
@@ -57,8 +58,7 @@ class _TokenShift(torch.autograd.Function):
         lib = _lib.load()
         x, prev, mix, length, new_starts = ctx.saved_tensors
         B, T, D, M = ctx.dims
-        gout = gout.to(x.dtype).contiguous()
-        gstate = None if gstate is None else gstate.to(x.dtype).contiguous()
+        gout, gstate = _cotangent(gout, x.dtype), _cotangent(gstate, x.dtype)
         gx, gprev = torch.empty_like(x), torch.empty_like(prev)
         ntile = (T + SHIFT_TILE - 1) // SHIFT_TILE
         gmix = torch.empty((B, ntile, M, D), dtype=torch.float32, device=x.device)
