@@ -4,8 +4,9 @@
 // A call through torch.autograd.Function in Python costs 80-100 us forward and 350 us for a forward and backward,
 // a ctypes call of a decoding step 30 us: more than most kernels behind them.  The same work from C++ costs a
 // few microseconds per call.  Every function here returns None when it is handed something out of the ordinary
-// (arguments that are no plain tensors, a functorch transform or a dispatch mode in force, shapes or types that do
-// not fit); the Python functions that call them then take their own path, which handles vmap and raises the errors.
+// (arguments that are no plain tensors or carry a tangent, a functorch transform, a dispatch mode or a tracer in force,
+// shapes or types that do not fit); the Python functions that call them then take their own path, which handles vmap
+// and raises the errors.
 #include <torch/csrc/python_headers.h>
 
 #include <array>
@@ -64,11 +65,13 @@ Tensor bytes(size_t n, const Tensor& like) { return fresh({(int64_t)n}, at::kByt
 int dtype_code(const Tensor& t) { return t.scalar_type() == at::kFloat ? B200WKV_F32 : B200WKV_BF16; }
 cudaStream_t stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 
-// The plain case: no functorch transform, no dispatch mode.
+// The plain case: no functorch transform, no dispatch mode, nothing that records a trace.
 bool plain_mode() {
     return !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) &&
-           !c10::impl::dispatch_mode_enabled();
+           !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::Tracer) && !c10::impl::dispatch_mode_enabled();
 }
+// A dual tensor of forward-mode differentiation: what runs below the dispatcher would drop its tangent without a word.
+bool has_tangent(const Tensor& t) { return t._fw_grad(/*level=*/0).defined(); }
 // One floating type the kernels know, one CUDA device, contiguous enough to be made so by contiguous().
 bool same_kind(const Tensor* t, int n) {
     const auto type = t[0].scalar_type();
@@ -814,6 +817,7 @@ bool take(PyObject* const* args, int n, Tensor* to) {
     for (int i = 0; i < n; ++i) {
         if (!THPVariable_CheckExact(args[i])) return false;
         to[i] = THPVariable_Unpack(args[i]);
+        if (has_tangent(to[i])) return false;
     }
     return plain_mode();
 }
