@@ -46,9 +46,11 @@ int wkv6_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r,
                  void* du, void* ds0, const int* run_if, bool rest_only = false);
 // A constant decay (versions 5, 5.2): fp32-accurate, run-parallel; `rest_only` above: what of the call these two left out
 size_t wkv5_exact_partial_bytes(int B, int T, int H);
+size_t wkv5_states_bytes(int B, int T, int H);
 bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands);
 int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
-                   const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark);
+                   const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark,
+                   void* workspace);
 int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
                    const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* partial,
                    void* dr, void* dk, void* dv, void* dw, void* du, void* ds0);
@@ -126,6 +128,57 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
     }
     return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out,
                         residual, nullptr, 0, nullptr);
+}
+
+size_t wkv6_workspace_bytes(int dtype, bool per_token, int B, int T, int H) {
+    if (dtype != B200WKV_BF16 || per_token) return 0;
+    return wkv5_exact_takes(T, {}) ? wkv5_states_bytes(B, T, H) : 16;   // (16: the token-sequential kernels, which want no room)
+}
+
+int wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int N, const void* r, const void* k,
+                 const void* v, const void* w, const void* u, const void* s0, const uint32_t* length,
+                 const uint8_t* new_starts, void* y, void* s_out, void* residual, size_t residual_bytes,
+                 unsigned flags, void* workspace) {
+    int st = check_dims(dtype, B, T, H, N);
+    if (st != B200WKV_OK) return st;
+    if (version != 5 && version != 6) return B200WKV_EUNSUPPORTED;
+    if (!r || !k || !v || !w || !u || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
+    if (residual != nullptr && residual_bytes < b200wkv6_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
+    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
+    const bool exact = !sequential && version != 6 && (residual != nullptr || workspace != nullptr);      // wkv5_exact.cu, see below
+    if (!aligned(sequential || exact ? vec4_bytes(dtype) : 16, {r, k, v, y}) || !aligned(version == 6 && !sequential ? 16 : vec4_bytes(dtype), {w}) ||
+        !aligned(16, {residual, workspace}))
+        return B200WKV_EUNSUPPORTED;
+    if (dtype == B200WKV_BF16) {
+        int* mark = residual_mark_of(residual, b200wkv6_residual_bytes(dtype, B, T, H, N));
+        // With a constant decay (versions 5, 5.2) the decay's gradient is a sum over ALL tokens of per-token terms that
+        // largely cancel; taken from bf16 tensor-core products it is only good to a few percent (10 % on short
+        // sequences), so training calls of those versions take the fp32-accurate kernels of wkv5_exact.cu, with the
+        // token-sequential ones for heads outside their domain (same checkpoints, marked as such) and for operands that the
+        // wider accesses of the former do not suit.  So do calls without a residual that bring a workspace (the host path's,
+        // which give the same bits with and without gradients).  Without either, and for everything of version 6: the
+        // chunked kernels.
+        if (exact && wkv5_exact_takes(T, {r, k, v, y, s0, s_out})) {
+            st = wkv5_exact_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, s0, length, new_starts, y, s_out, residual, mark, workspace);
+            if (st != B200WKV_OK) return st;
+            return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, s0, length, new_starts, y, s_out, residual, nullptr, 0,
+                                mark, true);
+        }
+        if (sequential || exact)
+            return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
+                                s_out, residual, nullptr, 0, mark);
+        // the chunked tensor-core kernel, and behind it the sequential kernel, which runs only if the chunked one met
+        // something outside its domain (it then redoes the whole call and marks the residual as its own)
+        int* flag = nullptr;
+        int ticket = 0;
+        st = wkv6_chunk_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y, s_out,
+                            residual, mark, &flag, &ticket);
+        if (st != B200WKV_OK) return st;
+        return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
+                            s_out, residual, flag, ticket, mark);
+    }
+    return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
+                        s_out, residual, nullptr, 0, nullptr);
 }
 }  // namespace b200wkv
 
@@ -218,45 +271,7 @@ int b200wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int 
                  const void* v, const void* w, const void* u, const void* s0, const uint32_t* length,
                  const uint8_t* new_starts, void* y, void* s_out, void* residual, size_t residual_bytes,
                  unsigned flags) {
-    int st = check_dims(dtype, B, T, H, N);
-    if (st != B200WKV_OK) return st;
-    if (version != 5 && version != 6) return B200WKV_EUNSUPPORTED;
-    if (!r || !k || !v || !w || !u || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
-    if (residual != nullptr && residual_bytes < b200wkv6_residual_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
-    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
-    const bool exact = !sequential && version != 6 && residual != nullptr;      // wkv5_exact.cu, see below
-    if (!aligned(sequential || exact ? vec4_bytes(dtype) : 16, {r, k, v, y}) || !aligned(version == 6 && !sequential ? 16 : vec4_bytes(dtype), {w}) ||
-        !aligned(16, {residual}))
-        return B200WKV_EUNSUPPORTED;
-    if (dtype == B200WKV_BF16) {
-        int* mark = residual_mark_of(residual, b200wkv6_residual_bytes(dtype, B, T, H, N));
-        // With a constant decay (versions 5, 5.2) the decay's gradient is a sum over ALL tokens of per-token terms that
-        // largely cancel; taken from bf16 tensor-core products it is only good to a few percent (10 % on short
-        // sequences), so training calls of those versions take the fp32-accurate kernels of wkv5_exact.cu, with the
-        // token-sequential ones for heads outside their domain (same checkpoints, marked as such) and for operands that the
-        // wider accesses of the former do not suit.  Their inference
-        // calls, and everything of version 6, take the chunked kernels.
-        if (exact && wkv5_exact_takes(T, {r, k, v, y, s0, s_out})) {
-            st = wkv5_exact_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, s0, length, new_starts, y, s_out, residual, mark);
-            if (st != B200WKV_OK) return st;
-            return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, s0, length, new_starts, y, s_out, residual, nullptr, 0,
-                                mark, true);
-        }
-        if (sequential || exact)
-            return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
-                                s_out, residual, nullptr, 0, mark);
-        // the chunked tensor-core kernel, and behind it the sequential kernel, which runs only if the chunked one met
-        // something outside its domain (it then redoes the whole call and marks the residual as its own)
-        int* flag = nullptr;
-        int ticket = 0;
-        st = wkv6_chunk_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y, s_out,
-                            residual, mark, &flag, &ticket);
-        if (st != B200WKV_OK) return st;
-        return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
-                            s_out, residual, flag, ticket, mark);
-    }
-    return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
-                        s_out, residual, nullptr, 0, nullptr);
+    return b200wkv::wkv6_fwd(stream, dtype, version, B, T, H, N, r, k, v, w, u, s0, length, new_starts, y, s_out, residual, residual_bytes, flags, nullptr);
 }
 
 int b200wkv6_bwd(void* stream, int dtype, int version, int B, int T, int H, int N, const void* r, const void* k,

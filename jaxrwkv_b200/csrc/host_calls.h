@@ -12,6 +12,13 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
              const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
              void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace);
 
+// b200wkv6_fwd; a call without a residual may bring a workspace of wkv6_workspace_bytes() (0: it wants none, NULL) and then has
+// the arithmetic of a call with one.
+size_t wkv6_workspace_bytes(int dtype, bool per_token, int B, int T, int H);
+int wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int N, const void* r, const void* k, const void* v,
+             const void* w, const void* u, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
+             void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace);
+
 // RWKV-4 with the receptance product inside (y = r * wkv; r NULL: without) and, with `raw_w`, the decay parameter w
 // before -exp().  The backward writes dr when r is given, and per-sequence sums of dw' and du (B, C).
 int wkv4_fwd(cudaStream_t st, int dtype, int B, int T, int C, bool raw_w, const void* w, const void* u, const void* r, const void* k,

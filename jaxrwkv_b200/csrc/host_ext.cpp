@@ -276,9 +276,12 @@ struct Wkv6Versioned {
         Tensor y = fresh_like(k), s_out = fresh_like(t[5]);
         const size_t rbytes = residual ? b200wkv6_residual_bytes(dtype_code(k), d.B, d.T, d.H, d.N) : 0;
         if (residual) *residual = bytes(rbytes, k);
-        check(b200wkv6_fwd(stream_of(k), dtype_code(k), per_token ? 6 : 5, d.B, d.T, d.H, d.N, in(c[0]), in(c[1]), in(c[2]),
-                           in(c[3]), in(c[4]), in(c[5]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), out(y),
-                           out(s_out), residual ? out(*residual) : nullptr, rbytes, 0));
+        // a constant decay (5, 5.2) without gradients: the arithmetic of a training call, with room for the states between its runs
+        const size_t wbytes = residual || d.N != 64 ? 0 : b200wkv::wkv6_workspace_bytes(dtype_code(k), per_token, d.B, d.T, d.H);
+        const Tensor scratch = wbytes ? bytes(wbytes, k) : Tensor();
+        check(b200wkv::wkv6_fwd(stream_of(k), dtype_code(k), per_token ? 6 : 5, d.B, d.T, d.H, d.N, in(c[0]), in(c[1]), in(c[2]),
+                                in(c[3]), in(c[4]), in(c[5]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), out(y),
+                                out(s_out), residual ? out(*residual) : nullptr, rbytes, 0, wbytes ? out(scratch) : nullptr));
         return {s_out, y};
     }
     static variable_list gradients(bool per_token, const variable_list& saved, const variable_list& grads) {
@@ -854,14 +857,12 @@ PyObject* py_wkv6(PyObject*, PyObject* const* args, Py_ssize_t n) {   // (per_to
     if (!take(args + 1, 8, t) || !Wkv6Versioned::fits(per_token, t)) Py_RETURN_NONE;
     {
         pybind11::gil_scoped_release no_gil;
-        // a constant decay (5, 5.2) without gradients also asks for a residual: the kernels of that call compute in fp32
         if (any_grad(t, 6)) {
             variable_list o = per_token ? Wkv6Node<true>::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7])
                                         : Wkv6Node<false>::apply(t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7]);
             s_out = o[0]; y = o[1];
         } else {
-            Tensor residual;
-            std::tie(s_out, y) = Wkv6Versioned::forward(per_token, t, t[6], t[7], per_token ? nullptr : &residual);
+            std::tie(s_out, y) = Wkv6Versioned::forward(per_token, t, t[6], t[7], nullptr);
         }
     }
     return pair(s_out, y);

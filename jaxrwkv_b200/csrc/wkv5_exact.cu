@@ -1,8 +1,8 @@
-// RWKV-5 / 5.2 (one constant decay per key channel), bf16 streams, training: fp32-accurate matrix products in runs of 64
-// tokens that are walked side by side.
+// RWKV-5 / 5.2 (one constant decay per key channel), bf16 streams: fp32-accurate matrix products in runs of 64 tokens that are
+// walked side by side.
 //
-// The gradient of a constant decay is a sum over ALL tokens of terms that largely cancel, so these calls keep fp32
-// accuracy throughout.  Token by token on CUDA cores (wkv6_seq.cu) that costs 0.5 us per token and head forward and
+// The gradient of a constant decay is a sum over ALL tokens of terms that largely cancel, so training calls keep
+// fp32 accuracy throughout, and so do the host path's calls without gradients, whose results are the same bits.  Token by token on CUDA cores (wkv6_seq.cu) that costs 0.5 us per token and head forward and
 // 1.1 us backward on a chain as long as the sequence.  Here a chunk of 16 tokens is a handful of matrix products on
 // mma.sync m16n8k8 tf32 tiles; every fp32 factor goes in as two tf32 numbers (x = hi + lo, 22 bits), products of two such
 // factors as hi hi + hi lo + lo hi; bf16 values are exact in tf32.  With d = the decay, t, s local to the chunk, m = 8:
@@ -221,14 +221,16 @@ struct FwdSmem5 {
     uint32_t starts[kRunChunks];
 };
 
-// kOutputs false: the state that the run's tokens leave from zero, into the checkpoint slot of the run behind (no CTA for
+// `states`: n_states fp32 states per head, per_run of them per run, the first of which is the one entering the run.  A call whose
+// residual they are keeps one per chunk (per_run = kRunChunks: the checkpoints), a call without a residual one per run.
+// kOutputs false: the state that the run's tokens leave from zero, into the slot of the run behind (no CTA for
 // the last run).  True: y, the checkpoints of the run's chunks behind the first, and the returned state.
 // 128 threads; warp w holds the rows j = 16 w .. of S^T[j][i] as accumulator tiles.
 template <bool kOutputs>
 __global__ void __launch_bounds__(128, 4)
-wkv5_fwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
+wkv5_fwd_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
                 const bf* __restrict__ w, const bf* __restrict__ u, const bf* __restrict__ s0, const uint32_t* __restrict__ length,
-                const uint8_t* __restrict__ new_starts, bf* __restrict__ y, bf* __restrict__ s_out, float* __restrict__ ckpt,
+                const uint8_t* __restrict__ new_starts, bf* __restrict__ y, bf* __restrict__ s_out, float* __restrict__ states,
                 int* __restrict__ residual_mark) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FwdSmem5& sm = *reinterpret_cast<FwdSmem5*>(smem_raw);
@@ -237,12 +239,12 @@ wkv5_fwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
     if (kOutputs && residual_mark != nullptr && blockIdx.x == 0 && tid == 0) *residual_mark = 1;   // fp32 checkpoints
     if (!in_domain(w + (size_t)h * kN)) return;
     const size_t stride = (size_t)H * kN, base = (size_t)bi * Tlen * stride + (size_t)h * kN;
-    const int t_run = run * kRun, nC = (Tlen + kC - 1) / kC, L = min((int)length[bi], Tlen);
-    float* const slots = ckpt + (size_t)bh * nC * kN * kN;
+    const int t_run = run * kRun, L = min((int)length[bi], Tlen);
+    float* const slots = states + (size_t)bh * n_states * kN * kN;
     float acc[8][4];             // acc[ni][e] = S[i = 8 ni + 2 q + (e & 1)][j = j0 + g + 8 (e >> 1)]
     auto element = [&](int ni, int e) { return (8 * ni + 2 * q + (e & 1)) * kN + j0 + g + 8 * (e >> 1); };
     if (kOutputs) {
-        const float* from = slots + (size_t)run * kRunChunks * kN * kN;
+        const float* from = slots + (size_t)run * per_run * kN * kN;
 #pragma unroll
         for (int ni = 0; ni < 8; ++ni)
 #pragma unroll
@@ -289,7 +291,7 @@ wkv5_fwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
         __syncthreads();
         if (c + 1 < kRunChunks) fetch(t0 + kC);
         const uint32_t starts = sm.starts[c];
-        if (kOutputs && c > 0) {
+        if (kOutputs && c > 0 && per_run == kRunChunks) {
             float* to = slots + (size_t)(run * kRunChunks + c) * kN * kN;
 #pragma unroll
             for (int ni = 0; ni < 8; ++ni)
@@ -398,7 +400,7 @@ wkv5_fwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
         }
     }
     if (!kOutputs) {
-        float* to = slots + (size_t)(run + 1) * kRunChunks * kN * kN;
+        float* to = slots + (size_t)(run + 1) * per_run * kN * kN;
 #pragma unroll
         for (int ni = 0; ni < 8; ++ni)
 #pragma unroll
@@ -407,15 +409,15 @@ wkv5_fwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
 }
 
 // The scan over the runs of one head: slot(next) = keep d^64 slot(this) + slot(next), for `steps` steps.  Forward: this =
-// the state entering a run (the first from s0), slots in the checkpoints.  Backward (kForward false): from the last run but
+// the state entering a run (the first from s0), slots in `states`.  Backward (kForward false): from the last run but
 // one down, slots in the rows of dr and dk (see run_slot()).  Four elements of a row per thread.
 __device__ __forceinline__ float* run_slot(bf* dr, bf* dk, size_t base, size_t stride, int run, int i, int j) {
     return reinterpret_cast<float*>((j < 32 ? dr : dk) + base + (size_t)(run * kRun + i) * stride) + (j & 31);
 }
 template <bool kForward>
 __global__ void __launch_bounds__(256)
-wkv5_scan_kernel(int Tlen, int H, int runs, const bf* __restrict__ w, const bf* __restrict__ s0, const uint8_t* __restrict__ new_starts,
-                 float* __restrict__ ckpt, bf* dr, bf* dk) {
+wkv5_scan_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* __restrict__ w, const bf* __restrict__ s0,
+                 const uint8_t* __restrict__ new_starts, float* __restrict__ states, bf* dr, bf* dk) {
     extern __shared__ unsigned char keep[];      // per run: no start flag inside
     const int bh = blockIdx.x, bi = bh / H, h = bh % H, tid = threadIdx.x;
     if (!in_domain(w + (size_t)h * kN)) return;
@@ -432,10 +434,9 @@ wkv5_scan_kernel(int Tlen, int H, int runs, const bf* __restrict__ w, const bf* 
 #pragma unroll
     for (int e = 1; e < kRun; e *= 2) d *= d;
     const float dn = (float)d;
-    const int nC = (Tlen + kC - 1) / kC;
     const size_t stride = (size_t)H * kN, base = (size_t)bi * Tlen * stride + (size_t)h * kN;
     auto slot = [&](int rn) {
-        return reinterpret_cast<float4*>(kForward ? ckpt + ((size_t)bh * nC + (size_t)rn * kRunChunks) * kN * kN + at
+        return reinterpret_cast<float4*>(kForward ? states + ((size_t)bh * n_states + (size_t)rn * per_run) * kN * kN + at
                                                   : run_slot(dr, dk, base, stride, rn, i, j));
     };
     auto step = [&](float4& x, const float4& add, int rn) {
@@ -853,8 +854,13 @@ bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands) {
     return (bits & 15u) == 0 && runs_of(T) <= 48 * 1024;
 }
 
+// What a call without a residual needs to keep: the states between its runs.
+size_t wkv5_states_bytes(int B, int T, int H) { return (size_t)B * H * runs_of(T) * kN * kN * sizeof(float); }
+
+// Exactly one of `residual` (the checkpoints, a state per chunk, stay there for the backward) and `workspace` is given.
 int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
-                   const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark) {
+                   const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark,
+                   void* workspace) {
     static DeviceOnce attr;
     if (!attr.ok([]() {
             cudaError_t e = cudaFuncSetAttribute(wkv5_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FwdSmem5));
@@ -862,13 +868,15 @@ int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
             return e;
         }))
         return B200WKV_ELAUNCH;
-    const int runs = runs_of(T), heads = B * H;
+    const int runs = runs_of(T), heads = B * H, per_run = residual != nullptr ? kRunChunks : 1;
+    const int n_states = residual != nullptr ? (T + kC - 1) / kC : runs;
+    float* const states = (float*)(residual != nullptr ? residual : workspace);
     auto launch = [&](auto kern, int n) {
-        kern<<<heads * n, 128, sizeof(FwdSmem5), st>>>(T, H, n, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u, (const bf*)s0,
-                                                       length, ns, (bf*)y, (bf*)s_out, (float*)residual, residual_mark);
+        kern<<<heads * n, 128, sizeof(FwdSmem5), st>>>(T, H, n, n_states, per_run, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u, (const bf*)s0,
+                                                       length, ns, (bf*)y, (bf*)s_out, states, residual_mark);
     };
     if (runs > 1) launch(wkv5_fwd_kernel<false>, runs - 1);
-    wkv5_scan_kernel<true><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, (const bf*)w, (const bf*)s0, ns, (float*)residual, nullptr, nullptr);
+    wkv5_scan_kernel<true><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, n_states, per_run, (const bf*)w, (const bf*)s0, ns, states, nullptr, nullptr);
     launch(wkv5_fwd_kernel<true>, runs);
     return done();
 }
@@ -891,7 +899,7 @@ int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
     };
     if (runs > 1) {
         launch(wkv5_bwd_kernel<false>, runs - 1);
-        wkv5_scan_kernel<false><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, (const bf*)w, nullptr, ns, nullptr, (bf*)dr, (bf*)dk);
+        wkv5_scan_kernel<false><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, 0, 0, (const bf*)w, nullptr, ns, nullptr, (bf*)dr, (bf*)dk);
     }
     launch(wkv5_bwd_kernel<true>, runs);
     wkv5_sum_runs_kernel<<<heads, 128, 0, st>>>(H, runs, (const bf*)w, (const float*)partial, (float*)dw, (float*)du);
