@@ -115,14 +115,18 @@ __device__ __forceinline__ float decay_of(T w, bool raw) {
     return raw ? to_f32(from_f32<T>(-expf(to_f32(w)))) : to_f32(w);
 }
 
-// state (a, b, p) followed by a stretch of tokens with summary (xa, xb, xp) that decays it by `decay` or, with `cut`, drops it
+// The log-decay over n tokens: 0 over none, also where one token's is infinite (exp(w) out of range).
+__device__ __forceinline__ float decay_over(int n, float ww) { return n > 0 ? (float)n * ww : 0.f; }
+// State (a, b, p) followed by a stretch of tokens with summary (xa, xb, xp) that decays it by `decay` or, with `cut`, drops it
+// (whatever it is: a NaN in front of a start flag ends there).
 __device__ __forceinline__ void combine(float& a, float& b, float& p, bool cut, float decay, float xa, float xb, float xp) {
     float e1, e2;
-    const float x = cut ? kEmpty : p + decay;
+    const float x = p + decay;
     split_weights(x, xp, e1, e2);
-    if (cut) e1 = 0.f;
-    a = e1 * a + e2 * xa; b = e1 * b + e2 * xb; p = fmaxf(x, xp);
+    a = cut ? xa : e1 * a + e2 * xa; b = cut ? xb : e1 * b + e2 * xb; p = cut ? xp : fmaxf(x, xp);
 }
+// factor x, with nothing left of x where the factor is 0: a start flag lies between
+__device__ __forceinline__ float carried(float factor, float x) { return factor != 0.f ? factor * x : 0.f; }
 
 template <typename T>
 __global__ void __launch_bounds__(kWarps * 32, 3)
@@ -189,7 +193,7 @@ wkv4_fwd_kernel(int Tlen, int C, bool raw_w, const T* __restrict__ w, const T* _
             if (j == warp) { a = xa; b = xb; p = xp; own_cut = cut; own_n = cta_n; }
             const int nj = max(0, min(kSeg, Tlen - (g0 + j) * kSeg));
             const bool rj = sreset[j] != 0;
-            combine(xa, xb, xp, rj, (float)nj * ww, sa[j][lane], sb[j][lane], sp[j][lane]);
+            combine(xa, xb, xp, rj, decay_over(nj, ww), sa[j][lane], sb[j][lane], sp[j][lane]);
             cut |= rj;
             cta_n += nj;
         }
@@ -209,12 +213,12 @@ wkv4_fwd_kernel(int Tlen, int C, bool raw_w, const T* __restrict__ w, const T* _
                 qr = *cluster.map_shared_rank(&cta_reset, q) != 0;
             }
             const int nq = max(0, min(kWarps * kSeg, Tlen - (g00 + q * kWarps) * kSeg));
-            combine(ca, cb, cp, qr, (float)nq * ww, qa, qb, qp);
+            combine(ca, cb, cp, qr, decay_over(nq, ww), qa, qb, qp);
         }
         {
             const float xa2 = a, xb2 = b, xp2 = p;
             a = ea; b = eb; p = ep;
-            combine(a, b, p, own_cut, (float)own_n * ww, xa2, xb2, xp2);
+            combine(a, b, p, own_cut, decay_over(own_n, ww), xa2, xb2, xp2);
         }
         // 3. outputs
         if (n > 0 && ckpt != nullptr && live) {
@@ -316,23 +320,23 @@ wkv4_bwd_kernel(int Tlen, int C, bool raw_w, const T* __restrict__ w, const T* _
                     const float num = e1 * a + e2 * vt, inv = reciprocal(e1 * b + e2);
                     hinv[i] = inv;
                     const float gnum = gr_[i].x() * gr_[i].y() * inv, gden = -gnum * num * inv;
-                    xa += pe * (e1 * gnum); xb += pe * (e1 * gden);
+                    xa += carried(pe, e1 * gnum); xb += carried(pe, e1 * gden);
                     const float x = p + ww;
                     hs[i] = signed_weight(x, kt);
                     const bool first = from_signed(hs[i], e1, e2);
                     a = e1 * a + e2 * vt; b = e1 * b + e2; p = fmaxf(x, kt);
-                    pe *= e1;
+                    pe = carried(pe, e1);
                     if (!first) pf = 0.f;
                     if (!full.value && t0 + i == L - 1) {    // the returned state's cotangent enters behind token L - 1
-                        xa += pe * gsa; xb += pe * gsb;
-                        xz += pf * (gsp - a * gsa - b * gsb);
+                        xa += carried(pe, gsa); xb += carried(pe, gsb);
+                        xz += carried(pf, gsp - a * gsa - b * gsb);
                     }
                 }
         };
         if (full_seg) replay(Full()); else if (n > 0) replay(Ragged());
         if (ends) {
-            xa += pe * gsa; xb += pe * gsb;
-            xz += pf * (gsp - a * gsa - b * gsb);
+            xa += carried(pe, gsa); xb += carried(pe, gsb);
+            xz += carried(pf, gsp - a * gsa - b * gsb);
         }
         sa[warp][lane] = xa; sb[warp][lane] = xb; sz[warp][lane] = xz; se[warp][lane] = pe; sf[warp][lane] = pf;
         __syncthreads();
@@ -343,8 +347,8 @@ wkv4_bwd_kernel(int Tlen, int C, bool raw_w, const T* __restrict__ w, const T* _
         for (int j = kWarps - 1; j >= 0; --j) {
             if (j == warp) { own_e = qe; own_f = qf; ga = qa; gb = qb; z = qz; }
             const float ej = se[j][lane], fj = sf[j][lane];
-            qa = ej * qa + sa[j][lane]; qb = ej * qb + sb[j][lane]; qz = fj * qz + sz[j][lane];
-            qe *= ej; qf *= fj;
+            qa = carried(ej, qa) + sa[j][lane]; qb = carried(ej, qb) + sb[j][lane]; qz = carried(fj, qz) + sz[j][lane];
+            qe = qe != 0.f ? carried(ej, qe) : 0.f; qf *= fj;
         }
         if (ranks > 1) {
             if (warp == 0) { cta_sum[0][lane] = qa; cta_sum[1][lane] = qb; cta_sum[2][lane] = qz; cta_sum[3][lane] = qe; cta_sum[4][lane] = qf; }
@@ -358,9 +362,9 @@ wkv4_bwd_kernel(int Tlen, int C, bool raw_w, const T* __restrict__ w, const T* _
                 const float* from = cluster.map_shared_rank(&cta_sum[0][0], q) + lane;
                 ra = from[0]; rb = from[32]; rz = from[64]; re = from[96]; rf = from[128];
             }
-            ca = re * ca + ra; cb = re * cb + rb; cz = rf * cz + rz;
+            ca = carried(re, ca) + ra; cb = carried(re, cb) + rb; cz = carried(rf, cz) + rz;
         }
-        ga += own_e * ia; gb += own_e * ib; z += own_f * iz;
+        ga += carried(own_e, ia); gb += carried(own_e, ib); z += carried(own_f, iz);
         // 3. gradients, walking back through the segment
         if (ends) { ga += gsa; gb += gsb; z += gsp - a * gsa - b * gsb; }   // (a, b): the state behind the segment
         auto gradients = [&](auto full) {
