@@ -430,28 +430,6 @@ int b200wkv_debug_step_residency(int dtype, int* grid_per_sm, int* fit_per_sm) {
     return wkv7_step_stream_residency(dtype, grid_per_sm, fit_per_sm);
 }
 
-int b200wkv_debug_split_plan(int chains, int n_blk, int per_sm, int* grid, int* seg) {
-    if (chains < 1 || n_blk < 1 || per_sm < 1 || !grid || !seg) return B200WKV_ESHAPE;
-    const SplitPlan p = plan_split(chains, n_blk, per_sm, sm_count_of_current_device());
-    *grid = p.grid;
-    *seg = p.seg;
-    return B200WKV_OK;
-}
-
-int b200wkv_debug_runs(int chains, int seg, int grid, int cta, int* runs, int capacity) {
-    if (chains < 1 || seg < 1 || grid < 1 || cta < 0 || cta >= grid || !runs) return B200WKV_ESHAPE;
-    const long long lo = (long long)chains * seg * cta / grid, hi = (long long)chains * seg * (cta + 1) / grid;
-    if (hi <= lo) return 0;
-    const int n = run_count(lo, hi, seg);
-    for (int order = 0; order < n && order < capacity; ++order) {
-        const RunPlan r = run_at(lo, hi, seg, order);
-        runs[3 * order] = r.chain;
-        runs[3 * order + 1] = r.seg_from;
-        runs[3 * order + 2] = r.seg_to;
-    }
-    return n;
-}
-
 static int check_shift(int dtype, int B, int T, int D, int M) {
     if (dtype != B200WKV_F32 && dtype != B200WKV_BF16) return B200WKV_EDTYPE;
     if (B < 1 || T < 1 || D < 4 || (D % 4) != 0 || M < 1 || M > 8 || (long long)B * T > 2147483647LL || B > 65535) return B200WKV_ESHAPE;

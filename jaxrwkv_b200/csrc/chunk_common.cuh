@@ -29,7 +29,6 @@ constexpr float kLn2 = 0.6931471805599453f;
 //   fscr     [kGradCtas][4 tiles]       scratch of the gradient kernel, one set per CTA: the decay factors 1/L_t, L_t,
 //                                       L_{t-1} and the log-decay of the block in hand (written when the operands are
 //                                       scaled, read back by the last epilogue; it lives in L2)
-constexpr int kHandoffSlots = 512;
 constexpr int SAVED_T = 0, SAVED_AAK = 1, SAVED_PRB = 2, SAVED_PRK = 3, SAVED_SA = 4, SAVED_S0 = 5;
 constexpr int GCB = kC * 16;          // column-block pitch of a tile in global memory (1024)
 constexpr int GTILE = 8 * GCB;        // 8192
@@ -66,55 +65,6 @@ __host__ __device__ __forceinline__ Slot slot_tokens(int slot, int T, int L) {
     int end = p + kC < T ? p + kC : T;
     if (cut >= 0 && slot == bl) end = cut;
     return Slot{p, end - p};
-}
-
-// What the schedule queries of b200wkv_debug.h answer: how sequences could be cut into runs of blocks over fewer CTAs.
-// Host side of the split: grid size and segments per sequence for `chains` sequences of `n_blk`
-// blocks with `per_sm` resident CTAs per SM on a device of `sm_count` SMs (the launchers pass the
-// count of the device that is current, looked up once per device).
-struct SplitPlan {
-    int grid;
-    int seg;
-};
-inline SplitPlan plan_split(int chains, int n_blk, int per_sm, int sm_count) {
-    const int slots = sm_count * per_sm;
-    SplitPlan p{chains, 1};
-    if (chains <= slots) return p;            // every sequence gets its own resident CTA
-    p.grid = slots;
-    if (chains % slots == 0 || slots > kHandoffSlots) return p;
-    // makespan in sequence lengths is ceil(chains * seg / slots) / seg: take the smallest seg that helps
-    double best = (double)((chains + slots - 1) / slots);
-    for (int seg = 2; seg <= 8 && seg <= n_blk; seg *= 2) {
-        const double m = (double)(((long long)chains * seg + slots - 1) / slots) / seg;
-        if (m < best * 0.98) {
-            best = m;
-            p.seg = seg;
-        }
-    }
-    return p;
-}
-
-// Work split of U = (sequences x segments) units over G CTAs: CTA c owns units [U c / G, U (c+1) / G).
-// Units are numbered sequence-major; the consecutive units of one sequence inside a CTA's range form
-// a run that the CTA walks as one piece.  A CTA whose range ends inside a sequence walks that run
-// FIRST and hands its carry to the next CTA (slot c); the run at the start of its range that begins
-// inside a sequence comes LAST and takes the carry of slot c - 1.  No CTA waits before it has
-// produced what its neighbour needs, so the waits cannot form a cycle.
-struct RunPlan {
-    int chain;      // sequence index (batch * H + head)
-    int seg_from;   // first segment of the run, in walking order
-    int seg_to;     // one past the last segment
-};
-__host__ __device__ __forceinline__ int run_count(long long lo, long long hi, int seg) { return (int)((hi - 1) / seg - lo / seg) + 1; }
-__host__ __device__ __forceinline__ RunPlan run_at(long long lo, long long hi, int seg, int order) {
-    const int first = (int)(lo / seg), n = run_count(lo, hi, seg);
-    // walking order: the last run of the range, the middle runs, the first run of the range
-    const int ri = (n == 1) ? 0 : (order == 0 ? n - 1 : (order == n - 1 ? 0 : order));
-    RunPlan r;
-    r.chain = first + ri;
-    r.seg_from = (ri == 0) ? (int)(lo % seg) : 0;
-    r.seg_to = (ri == n - 1) ? (int)((hi - 1) % seg) + 1 : seg;
-    return r;
 }
 
 __device__ __forceinline__ uint32_t pack2(float x, float y) {

@@ -477,9 +477,9 @@ def test_bwd_headline_shape_against_oracle_slices():
 
 @pytest.mark.parametrize("T", [300, 512])
 def test_chunk_bwd_sequences_split_across_ctas(T):
-    """More sequences than SMs and not a multiple of them: the tensor-core backward cuts sequences
-    into runs of blocks owned by neighbouring CTAs.  Ragged lengths and start flags; every gradient
-    against the token-sequential kernels on the same inputs."""
+    """More sequences than SMs and not a multiple of them: the blocks of one sequence are taken by several
+    CTAs of the gradient kernel.  Ragged lengths and start flags; every gradient against the token-sequential
+    kernels on the same inputs."""
     B, H = 5, 37
     d = wkv7_case(B, T, H, seed=4321 + T, s0_scale=0.3, p_start=1 / 100, random_length=True)
     t = to_dev(d, torch.bfloat16)
@@ -497,8 +497,8 @@ def test_chunk_bwd_sequences_split_across_ctas(T):
 
 
 def test_forward_backward_replay_from_a_cuda_graph():
-    """The calls only enqueue work (kernels, one small memset), so a forward + backward pair can be captured
-    into a CUDA graph and replayed on new data; shape chosen so that the backward runs in its split mode."""
+    """The calls only enqueue kernels, so a forward + backward pair can be captured into a CUDA graph and
+    replayed on new data; more sequences than SMs, ragged lengths and start flags."""
     B, T, H = 5, 256, 37
     d = wkv7_case(B, T, H, seed=77, s0_scale=0.3, p_start=1 / 100, random_length=True)
     t = to_dev(d, torch.bfloat16)
