@@ -56,6 +56,11 @@ NCU_TRAFFIC = {"sources": "20d31d569af8", "B": 8, "wkv7_fwd": 1974.2e6, "wkv7_bw
 # gives each kernel's share.  Traffic of the backward is the sum over both kernels.
 KERNELS = {"wkv7_fwd": ["wkv7_chunk_fwd_kernel"], "wkv7_bwd": ["wkv7_carry_bwd_kernel<3>", "wkv7_grad_bwd_kernel"]}
 
+# Kernel launches of one step (Headline.step): forward, the chunked kernel and the fp32 one that redoes the call when a decay left
+# the chunked kernel's range (it returns at once otherwise); backward, state-gradient carry, gradient kernel, and the fp32
+# backward under the same condition.
+LAUNCHES_PER_STEP = 5
+
 
 def kernel_source_hash():
     h = hashlib.sha1()
@@ -263,7 +268,7 @@ def bench_configs(torch, dev, world, rank, peak):
         x = make_wkv7_device_inputs(2, 256, 4, N, torch.float32, dev, 1234, s0_scale=0.0, grads=False)
         ms = cuda_ms(torch, lambda: rwkv7.batched_wkv7_fwd(*[x[n] for n in order], x["length"], x["new_starts"], 2, need_residual=False), 3, 20)
         nb = 2 * (256 * 7 * 4 * N * 4 + 2 * 4 * N * N * 4)
-        out["config1"] = {"workload": "wkv7 forward, fp32, B=2, T=256, H=4 (sequential fp32 kernel; 8 sequences on 148 SMs)",
+        out["config1"] = {"workload": "wkv7 forward, fp32, B=2, T=256, H=4 (fp32 token chains, the rows of 8 sequences split over 64 CTAs)",
                           "ms": ms, "tokens_per_s": 2 * 256 / (ms / 1e3), "algorithmic_bytes": nb, "roofline_frac": gb(nb, ms) / peak}
         # ---- config 2: bf16 forward, B=8, T=1024, H=12, Bernoulli(1/256) starts, ragged lengths
         xs = [make_wkv7_device_inputs(8, 1024, 12, N, torch.bfloat16, dev, 1235 + i, p_start=1 / 256, random_length=True,
@@ -708,13 +713,8 @@ def main():
             "value_per_gpu": value / world, "e2e": e2e, "roofline": roofline, "cpu_baseline": cpu,
             "clocks": clocks, "sustained": sustained, "strong": strong, "configs": configs,
             "device_status": status,
-            # launches of this library's kernels per step and rank inside the device-timed region.  Forward call:
-            # the chunked kernel and the sequential kernel that redoes the call when a decay left the chunked
-            # kernel's range (it returns at once otherwise).  Backward call: state-gradient carry, gradient kernel,
-            # the one-kernel backward for sequences the forward did not mark as fast (none here: it returns at
-            # once) and the sequential backward under the same condition as the forward's; plus one memset node
-            # clearing the one-kernel backward's hand-over flags.
-            "gpu_launches": 6 * args.steps * world, "memset_nodes": args.steps * world}
+            # launches of this library's kernels inside the device-timed region, over all ranks
+            "gpu_launches": LAUNCHES_PER_STEP * args.steps * world}
     print(json.dumps(line), flush=True)
     if world > 1:
         dist.destroy_process_group()
