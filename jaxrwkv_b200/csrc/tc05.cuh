@@ -1,6 +1,7 @@
 // Thin inline-PTX layer over the Blackwell tensor-core path used by the chunked WKV kernels:
 // tcgen05.mma with shared-memory operand descriptors, TMEM allocation and load/store,
-// tcgen05.commit onto an mbarrier, and the fences between the generic and async proxies.
+// tcgen05.commit onto an mbarrier, and the fences between the generic and async proxies; and over the warp-wide matrix
+// instructions of the kernels whose tiles are smaller than tcgen05 has.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -63,6 +64,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_init_fence() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // Bounded wait for the phase with the given parity.  Returns false if the limit ran out (the
 // caller records an error and carries on so that the kernel always terminates).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t max_tries = (1u << 22)) {
@@ -81,6 +86,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
         if (ok) return true;
     }
     return false;
+}
+
+// ---- warp-wide matrix instructions ----------------------------------------------------------------
+// four 8x8 tiles of 16-bit elements: lane l gives the row address of tile l / 8
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
+}
+// D(16x8, fp32) += A(16x16, bf16, row) B(16x8, bf16, col)
+__device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) { mma_bf16(d, a[0], a[1], a[2], a[3], b0, b1); }
+// 16 bytes from global to shared memory (cp.async), zeros where not valid
+__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "r"(valid ? 16 : 0)
+                 : "memory");
 }
 
 // ---- bulk asynchronous copies (TMA, untiled) ----------------------------------------------------

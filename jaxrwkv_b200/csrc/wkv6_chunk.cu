@@ -34,21 +34,14 @@ int* wkv_call_flag(int* ticket);   // wkv7_chunk.cu: a slot of the per-device fl
 namespace {
 
 typedef __nv_bfloat16 bf;
+using tc::ldmatrix_x4;
+using tc::ldmatrix_x4_trans;
+using tc::mma_bf16;
 constexpr int kC6 = 16;          // tokens per chunk
 constexpr int kRunLen6 = 16;    // chunks per run of the run-parallel backward
 constexpr int PITCH = 72;        // bf16 per shared-memory row (144 bytes): 4-byte fragment reads and ldmatrix rows hit 32 banks
 constexpr float kMaxHalfDecay = 80.f;   // |sum of lw over half a chunk| the scaling can represent
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
-}
 // One 16-token x 16-channel block of a row-major [token][channel] tile, f[0..3] = (tokens 0-7 | 8-15) x (channels 0-7 |
 // 8-15) in the order (0-7, 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15).  As a LEFT operand (rows = tokens) the four
 // are a0..a3; as a RIGHT operand (n = token, k = channel) tokens 0-7 take (f[0], f[2]) and tokens 8-15 (f[1], f[3]).
@@ -59,12 +52,6 @@ __device__ __forceinline__ void mma_ab(float* d, const Frag& a, const Frag& b, i
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a.f[0]), "r"(a.f[1]), "r"(a.f[2]), "r"(a.f[3]), "r"(b.f[nt]), "r"(b.f[nt + 2]));
-}
-// D(16x8, fp32) += A(16x16, bf16, row) B(16x8, bf16, col)
-__device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);

@@ -22,27 +22,11 @@ int* wkv7_chunk_status_word();
 namespace {
 
 typedef __nv_bfloat16 bf;
-
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
-}
-// D(16x8, fp32) += A(16x16, bf16, row) B(16x8, bf16, col)
-__device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
-}
+using tc::cp_async16;
+using tc::ldmatrix_x4;
+using tc::ldmatrix_x4_trans;
+using tc::mbar_arrive;
+using tc::mma_bf16;
 
 // ------------------------------------------------------------------ the chain --------
 constexpr int kChainStages = 3;
@@ -227,10 +211,6 @@ struct OutSmem {
     bf w[8][kC][8];                             // W~[t][j], likewise
     bf rows[kC][kRowPitch];                     // R-[t][j], then the outputs
 };
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, bool valid) {   // zeros where not valid
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
-}
 
 // One CTA of four warps per slot, each warp 16 tokens.  Bound by the traffic of its tiles (40 KB per slot, 80 KB with a
 // residual), most of which the chain has just left in L2.

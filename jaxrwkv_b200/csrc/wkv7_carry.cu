@@ -20,10 +20,16 @@
 #include "common.cuh"
 #include "chunk_common.cuh"
 #include "device_once.cuh"
+#include "tc05.cuh"
 
 namespace b200wkv {
 
 namespace {
+
+using tc::cp_async16;
+using tc::ldmatrix_x4;
+using tc::ldmatrix_x4_trans;
+using tc::mma_bf16;
 
 constexpr int PITCH = 72;                       // bf16 per shared-memory row (144 bytes): ldmatrix and 4-byte reads hit 32 different banks
 // Depth of the cp.async ring: three stages (two CTAs per SM) while every sequence has a resident CTA anyway, two stages
@@ -38,30 +44,10 @@ struct CarryStage {
 template <int kStages>
 constexpr int carry_smem() { return kStages * (int)sizeof(CarryStage); }
 
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, bool valid) {   // zeros where not valid
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src), "r"(valid ? 16 : 0)
-                 : "memory");
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3, const void* row) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-                 : "r"((uint32_t)__cvta_generic_to_shared(row)));
-}
-// D(16x8, fp32) += A(16x16, bf16, row) B(16x8, bf16, col)
-__device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 template <int kStages>
 __global__ void __launch_bounds__(128)

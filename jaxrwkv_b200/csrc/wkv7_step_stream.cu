@@ -92,9 +92,6 @@ static_assert(kCtasPerSm * (smem_bytes<__nv_bfloat16>() + kSmemPerCta) <= kSmemO
               "kCtasPerSm CTAs fit");
 
 __device__ __forceinline__ void compute_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kComputeThreads) : "memory"); }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(bar)) : "memory");
-}
 // 32 bytes to global memory in one instruction: a whole sector per lane
 __device__ __forceinline__ void store32(void* dst, const uint4& lo, const uint4& hi) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(__cvta_generic_to_global(dst)), "r"(lo.x),
@@ -217,7 +214,7 @@ wkv7_step_stream_kernel(int BH, int H, const T* __restrict__ w, const T* __restr
 #pragma unroll
             for (int q = 0; q < kChunks; ++q) TL::unpack(*reinterpret_cast<const uint4*>(stage + chunk_off(g, q)), &S[g][q * kCE]);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sm.done[s]);   // this warp has its half of the stage in registers
+        if (lane == 0) tc::mbar_arrive(&sm.done[s]);   // this warp has its half of the stage in registers
         T* const out = s_out + state_off(bh) + (size_t)row0 * kN + 16 * p;
         // register slot q of a lane of odd rsel holds chunk q ^ 1: such a lane stores its slots swapped
         auto write_state = [&]() {
