@@ -170,7 +170,11 @@ static void* wkv7_workspace(Tensor& scratch, const Tensor& like, int B, int T, i
     if (like.scalar_type() != at::kBFloat16 || N != 64 || B < 1 || T < 2 || H < 1) return nullptr;
     const size_t n = b200wkv::wkv7_blocks_bytes(B, T, H, residual);
     if (n == 0) return nullptr;
-    scratch = bytes(n, like);
+    try {
+        scratch = bytes(n, like);
+    } catch (const c10::OutOfMemoryError&) {
+        return nullptr;                           // no room for it (up to 2 GiB): the walk needs none
+    }
     return out(scratch);
 }
 
