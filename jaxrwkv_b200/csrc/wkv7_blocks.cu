@@ -55,7 +55,7 @@ wkv7_chain_blocks_kernel(int Tlen, int H, int n_seq, int pieces, const uint32_t*
                          const bf* __restrict__ s0, const bf* __restrict__ mprime, const uint4* __restrict__ m_low,
                          const float4* __restrict__ u, const float* __restrict__ lam, unsigned char* __restrict__ s0_tiles,
                          size_t s0_stride, bf* __restrict__ s_out, float* __restrict__ s_at_len, int* __restrict__ status,
-                         const int* __restrict__ range_flag, int range_ticket) {
+                         int* __restrict__ range_flag, int range_ticket) {
     let_next_in();
     if (word_behind(range_flag) == range_ticket) return;       // a decay outside the range: the call is redone
 
@@ -157,10 +157,12 @@ wkv7_chain_blocks_kernel(int Tlen, int H, int n_seq, int pieces, const uint32_t*
             landed = false;
             break;
         }
+        bool flagged = false;                   // (L_C is 0 in every channel then)
         float low[8][4];
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
             const float2 l2 = *reinterpret_cast<const float2*>(&s.lam[nt * 8 + 2 * q]);
+            if (nt == 0) flagged = l2.x == 0.f;
             const float4* const column = s.u[2 * nt + (q >> 1)];
             const float2 ulo = reinterpret_cast<const float2*>(column + i0 + g)[q & 1], uhi = reinterpret_cast<const float2*>(column + i0 + g + 8)[q & 1];
             acc[nt][0] = fmaf(acc[nt][0], l2.x, ulo.x);
@@ -185,6 +187,12 @@ wkv7_chain_blocks_kernel(int Tlen, int H, int n_seq, int pieces, const uint32_t*
             }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sm.empty[stage]);
+        if (flagged) {                          // of a state that is no number, 0 x NaN has gone on (see wkv7_chunk.cu)
+            bool odd = false;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) odd |= (a[e >> 2][e & 3] & 0x7f80u) == 0x7f80u || (a[e >> 2][e & 3] & 0x7f800000u) == 0x7f800000u;
+            if (odd) atomicExch(range_flag, range_ticket);
+        }
         if (m > first || piece == 0) {
             unsigned char* const out = s0_tiles + (slot0 + sl) * s0_stride;
 #pragma unroll
@@ -294,9 +302,8 @@ wkv7_block_outputs_kernel(int Tlen, int H, int n_blk_slots, const uint32_t* __re
 
 }  // namespace
 
-int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, const int* range_flag, int range_ticket,
-                       const BlocksCall& c, void* y,
-                       void* s_out, float* s_at_len) {
+int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, int* range_flag, int range_ticket,
+                       const BlocksCall& c, void* y, void* s_out, float* s_at_len) {
     static DeviceOnce smem_attr;
     if (!smem_attr.ok([]() { return cudaFuncSetAttribute(wkv7_chain_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(ChainSmem)); }))
         return B200WKV_ELAUNCH;

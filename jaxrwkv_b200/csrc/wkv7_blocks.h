@@ -38,7 +38,7 @@ struct BlocksCall {
     size_t s0_stride;
     unsigned char* saved;
 };
-int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, const int* range_flag, int range_ticket,
+int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, int* range_flag, int range_ticket,
                        const BlocksCall& call, void* y,
                        void* s_out, float* s_at_len);
 

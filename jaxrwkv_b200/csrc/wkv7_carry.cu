@@ -134,11 +134,22 @@ wkv7_carry_bwd_kernel(int Tlen, int H, const uint32_t* __restrict__ length,
                 afrag[nt >> 1][(nt & 1) * 2 + 1] = hi;
             }
         }
-        // dS diag(L_C) in fp32
+        // dS diag(L_C) in fp32; at a start flag (L_C is 0 in every channel) nothing of dS goes on, not even what is no number
+        float2 l2[8];
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) l2[nt] = *reinterpret_cast<const float2*>(&s.lam[nt * 8 + 2 * q]);
+        if (l2[0].x == 0.f) {
+#pragma unroll
+            for (int nt = 0; nt < 8; ++nt)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    acc[nt][e] = 0.f;
+                    afrag[nt >> 1][(nt & 1) * 2 + (e >> 1)] = 0u;
+                }
+        }
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
-            const float2 l2 = *reinterpret_cast<const float2*>(&s.lam[nt * 8 + 2 * q]);
-            acc[nt][0] *= l2.x; acc[nt][1] *= l2.y; acc[nt][2] *= l2.x; acc[nt][3] *= l2.y;
+            acc[nt][0] *= l2[nt].x; acc[nt][1] *= l2[nt].y; acc[nt][2] *= l2[nt].x; acc[nt][3] *= l2[nt].y;
         }
         // += dS M'^T : B[k = j'][n = j] = M'[j][j'], read along the rows of M'
         // (one ldmatrix.x4 fetches the two 8x8 blocks of each of two column tiles: rows j of M', 16 values of j')

@@ -123,6 +123,26 @@ __device__ __noinline__ void mask_state_products(uint32_t taddr, uint64_t mask, 
     tc::tmem_st32(taddr, g);
     tc::tmem_wait_st();
 }
+// The masks put zeros where a start flag cuts, and the products that follow multiply them: 0 x NaN would carry what is not
+// a number over the flag.  So where this thread's 32 columns of a row of sa, W~ (NULL: not wanted) or V, in their slabs, hold any,
+// the call is redone by the token-sequential kernel, which drops the state at a flag whatever it is.
+__device__ __noinline__ void leave_to_sequential_if_odd(const unsigned char* sa, const unsigned char* w_tilde, const unsigned char* v, int* range_flag,
+                                                        int range_ticket) {
+    bool odd = false;
+    auto look = [&](const unsigned char* row) {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint4 x = *reinterpret_cast<const uint4*>(row + c * CB64);
+            const uint32_t words[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) odd |= (words[e] & 0x7f80u) == 0x7f80u || (words[e] & 0x7f800000u) == 0x7f800000u;
+        }
+    };
+    look(sa);
+    look(v);
+    if (w_tilde != nullptr) look(w_tilde);
+    if (odd) atomicExch(range_flag, range_ticket);
+}
 // 32 columns in TMEM added in fp32 onto a bf16 row in global memory; the whole warp calls it
 __device__ __noinline__ void add_to_row(uint32_t taddr, __nv_bfloat16* row, bool live) {
     float m[32];
@@ -388,7 +408,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             // A decay so strong that 1 / L leaves the range the products can carry (never reached by decays
             // of the model's own parametrisation): the chunked form cannot represent this chunk.  Record it;
             // the token-sequential kernel launched behind this one redoes the call when it finds the mark.
-            if (total < kCumFloor) atomicExch(range_flag, range_ticket);
+            if (!(total >= kCumFloor)) atomicExch(range_flag, range_ticket);   // (or is no number)
             const float t2 = fmaxf(total, kCumFloor);
             sm.tot[tid] = t2;
             const float lam_c = ex2(t2);
@@ -615,6 +635,10 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             tc::commit(&sm.bar[3]);
         }
         if (tid < 64) flag_ahead = (more && np + tid < Tlen) ? new_starts[(size_t)nbi * Tlen + np + tid] : 0;   // next chunk's start flags
+        if (flagged && quad < 2) {
+            const int at = hsel * 4 * CB64 + row * 16;
+            leave_to_sequential_if_odd(smem + OFF_SA + at, affine ? smem + OFF_G + at : nullptr, smem + OFF_V + at, range_flag, range_ticket);
+        }
         if (!tc::mbar_wait(&sm.bar[3], par)) failed = true;
         tc::fence_after_sync();
         if constexpr (kBlocks) {
