@@ -39,20 +39,21 @@ size_t wkv6_seq_residual_bytes(int B, int T, int H);
 int wkv6_seq_fwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r, const void* k, const void* v,
                  const void* w, int per_token, const void* u, const void* s0, const uint32_t* length,
                  const uint8_t* ns, void* y, void* s_out, void* residual, const int* run_if, int run_ticket,
-                 int* residual_mark, bool rest_only = false);
+                 int* residual_mark, const int* rest_of = nullptr);
 int wkv6_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r, const void* k, const void* v,
                  const void* w, int per_token, const void* u, const uint32_t* length, const uint8_t* ns,
                  const void* dy, const void* ds_out, const void* residual, void* dr, void* dk, void* dv, void* dw,
-                 void* du, void* ds0, const int* run_if, bool rest_only = false);
-// A constant decay (versions 5, 5.2): fp32-accurate, run-parallel; `rest_only` above: what of the call these two left out
+                 void* du, void* ds0, const int* run_if, const int* rest_of = nullptr);
+// A constant decay (versions 5, 5.2): fp32-accurate, run-parallel; `rest_of` above: their words per head, and only what these two left out is done
 size_t wkv5_exact_partial_bytes(int B, int T, int H);
 size_t wkv5_states_bytes(int B, int T, int H);
+int* wkv5_odd_heads(int B, int T, int H, void* residual, void* workspace);
 bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands);
 int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
                    const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual, int* residual_mark,
                    void* workspace);
 int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
-                   const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* partial,
+                   const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual, void* partial,
                    void* dr, void* dk, void* dv, void* dw, void* du, void* ds0);
 size_t wkv6_chunk_residual_bytes(int B, int T, int H);
 int wkv6_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w,
@@ -162,8 +163,11 @@ int wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int N, c
             st = wkv5_exact_fwd((cudaStream_t)stream, B, T, H, r, k, v, w, u, s0, length, new_starts, y, s_out, residual, mark, workspace);
             if (st != B200WKV_OK) return st;
             return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, s0, length, new_starts, y, s_out, residual, nullptr, 0,
-                                mark, true);
+                                mark, wkv5_odd_heads(B, T, H, residual, workspace));
         }
+        if (exact && residual != nullptr &&     // the backward may take them all the same: no head is to be left out
+            cudaMemsetAsync(wkv5_odd_heads(B, T, H, residual, nullptr), 0, (size_t)B * H * sizeof(int), (cudaStream_t)stream) != cudaSuccess)
+            return B200WKV_ELAUNCH;
         if (sequential || exact)
             return wkv6_seq_fwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, version == 6, u, s0, length, new_starts, y,
                                 s_out, residual, nullptr, 0, mark);
@@ -297,7 +301,7 @@ int b200wkv6_bwd(void* stream, int dtype, int version, int B, int T, int H, int 
             if (st != B200WKV_OK) return st;
         }
         return wkv6_seq_bwd((cudaStream_t)stream, dtype, B, T, H, r, k, v, w, 0, u, length, new_starts, dy, ds_out, residual, dr, dk, dv, dw, du,
-                            ds0, nullptr, !sequential);
+                            ds0, nullptr, sequential ? nullptr : wkv5_odd_heads(B, T, H, residual, nullptr));
     }
     if (dtype == B200WKV_BF16) {
         // the forward's mark decides on the device which of the two runs; the other returns at once

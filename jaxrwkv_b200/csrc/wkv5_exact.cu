@@ -45,6 +45,22 @@ __device__ __forceinline__ bool in_domain(const bf* w_head) {   // of the whole 
     return __syncthreads_and(d >= 1e-4f && d <= 1.f) != 0;
 }
 
+// What is not a number ends at a start flag in the token-sequential kernels, but 0 x NaN would carry it on here.  A chunk with
+// flags that meets any in what the masks' zeros are multiplied with sets its head's word, and the head is left to wkv6_seq.cu.
+__device__ __forceinline__ bool odd(uint32_t two) { return (two & 0x7f80u) == 0x7f80u || (two & 0x7f800000u) == 0x7f800000u; }   // bf16
+__device__ __forceinline__ bool odd_rows(const bf* tile_at) {          // 8 elements
+    const uint4 x = *reinterpret_cast<const uint4*>(tile_at);
+    return odd(x.x) || odd(x.y) || odd(x.z) || odd(x.w);
+}
+__device__ __forceinline__ bool odd_tiles(const float (*acc)[4]) {
+    float z = 0.f;
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z = fmaf(acc[n][e], 0.f, z);
+    return z != 0.f;
+}
+
 struct Pow {
     float p[kPow][kN], n[kNeg + 1][kN];    // d^e, d^-e
     __device__ __forceinline__ float at(int e, int i) const { return e >= 0 ? p[e][i] : n[-e][i]; }
@@ -231,7 +247,7 @@ __global__ void __launch_bounds__(128, 4)
 wkv5_fwd_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
                 const bf* __restrict__ w, const bf* __restrict__ u, const bf* __restrict__ s0, const uint32_t* __restrict__ length,
                 const uint8_t* __restrict__ new_starts, bf* __restrict__ y, bf* __restrict__ s_out, float* __restrict__ states,
-                int* __restrict__ residual_mark) {
+                int* __restrict__ odd_heads, int* __restrict__ residual_mark) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FwdSmem5& sm = *reinterpret_cast<FwdSmem5*>(smem_raw);
     const int bh = blockIdx.x / runs, run = blockIdx.x % runs, bi = bh / H, h = bh % H;
@@ -291,6 +307,7 @@ wkv5_fwd_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* 
         __syncthreads();
         if (c + 1 < kRunChunks) fetch(t0 + kC);
         const uint32_t starts = sm.starts[c];
+        if (kOutputs && starts != 0 && (odd_tiles(acc) || odd_rows(&sm.v[tid >> 3][(tid & 7) * 8]))) odd_heads[bh] = 1;
         if (kOutputs && c > 0 && per_run == kRunChunks) {
             float* to = slots + (size_t)(run * kRunChunks + c) * kN * kN;
 #pragma unroll
@@ -417,9 +434,10 @@ __device__ __forceinline__ float* run_slot(bf* dr, bf* dk, size_t base, size_t s
 template <bool kForward>
 __global__ void __launch_bounds__(256)
 wkv5_scan_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* __restrict__ w, const bf* __restrict__ s0,
-                 const uint8_t* __restrict__ new_starts, float* __restrict__ states, bf* dr, bf* dk) {
+                 const uint8_t* __restrict__ new_starts, float* __restrict__ states, int* __restrict__ odd_heads, bf* dr, bf* dk) {
     extern __shared__ unsigned char keep[];      // per run: no start flag inside
     const int bh = blockIdx.x, bi = bh / H, h = bh % H, tid = threadIdx.x;
+    if (kForward && blockIdx.y == 0 && tid == 0) odd_heads[bh] = 0;
     if (!in_domain(w + (size_t)h * kN)) return;
     for (int rn = tid >> 5; rn < runs; rn += 8) {
         const int t = rn * kRun + (tid & 31);
@@ -499,7 +517,8 @@ __global__ void __launch_bounds__(128, 3)
 wkv5_bwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
                 const bf* __restrict__ w, const bf* __restrict__ u, const uint32_t* __restrict__ length,
                 const uint8_t* __restrict__ new_starts, const bf* __restrict__ dy, const bf* __restrict__ ds_out,
-                const float* __restrict__ ckpt, bf* dr, bf* dk, bf* __restrict__ dv, float* __restrict__ part, bf* __restrict__ ds0) {
+                const float* __restrict__ ckpt, int* __restrict__ odd_heads, bf* dr, bf* dk, bf* __restrict__ dv, float* __restrict__ part,
+                bf* __restrict__ ds0) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BwdSmem5& sm = *reinterpret_cast<BwdSmem5*>(smem_raw);
     const int n_here = kGrads ? runs : runs - 1;
@@ -575,6 +594,10 @@ wkv5_bwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
             for (int nj = 0; nj < 8; ++nj)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) acc[nj][e] += m[nj][e];
+        }
+        if (kGrads && starts != 0) {
+            const int at = (tid >> 3) * kPitch + (tid & 7) * 8;
+            if (odd_tiles(acc) || odd_rows(&sm.r[0][0] + at) || odd_rows(&sm.k[0][0] + at) || odd_rows(vv + at) || odd_rows(gy + at)) odd_heads[bh] = 1;
         }
         // ---- operand tiles
         auto hats = [&](int hi) {                  // K^ of a state gradient that stands behind token hi - 1
@@ -845,7 +868,15 @@ int done() { return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELA
 int runs_of(int T) { return (T + kRun - 1) / kRun; }
 }  // namespace
 
-size_t wkv5_exact_partial_bytes(int B, int T, int H) { return (size_t)B * H * runs_of(T) * 2 * kN * sizeof(float); }
+// Behind a residual's checkpoints: the runs' shares of dw and du, and a word per head.
+size_t wkv5_exact_partial_bytes(int B, int T, int H) { return (size_t)B * H * (runs_of(T) * (size_t)(2 * kN) * sizeof(float) + sizeof(int)); }
+// The words per head (see odd() above) of a call with this residual, or with this workspace.
+int* wkv5_odd_heads(int B, int T, int H, void* residual, void* workspace) {
+    const size_t BH = (size_t)B * H;
+    char* const base = static_cast<char*>(residual != nullptr ? residual : workspace);
+    const size_t behind = residual != nullptr ? ((size_t)((T + kC - 1) / kC) * kN * kN + (size_t)runs_of(T) * 2 * kN) : (size_t)runs_of(T) * kN * kN;
+    return reinterpret_cast<int*>(base + BH * behind * sizeof(float));
+}
 
 // Rows travel in 16-byte pieces here (8 bytes in the token-sequential kernels), and the scan keeps a byte per run in shared memory.
 bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands) {
@@ -854,8 +885,8 @@ bool wkv5_exact_takes(int T, std::initializer_list<const void*> operands) {
     return (bits & 15u) == 0 && runs_of(T) <= 48 * 1024;
 }
 
-// What a call without a residual needs to keep: the states between its runs.
-size_t wkv5_states_bytes(int B, int T, int H) { return (size_t)B * H * runs_of(T) * kN * kN * sizeof(float); }
+// What a call without a residual needs to keep: the states between its runs, and a word per head.
+size_t wkv5_states_bytes(int B, int T, int H) { return (size_t)B * H * (runs_of(T) * (size_t)kN * kN * sizeof(float) + sizeof(int)); }
 
 // Exactly one of `residual` (the checkpoints, a state per chunk, stay there for the backward) and `workspace` is given.
 int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
@@ -871,18 +902,19 @@ int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
     const int runs = runs_of(T), heads = B * H, per_run = residual != nullptr ? kRunChunks : 1;
     const int n_states = residual != nullptr ? (T + kC - 1) / kC : runs;
     float* const states = (float*)(residual != nullptr ? residual : workspace);
+    int* const odd_heads = wkv5_odd_heads(B, T, H, residual, workspace);
     auto launch = [&](auto kern, int n) {
         kern<<<heads * n, 128, sizeof(FwdSmem5), st>>>(T, H, n, n_states, per_run, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u, (const bf*)s0,
-                                                       length, ns, (bf*)y, (bf*)s_out, states, residual_mark);
+                                                       length, ns, (bf*)y, (bf*)s_out, states, odd_heads, residual_mark);
     };
     if (runs > 1) launch(wkv5_fwd_kernel<false>, runs - 1);
-    wkv5_scan_kernel<true><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, n_states, per_run, (const bf*)w, (const bf*)s0, ns, states, nullptr, nullptr);
+    wkv5_scan_kernel<true><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, n_states, per_run, (const bf*)w, (const bf*)s0, ns, states, odd_heads, nullptr, nullptr);
     launch(wkv5_fwd_kernel<true>, runs);
     return done();
 }
 
 int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
-                   const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, const void* residual, void* partial,
+                   const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual, void* partial,
                    void* dr, void* dk, void* dv, void* dw, void* du, void* ds0) {
     static DeviceOnce attr;
     if (!attr.ok([]() {
@@ -892,14 +924,15 @@ int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
         }))
         return B200WKV_ELAUNCH;
     const int runs = runs_of(T), heads = B * H;
+    int* const odd_heads = wkv5_odd_heads(B, T, H, residual, nullptr);
     auto launch = [&](auto kern, int n) {
         kern<<<heads * n, 128, sizeof(BwdSmem5), st>>>(T, H, runs, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u, length, ns,
-                                                       (const bf*)dy, (const bf*)ds_out, (const float*)residual, (bf*)dr, (bf*)dk, (bf*)dv,
+                                                       (const bf*)dy, (const bf*)ds_out, (const float*)residual, odd_heads, (bf*)dr, (bf*)dk, (bf*)dv,
                                                        (float*)partial, (bf*)ds0);
     };
     if (runs > 1) {
         launch(wkv5_bwd_kernel<false>, runs - 1);
-        wkv5_scan_kernel<false><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, 0, 0, (const bf*)w, nullptr, ns, nullptr, (bf*)dr, (bf*)dk);
+        wkv5_scan_kernel<false><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, 0, 0, (const bf*)w, nullptr, ns, nullptr, nullptr, (bf*)dr, (bf*)dk);
     }
     launch(wkv5_bwd_kernel<true>, runs);
     wkv5_sum_runs_kernel<<<heads, 128, 0, st>>>(H, runs, (const bf*)w, (const float*)partial, (float*)dw, (float*)du);

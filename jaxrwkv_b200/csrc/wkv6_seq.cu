@@ -19,11 +19,12 @@ struct DecaySrc {
     int per_token;        // 1: index by (b,t,h) and apply exp ; 0: index by h only, use as is
 };
 
-// Behind the run-parallel kernels of a constant decay (wkv5_exact.cu): only the heads outside their domain are left.
+// Behind the run-parallel kernels of a constant decay (wkv5_exact.cu): only the heads outside their domain are left, and those
+// whose word they set.
 template <typename T>
-__device__ __forceinline__ bool done_by_runs(const T* w_head) {
+__device__ __forceinline__ bool done_by_runs(const T* w_head, int odd_head) {
     const float d = to_f32(w_head[threadIdx.x & 63]);
-    return __syncthreads_and(d >= 1e-4f && d <= 1.f) != 0;
+    return __syncthreads_and(d >= 1e-4f && d <= 1.f && odd_head == 0) != 0;
 }
 
 // ------------------------------------------------------------------ forward ---------
@@ -44,12 +45,12 @@ wkv6_seq_fwd_kernel(int Tlen, int H, const T* __restrict__ r, const T* __restric
                     const T* __restrict__ w, int w_per_token, const T* __restrict__ u, const T* __restrict__ s0,
                     const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts, T* __restrict__ y,
                     T* __restrict__ s_out, float* __restrict__ ckpt, const int* __restrict__ run_if, int run_ticket,
-                    int* __restrict__ residual_mark, bool rest_only) {
+                    int* __restrict__ residual_mark, const int* __restrict__ rest_of) {
     // As the fallback behind the chunked kernel: run only when that kernel left its ticket in *run_if, and
     // mark the residual as being in this kernel's format.
     if (run_if != nullptr && *run_if != run_ticket) return;
     if (residual_mark != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *residual_mark = 1;
-    if (rest_only && done_by_runs(w + (size_t)(blockIdx.x % H) * kN)) return;
+    if (rest_of != nullptr && done_by_runs(w + (size_t)(blockIdx.x % H) * kN, rest_of[blockIdx.x])) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Fwd6Smem& sm = *reinterpret_cast<Fwd6Smem*>(smem_raw);
     const int bh = blockIdx.x, bi = bh / H, h = bh % H;
@@ -180,9 +181,9 @@ wkv6_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ r, const T* __restric
                     const T* __restrict__ dy, const T* __restrict__ ds_out, const float* __restrict__ ckpt,
                     T* __restrict__ dr, T* __restrict__ dk, T* __restrict__ dv, T* __restrict__ dw_tok,
                     float* __restrict__ dw_head, float* __restrict__ du_head, T* __restrict__ ds0,
-                    const int* __restrict__ run_if, bool rest_only) {
+                    const int* __restrict__ run_if, const int* __restrict__ rest_of) {
     if (run_if != nullptr && *run_if == 0) return;   // the residual is in the chunked kernels' format
-    if (rest_only && done_by_runs(w + (size_t)(blockIdx.x % H) * kN)) return;
+    if (rest_of != nullptr && done_by_runs(w + (size_t)(blockIdx.x % H) * kN, rest_of[blockIdx.x])) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Bwd6Smem& sm = *reinterpret_cast<Bwd6Smem*>(smem_raw);
     const int bh = blockIdx.x, bi = bh / H, h = bh % H;
@@ -391,14 +392,14 @@ wkv6_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ r, const T* __restric
 template <typename T>
 int launch_fwd6(cudaStream_t st, int B, int Tlen, int H, const void* r, const void* k, const void* v, const void* w,
                 int per_token, const void* u, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
-                void* s_out, void* residual, const int* run_if, int run_ticket, int* residual_mark, bool rest_only) {
+                void* s_out, void* residual, const int* run_if, int run_ticket, int* residual_mark, const int* rest_of) {
     auto kern = wkv6_seq_fwd_kernel<T>;
     static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
     if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Fwd6Smem)); }))
         return B200WKV_ELAUNCH;
     kern<<<B * H, 192, sizeof(Fwd6Smem), st>>>(Tlen, H, (const T*)r, (const T*)k, (const T*)v, (const T*)w, per_token,
                                                (const T*)u, (const T*)s0, length, ns, (T*)y, (T*)s_out, (float*)residual,
-                                               run_if, run_ticket, residual_mark, rest_only);
+                                               run_if, run_ticket, residual_mark, rest_of);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
@@ -406,7 +407,7 @@ template <typename T>
 int launch_bwd6(cudaStream_t st, int B, int Tlen, int H, const void* r, const void* k, const void* v, const void* w,
                 int per_token, const void* u, const uint32_t* length, const uint8_t* ns, const void* dy,
                 const void* ds_out, const void* residual, void* dr, void* dk, void* dv, void* dw, void* du, void* ds0,
-                const int* run_if, bool rest_only) {
+                const int* run_if, const int* rest_of) {
     auto kern = wkv6_seq_bwd_kernel<T>;
     static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
     if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Bwd6Smem)); }))
@@ -415,7 +416,7 @@ int launch_bwd6(cudaStream_t st, int B, int Tlen, int H, const void* r, const vo
                                                (const T*)u, length, ns, (const T*)dy, (const T*)ds_out,
                                                (const float*)residual, (T*)dr, (T*)dk, (T*)dv,
                                                per_token ? (T*)dw : nullptr, per_token ? nullptr : (float*)dw,
-                                               (float*)du, (T*)ds0, run_if, rest_only);
+                                               (float*)du, (T*)ds0, run_if, rest_of);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 }  // namespace
@@ -427,21 +428,21 @@ size_t wkv6_seq_residual_bytes(int B, int T, int H) {
 int wkv6_seq_fwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r, const void* k, const void* v,
                  const void* w, int per_token, const void* u, const void* s0, const uint32_t* length,
                  const uint8_t* ns, void* y, void* s_out, void* residual, const int* run_if, int run_ticket,
-                 int* residual_mark, bool rest_only) {
+                 int* residual_mark, const int* rest_of) {
     if (dtype == B200WKV_F32)
-        return launch_fwd6<float>(st, B, T, H, r, k, v, w, per_token, u, s0, length, ns, y, s_out, residual, run_if, run_ticket, residual_mark, rest_only);
+        return launch_fwd6<float>(st, B, T, H, r, k, v, w, per_token, u, s0, length, ns, y, s_out, residual, run_if, run_ticket, residual_mark, rest_of);
     return launch_fwd6<__nv_bfloat16>(st, B, T, H, r, k, v, w, per_token, u, s0, length, ns, y, s_out, residual, run_if, run_ticket,
-                                      residual_mark, rest_only);
+                                      residual_mark, rest_of);
 }
 
 int wkv6_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* r, const void* k, const void* v,
                  const void* w, int per_token, const void* u, const uint32_t* length, const uint8_t* ns,
                  const void* dy, const void* ds_out, const void* residual, void* dr, void* dk, void* dv, void* dw,
-                 void* du, void* ds0, const int* run_if, bool rest_only) {
+                 void* du, void* ds0, const int* run_if, const int* rest_of) {
     if (dtype == B200WKV_F32)
-        return launch_bwd6<float>(st, B, T, H, r, k, v, w, per_token, u, length, ns, dy, ds_out, residual, dr, dk, dv, dw, du, ds0, run_if, rest_only);
+        return launch_bwd6<float>(st, B, T, H, r, k, v, w, per_token, u, length, ns, dy, ds_out, residual, dr, dk, dv, dw, du, ds0, run_if, rest_of);
     return launch_bwd6<__nv_bfloat16>(st, B, T, H, r, k, v, w, per_token, u, length, ns, dy, ds_out, residual, dr, dk, dv, dw, du, ds0,
-                                      run_if, rest_only);
+                                      run_if, rest_of);
 }
 
 }  // namespace b200wkv
