@@ -20,7 +20,7 @@
 // the rows in front of the last flag, and the decayed entering state is dropped.  (Ending the chunk in front of every
 // flag instead, as an earlier form did, costs a whole chunk's time per flag, and a backward that can follow it: forward and
 // backward at B=6, T=2043, H=32 with a flag every 512 tokens took 970-990 us so, and take 676 us with the masks, while
-// a forward without flags, B=8, T=4096, H=32, takes 595 us in that form and 597 with the masks.)  The
+// a forward without flags, B=8, T=4096, H=32, takes 595 us in that form and 594-597 with the masks.)  The
 // cumulative decay is not restarted: only ratios inside a segment survive the masks.  A chunk ends early only where the
 // state is wanted, at `length`, and at the end of the sequence; the rows behind its end are zero.
 //
@@ -88,7 +88,7 @@ static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "two CTAs per SM");
 // What only chunks with start flags and chunks of fewer than 64 tokens need is kept out of the walk's loop: the passes over TMEM
 // are functions that are not inlined, and the flags are read back from shared memory where a flagged chunk needs them.  With the
 // passes inlined and the flags' 64 bits live across the loop body, every chunk WITHOUT flags paid 1 % (forward with a residual at
-// B=8, T=4096, H=32: 603-607 -> 597 us; without a residual 543 -> 531; B=6, T=2043 with a flag every 512 tokens 321 -> 318).  A second copy of the loop body for full chunks without flags is no faster on such sequences and
+// B=8, T=4096, H=32: 603-607 -> 594-597 us; without a residual 543 -> 531; B=6, T=2043 with a flag every 512 tokens 321 -> 318).  A second copy of the loop body for full chunks without flags is no faster on such sequences and
 // loses where both kinds mix, the two bodies evicting each other's instructions (B=8, T=1024, H=32, a flag every 100 tokens: 200 us
 // against 178).
 __device__ __forceinline__ uint64_t start_mask(const Small& sm) {   // bit t: a flag on token t of the chunk
@@ -124,24 +124,24 @@ __device__ __noinline__ void mask_state_products(uint32_t taddr, uint64_t mask, 
     tc::tmem_wait_st();
 }
 // The masks put zeros where a start flag cuts, and the products that follow multiply them: 0 x NaN would carry what is not
-// a number over the flag.  So where this thread's 32 columns of a row of sa, W~ (NULL: not wanted) or V, in their slabs, hold any,
-// the call is redone by the token-sequential kernel, which drops the state at a flag whatever it is.
+// a number over the flag.  So a flagged chunk that meets any in k, v, a, b or its entering state leaves the call to the
+// token-sequential kernel, which drops the state at a flag whatever it is.  (The walk looks at the operands in registers; blocks
+// side by side, whose body that costs 4 us of 57, at what came of them.)  The sums stay 0 for numbers and are NaN otherwise.
+__device__ __forceinline__ void add_odd(__nv_bfloat162& sum, const uint4& x) {
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&x);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) sum = __hfma2(h[i], zero, sum);
+}
+__device__ __forceinline__ bool is_odd(const __nv_bfloat162& sum) { return __low2float(sum) + __high2float(sum) != 0.f; }
+// this thread's 32 columns of a row of sa, W~ and V in their slabs
 __device__ __noinline__ void leave_to_sequential_if_odd(const unsigned char* sa, const unsigned char* w_tilde, const unsigned char* v, int* range_flag,
                                                         int range_ticket) {
-    bool odd = false;
-    auto look = [&](const unsigned char* row) {
+    __nv_bfloat162 odd = __floats2bfloat162_rn(0.f, 0.f);
+    for (const unsigned char* row : {sa, w_tilde, v})
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const uint4 x = *reinterpret_cast<const uint4*>(row + c * CB64);
-            const uint32_t words[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) odd |= (words[e] & 0x7f80u) == 0x7f80u || (words[e] & 0x7f800000u) == 0x7f800000u;
-        }
-    };
-    look(sa);
-    look(v);
-    if (w_tilde != nullptr) look(w_tilde);
-    if (odd) atomicExch(range_flag, range_ticket);
+        for (int c = 0; c < 4; ++c) add_odd(odd, *reinterpret_cast<const uint4*>(row + c * CB64));
+    if (is_odd(odd)) atomicExch(range_flag, range_ticket);
 }
 // 32 columns in TMEM added in fp32 onto a bf16 row in global memory; the whole warp calls it
 __device__ __noinline__ void add_to_row(uint32_t taddr, __nv_bfloat16* row, bool live) {
@@ -456,9 +456,13 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             }
             if (flagged) {   // the rare chunk with start flags: the masked rows are written over
                 const uint64_t m = start_mask(sm);
+                __nv_bfloat162 odd = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
                     const int t = q * 32 + tsub;
+#pragma unroll
+                    for (int i = 1; i < 5; ++i)
+                        if (!kBlocks) add_odd(odd, raw[q][i]);
                     const uint4 none = make_uint4(0, 0, 0, 0);
                     if (affine && !in_first(m, t)) {   // what carries the dependence on S0: nothing from the first flag on
                         slab_store(smem + OFF_SA, CB64, t, jb, none);
@@ -470,6 +474,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                         slab_store(smem + OFF_KH, CB64, t, jb, none);
                     }
                 }
+                if (!kBlocks && is_odd(odd)) atomicExch(range_flag, range_ticket);
             }
         }
         // ================= entering state: bf16 copy for the products, decayed fp32 copy back to TMEM =====
@@ -484,6 +489,12 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             }
 #pragma unroll
             for (int c = 0; c < 4; ++c) slab_store(smem + OFF_S0, CB64, row, hsel * 4 + c, pack8(&s[c * 8]));
+            if (flagged) {
+                float odd = 0.f;
+#pragma unroll
+                for (int c = 0; c < 32; ++c) odd = fmaf(s[c], 0.f, odd);
+                if (odd != 0.f) atomicExch(range_flag, range_ticket);
+            }
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
                 const float4 l4 = *reinterpret_cast<const float4*>(&sm.lam[hsel * 32 + c * 4]);
@@ -635,9 +646,9 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             tc::commit(&sm.bar[3]);
         }
         if (tid < 64) flag_ahead = (more && np + tid < Tlen) ? new_starts[(size_t)nbi * Tlen + np + tid] : 0;   // next chunk's start flags
-        if (flagged && quad < 2) {
+        if (kBlocks && flagged && quad < 2) {
             const int at = hsel * 4 * CB64 + row * 16;
-            leave_to_sequential_if_odd(smem + OFF_SA + at, affine ? smem + OFF_G + at : nullptr, smem + OFF_V + at, range_flag, range_ticket);
+            leave_to_sequential_if_odd(smem + OFF_SA + at, smem + OFF_G + at, smem + OFF_V + at, range_flag, range_ticket);
         }
         if (!tc::mbar_wait(&sm.bar[3], par)) failed = true;
         tc::fence_after_sync();
