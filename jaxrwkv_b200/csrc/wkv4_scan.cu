@@ -25,8 +25,10 @@
 // That is linear in (gaa, gbb, z) with a scalar factor per segment, so the same three steps apply, in reverse order of
 // segments; step 1 can be computed walking FORWARD with the running product of the factors, together with the replay
 // of the states.  What the replay computed (states, weights, reciprocals) stays in registers for step 3.
-// Bound by instruction issue and the registers' worth of warps: 1340 us -> 45 us forward + 96 us backward at B=8, T=1024,
-// C=768, bf16 (75 and 102 MB of streams).
+// 1340 us -> 48 us forward + 94 us backward at B=8, T=1024, C=768, bf16 (75 and 102 MB of streams; under ncu, cold).  No unit is
+// full: issue slots 59 and 47 %, DRAM 10 %, 21 and 15 warps per SM (80 and 128 registers).  Per issued instruction a warp waits
+// 2.1 and 1.4 cycles for its rows out of global memory, which all come at a segment's start, and 1.0 and 0.8 for the cluster's
+// fences.
 #include <cooperative_groups.h>
 #include "common.cuh"
 #include "host_calls.h"

@@ -21,8 +21,11 @@
 // are interchangeable per head.  Backward: the same three steps in reverse; the state gradients between runs lie in the
 // rows of dr and dk of the run in front, which that run reads before it writes them.
 //
-// Measured at B=4, T=1024, H=32: forward 515 -> 24 + 9 + 80 us, backward 1127 -> 30 + 9 + 194 + 3 us; bound by the
-// shared-memory path (61 % of its peak) and instruction issue (45 %) together, the tensor pipe at 37 %.
+// Measured at B=4, T=1024, H=32: forward 515 -> 24 + 9 + 80 us, backward 1127 -> 30 + 9 + 194 + 3 us.  The outputs and the
+// gradients use the shared-memory path to 78 and 76 % of its peak and 48 and 43 % of the issue slots; the gradient kernel's
+// warps wait longest for the checkpoint's rows out of global memory (1.3 cycles per issued instruction), then for shared memory (1.1).
+// A 64-term product of a split fp32 factor with a bf16 row has a relative error of 1.3e-7 (an fp32 fma chain 1.5e-7), of two
+// split factors 3.5e-7; results are rounded to bf16, 1.7e-3.
 // Powers of d outside d^{+-8} fp32 range: a head with a channel outside [1e-4, 1] is left to wkv6_seq.cu.
 #include <initializer_list>
 #include "common.cuh"

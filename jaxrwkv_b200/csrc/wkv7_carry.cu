@@ -14,7 +14,7 @@
 // leaving every block goes to global memory in bf16; the second part (wkv7_grad.cu) turns it, block by
 // block and in parallel over all blocks, into the gradients of the six streams.
 //
-// Start flags need nothing here: a block with one has L_C = 0, M' = 0 and R- zero from the first flag on.
+// A block with a start flag has L_C = 0, M' = 0 and R- zero from the first flag on; dS is dropped there by a select.
 //
 // Semantics: reverse-mode derivative of BaseRWKV.inner_loop of jaxrwkv (src/jaxrwkv/rwkv7.py:199-220).
 #include "common.cuh"

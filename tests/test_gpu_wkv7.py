@@ -396,9 +396,9 @@ def test_chunk_bwd_full_size_properties():
 @pytest.mark.parametrize("T", [64, 192, 512])
 def test_bwd_carry_and_gradient_kernels(T):
     """Sequences made of whole 64-token blocks (start flags only at multiples of 64, `length` 0, a multiple of 64
-    or beyond T) take the two-kernel backward: the sequential state-gradient carry, then the gradients of all
-    blocks in parallel.  Rows of other kinds in the same call (a flag or `length` inside a block) take the
-    one-kernel backward; every gradient of every row against the oracle."""
+    or beyond T) and rows of other kinds in the same call (a flag or `length` inside a block): the sequential
+    state-gradient carry, then the gradients of all blocks in parallel; every gradient of every row against the
+    oracle."""
     nb = T // 64
     starts = [[0], [], [0, 64 * (nb // 2)], [64 * (nb - 1)], [0, 5], []]
     lengths = [T, T + 7, 64 * max(nb - 1, 0), 0, T, T - 3]
@@ -406,7 +406,7 @@ def test_bwd_carry_and_gradient_kernels(T):
     check_bwd(d, torch.bfloat16)
     check_bwd(d, torch.bfloat16, use_gy=True, use_gs=False)
     # With dy = 0 and a 64 x 64 state cotangent the decay gradient is the small difference of large running sums
-    # D_t = sum_i dS_t S_t (|dw| is a tenth of |dk|): every tensor-core backward here, one-kernel or split, lands
+    # D_t = sum_i dS_t S_t (|dw| is a tenth of |dk|): the tensor-core backward lands
     # near 2.5 % on it (the fp32 sequential kernels at 0.2 %), so this one gradient gets 4e-2 in this one variant.
     check_bwd(d, torch.bfloat16, use_gy=False, use_gs=True, tol_dw=4e-2)
 
