@@ -71,7 +71,11 @@ bool plain_mode() {
     return (c10::impl::tls_local_dispatch_key_set().included_ & special).empty() && !c10::impl::dispatch_mode_enabled();
 }
 // A dual tensor of forward-mode differentiation: what runs below the dispatcher would drop its tangent without a word.
-bool has_tangent(const Tensor& t) { return t._fw_grad(/*level=*/0).defined(); }
+bool has_tangent(const Tensor& t) {
+    // (the general look takes a lock; most tensors have no autograd record, or one without any tangent that is no view's)
+    const auto* const meta = torch::autograd::impl::get_autograd_meta(t);
+    return meta != nullptr && (meta->fw_grad_ != nullptr || meta->is_view_) && t._fw_grad(/*level=*/0).defined();
+}
 // One floating type the kernels know, one CUDA device, contiguous enough to be made so by contiguous().
 bool same_kind(const Tensor* t, int n) {
     const auto type = t[0].scalar_type();
