@@ -3,6 +3,7 @@
 #include "common.cuh"
 #include "chunk_common.cuh"
 #include "host_calls.h"
+#include "wkv7_blocks.h"
 #include "../../include/b200wkv_debug.h"
 
 namespace b200wkv {
@@ -16,6 +17,17 @@ int wkv7_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w,
                  const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
                  const uint8_t* ns, const void* dy, const void* ds_out, void* residual, size_t residual_bytes, void* dw, void* dr,
                  void* dk, void* dv, void* da, void* db, void* ds0, const int* run_if);
+
+// fp32 from wkv7_fp32_takes() tokens on: 16 tokens at a time (wkv7_fp32.cu)
+bool wkv7_fp32_takes(int T);
+size_t wkv7_fp32_workspace_bytes(int B, int T, int H);
+size_t wkv7_fp32_residual_bytes(int B, int T, int H);
+int wkv7_fp32_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
+                  const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual,
+                  void* workspace);
+int wkv7_fp32_bwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
+                  const void* b, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual, void* dw,
+                  void* dr, void* dk, void* dv, void* da, void* db, void* ds0);
 
 int wkv7_step(cudaStream_t st, int dtype, int B, int H, const void* w, const void* r, const void* k, const void* v,
               const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
@@ -127,8 +139,16 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
         return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual,
                             range_flag, ticket, mark);
     }
+    // 16 tokens at a time where the residual has all its room, or a workspace was brought
+    if (dtype == B200WKV_F32 && wkv7_fp32_takes(T) && (residual != nullptr ? residual_bytes >= wkv7_fp32_residual_bytes(B, T, H) : workspace != nullptr))
+        return wkv7_fp32_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, workspace);
     return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out,
                         residual, nullptr, 0, nullptr);
+}
+
+size_t wkv7_workspace_bytes(int dtype, int B, int T, int H, bool residual) {
+    if (dtype == B200WKV_F32) return residual ? 0 : wkv7_fp32_workspace_bytes(B, T, H);
+    return wkv7_blocks_bytes(B, T, H, residual);
 }
 
 size_t wkv6_workspace_bytes(int dtype, bool per_token, int B, int T, int H) {
@@ -211,9 +231,10 @@ int b200wkv_device_status(void) { return wkv7_chunk_status(); }
 
 size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N) {
     if (check_dims(dtype, B, T, H, N) != B200WKV_OK) return 0;
-    // fp32 uses the sequential kernels (a state every 16 tokens); bf16 uses the chunked tensor-core
+    // fp32 keeps a state every 16 tokens; bf16 uses the chunked tensor-core
     // kernels (a state every 64 tokens) unless B200WKV_FLAG_SEQUENTIAL asks otherwise, so size for both
-    // (fp32: and for the state gradients between the chunks that the backward walks side by side, where it does)
+    // (fp32: and for what the backward that works on all chunks side by side wants besides, where it does)
+    if (dtype == B200WKV_F32 && wkv7_fp32_takes(T)) return wkv7_fp32_residual_bytes(B, T, H);
     const size_t seq = wkv7_seq_residual_bytes(B, T, H);
     if (dtype == B200WKV_F32) return seq + wkv7_seq_carry_bytes(B, T, H);
     const size_t chk = wkv7_chunk_residual_bytes(B, T, H);
@@ -255,6 +276,8 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
         return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
                             residual, b200wkv7_residual_bytes(dtype, B, T, H, N) - kResidualMarkBytes, dw, dr, dk, dv, da, db, ds0, mark);
     }
+    if (dtype == B200WKV_F32 && wkv7_fp32_takes(T) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H))
+        return wkv7_fp32_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, ds_out, residual, dw, dr, dk, dv, da, db, ds0);
     return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
                         residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, nullptr);
 }

@@ -64,8 +64,9 @@ cudaError_t launch_behind(void (*kernel)(P...), unsigned grid, unsigned block, s
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 #ifdef __CUDACC__
+__device__ __forceinline__ void wait_for_grid_in_front() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ int word_behind(const int* word) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    wait_for_grid_in_front();
     return *static_cast<const volatile int*>(word);
 }
 __device__ __forceinline__ void let_next_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -6,8 +6,8 @@
 
 namespace b200wkv {
 
-// b200wkv7_fwd with a workspace of wkv7_blocks_bytes() (0: the call wants none, workspace NULL).
-size_t wkv7_blocks_bytes(int B, int T, int H, bool residual);
+// b200wkv7_fwd with a workspace of wkv7_workspace_bytes() (0: the call wants none, workspace NULL).
+size_t wkv7_workspace_bytes(int dtype, int B, int T, int H, bool residual);
 int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k, const void* v,
              const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
              void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace);

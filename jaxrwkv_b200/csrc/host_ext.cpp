@@ -169,10 +169,10 @@ variable_list gradients_of(AutogradContext* ctx, const variable_list& grads) {
 
 // ------------------------------------------------------------------------------------------------- RWKV-7
 // Streams (lead, T, H, N), state (lead, H, N, N), any number of leading batch axes.
-// the workspace of a forward call over few sequences (NULL: it wants none); `scratch` keeps it until the call is enqueued
+// the workspace of a forward call (NULL: it wants none); `scratch` keeps it until the call is enqueued
 static void* wkv7_workspace(Tensor& scratch, const Tensor& like, int B, int T, int H, int N, bool residual) {
-    if (like.scalar_type() != at::kBFloat16 || N != 64 || B < 1 || T < 2 || H < 1) return nullptr;
-    const size_t n = b200wkv::wkv7_blocks_bytes(B, T, H, residual);
+    if (N != 64 || B < 1 || T < 2 || H < 1) return nullptr;
+    const size_t n = b200wkv::wkv7_workspace_bytes(dtype_code(like), B, T, H, residual);
     if (n == 0) return nullptr;
     try {
         scratch = bytes(n, like);

@@ -38,6 +38,8 @@ struct BlocksCall {
     size_t s0_stride;
     unsigned char* saved;
 };
+// Bytes of workspace with which a call takes this form (0: it does not)
+size_t wkv7_blocks_bytes(int B, int T, int H, bool residual);
 int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, int* range_flag, int range_ticket,
                        const BlocksCall& call, void* y,
                        void* s_out, float* s_at_len);

@@ -32,33 +32,6 @@ enum { kW, kA, kB, kK, kR };
 struct Plain { static constexpr bool value = true; };
 struct Marked { static constexpr bool value = false; };
 
-// two fp32 values in a 64-bit register: fma.rn.f32x2 rounds each as fmaf does
-struct Pair { unsigned long long u; };
-__device__ __forceinline__ Pair pair(float a, float b) {
-    Pair p;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(p.u) : "f"(a), "f"(b));
-    return p;
-}
-__device__ __forceinline__ float2 unpack(Pair p) {
-    float2 f;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p.u));
-    return f;
-}
-__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
-    Pair d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.u) : "l"(a.u), "l"(b.u), "l"(c.u));
-    return d;
-}
-__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
-    Pair d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
-    return d;
-}
-__device__ __forceinline__ Pair add2(Pair a, Pair b) {
-    Pair d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d.u) : "l"(a.u), "l"(b.u));
-    return d;
-}
 // a lane's eight columns of a row: 4 p + 32 q .. + 3 for q = 0, 1, so that the eight lanes' loads are 128 contiguous bytes
 struct Cols { Pair v[4]; };
 __device__ __forceinline__ Cols cols(const float* row, int p) {
@@ -96,9 +69,6 @@ __device__ __forceinline__ float dot(const Cols& a, const Cols& b) {
     return s.x + s.y;
 }
 
-__device__ __forceinline__ float4 decay4(float4 w) {
-    return make_float4(expf(-expf(w.x)), expf(-expf(w.y)), expf(-expf(w.z)), expf(-expf(w.w)));
-}
 __device__ __forceinline__ float sum8(float x) {   // over the eight lanes of a row
     x += __shfl_xor_sync(0xffffffffu, x, 1);
     x += __shfl_xor_sync(0xffffffffu, x, 2);
