@@ -48,20 +48,26 @@ struct DeviceOnce {
 // (launch_behind), so that its CTAs are set up while the one in front of it finishes, and starts with word_behind(), which
 // waits until that one has completed and then reads the word that decides whether there is anything to do.  The read is
 // volatile and everything else comes behind the caller's branch on it, so that no load can be moved in front of the wait.
-// A kernel that others are launched behind lets them in with let_next_in().
+// A kernel that others are launched behind lets them in with let_next_in().  Every CTA waits before it ends, so that a kernel's
+// completion stands for that of all in front of it; what it does in front of the wait must not touch what they write or read, and what they
+// have written is not read through a __restrict__ pointer, which would let the compiler move the read in front of the wait.
 template <typename... P, typename... A>
-cudaError_t launch_behind(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+cudaError_t launch_in_chain(bool first, void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = first ? 0 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    return launch_in_chain(false, kernel, grid, block, smem, st, args...);
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void wait_for_grid_in_front() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

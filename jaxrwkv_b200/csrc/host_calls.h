@@ -19,6 +19,10 @@ int wkv6_fwd(void* stream, int dtype, int version, int B, int T, int H, int N, c
              const void* w, const void* u, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
              void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace);
 
+// dw and du of operands shared by the batch (C channels) in the element type, from b200wkv6_bwd's sums per sequence; directly behind it in
+// the stream.  gw NULL: du alone
+int wkv6_parameter_grads(cudaStream_t st, int dtype, int B, int C, const float* gw, const float* gu, void* dw, void* du);
+
 // RWKV-4 with the receptance product inside (y = r * wkv; r NULL: without) and, with `raw_w`, the decay parameter w
 // before -exp().  The backward writes dr when r is given, and per-sequence sums of dw' and du (B, C).
 int wkv4_fwd(cudaStream_t st, int dtype, int B, int T, int C, bool raw_w, const void* w, const void* u, const void* r, const void* k,

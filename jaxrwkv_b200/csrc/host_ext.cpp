@@ -307,6 +307,12 @@ struct Wkv6Versioned {
                            in(c[3]), in(c[4]), in(c[5]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), in(gy), in(gs),
                            out(res), (size_t)res.numel(), out(gr), out(gk), out(gv), out(gw), out(gu), out(gs0), 0));
         // gradients of the shared operands: summed over the batch, and over the channels of a per-head constant
+        if (u.size(1) == d.N && (per_token || w.size(1) == d.N)) {
+            const Tensor du = fresh_like(u), dw = per_token ? gw : fresh_like(w);
+            check(b200wkv::wkv6_parameter_grads(stream_of(k), dtype_code(k), d.B, d.H * d.N, per_token ? nullptr : (const float*)in(gw), (const float*)in(gu),
+                                                per_token ? nullptr : out(dw), out(du)));
+            return {gr, gk, gv, dw, du, gs0};
+        }
         const auto shared = [&](const Tensor& g, const Tensor& p) {
             return (p.size(1) == 1 ? g.sum(at::IntArrayRef{0, 2}) : g.sum(0)).to(p.scalar_type()).view(p.sizes());
         };

@@ -31,6 +31,7 @@
 // fences.
 #include <cooperative_groups.h>
 #include "common.cuh"
+#include "device_once.cuh"
 #include "host_calls.h"
 
 namespace b200wkv {
@@ -433,8 +434,8 @@ wkv4_bwd_kernel(int Tlen, int C, bool raw_w, const T* __restrict__ w, const T* _
 }
 
 template <typename T>
-__global__ void wkv4_parameter_grads_kernel(int B, int C, const T* __restrict__ w, const float* __restrict__ gw,
-                                            const float* __restrict__ gu, T* __restrict__ dw, T* __restrict__ du) {
+__global__ void wkv4_parameter_grads_kernel(int B, int C, const T* __restrict__ w, const float* gw, const float* gu, T* __restrict__ dw, T* __restrict__ du) {
+    wait_for_grid_in_front();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     float sw = 0.f, su = 0.f;
@@ -465,7 +466,6 @@ int launch(Kernel kern, cudaStream_t st, int B, int Tlen, int C, Args... args) {
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kern, Tlen, C, args...) == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
-int done() { return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH; }
 }  // namespace
 
 size_t wkv4_residual_bytes(int B, int T, int C) { return (size_t)B * ((T + kSeg - 1) / kSeg) * 3 * C * sizeof(float); }
@@ -496,12 +496,11 @@ int wkv4_bwd(cudaStream_t st, int dtype, int B, int T, int C, bool raw_w, const 
                                                                                   residual, gw, gu, gr, gk, gv, gs);
 }
 int wkv4_parameter_grads(cudaStream_t st, int dtype, int B, int C, const void* w, const float* gw, const float* gu, void* dw, void* du) {
-    const int grid = (C + 63) / 64;
-    if (dtype == B200WKV_F32)
-        wkv4_parameter_grads_kernel<float><<<grid, 64, 0, st>>>(B, C, (const float*)w, gw, gu, (float*)dw, (float*)du);
-    else
-        wkv4_parameter_grads_kernel<__nv_bfloat16><<<grid, 64, 0, st>>>(B, C, (const __nv_bfloat16*)w, gw, gu, (__nv_bfloat16*)dw, (__nv_bfloat16*)du);
-    return done();
+    auto launch = [&](auto type) {                // directly behind the backward kernel
+        typedef decltype(type) T;
+        return launch_behind(wkv4_parameter_grads_kernel<T>, (C + 63) / 64, 64, 0, st, B, C, (const T*)w, gw, gu, (T*)dw, (T*)du);
+    };
+    return (dtype == B200WKV_F32 ? launch(float()) : launch(__nv_bfloat16())) == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 }  // namespace b200wkv

@@ -249,19 +249,33 @@ template <bool kOutputs>
 __global__ void __launch_bounds__(128, 4)
 wkv5_fwd_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* __restrict__ r, const bf* __restrict__ k, const bf* __restrict__ v,
                 const bf* __restrict__ w, const bf* __restrict__ u, const bf* __restrict__ s0, const uint32_t* __restrict__ length,
-                const uint8_t* __restrict__ new_starts, bf* __restrict__ y, bf* __restrict__ s_out, float* __restrict__ states,
+                const uint8_t* __restrict__ new_starts, bf* __restrict__ y, bf* __restrict__ s_out, float* states,
                 int* __restrict__ odd_heads, int* __restrict__ residual_mark) {
+    let_next_in();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     FwdSmem5& sm = *reinterpret_cast<FwdSmem5*>(smem_raw);
     const int bh = blockIdx.x / runs, run = blockIdx.x % runs, bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3, j0 = 16 * warp;
     if (kOutputs && residual_mark != nullptr && blockIdx.x == 0 && tid == 0) *residual_mark = 1;   // fp32 checkpoints
-    if (!in_domain(w + (size_t)h * kN)) return;
+    if (!in_domain(w + (size_t)h * kN)) {
+        wait_for_grid_in_front();
+        return;
+    }
     const size_t stride = (size_t)H * kN, base = (size_t)bi * Tlen * stride + (size_t)h * kN;
     const int t_run = run * kRun, L = min((int)length[bi], Tlen);
     float* const slots = states + (size_t)bh * n_states * kN * kN;
     float acc[8][4];             // acc[ni][e] = S[i = 8 ni + 2 q + (e & 1)][j = j0 + g + 8 (e >> 1)]
     auto element = [&](int ni, int e) { return (8 * ni + 2 * q + (e & 1)) * kN + j0 + g + 8 * (e >> 1); };
+    Ahead r_next, k_next, v_next;
+    auto fetch = [&](int t0) {
+        if (kOutputs) r_next.fetch(r, base, stride, t0, Tlen);
+        k_next.fetch(k, base, stride, t0, Tlen);
+        v_next.fetch(v, base, stride, t0, Tlen);
+    };
+    fetch(t_run);
+    load_starts(sm.starts, new_starts + (size_t)bi * Tlen, t_run, Tlen);
+    fill_powers(sm.pw, w + (size_t)h * kN);
+    wait_for_grid_in_front();    // (what is above depends on the operands alone)
     if (kOutputs) {
         const float* from = slots + (size_t)run * per_run * kN * kN;
 #pragma unroll
@@ -274,15 +288,6 @@ wkv5_fwd_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* 
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[ni][e] = 0.f;
     }
-    Ahead r_next, k_next, v_next;
-    auto fetch = [&](int t0) {
-        if (kOutputs) r_next.fetch(r, base, stride, t0, Tlen);
-        k_next.fetch(k, base, stride, t0, Tlen);
-        v_next.fetch(v, base, stride, t0, Tlen);
-    };
-    fetch(t_run);
-    load_starts(sm.starts, new_starts + (size_t)bi * Tlen, t_run, Tlen);
-    fill_powers(sm.pw, w + (size_t)h * kN);
     auto write_state = [&](bf* to) {
 #pragma unroll
         for (int ni = 0; ni < 8; ++ni)
@@ -437,11 +442,15 @@ __device__ __forceinline__ float* run_slot(bf* dr, bf* dk, size_t base, size_t s
 template <bool kForward>
 __global__ void __launch_bounds__(256)
 wkv5_scan_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf* __restrict__ w, const bf* __restrict__ s0,
-                 const uint8_t* __restrict__ new_starts, float* __restrict__ states, int* __restrict__ odd_heads, bf* dr, bf* dk) {
+                 const uint8_t* __restrict__ new_starts, float* states, int* __restrict__ odd_heads, bf* dr, bf* dk) {
     extern __shared__ unsigned char keep[];      // per run: no start flag inside
     const int bh = blockIdx.x, bi = bh / H, h = bh % H, tid = threadIdx.x;
+    let_next_in();
     if (kForward && blockIdx.y == 0 && tid == 0) odd_heads[bh] = 0;
-    if (!in_domain(w + (size_t)h * kN)) return;
+    if (!in_domain(w + (size_t)h * kN)) {
+        wait_for_grid_in_front();
+        return;
+    }
     for (int rn = tid >> 5; rn < runs; rn += 8) {
         const int t = rn * kRun + (tid & 31);
         const uint8_t* ns = new_starts + (size_t)bi * Tlen;
@@ -455,6 +464,7 @@ wkv5_scan_kernel(int Tlen, int H, int runs, int n_states, int per_run, const bf*
 #pragma unroll
     for (int e = 1; e < kRun; e *= 2) d *= d;
     const float dn = (float)d;
+    wait_for_grid_in_front();
     const size_t stride = (size_t)H * kN, base = (size_t)bi * Tlen * stride + (size_t)h * kN;
     auto slot = [&](int rn) {
         return reinterpret_cast<float4*>(kForward ? states + ((size_t)bh * n_states + (size_t)rn * per_run) * kN * kN + at
@@ -522,16 +532,33 @@ wkv5_bwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
                 const uint8_t* __restrict__ new_starts, const bf* __restrict__ dy, const bf* __restrict__ ds_out,
                 const float* __restrict__ ckpt, int* __restrict__ odd_heads, bf* dr, bf* dk, bf* __restrict__ dv, float* __restrict__ part,
                 bf* __restrict__ ds0) {
+    let_next_in();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BwdSmem5& sm = *reinterpret_cast<BwdSmem5*>(smem_raw);
     const int n_here = kGrads ? runs : runs - 1;
     const int bh = blockIdx.x / n_here, run = blockIdx.x % n_here + (kGrads ? 0 : 1), bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, q = lane & 3, i0 = 16 * warp;
-    if (!in_domain(w + (size_t)h * kN)) return;
+    if (!in_domain(w + (size_t)h * kN)) {
+        wait_for_grid_in_front();
+        return;
+    }
     const size_t stride = (size_t)H * kN, base = (size_t)bi * Tlen * stride + (size_t)h * kN;
     const int t_run = run * kRun, nC = (Tlen + kC - 1) / kC, L = min((int)length[bi], Tlen);
     float acc[8][4];             // acc[nj][e] = dS[i = i0 + g + 8 (e >> 1)][j = 8 nj + 2 q + (e & 1)]
     const int row_u = i0 + g, row_d = i0 + g + 8;
+    Ahead r_next, k_next, v_next, dy_next;
+    auto fetch = [&](int t0) {
+        r_next.fetch(r, base, stride, t0, Tlen);
+        dy_next.fetch(dy, base, stride, t0, Tlen);
+        if (kGrads) {
+            k_next.fetch(k, base, stride, t0, Tlen);
+            v_next.fetch(v, base, stride, t0, Tlen);
+        }
+    };
+    fetch(t_run + (kRunChunks - 1) * kC);
+    load_starts(sm.starts, new_starts + (size_t)bi * Tlen, t_run, Tlen);
+    fill_powers(sm.pw, w + (size_t)h * kN);
+    wait_for_grid_in_front();    // (what is above depends on the operands alone)
     if (kGrads && run + 1 < runs) {
 #pragma unroll
         for (int nj = 0; nj < 8; ++nj) {
@@ -545,18 +572,6 @@ wkv5_bwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[nj][e] = 0.f;
     }
-    Ahead r_next, k_next, v_next, dy_next;
-    auto fetch = [&](int t0) {
-        r_next.fetch(r, base, stride, t0, Tlen);
-        dy_next.fetch(dy, base, stride, t0, Tlen);
-        if (kGrads) {
-            k_next.fetch(k, base, stride, t0, Tlen);
-            v_next.fetch(v, base, stride, t0, Tlen);
-        }
-    };
-    fetch(t_run + (kRunChunks - 1) * kC);
-    load_starts(sm.starts, new_starts + (size_t)bi * Tlen, t_run, Tlen);
-    fill_powers(sm.pw, w + (size_t)h * kN);
     auto load_cotangent = [&](float (*m)[4]) {
 #pragma unroll
         for (int nj = 0; nj < 8; ++nj) {
@@ -859,15 +874,16 @@ wkv5_bwd_kernel(int Tlen, int H, int runs, const bf* __restrict__ r, const bf* _
 
 // The runs' shares of dw and du of one head, added in order.
 __global__ void __launch_bounds__(128)
-wkv5_sum_runs_kernel(int H, int runs, const bf* __restrict__ w, const float* __restrict__ part, float* __restrict__ dw, float* __restrict__ du) {
+wkv5_sum_runs_kernel(int H, int runs, const bf* __restrict__ w, const float* part, float* __restrict__ dw, float* __restrict__ du) {
     const int bh = blockIdx.x, i = threadIdx.x & 63;
+    let_next_in();
+    wait_for_grid_in_front();
     if (!in_domain(w + (size_t)(bh % H) * kN)) return;
     float s = 0.f;
     for (int rn = 0; rn < runs; ++rn) s += part[((size_t)bh * runs + rn) * 2 * kN + threadIdx.x];
     (threadIdx.x < kN ? dw : du)[(size_t)bh * kN + i] = s;
 }
 
-int done() { return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH; }
 int runs_of(int T) { return (T + kRun - 1) / kRun; }
 }  // namespace
 
@@ -906,14 +922,17 @@ int wkv5_exact_fwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
     const int n_states = residual != nullptr ? (T + kC - 1) / kC : runs;
     float* const states = (float*)(residual != nullptr ? residual : workspace);
     int* const odd_heads = wkv5_odd_heads(B, T, H, residual, workspace);
-    auto launch = [&](auto kern, int n) {
-        kern<<<heads * n, 128, sizeof(FwdSmem5), st>>>(T, H, n, n_states, per_run, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u, (const bf*)s0,
-                                                       length, ns, (bf*)y, (bf*)s_out, states, odd_heads, residual_mark);
+    cudaError_t e = cudaSuccess;
+    auto launch = [&](bool first, auto kern, int n) {
+        e = launch_in_chain(first, kern, heads * n, 128, sizeof(FwdSmem5), st, T, H, n, n_states, per_run, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w,
+                            (const bf*)u, (const bf*)s0, length, ns, (bf*)y, (bf*)s_out, states, odd_heads, residual_mark);
     };
-    if (runs > 1) launch(wkv5_fwd_kernel<false>, runs - 1);
-    wkv5_scan_kernel<true><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, n_states, per_run, (const bf*)w, (const bf*)s0, ns, states, odd_heads, nullptr, nullptr);
-    launch(wkv5_fwd_kernel<true>, runs);
-    return done();
+    if (runs > 1) launch(true, wkv5_fwd_kernel<false>, runs - 1);
+    if (e == cudaSuccess)
+        e = launch_in_chain(runs == 1, wkv5_scan_kernel<true>, dim3(heads, kN * kN / 1024), 256, runs, st, T, H, runs, n_states, per_run, (const bf*)w,
+                            (const bf*)s0, ns, states, odd_heads, (bf*)nullptr, (bf*)nullptr);
+    if (e == cudaSuccess) launch(false, wkv5_fwd_kernel<true>, runs);
+    return e == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const void* k, const void* v, const void* w, const void* u,
@@ -928,18 +947,21 @@ int wkv5_exact_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
         return B200WKV_ELAUNCH;
     const int runs = runs_of(T), heads = B * H;
     int* const odd_heads = wkv5_odd_heads(B, T, H, residual, nullptr);
-    auto launch = [&](auto kern, int n) {
-        kern<<<heads * n, 128, sizeof(BwdSmem5), st>>>(T, H, runs, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u, length, ns,
-                                                       (const bf*)dy, (const bf*)ds_out, (const float*)residual, odd_heads, (bf*)dr, (bf*)dk, (bf*)dv,
-                                                       (float*)partial, (bf*)ds0);
+    cudaError_t e = cudaSuccess;
+    auto launch = [&](bool first, auto kern, int n) {
+        e = launch_in_chain(first, kern, heads * n, 128, sizeof(BwdSmem5), st, T, H, runs, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)w, (const bf*)u,
+                            length, ns, (const bf*)dy, (const bf*)ds_out, (const float*)residual, odd_heads, (bf*)dr, (bf*)dk, (bf*)dv, (float*)partial,
+                            (bf*)ds0);
     };
     if (runs > 1) {
-        launch(wkv5_bwd_kernel<false>, runs - 1);
-        wkv5_scan_kernel<false><<<dim3(heads, kN * kN / 1024), 256, runs, st>>>(T, H, runs, 0, 0, (const bf*)w, nullptr, ns, nullptr, nullptr, (bf*)dr, (bf*)dk);
+        launch(true, wkv5_bwd_kernel<false>, runs - 1);
+        if (e == cudaSuccess)
+            e = launch_behind(wkv5_scan_kernel<false>, dim3(heads, kN * kN / 1024), 256, runs, st, T, H, runs, 0, 0, (const bf*)w, (const bf*)nullptr, ns,
+                              (float*)nullptr, (int*)nullptr, (bf*)dr, (bf*)dk);
     }
-    launch(wkv5_bwd_kernel<true>, runs);
-    wkv5_sum_runs_kernel<<<heads, 128, 0, st>>>(H, runs, (const bf*)w, (const float*)partial, (float*)dw, (float*)du);
-    return done();
+    if (e == cudaSuccess) launch(runs == 1, wkv5_bwd_kernel<true>, runs);
+    if (e == cudaSuccess) e = launch_behind(wkv5_sum_runs_kernel, heads, 128, 0, st, H, runs, (const bf*)w, (const float*)partial, (float*)dw, (float*)du);
+    return e == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
 
 }  // namespace b200wkv

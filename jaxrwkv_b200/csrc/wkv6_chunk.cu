@@ -476,9 +476,10 @@ __global__ void __launch_bounds__(128, 3)
 wkv6_chunk_bwd_kernel(int Tlen, int H, const bf* __restrict__ u, const uint32_t* __restrict__ length, const uint8_t* __restrict__ new_starts, int has_dy, const bf* __restrict__ ds_out, const bf* __restrict__ ckpt, const uint4* __restrict__ scores,
                       const int* __restrict__ residual_mark, bf* __restrict__ dr, bf* __restrict__ dk, bf* __restrict__ dv,
                       bf* __restrict__ dw, float* __restrict__ du_head, bf* __restrict__ ds0,
-                      int n_runs, int run_len, const bf* __restrict__ dsck, float* __restrict__ partial, int* __restrict__ status,
+                      int n_runs, int run_len, const bf* dsck, float* __restrict__ partial, int* __restrict__ status,
                       const __grid_constant__ SeqMaps maps) {
-    if (*residual_mark != 0) return;          // the forward fell back to the sequential kernels
+    let_next_in();
+    if (word_behind(residual_mark) != 0) return;          // the forward fell back to the sequential kernels
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Bwd6cSmem& sm = *reinterpret_cast<Bwd6cSmem*>(smem_raw);
     // n_runs > 1: a sequence is walked by n_runs CTAs, run rho = chunks [rho run_len, (rho + 1) run_len), each starting
@@ -923,6 +924,7 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const uint32_t*
                       const uint8_t* __restrict__ new_starts, int has_dy, const bf* __restrict__ ds_out,
                       const int* __restrict__ residual_mark, int n_runs, int run_len, bf* __restrict__ dsck, int* __restrict__ status,
                       const __grid_constant__ SeqMaps maps) {
+    let_next_in();
     if (*residual_mark != 0) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     Carry6Smem& sm = *reinterpret_cast<Carry6Smem*>(smem_raw);
@@ -1103,9 +1105,10 @@ wkv6_carry_bwd_kernel(int Tlen, int H, const bf* __restrict__ r, const uint32_t*
 }
 
 // du of a (batch, head): the runs' shares added in a fixed order
-__global__ void wkv6_reduce_runs_kernel(int BH, int n_runs, const float* __restrict__ partial, const int* __restrict__ residual_mark,
+__global__ void wkv6_reduce_runs_kernel(int BH, int n_runs, const float* partial, const int* __restrict__ residual_mark,
                                         float* __restrict__ du_head) {
-    if (*residual_mark != 0) return;
+    let_next_in();
+    if (word_behind(residual_mark) != 0) return;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= BH * kN) return;
     const int bh = idx / kN, i = idx % kN;
@@ -1182,13 +1185,16 @@ int wkv6_chunk_bwd(cudaStream_t st, int B, int T, int H, const void* r, const vo
     const void* streams[9] = {r, k, v, w, dy, dr, dk, dv, dw};
     SeqMaps maps;
     if (!make_seq_maps(&maps, streams, 9, B, T, H, kC6)) return B200WKV_ELAUNCH;
-    wkv6_chunk_bwd_kernel<<<B * H * n_runs, 128, sizeof(Bwd6cSmem), st>>>(
-        T, H, (const bf*)u, length, ns, dy != nullptr ? 1 : 0, (const bf*)ds_out, (const bf*)(base + lay.states), (const uint4*)(base + lay.scores), residual_mark, (bf*)dr, (bf*)dk, (bf*)dv, (bf*)dw, (float*)du, (bf*)ds0, n_runs, n_runs > 1 ? kRunLen : (T + kC6 - 1) / kC6, dsck, partial, wkv7_chunk_status_word(), maps);
-    if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
+    // (behind the carry, where there is one)
+    if (launch_in_chain(n_runs == 1, wkv6_chunk_bwd_kernel, B * H * n_runs, 128, sizeof(Bwd6cSmem), st, T, H, (const bf*)u, length, ns, dy != nullptr ? 1 : 0,
+                        (const bf*)ds_out, (const bf*)(base + lay.states), (const uint4*)(base + lay.scores), residual_mark, (bf*)dr, (bf*)dk, (bf*)dv,
+                        (bf*)dw, (float*)du, (bf*)ds0, n_runs, n_runs > 1 ? kRunLen : (T + kC6 - 1) / kC6, dsck, partial, wkv7_chunk_status_word(),
+                        maps) != cudaSuccess)
+        return B200WKV_ELAUNCH;
     if (n_runs > 1) {
         const int total = B * H * kN;
-        wkv6_reduce_runs_kernel<<<(total + 255) / 256, 256, 0, st>>>(B * H, n_runs, partial, residual_mark, (float*)du);
-        if (cudaGetLastError() != cudaSuccess) return B200WKV_ELAUNCH;
+        if (launch_behind(wkv6_reduce_runs_kernel, (total + 255) / 256, 256, 0, st, B * H, n_runs, partial, residual_mark, (float*)du) != cudaSuccess)
+            return B200WKV_ELAUNCH;
     }
     return B200WKV_OK;
 }

@@ -48,9 +48,11 @@ wkv6_seq_fwd_kernel(int Tlen, int H, const T* __restrict__ r, const T* __restric
                     int* __restrict__ residual_mark, const int* __restrict__ rest_of) {
     // As the fallback behind the chunked kernel: run only when that kernel left its ticket in *run_if, and
     // mark the residual as being in this kernel's format.
-    if (run_if != nullptr && *run_if != run_ticket) return;
+    let_next_in();
+    if (run_if != nullptr && word_behind(run_if) != run_ticket) return;
+    const int odd = rest_of != nullptr ? word_behind(rest_of + blockIdx.x) : 0;
     if (residual_mark != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *residual_mark = 1;
-    if (rest_of != nullptr && done_by_runs(w + (size_t)(blockIdx.x % H) * kN, rest_of[blockIdx.x])) return;
+    if (rest_of != nullptr && done_by_runs(w + (size_t)(blockIdx.x % H) * kN, odd)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Fwd6Smem& sm = *reinterpret_cast<Fwd6Smem*>(smem_raw);
     const int bh = blockIdx.x, bi = bh / H, h = bh % H;
@@ -182,8 +184,10 @@ wkv6_seq_bwd_kernel(int Tlen, int H, const T* __restrict__ r, const T* __restric
                     T* __restrict__ dr, T* __restrict__ dk, T* __restrict__ dv, T* __restrict__ dw_tok,
                     float* __restrict__ dw_head, float* __restrict__ du_head, T* __restrict__ ds0,
                     const int* __restrict__ run_if, const int* __restrict__ rest_of) {
-    if (run_if != nullptr && *run_if == 0) return;   // the residual is in the chunked kernels' format
-    if (rest_of != nullptr && done_by_runs(w + (size_t)(blockIdx.x % H) * kN, rest_of[blockIdx.x])) return;
+    let_next_in();
+    if (run_if != nullptr && word_behind(run_if) == 0) return;   // the residual is in the chunked kernels' format
+    const int odd = rest_of != nullptr ? word_behind(rest_of + blockIdx.x) : 0;
+    if (rest_of != nullptr && done_by_runs(w + (size_t)(blockIdx.x % H) * kN, odd)) return;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Bwd6Smem& sm = *reinterpret_cast<Bwd6Smem*>(smem_raw);
     const int bh = blockIdx.x, bi = bh / H, h = bh % H;
@@ -397,10 +401,11 @@ int launch_fwd6(cudaStream_t st, int B, int Tlen, int H, const void* r, const vo
     static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
     if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Fwd6Smem)); }))
         return B200WKV_ELAUNCH;
-    kern<<<B * H, 192, sizeof(Fwd6Smem), st>>>(Tlen, H, (const T*)r, (const T*)k, (const T*)v, (const T*)w, per_token,
-                                               (const T*)u, (const T*)s0, length, ns, (T*)y, (T*)s_out, (float*)residual,
-                                               run_if, run_ticket, residual_mark, rest_of);
-    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+    const bool alone = run_if == nullptr && rest_of == nullptr;      // (else: the fallback behind other kernels of the call)
+    return launch_in_chain(alone, kern, B * H, 192, sizeof(Fwd6Smem), st, Tlen, H, (const T*)r, (const T*)k, (const T*)v, (const T*)w, per_token, (const T*)u,
+                           (const T*)s0, length, ns, (T*)y, (T*)s_out, (float*)residual, run_if, run_ticket, residual_mark, rest_of) == cudaSuccess
+               ? B200WKV_OK
+               : B200WKV_ELAUNCH;
 }
 
 template <typename T>
@@ -412,14 +417,38 @@ int launch_bwd6(cudaStream_t st, int B, int Tlen, int H, const void* r, const vo
     static DeviceOnce smem_attr;   // one per template instance; the attribute is per device
     if (!smem_attr.ok([kern]() { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Bwd6Smem)); }))
         return B200WKV_ELAUNCH;
-    kern<<<B * H, 256, sizeof(Bwd6Smem), st>>>(Tlen, H, (const T*)r, (const T*)k, (const T*)v, (const T*)w, per_token,
-                                               (const T*)u, length, ns, (const T*)dy, (const T*)ds_out,
-                                               (const float*)residual, (T*)dr, (T*)dk, (T*)dv,
-                                               per_token ? (T*)dw : nullptr, per_token ? nullptr : (float*)dw,
-                                               (float*)du, (T*)ds0, run_if, rest_of);
-    return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+    const bool alone = run_if == nullptr && rest_of == nullptr;
+    return launch_in_chain(alone, kern, B * H, 256, sizeof(Bwd6Smem), st, Tlen, H, (const T*)r, (const T*)k, (const T*)v, (const T*)w, per_token, (const T*)u,
+                           length, ns, (const T*)dy, (const T*)ds_out, (const float*)residual, (T*)dr, (T*)dk, (T*)dv, per_token ? (T*)dw : (T*)nullptr,
+                           per_token ? (float*)nullptr : (float*)dw, (float*)du, (T*)ds0, run_if, rest_of) == cudaSuccess
+               ? B200WKV_OK
+               : B200WKV_ELAUNCH;
+}
+// The gradients of operands that all sequences share, from the sums per sequence (B, C): one launch for both, where the
+// framework's reductions and conversions are four and take 17 us of a backward of 250.
+template <typename T>
+__global__ void __launch_bounds__(64)
+wkv6_parameter_grads_kernel(int B, int C, const float* gw, const float* gu, T* __restrict__ dw, T* __restrict__ du) {
+    wait_for_grid_in_front();
+    const int c = blockIdx.x * 64 + threadIdx.x;
+    const float* const from = blockIdx.y == 0 ? gu : gw;
+    if (c >= C) return;
+    float sum = 0.f;
+#pragma unroll 4
+    for (int b = 0; b < B; ++b) sum += from[(size_t)b * C + c];
+    (blockIdx.y == 0 ? du : dw)[c] = from_f32<T>(sum);
 }
 }  // namespace
+
+// Behind wkv6_bwd (the same stream, nothing in between); gw NULL: du alone
+int wkv6_parameter_grads(cudaStream_t st, int dtype, int B, int C, const float* gw, const float* gu, void* dw, void* du) {
+    const dim3 grid((C + 63) / 64, gw != nullptr ? 2 : 1);
+    auto launch = [&](auto type) {
+        typedef decltype(type) T;
+        return launch_behind(wkv6_parameter_grads_kernel<T>, grid, 64, 0, st, B, C, gw, gu, (T*)dw, (T*)du);
+    };
+    return (dtype == B200WKV_F32 ? launch(float()) : launch(__nv_bfloat16())) == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+}
 
 size_t wkv6_seq_residual_bytes(int B, int T, int H) {
     return (size_t)B * H * ((T + kCk6 - 1) / kCk6) * kN * kN * sizeof(float);

@@ -663,7 +663,7 @@ struct OutSmem {
     float rbar[kC][kN];
 };
 __global__ void __launch_bounds__(128)
-wkv7_fp32_outputs_kernel(const Operands op, const Tiles tiles, const float* __restrict__ slots, float* __restrict__ y) {
+wkv7_fp32_outputs_kernel(const Operands op, const Tiles tiles, const float* slots, float* y) {
     __shared__ __align__(16) OutSmem sm;
     const int nC = (op.T + kC - 1) / kC, bh = blockIdx.x / nC, c = blockIdx.x % nC, bi = bh / op.H, h = bh % op.H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t0 = c * kC;
@@ -726,7 +726,7 @@ struct GradSmem {
 };
 __global__ void __launch_bounds__(kGradThreads, 2)
 wkv7_fp32_grads_kernel(const Operands op, const float* __restrict__ vv, const float* __restrict__ ds_out, const float* __restrict__ ckpt,
-                       const float* __restrict__ carry, const float* __restrict__ sums, float* __restrict__ dw, float* __restrict__ dr,
+                       const float* carry, const float* sums, float* __restrict__ dw, float* __restrict__ dr,
                        float* __restrict__ dk, float* dv, float* __restrict__ da, float* __restrict__ db) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     GradSmem& sm = *reinterpret_cast<GradSmem*>(smem_raw);
