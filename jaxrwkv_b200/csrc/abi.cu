@@ -18,8 +18,8 @@ int wkv7_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w,
                  const uint8_t* ns, const void* dy, const void* ds_out, void* residual, size_t residual_bytes, void* dw, void* dr,
                  void* dk, void* dv, void* da, void* db, void* ds0, const int* run_if);
 
-// fp32 from wkv7_fp32_takes() tokens on: 16 tokens at a time (wkv7_fp32.cu)
-bool wkv7_fp32_takes(int T);
+// fp32 where wkv7_fp32_takes() says so: 16 tokens at a time (wkv7_fp32.cu)
+bool wkv7_fp32_takes(int B, int T, int H);
 size_t wkv7_fp32_workspace_bytes(int B, int T, int H);
 size_t wkv7_fp32_residual_bytes(int B, int T, int H);
 int wkv7_fp32_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
@@ -140,7 +140,8 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
                             range_flag, ticket, mark);
     }
     // 16 tokens at a time where the residual has all its room, or a workspace was brought
-    if (dtype == B200WKV_F32 && wkv7_fp32_takes(T) && (residual != nullptr ? residual_bytes >= wkv7_fp32_residual_bytes(B, T, H) : workspace != nullptr))
+    if (dtype == B200WKV_F32 &&
+        (residual != nullptr ? wkv7_fp32_takes(B, T, H) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H) : workspace != nullptr))
         return wkv7_fp32_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, workspace);
     return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out,
                         residual, nullptr, 0, nullptr);
@@ -234,7 +235,7 @@ size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N) {
     // fp32 keeps a state every 16 tokens; bf16 uses the chunked tensor-core
     // kernels (a state every 64 tokens) unless B200WKV_FLAG_SEQUENTIAL asks otherwise, so size for both
     // (fp32: and for what the backward that works on all chunks side by side wants besides, where it does)
-    if (dtype == B200WKV_F32 && wkv7_fp32_takes(T)) return wkv7_fp32_residual_bytes(B, T, H);
+    if (dtype == B200WKV_F32 && wkv7_fp32_takes(B, T, H)) return wkv7_fp32_residual_bytes(B, T, H);
     const size_t seq = wkv7_seq_residual_bytes(B, T, H);
     if (dtype == B200WKV_F32) return seq + wkv7_seq_carry_bytes(B, T, H);
     const size_t chk = wkv7_chunk_residual_bytes(B, T, H);
@@ -276,7 +277,7 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
         return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
                             residual, b200wkv7_residual_bytes(dtype, B, T, H, N) - kResidualMarkBytes, dw, dr, dk, dv, da, db, ds0, mark);
     }
-    if (dtype == B200WKV_F32 && wkv7_fp32_takes(T) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H))
+    if (dtype == B200WKV_F32 && wkv7_fp32_takes(B, T, H) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H))
         return wkv7_fp32_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, ds_out, residual, dw, dr, dk, dv, da, db, ds0);
     return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
                         residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, nullptr);

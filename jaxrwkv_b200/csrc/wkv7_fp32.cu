@@ -142,9 +142,12 @@ wkv7_fp32_prepare_kernel(const Operands op, const Tiles tiles, float* __restrict
     const int tid = threadIdx.x, t0 = c * kC, row = tid >> 4, lane16 = tid & 15, col = lane16 * 4;
     const int L = min((int)op.length[bi], op.T);
     const bool flag = tid > 0 && tid < kC && t0 + tid < op.T && op.new_starts[(size_t)bi * op.T + t0 + tid] != 0;
-    if (__syncthreads_or(flag) || kind_of(0, t0, op.T, L) == kWalked) return;
     const size_t seq = (size_t)bi * op.T * op.H * kN + (size_t)h * kN, tok = (size_t)op.H * kN;
     const size_t mine = seq + (size_t)(t0 + row) * tok + col;
+    if (__syncthreads_or(flag) || kind_of(0, t0, op.T, L) == kWalked) {      // only the decays, which every warp of the chain needs
+        if (t0 + row < op.T) put4(tiles.left + bh * tiles.head_stride + c * tiles.chunk_stride + row * kN + col, decay4(at4(op.w + mine)));
+        return;
+    }
     {
         const float4 w = at4(op.w + mine), a = at4(op.a + mine), b = at4(op.b + mine), r = at4(op.r + mine);
         const float4 k = kForward ? at4(op.k + mine) : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -389,7 +392,7 @@ struct ChainSmem {
     struct Stage {
         float left[kC][kN], right[kC][kN], decay[kN], d[kRows][kN];
     } st[kStages];
-    float raw[6][kC][kN];                            // w, a, b, r, v, k of a chunk that is walked
+    float raw[6][kC][kN];                            // decay, a, b, r, v, k of a chunk that is walked
     float s[kRows][kC];
     uint64_t full[kStages], empty[kStages], raw_full, raw_empty;
     int kind[kStages];
@@ -427,7 +430,7 @@ template <bool kForward, class Smem>
 __device__ __forceinline__ bool fetch_chunks(Smem& sm, const Operands& op, const Tiles& tiles, const Place<kForward>& at, const float* slots) {
     const int lane = threadIdx.x & 31;
     const uint8_t* const ns = op.new_starts + (size_t)at.bi * op.T;
-    const float* const raw[6] = {op.w, op.a, op.b, op.r, op.v, op.k};
+    const float* const raw[5] = {op.a, op.b, op.r, op.v, op.k};
     const int n_raw = kForward ? 6 : op.v != nullptr ? 5 : 4;
     uint32_t ahead = 0;                              // flags of 32 chunks, one per lane
     int walked = 0;
@@ -458,12 +461,13 @@ __device__ __forceinline__ bool fetch_chunks(Smem& sm, const Operands& op, const
             }
         }
         __syncwarp();
+        const size_t tile = at.bh * tiles.head_stride + at.chunk(it) * tiles.chunk_stride;
         if (kind == kWalked) {
             ++walked;
-            for (int i = lane; i < n_raw * n; i += 32)
-                tc::bulk_load(sm.raw[i / n][i % n], raw[i / n] + at.seq + (size_t)(t0 + i % n) * at.tok, kN * 4, &sm.raw_full);
+            if (lane == 0) tc::bulk_load(sm.raw[0], tiles.left + tile, (uint32_t)(n * kN * 4), &sm.raw_full);
+            for (int i = lane; i < (n_raw - 1) * n; i += 32)
+                tc::bulk_load(sm.raw[1 + i / n][i % n], raw[i / n] + at.seq + (size_t)(t0 + i % n) * at.tok, kN * 4, &sm.raw_full);
         } else {
-            const size_t tile = at.bh * tiles.head_stride + at.chunk(it) * tiles.chunk_stride;
             if (lane == 0) tc::bulk_load(s.left, tiles.left + tile, kTile * 4, bar);
             else if (lane == 1) tc::bulk_load(s.right, tiles.right + tile, kTile * 4, bar);
             else if (lane == 2) tc::bulk_load(s.decay, tiles.decay + tile, kN * 4, bar);
@@ -473,11 +477,6 @@ __device__ __forceinline__ bool fetch_chunks(Smem& sm, const Operands& op, const
     return true;
 }
 
-__device__ __forceinline__ float sum16(float x) {
-#pragma unroll
-    for (int m = 1; m < 16; m <<= 1) x += __shfl_xor_sync(0xffffffffu, x, m);
-    return x;
-}
 // A lane's four columns of R rows
 template <int R>
 struct Slice {
@@ -504,52 +503,98 @@ struct Slice {
     }
 };
 
-// A chunk token by token
+// A chunk token by token.  What a token waits for is one sum over 16 lanes, 150 cycles, which all rows of a lane take together; the
+// operands of four tokens are in registers before the first of them, and the outputs' sums, which nothing waits for, are
+// taken for four tokens at once.  A flag in 300 tokens of 4 heads costs 4.4 us so, 12.1 where every lane takes its own decays and
+// the sums one after the other (T=2048 with a flag every 256 tokens 144 and 168 us, 64 heads, T=300, forward and backward 254 and 268).
+template <int R>
+__device__ __forceinline__ void sum16(float* x) {
+#pragma unroll
+    for (int bit = 1; bit < 16; bit <<= 1)
+#pragma unroll
+        for (int m = 0; m < R; ++m) x[m] += __shfl_xor_sync(0xffffffffu, x[m], bit);
+}
 template <bool kForward, int R, class Smem>
 __device__ __forceinline__ void walk(Slice<R>& x, const Smem& sm, const Operands& op, const Place<kForward>& at, int t0, uint32_t starts, int row, int col,
                                      const float* x0, float* sums, float* y, float* out) {
-    const int n = min(kC, op.T - t0);
+    constexpr int kStep = 4;
+    const int n = min(kC, op.T - t0), l = col >> 2;
     const size_t state_at = ((size_t)at.bh * kN + row) * kN + col;
     auto axpy = [](Pair f, const Row4& a, const Row4& b) { return Row4{fma2(f, a.lo, b.lo), fma2(f, a.hi, b.hi)}; };
 #pragma unroll 1
-    for (int i = 0; i < n; ++i) {
-        const int t = kForward ? i : n - 1 - i;
-        const float4 wd = decay4(at4(&sm.raw[0][t][col]));
-        const Row4 w{pair(wd.x, wd.y), pair(wd.z, wd.w)}, a = row4(&sm.raw[1][t][col]), b = row4(&sm.raw[2][t][col]), r = row4(&sm.raw[3][t][col]);
-        float v[R], sum[R], o[R];
+    for (int i0 = 0; i0 < n; i0 += kStep) {
+        Row4 w[kStep], a[kStep], b[kStep], r[kStep], k[kStep];
+        float v[kStep][R], o[R][kStep];
 #pragma unroll
-        for (int m = 0; m < R; ++m) v[m] = op.v != nullptr ? sm.raw[4][t][row + m] : 0.f;
-        if (kForward) {
-            const Row4 k = row4(&sm.raw[5][t][col]);
-            if ((starts >> t) & 1u) x.clear();
-#pragma unroll
-            for (int m = 0; m < R; ++m) {
-                sum[m] = sum16(dot(x.x[m], a));
-                const Pair V = pair(v[m], v[m]);
-                const Row4 kept{fma2(x.x[m].lo, w.lo, mul2(V, k.lo)), fma2(x.x[m].hi, w.hi, mul2(V, k.hi))};
-                x.x[m] = axpy(pair(sum[m], sum[m]), b, kept);
-                o[m] = sum16(dot(x.x[m], r));
-            }
-            if (col == 0) {
-#pragma unroll
-                for (int m = 0; m < R; ++m) y[at.seq + (size_t)(t0 + t) * at.tok + row + m] = o[m];
-            }
-            if (t0 + t == at.L - 1) x.store(out + state_at);
-        } else {
-            if (t0 + t == at.L - 1 && x0 != nullptr) x.add(x0 + state_at);
+        for (int e = 0; e < kStep; ++e) {
+            const int i = min(i0 + e, n - 1), t = kForward ? i : n - 1 - i;
+            w[e] = row4(&sm.raw[0][t][col]);
+            a[e] = row4(&sm.raw[1][t][col]);
+            b[e] = row4(&sm.raw[2][t][col]);
+            r[e] = row4(&sm.raw[3][t][col]);
+            if (kForward) k[e] = row4(&sm.raw[5][t][col]);
 #pragma unroll
             for (int m = 0; m < R; ++m) {
-                x.x[m] = axpy(pair(v[m], v[m]), r, x.x[m]);
-                sum[m] = sum16(dot(x.x[m], b));
-                const Pair S = pair(sum[m], sum[m]);
-                x.x[m] = Row4{fma2(x.x[m].lo, w.lo, mul2(S, a.lo)), fma2(x.x[m].hi, w.hi, mul2(S, a.hi))};
+                v[e][m] = op.v != nullptr ? sm.raw[4][t][row + m] : 0.f;
+                o[m][e] = 0.f;
             }
-            if ((starts >> t) & 1u) x.clear();
         }
-        if (sums != nullptr && col == 0) {
-            float* const to = sums + at.sum(op, t0 + t) + row;
 #pragma unroll
-            for (int m = 0; m < R; ++m) to[m] = sum[m];
+        for (int e = 0; e < kStep; ++e) {
+            if (i0 + e >= n) break;
+            const int t = kForward ? i0 + e : n - 1 - i0 - e;
+            float sum[R];
+            if (kForward) {
+                if ((starts >> t) & 1u) x.clear();
+#pragma unroll
+                for (int m = 0; m < R; ++m) sum[m] = dot(x.x[m], a[e]);
+                sum16<R>(sum);
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    const Pair V = pair(v[e][m], v[e][m]);
+                    const Row4 kept{fma2(x.x[m].lo, w[e].lo, mul2(V, k[e].lo)), fma2(x.x[m].hi, w[e].hi, mul2(V, k[e].hi))};
+                    x.x[m] = axpy(pair(sum[m], sum[m]), b[e], kept);
+                    o[m][e] = dot(x.x[m], r[e]);
+                }
+                if (t0 + t == at.L - 1) x.store(out + state_at);
+            } else {
+                if (t0 + t == at.L - 1 && x0 != nullptr) x.add(x0 + state_at);
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    x.x[m] = axpy(pair(v[e][m], v[e][m]), r[e], x.x[m]);
+                    sum[m] = dot(x.x[m], b[e]);
+                }
+                sum16<R>(sum);
+#pragma unroll
+                for (int m = 0; m < R; ++m) {
+                    const Pair S = pair(sum[m], sum[m]);
+                    x.x[m] = Row4{fma2(x.x[m].lo, w[e].lo, mul2(S, a[e].lo)), fma2(x.x[m].hi, w[e].hi, mul2(S, a[e].hi))};
+                }
+                if ((starts >> t) & 1u) x.clear();
+            }
+            if (sums != nullptr && col == 0) {
+                float* const to = sums + at.sum(op, t0 + t) + row;
+#pragma unroll
+                for (int m = 0; m < R; ++m) to[m] = sum[m];
+            }
+        }
+        if (kForward) {                              // lane l ends with the outputs of token l % 4
+            float q[R];
+#pragma unroll
+            for (int m = 0; m < R; ++m) {
+                const bool odd = l & 1;
+                const float even = (odd ? o[m][1] : o[m][0]) + __shfl_xor_sync(0xffffffffu, odd ? o[m][0] : o[m][1], 1);
+                const float late = (odd ? o[m][3] : o[m][2]) + __shfl_xor_sync(0xffffffffu, odd ? o[m][2] : o[m][3], 1);
+                q[m] = (l & 2 ? late : even) + __shfl_xor_sync(0xffffffffu, l & 2 ? even : late, 2);
+            }
+#pragma unroll
+            for (int bit = 4; bit < 16; bit <<= 1)
+#pragma unroll
+                for (int m = 0; m < R; ++m) q[m] += __shfl_xor_sync(0xffffffffu, q[m], bit);
+            if (l < kStep && i0 + l < n) {
+#pragma unroll
+                for (int m = 0; m < R; ++m) y[at.seq + (size_t)(t0 + i0 + l) * at.tok + row + m] = q[m];
+            }
         }
     }
 }
@@ -1007,16 +1052,21 @@ int launch_chain(cudaStream_t st, int heads, A... args) {
 }  // namespace
 
 // Whether calls with gradients take these kernels (the rest of wkv7_chain.cu and wkv7_seq.cu: fewer tokens, and residuals without
-// their room).  Forward and backward, token by token / here, us: 4 heads 127 / 122 at T=64 (host time), 160 heads 180 / 128 at T=64,
-// 2389 / 1527 at 1024, 640 heads 534 / 414 at 64, 2003 / 1446 at 256.
-bool wkv7_fp32_takes(int T) { return chunks_of(T) >= 4; }
+// their room).  Where the host's launches take longer than the device (some 100 us for a forward and backward), the four
+// kernels more are 6 us lost; the line is where the token-by-token kernels are at 105-110 us.  Those / here, us: 8 heads 99 / 106
+// at T=256, 125 / 107 at 320; 24 heads 102 / 107 at 160, 134 / 107 at 208; 40 heads 101 / 107 at 104, 129 / 104 at 160; 64 heads 100 / 104
+// at 64, 115 / 105 at 104; 160 heads 177 / 122 at 64, 774 / 480 at 320; 640 heads 534 / 395 at 64.
+bool wkv7_fp32_takes(int B, int T, int H) { return chunks_of(T) >= 4 && chunks_of(T) * ((long long)B * H + 16) >= 440; }
 
 // What a forward call without a residual wants as a workspace (0: it takes the token-by-token chain).  Measured, us, that chain /
-// here: 4 heads 19 / 21 at T=128, 33 / 25 at 256, 117 / 60 at 1024; 48 heads 27 / 27, 49 / 47, 179 / 156; 160 heads 66 / 63, 124 / 117,
-// 476 / 436; 640 heads 170 / 213, 312 / 398: a chain fills the device by itself there, and what is done beside it here
-// comes on top.  The last limit bounds the workspace, 2 GiB.
+// here, and with a flag every 256 tokens and lengths of T / 2 to T: 4 heads 27 / 23 and 27 / 29 at T=200, 37 / 29 and 37 / 33 at
+// 300, 115 / 60 and 115 / 80 at 1000; 32 heads 41 / 37 and 42 / 44 at 256, 76 / 61 and 78 / 82 at 512, 283 / 217 and 289 / 246 at 2000;
+// 48 heads 107 / 95 and 109 / 114 at 600; 64 heads 58 / 60 and 59 / 84 at 300, 176 / 179 and 179 / 216 at 1000.  That chain takes the same
+// time up to a head per SM and doesn't mind flags, this one shares the device with what is done beside it: up to a quarter of a
+// head per SM, from 16 chunks on, and as many as heads.  The last limit bounds the workspace, 2 GiB.
 size_t wkv7_fp32_workspace_bytes(int B, int T, int H) {
-    if (chunks_of(T) < 10 || (long long)B * H > sm_count_of_current_device()) return 0;
+    const long long heads = (long long)B * H;
+    if (chunks_of(T) < 16 || chunks_of(T) < heads || 4 * heads > sm_count_of_current_device()) return 0;
     const size_t bytes = (size_t)B * H * chunks_of(T) * (kN * kN + kTileFloats) * sizeof(float);
     return bytes <= ((size_t)2 << 30) ? bytes : 0;
 }

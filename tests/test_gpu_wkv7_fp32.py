@@ -38,27 +38,28 @@ def check(d, H, gy=True, gs=True):
         assert rel_err(npf(a), b) < TOL, n
 
 
-@pytest.mark.parametrize("T", [63, 64, 65, 95, 160, 177])    # token by token; whole chunks; ragged ones; without gradients too
-@pytest.mark.parametrize("B,H", [(1, 2), (3, 5), (4, 8), (4, 10)])   # each split of a head's rows on 148 SMs
+# each split of a head's rows on 148 SMs; token by token, whole chunks, ragged ones; without gradients from as many chunks as heads on
+@pytest.mark.parametrize("B,H,T", [(1, 2, 384), (1, 2, 385), (1, 2, 400), (3, 5, 224), (3, 5, 225), (3, 5, 256), (3, 5, 271), (4, 8, 161), (4, 8, 512),
+                                   (4, 8, 527), (4, 10, 112), (4, 10, 113), (4, 10, 143), (16, 10, 63), (16, 10, 64), (16, 10, 65)])
 def test_sizes(B, H, T):
     check(wkv7_case(B, T, H, seed=T + B, s0_scale=0.3), H)
 
 
 @pytest.mark.parametrize("B,H", [(4, 1), (4, 4)])
 def test_flags_and_lengths_at_chunk_edges(B, H):
-    T = 176
-    starts = [[0, 16, 32], [15, 31, 175], [1, 48, 49, 96], []]
+    T = 352
+    starts = [[0, 16, 32], [15, 31, 351], [1, 48, 49, 96], []]
     lengths = [0, 48, 47, 97]                                # none; the end of a chunk; inside one; its first token
     check(wkv7_case(B, T, H, seed=H, s0_scale=0.3, starts=starts, lengths=lengths), H)
 
 
 @pytest.mark.parametrize("gy,gs", [(True, False), (False, True)])
 def test_one_cotangent(gy, gs):
-    check(wkv7_case(2, 100, 2, seed=4, p_start=0.02, random_length=True, s0_scale=0.3), 2, gy, gs)
+    check(wkv7_case(2, 340, 2, seed=4, p_start=0.02, random_length=True, s0_scale=0.3), 2, gy, gs)
 
 
 def test_decays_that_vanish():
-    d = wkv7_case(2, 96, 2, seed=9, s0_scale=0.3)
+    d = wkv7_case(2, 352, 2, seed=9, s0_scale=0.3)
     d["w"][:, ::3] = 6.0                                     # exp(-exp(6)) is 0 in 32 bits
     d["w"][:, 1::3] = 4.0                                    # 2e-24 a token
     check(d, 2)
@@ -66,7 +67,7 @@ def test_decays_that_vanish():
 
 @pytest.mark.parametrize("at", [16, 21])                     # the first token of a chunk; inside one
 def test_a_flag_holds_back_what_is_not_a_number(at):
-    B, T, H = 1, 96, 2
+    B, T, H = 1, 400, 2
     d = wkv7_case(B, T, H, seed=5, starts=[[at]], s0_scale=0.3)
     length, ns = (x.cuda() for x in flags(d))
     for name in ("k", "v", "a", "b", "w", "s0"):
