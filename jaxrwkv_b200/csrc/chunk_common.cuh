@@ -229,7 +229,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 // so stepping along K is one 32-bit add on the low word.
 struct Op { uint32_t lo, hi, step16; };
 __device__ __forceinline__ Op make_op(uint32_t addr, uint32_t step, uint32_t lbo, uint32_t sbo) {
-    return {(addr >> 4) | ((lbo >> 4) << 16), (sbo >> 4) | (1u << 14), step >> 4};
+    // (in a cluster the upper bits of a shared-memory address say whose it is)
+    return {((addr >> 4) & 0x3FFF) | ((lbo >> 4) << 16), (sbo >> 4) | (1u << 14), step >> 4};
 }
 __device__ __forceinline__ Op kmaj128(uint32_t a) { return make_op(a, 2 * CB128, CB128, 128); }   // rows = M/N, cols = K
 __device__ __forceinline__ Op kmaj64(uint32_t a) { return make_op(a, 2 * CB64, CB64, 128); }

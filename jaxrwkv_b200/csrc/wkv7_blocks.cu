@@ -9,6 +9,9 @@
 // mma.sync per warp behind one another's results) and the zero-state blocks fill the device: one sequence of 40 heads,
 // T=2048, 224 -> 122 us; of 4 heads, T=4096, 407 -> 103 us.  M' is carried as high + low bf16 parts, U, y' and sa' in fp32, so
 // that the split adds no rounding that the walk does not have in another place (errors against the oracle are the same).
+//
+// What a ring of CTAs does faster (see the rule in wkv7_chunk.cu) no longer comes here: long sequences of few heads stay, whose chain
+// the start flags cut.
 #include "common.cuh"
 #include "tc05.cuh"
 #include "chunk_common.cuh"

@@ -36,6 +36,7 @@
 #include "tmap.cuh"
 #include "wkv7_blocks.h"
 
+#include <algorithm>
 #include <atomic>
 
 namespace b200wkv {
@@ -72,12 +73,20 @@ static_assert(OFF_MT + GTILE <= OFF_M2A + SLAB64, "result tiles must lie over V 
 constexpr int STG_TILE = kC * kN * 2;
 static_assert(5 * STG_TILE <= 2 * SLAB128 + SLAB64 && STG_TILE <= SLAB128 - SLAB64, "staging tiles must fit their hosts");
 __device__ __forceinline__ int stage_off(int m) { return m < 5 ? OFF_AR + m * STG_TILE : OFF_M2A + SLAB64; }
+// A ring's step once the zero-state products are done (nothing here lies over the staging tiles):
+constexpr int OFF_IN = OFF_BH;                   // the entering state, fp32, 16 column pieces of [64 rows][16 bytes], written by the CTA in front
+constexpr int OFF_SB = OFF_SA;                   // the same in bf16         64-row slab
+constexpr int OFF_MH = OFF_V;                    // M', its bf16 part        64-row slab
+constexpr int OFF_ML = OFF_G;                    // M', what that rounds off 64-row slab (over W~)
+constexpr int OFF_WR = OFF_TP;                   // [W~ ; R-]                128-row slab
+static_assert(OFF_IN + kN * kN * 4 <= OFF_SB, "the entering state lies over B^ and K^");
 struct Small {
     float h1[kN];        // cumulative log-decay of tokens 0..31, stored [e][jb] for channel 8 jb + e
     float tot[kN];       // ... of the whole chunk
     float lam[kN];       // exp(tot)
     float lamt[kN];      // the same, stored [e][jb]
     uint64_t bar[5];   // 0..3 product rounds, 4 staging tiles
+    uint64_t ring[4];  // a ring's: state products, output products, the entering state has arrived, the next CTA is ready for one
     uint32_t nsm[2];
     uint32_t tmem;
 };
@@ -175,12 +184,30 @@ __device__ __forceinline__ void store_part(float4* tiles, size_t slot, int hsel,
     for (int c = 0; c < 8; ++c) tiles[slot * 1024 + (hsel * 8 + c) * 64 + row] = make_float4(x[c * 4], x[c * 4 + 1], x[c * 4 + 2], x[c * 4 + 3]);
 }
 
-// kBlocks: the blocks of all sequences as one list, each from a zero state; a CTA walks consecutive ones, and what depends on
-// the entering state is left to the kernels of wkv7_blocks.cu.  Otherwise a CTA walks one sequence (or piece of one).
+__device__ __forceinline__ void load_part(const float4* tiles, size_t slot, int hsel, int row, float* x) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float4 v = tiles[slot * 1024 + (hsel * 8 + c) * 64 + row];
+        x[c * 4] = v.x; x[c * 4 + 1] = v.y; x[c * 4 + 2] = v.z; x[c * 4 + 3] = v.w;
+    }
+}
+
+// kWalk: a CTA walks one sequence (or piece of one).  The others do everything of a block that does not depend on the entering
+// state S0 as if that were zero, which leaves, with U, y', sa' the zero-state results,
+//     S_C = S0 diag(L_C) + S0 M' + U          y_t = R-_t S0^T + y'_t          sa_t = W~_t S0^T + sa'_t,
+// M' as high + low bf16 parts and U, y', sa' in fp32, so that the split adds no rounding that the walk does not have elsewhere.
+// kBlocks: the blocks of all sequences as one list, a CTA has consecutive ones, and what depends on S0 is left to the kernels of
+// wkv7_blocks.cu.
+// kRing: a cluster of CTAs walks one sequence, whose blocks are dealt out in turn.  A CTA takes S0 out of its shared memory, where
+// the CTA with the block in front has put it, passes S_C on to the next one and then finishes its outputs.  A state's way through a
+// CTA takes 2700 cycles (330 to the operand slab, 870 products, 400 results, 1000 to the next CTA), a block 17 k of its CTA's, 13 k of
+// them before the state is needed.  One sequence of 40 heads, T=1999: 114 us in kBlocks, 83 by rings of six; 80 sequences,
+// T=1024: 111 walked, 96 by rings of three.
+enum Form { kWalkForm, kBlocksForm, kRingForm };
 //
 // 256 threads: warp = (quad, hsel); quad selects the 32 TMEM lanes (tile rows) the warp may access,
 // hsel the column half it works on, so every accumulator tile is shared by two warps per row group.
-template <bool kBlocks>
+template <Form kForm>
 __global__ void __launch_bounds__(256, 2)
 wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ r,
                       const __nv_bfloat16* __restrict__ k, const __nv_bfloat16* __restrict__ v,
@@ -193,7 +220,8 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                       int* __restrict__ range_flag, int range_ticket, int* __restrict__ residual_mark,
                       __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces,
                       const BlockParts parts) {
-    if (kBlocks) let_next_in();
+    constexpr bool kBlocks = kForm == kBlocksForm, kRing = kForm == kRingForm, kZero = kBlocks || kRing;
+    if (kZero) let_next_in();
     extern __shared__ __align__(1024) unsigned char smem[];   // (the swizzle of the output tile is a function of the address)
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
     // (all first pieces come first in the grid: where no cut exists the other pieces' CTAs return at once, and the
@@ -203,20 +231,28 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
     const int units = kBlocks ? n_seq * (nSlot - 1) : 0;
     int unit = kBlocks ? (int)((long long)units * blockIdx.x / gridDim.x) : 0;
     const int unit_end = kBlocks ? (int)((long long)units * (blockIdx.x + 1) / gridDim.x) : 0;
-    int bh = kBlocks ? unit / (nSlot - 1) : blockIdx.x % n_seq;
-    const int piece = kBlocks ? 0 : blockIdx.x / n_seq;
+    const uint32_t ring_rank = kRing ? tc::cluster_rank() : 0, ring_size = kRing ? tc::cluster_size() : 1;
+    int bh = kBlocks ? unit / (nSlot - 1) : kRing ? (int)(blockIdx.x / ring_size) : blockIdx.x % n_seq;
+    const int piece = kZero ? 0 : blockIdx.x / n_seq;
     int bi = bh / H, h = bh % H;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int quad = warp & 3, hsel = warp >> 2;
     const int row = quad * 32 + lane;
     int L = min((int)length[bi], Tlen);
+    // a ring's steps: the slots of the sequence in order of time, this CTA's are `step`, step + ring_size, ...
+    const int bl = L / kC;
+    const bool cut = kRing && slot_tokens(nSlot - 1, Tlen, L).n > 0;
+    const int steps = cut ? nSlot : nSlot - 1;
+    auto slot_of = [&](int m) { return !cut || m <= bl ? m : m == bl + 1 ? nSlot - 1 : m - 1; };
+    int step = (int)ring_rank;
     // ---- sequence-parallel mode (pieces > 1, calls without a residual): a start flag cuts every dependence, so a
     // sequence may be walked as independent pieces whose first token carries a start flag.  Cut k, k = 1..pieces-1,
     // is the start flag nearest to k T / pieces within half a piece of it, if there is one; every CTA of the
     // sequence finds the same cuts by itself, a CTA whose own cut does not exist has nothing to do.
     int t_begin = 0, t_end = Tlen;
     if (kBlocks) t_begin = (unit - bh * (nSlot - 1)) * kC;
-    if (!kBlocks && pieces > 1) {
+    if (kRing && step < steps) t_begin = slot_tokens(slot_of(step), Tlen, L).p;
+    if (!kZero && pieces > 1) {
         const uint8_t* ns_row = new_starts + (size_t)bi * Tlen;
         const int half = Tlen / (2 * pieces);
         auto find_cut = [&](int k) -> int {       // position of cut k, or -1; all threads of the CTA take part
@@ -248,12 +284,18 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
     if (tid == 0) {
 #pragma unroll
         for (int i = 0; i < 5; ++i) tc::mbar_init(&sm.bar[i], (i == 2 || i == 3) ? 2 : 1);   // M3, M4: two issuing threads
+        if (kRing) {
+            tc::mbar_init(&sm.ring[0], 1);
+            tc::mbar_init(&sm.ring[1], 1);
+            tc::mbar_init(&sm.ring[2], 1);
+            tc::mbar_init(&sm.ring[3], 1);
+        }
         tc::mbar_init_fence();
         if (blockIdx.x == 0 && residual_mark != nullptr) *residual_mark = 0;   // this residual is in the chunked format (so far)
     }
     if (warp == 0) tc::tmem_alloc(&sm.tmem, 256);
     tc::fence_before_sync();
-    __syncthreads();
+    if (kRing) tc::cluster_sync(); else __syncthreads();   // (the barriers of every CTA of the ring are there)
     tc::fence_after_sync();
     const uint32_t tbase = sm.tmem;
     const uint32_t lane_addr = tbase + ((uint32_t)(quad * 32) << 16);  // this warp's 32 TMEM lanes
@@ -261,7 +303,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
     bool failed = false;
 
     // ---- state into TMEM (rows 0..63 = S0 in fp32, rows 64..127 are never read) --------------
-    if (!kBlocks) {
+    if (!kZero) {
         float s[32];
         if (row < 64 && t_begin == 0) {
 #pragma unroll
@@ -309,6 +351,21 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         }
         pend_y = pend_m = pend_r = false;
     };
+    uint32_t in_par = 0, ready_par = 0, ring_par = 0;     // of the entering states, the next CTA's readiness, the state products
+    if (kRing && L == 0 && step == 0 && quad < 2) {      // the input state comes back as it was given
+        float s[32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const uint4 raw = *reinterpret_cast<const uint4*>(s0 + st_row + c * 8);
+            *reinterpret_cast<uint4*>(s_out + st_row + c * 8) = raw;
+            unpack8(raw, &s[c * 8]);
+        }
+        if (s_at_len != nullptr) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                *reinterpret_cast<float4*>(s_at_len + st_row + c * 4) = make_float4(s[c * 4], s[c * 4 + 1], s[c * 4 + 2], s[c * 4 + 3]);
+        }
+    }
     uint8_t flag_ahead = (tid < 64 && t_begin + tid < Tlen) ? new_starts[(size_t)bi * Tlen + t_begin + tid] : 0;
     // the 64 token rows from cp on of w, r, k, v, a, b into the staging tiles (thread 0; one tiled copy
     // per stream).  Rows past the chunk arrive too and are ignored.
@@ -319,11 +376,11 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             for (int m = 0; m < 6; ++m) tc::tensor_load_2d(smem + stage_off(m), &maps.m[m], ch * kN, cbi * Tlen + cp, &sm.bar[4]);
         }
     };
-    issue_stage(bi, h, t_begin);
+    if (!kRing || step < steps) issue_stage(bi, h, t_begin);
     while (true) {
         // ================= boundary at position p: TMEM holds the state after token p-1 =================
         // (of the pieces of a sequence, the one that has walked token L - 1 holds it; L == 0: the first)
-        const bool want_out = !kBlocks && (p == L) && (p > t_begin || t_begin == 0);
+        const bool want_out = !kZero && (p == L) && (p > t_begin || t_begin == 0);
         if (quad < 2 && want_out) {
             float s[32];
             tc::tmem_ld32(lane_addr + DS + hsel * 32, s);
@@ -336,15 +393,15 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                     *reinterpret_cast<float4*>(s_at_len + st_row + c * 4) = make_float4(s[c * 4], s[c * 4 + 1], s[c * 4 + 2], s[c * 4 + 3]);
             }
         }
-        if (kBlocks ? unit >= unit_end : p >= t_end) break;
+        if (kBlocks ? unit >= unit_end : kRing ? step >= steps : p >= t_end) break;
         // ================= extent of this chunk =================
         // (with a residual the chunks are the 64-token blocks of the sequence, so that the backward can number them)
         const int be = min(kBlocks || saved != nullptr ? ((p >> 6) + 1) << 6 : p + kC, t_end);
-        const int p1 = L > p && L < be ? L : be, n = p1 - p;
-        // what is walked next: the second part of this block, the next block, or the first of the next sequence
+        const int p1 = kRing ? p + slot_tokens(slot_of(step), Tlen, L).n : L > p && L < be ? L : be, n = p1 - p;
+        // what is walked next: the second part of this block, the next block, or the first of the next sequence; a ring's next step
         const bool next_seq = kBlocks && p1 == Tlen;
-        const bool more = kBlocks ? p1 < be || unit + 1 < unit_end : p1 < t_end;
-        const int np = next_seq ? 0 : p1, nh = next_seq ? (h + 1 == H ? 0 : h + 1) : h, nbi = next_seq && h + 1 == H ? bi + 1 : bi;
+        const bool more = kBlocks ? p1 < be || unit + 1 < unit_end : kRing ? step + (int)ring_size < steps : p1 < t_end;
+        const int np = kRing ? slot_tokens(slot_of(more ? step + (int)ring_size : step), Tlen, L).p : next_seq ? 0 : p1, nh = next_seq ? (h + 1 == H ? 0 : h + 1) : h, nbi = next_seq && h + 1 == H ? bi + 1 : bi;
         if (tid < 64) {
             // the flag byte of position p + tid was requested while the previous chunk's products ran
             const bool f = tid < n && flag_ahead != 0;
@@ -359,7 +416,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         // the second part of a block that `length` cuts (the only chunk that starts inside a block)
         const size_t blk_slot = (size_t)bh * nSlot + ((p & (kC - 1)) == 0 ? p >> 6 : nSlot - 1);
         unsigned char* const keep = saved != nullptr ? saved + blk_slot * kSavedBytes : nullptr;
-        const bool affine = kBlocks || keep != nullptr;   // M', R- and L_C are wanted
+        const bool affine = kZero || keep != nullptr;   // M', R- and L_C are wanted
         // ================= stage inputs (registers), log-decay into the scan buffer =================
         uint4 raw[2][5];   // r, k, v, a, b
         float lw[2][8];    // log2 of the decay: -exp(w) * log2(e)
@@ -462,7 +519,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                     const int t = q * 32 + tsub;
 #pragma unroll
                     for (int i = 1; i < 5; ++i)
-                        if (!kBlocks) add_odd(odd, raw[q][i]);
+                        if (!kZero) add_odd(odd, raw[q][i]);
                     const uint4 none = make_uint4(0, 0, 0, 0);
                     if (affine && !in_first(m, t)) {   // what carries the dependence on S0: nothing from the first flag on
                         slab_store(smem + OFF_SA, CB64, t, jb, none);
@@ -474,11 +531,11 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                         slab_store(smem + OFF_KH, CB64, t, jb, none);
                     }
                 }
-                if (!kBlocks && is_odd(odd)) atomicExch(range_flag, range_ticket);
+                if (!kZero && is_odd(odd)) atomicExch(range_flag, range_ticket);
             }
         }
         // ================= entering state: bf16 copy for the products, decayed fp32 copy back to TMEM =====
-        if (!kBlocks && quad < 2) {
+        if (!kZero && quad < 2) {
             float s[32];
             if (reset_here) {
 #pragma unroll
@@ -514,14 +571,14 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         if (tid == 0) {
             tc::fence_after_sync();
             mma_k64(tbase + D1, kmaj128(sAR), kmaj128(sBK), ID_128x128_KK, false);
-            if (!kBlocks) mma_k64(tbase + D2, kmaj128(sAR), kmaj64(sS0), ID_128x64_KK, false);
+            if (!kZero) mma_k64(tbase + D2, kmaj128(sAR), kmaj64(sS0), ID_128x64_KK, false);
             tc::commit(&sm.bar[0]);
         }
-        if (!kBlocks && keep != nullptr && warp == 7 && lane < 8) {   // the bf16 entering state goes to the residual as it is
+        if (!kZero && keep != nullptr && warp == 7 && lane < 8) {   // the bf16 entering state goes to the residual as it is
             tc::bulk_store(keep + (size_t)SAVED_S0 * GTILE + lane * GCB, smem + OFF_S0 + lane * CB64, 64 * 16);
             tc::bulk_commit();
         }
-        if (affine && tid < 64) lam_out[blk_slot * kN + tid] = flagged ? 0.f : sm.lam[tid];
+        if ((kRing ? keep != nullptr : affine) && tid < 64) lam_out[blk_slot * kN + tid] = flagged ? 0.f : sm.lam[tid];
         if (!tc::mbar_wait(&sm.bar[0], par)) failed = true;
         tc::fence_after_sync();
         // ================= E1: triangular masks, operands of the next products =================
@@ -548,7 +605,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 for (int c = 0; c < 8; ++c) slab_store(dst, CB128, row, c, pack8(&d[c * 8]));
             }
         }
-        if (!kBlocks && inner) mask_state_products(lane_addr + D2 + hsel * 32, start_mask(sm), row & 63);
+        if (!kZero && inner) mask_state_products(lane_addr + D2 + hsel * 32, start_mask(sm), row & 63);
         if (warp == 7) tc::bulk_wait_read<0>();   // the S0 slab has been read: the inverse writes over part of it next
         tc::fence_async_smem();
         tc::fence_before_sync();
@@ -556,7 +613,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         // ================= M2: G += A_ak V, Ypart += P_rk V ; meanwhile the triangular inverse =================
         if (tid == 0) {
             tc::fence_after_sync();
-            mma_k64(tbase + D2, kmaj128(sM2A), mnmaj64(sV), ID_128x64_KM, !kBlocks);
+            mma_k64(tbase + D2, kmaj128(sM2A), mnmaj64(sV), ID_128x64_KM, !kZero);
             tc::commit(&sm.bar[1]);
         }
         // A_ak, P_rk and P_rb leave for the residual as bulk copies out of their slabs (one 64-row column
@@ -609,7 +666,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             tc::tmem_wait_ld();
 #pragma unroll
             for (int c = 0; c < 4; ++c) slab_store(smem + OFF_SA, CB64, row, hsel * 4 + c, pack8(&sa[c * 8]));
-            if (kBlocks && keep != nullptr) store_part(parts.sa, blk_slot, hsel, row, sa);
+            if (kZero && keep != nullptr) store_part(parts.sa, blk_slot, hsel, row, sa);
             if (affine) {
                 tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, sa);
                 tc::tmem_wait_ld();
@@ -621,10 +678,11 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 }
             }
         }
+        if (kRing && warp == 7) tc::bulk_wait_read<0>();   // (T has left its slab, which is written over behind the next products)
         tc::fence_async_smem();
         tc::fence_before_sync();
         __syncthreads();
-        if (!kBlocks && keep != nullptr && warp == 7 && lane < 8) {   // sa
+        if (!kZero && keep != nullptr && warp == 7 && lane < 8) {   // sa
             tc::bulk_store(keep + (size_t)SAVED_SA * GTILE + lane * GCB, smem + OFF_SA + lane * CB64, 64 * 16);
             tc::bulk_commit();
         }
@@ -632,7 +690,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         if (tid == 0) {
             tc::fence_after_sync();
             mma_k64(tbase + D2, kmaj128(sTP), mnmaj64(sSA), ID_128x64_KM, true);
-            mma_k64(tbase + DS, mnmaj64(sSA), mnmaj64(sBH), ID_128x64_MM, !kBlocks);
+            mma_k64(tbase + DS, mnmaj64(sSA), mnmaj64(sBH), ID_128x64_MM, !kZero);
             mma_k64(tbase + DS, mnmaj64(sV), mnmaj64(sKH), ID_128x64_MM, true);
             tc::commit(&sm.bar[3]);
         } else if (tid == kIssuer2) {
@@ -646,7 +704,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
             tc::commit(&sm.bar[3]);
         }
         if (tid < 64) flag_ahead = (more && np + tid < Tlen) ? new_starts[(size_t)nbi * Tlen + np + tid] : 0;   // next chunk's start flags
-        if (kBlocks && flagged && quad < 2) {
+        if (kZero && flagged && quad < 2) {
             const int at = hsel * 4 * CB64 + row * 16;
             leave_to_sequential_if_odd(smem + OFF_SA + at, smem + OFF_G + at, smem + OFF_V + at, range_flag, range_ticket);
         }
@@ -691,6 +749,168 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                     if (t < n) to[c] = pack8(rf);
                 }
             }
+        } else if constexpr (kRing) {
+            // (the slabs that the entering state is put over have been read)
+            const uint32_t left = (ring_rank + ring_size - 1) % ring_size, right = (ring_rank + 1) % ring_size;
+            if (tid == 0 && step > 0) {
+                tc::mbar_expect_tx(&sm.ring[2], kN * kN * 4);
+                tc::mbar_arrive_in_cta(tc::in_cta(&sm.ring[3], left));
+            }
+            float x[32];
+            if (quad < 2) {
+                tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);          // M'[j][j'], row j = this thread's lane, as high + low parts
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint4 high = pack8(&x[c * 8]);
+                    float hf[8];
+                    unpack8(high, hf);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) hf[e] = x[c * 8 + e] - hf[e];
+                    slab_store(smem + OFF_MH, CB64, row, hsel * 4 + c, high);
+                    if (keep != nullptr) {
+                        reinterpret_cast<uint4*>(mprime)[blk_slot * 512 + (hsel * 4 + c) * 64 + row] = high;
+                        slab_store(smem + OFF_WR, CB128, row, hsel * 4 + c, *reinterpret_cast<const uint4*>(smem + OFF_G + (hsel * 4 + c) * CB64 + row * 16));
+                    }
+                    slab_store(smem + OFF_ML, CB64, row, hsel * 4 + c, pack8(hf));
+                }
+            } else {
+                const int t = row - 64;
+                uint4* const to = reinterpret_cast<uint4*>(rbar + seq_base + (size_t)(p + min(t, n - 1)) * tok_stride + hsel * 32);
+                uint4 rt[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) rt[c] = to[c];             // R~, stored when the operands were scaled
+                tc::tmem_ld32(lane_addr + D1 + 64 + hsel * 32, x);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    float rf[8];
+                    unpack8(rt[c], rf);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) rf[e] += x[c * 8 + e];
+                    const uint4 r_bar = pack8(rf);
+                    slab_store(smem + OFF_WR, CB128, row, hsel * 4 + c, r_bar);
+                    if (keep != nullptr && t < n) to[c] = r_bar;
+                }
+            }
+            // ---- the leaving state: of a flagged block U, which waits for nothing, otherwise what becomes of the entering one
+            auto pass_on = [&](const float* state) {
+                if (step + 1 < steps) {
+                    const uint32_t to = tc::in_cta(smem + OFF_IN, right), bar = tc::in_cta(&sm.ring[2], right);
+#pragma unroll
+                    for (int c = 0; c < 8; ++c)
+                        tc::store_in_cta(to + (uint32_t)((hsel * 8 + c) * 64 + row) * 16, make_float4(state[c * 4], state[c * 4 + 1], state[c * 4 + 2], state[c * 4 + 3]), bar);
+                }
+                if (p1 == L) {                 // the returned state
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(s_out + st_row + c * 8) = pack8(&state[c * 8]);
+                    if (s_at_len != nullptr) {
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            *reinterpret_cast<float4*>(s_at_len + st_row + c * 4) = make_float4(state[c * 4], state[c * 4 + 1], state[c * 4 + 2], state[c * 4 + 3]);
+                    }
+                }
+            };
+            if (flagged && quad < 2) {
+                if (step + 1 < steps && !tc::mbar_wait_cluster(&sm.ring[3], ready_par)) failed = true;
+                tc::tmem_ld32(lane_addr + DS + hsel * 32, x);
+                tc::tmem_wait_ld();
+                pass_on(x);
+            }
+            // ---- the entering state
+            float4* const entering = reinterpret_cast<float4*>(smem + OFF_IN);
+            if (quad < 2) {
+                if (step == 0) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) unpack8(*reinterpret_cast<const uint4*>(s0 + st_row + c * 8), &x[c * 8]);
+                    store_part(entering, 0, hsel, row, x);
+                } else {
+                    if (!tc::mbar_wait_cluster(&sm.ring[2], in_par)) failed = true;
+                    load_part(entering, 0, hsel, row, x);
+                }
+                if (flagged) {
+                    float odd = 0.f;
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) odd = fmaf(x[c], 0.f, odd);
+                    if (odd != 0.f) atomicExch(range_flag, range_ticket);
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) slab_store(smem + OFF_SB, CB64, row, hsel * 4 + c, reset_here ? make_uint4(0, 0, 0, 0) : pack8(&x[c * 8]));
+            }
+            if (step > 0) in_par ^= 1u;
+            tc::fence_async_smem();
+            tc::fence_before_sync();
+            __syncthreads();
+            if (tid == 0 && !flagged) {
+                tc::fence_after_sync();
+                mma_k64(tbase + DS, kmaj64(tc::smem_u32(smem + OFF_SB)), mnmaj64(tc::smem_u32(smem + OFF_ML)), ID_128x64_KM, true);
+                mma_k64(tbase + DS, kmaj64(tc::smem_u32(smem + OFF_SB)), mnmaj64(tc::smem_u32(smem + OFF_MH)), ID_128x64_KM, true);
+                tc::commit(&sm.ring[0]);
+            } else if (tid == kIssuer2) {      // what no other CTA waits for
+                tc::fence_after_sync();
+                mma_k64(tbase + D1, kmaj128(tc::smem_u32(smem + OFF_WR)), kmaj64(tc::smem_u32(smem + OFF_SB)), ID_128x64_KK, false);
+                tc::commit(&sm.ring[1]);
+            }
+            if (keep != nullptr && warp == 7 && lane < 8) {   // the bf16 entering state goes to the residual
+                tc::bulk_store(keep + (size_t)SAVED_S0 * GTILE + lane * GCB, smem + OFF_SB + lane * CB64, 64 * 16);
+                tc::bulk_commit();
+            }
+            if (!flagged) {
+                // (meanwhile: whether the next CTA can take the state, what remains of the entering one)
+                if (quad < 2) {
+                    if (step + 1 < steps && !tc::mbar_wait_cluster(&sm.ring[3], ready_par)) failed = true;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const float4 l4 = *reinterpret_cast<const float4*>(&sm.lam[hsel * 32 + c * 4]);
+                        x[c * 4] *= l4.x; x[c * 4 + 1] *= l4.y; x[c * 4 + 2] *= l4.z; x[c * 4 + 3] *= l4.w;
+                    }
+                }
+                if (!tc::mbar_wait(&sm.ring[0], ring_par)) failed = true;
+                ring_par ^= 1u;
+                tc::fence_after_sync();
+                if (quad < 2) {
+                    float s[32];
+                    tc::tmem_ld32(lane_addr + DS + hsel * 32, s);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int c = 0; c < 32; ++c) s[c] += x[c];
+                    pass_on(s);
+                }
+            }
+            if (step + 1 < steps) ready_par ^= 1u;
+            // ---- outputs (and sa)
+            if (!tc::mbar_wait(&sm.ring[1], par)) failed = true;
+            tc::fence_after_sync();
+            if (quad >= 2) {
+                const int t = row - 64;
+                float yv[32];
+                tc::tmem_ld32(lane_addr + D2 + hsel * 32, yv);
+                tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 32; ++c) yv[c] += x[c];
+                if (n == kC) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        *reinterpret_cast<uint4*>(smem + OFF_YT + t * 128 + (((hsel * 4 + c) ^ (t & 7)) << 4)) = pack8(&yv[c * 8]);
+                } else if (t < n) {
+                    __nv_bfloat16* dst = y + seq_base + (size_t)(p + t) * tok_stride + hsel * 32;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(dst + c * 8) = pack8(&yv[c * 8]);
+                }
+            } else if (keep != nullptr) {
+                float s[32];
+                tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);
+                load_part(parts.sa, blk_slot, hsel, row, s);
+                tc::tmem_wait_ld();
+#pragma unroll
+                for (int c = 0; c < 32; ++c) s[c] += x[c];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    *reinterpret_cast<uint4*>(keep + (size_t)SAVED_SA * GTILE + (hsel * 4 + c) * GCB + row * 16) = pack8(&s[c * 8]);
+            }
+            pend_y = (n == kC);
+            pend_p = p;
         } else {
         if (quad >= 2) {
             const int t = row - 64;
@@ -737,6 +957,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
         tc::fence_before_sync();
         if (warp == 7) tc::bulk_wait_read<0>();   // the slabs copied out may be rewritten after the next barrier
         p = np;
+        if (kRing) step += (int)ring_size;
         if (kBlocks) {
             if (p1 == be) ++unit;
             if (next_seq) {
@@ -754,7 +975,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
     if (warp == 7) tc::bulk_wait_all<0>();   // every copy to the residual has landed before the CTA retires
     if (failed) atomicExch(&g_status, 1);
     tc::fence_before_sync();
-    __syncthreads();
+    if (kRing) tc::cluster_sync(); else __syncthreads();   // (no CTA of a ring leaves while another one may still write to it)
     if (warp == 0) tc::tmem_dealloc(tbase, 256);
 }
 
@@ -792,7 +1013,7 @@ int* wkv_call_flag(int* ticket) {
     return ring + (t & 63u);
 }
 
-// The rule between the two forms, as the bytes of workspace that the block-parallel one wants (0: the sequential walk).
+// The rule between the three forms, as the bytes of workspace that rings and blocks side by side want (0: the sequential walk).
 // Walking a sequence takes 6.6 us per block whatever else runs, up to one sequence per SM; side by side, a block costs 0.04 us
 // of the device and a step of the chain 1.2-1.5 us, and two more launches and the workspace some 10 us of host time.  Measured
 // (us, walk / side by side, forward of BH sequences without start flags): T=256: 37 / 36 at BH=40, 39 / 48 at 96; T=1024:
@@ -801,13 +1022,42 @@ int* wkv_call_flag(int* ticket) {
 // at 4096).  Without one, the walk is cut at start flags where there are any, and then wins where there are many blocks
 // (a flag every 256 tokens: 156 / 138 at BH=64, T=2048; 163 / 164 at 40, 181 / 227 at 64, T=4096): up to nine blocks per CTA
 // slot.  The last limit bounds the workspace, 2 GiB.
+//
+// Rings take precedence.  A ring has as many CTAs as the device has room for: seven eighths of the two slots per SM, because a
+// cluster stays within a GPC (BH=32, T=2048: 83 us by six, 72 by seven, 68 by eight; 114 by nine, which do not fit at once;
+// BH=80: three, and two CTAs only wait for one another).  Nine are enough to keep a state moving (17 k cycles for a block, 2.7 k for
+// a hop); up to a sixteenth of a sequence per SM there is room for sixteen, which halves the time between start flags.  Without
+// flags a ring is never slower than the other two.  With many, blocks side by side and the walk in pieces are cut into shorter
+// chains, a ring isn't, and its few CTAs lose in long sequences.  The limits in blocks are where both are equal at a flag every
+// 256 tokens (us, walk or side by side / ring, without flags and with):
+//     BH=4:   T=2048 60 / 56, 42 / 42      4096 99 / 99, 52 / 60         BH=16:  T=1600 68 / 54, 54 / 50    4096 137 / 110, 85 / 104
+//     BH=32:  T=4096 185 / 123, 130 / 125                                BH=40:  T=3000 157 / 119, 124 / 124  4096 201 / 157, 158 / 163
+//     BH=48:  T=2000 126 / 101, 115 / 106  4096 418 / 187, 161 / 201     BH=64:  T=2000 145 / 127, 133 / 136  4096 419 / 242, 170 / 258
+//     BH=80:  T=1024 112 / 94, 124 / 97    2000 216 / 171, 138 / 180     BH=72 (side by side):  T=2000 158 / 170, 153 / 183
+// From three blocks on (T=192: 25.3 / 19; two: 19.2 / 17-21), with a residual from four: there the host, who has a workspace to
+// allocate, is what such a call waits for.
+static int ring_size(int B, int T, int H, bool residual) {
+    const long long sms = sm_count_of_current_device(), seqs = (long long)B * H, blocks = block_slots(T) - 1;
+    const long long n = 16 * seqs <= sms ? 16 : std::min(7 * sms / 4 / seqs, 9LL);
+    const long long longest = n * seqs < 4 * sms / 3 ? 24 : n >= 7 ? 65535 : n == 6 ? 48 : n > 3 ? 32 : 2 * seqs > sms ? 16 : 0;
+    if (n < 3 || blocks < (residual ? 4 : 3) || blocks > longest) return 1;
+    return (int)std::min(n, blocks);
+}
+// A ring's workspace.  With a residual: sa' of every slot, which waits there for the entering state.  Without: R~ of every token, which
+// the residual would have room for.
+static size_t ring_bytes(int B, int T, int H, bool residual) {
+    return (size_t)B * H * (residual ? (size_t)block_slots(T) * (kC * kN * sizeof(float)) : (size_t)T * (kN * sizeof(__nv_bfloat16)));
+}
+
 size_t wkv7_blocks_bytes(int B, int T, int H, bool residual) {
+    const size_t most = (size_t)2 << 30;
+    if (ring_size(B, T, H, residual) > 1 && ring_bytes(B, T, H, residual) <= most) return ring_bytes(B, T, H, residual);
     const long long sms = sm_count_of_current_device(), seqs = (long long)B * H, blocks = block_slots(T) - 1;
     if (blocks < 4 || blocks >= 65536) return 0;
     if (2 * seqs > sms && !(residual && blocks >= 24 && 3 * seqs <= 2 * sms)) return 0;
     if (!residual && seqs * blocks > 9 * 2 * sms) return 0;
     const size_t bytes = blocks_layout(B, T, H, residual).end;
-    return bytes <= ((size_t)2 << 30) ? bytes : 0;
+    return bytes <= most ? bytes : 0;
 }
 
 int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v,
@@ -816,9 +1066,13 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
     typedef __nv_bfloat16 bf;
     static DeviceOnce smem_attr;   // the opt-in to large dynamic shared memory is a per-device function attribute
     if (!smem_attr.ok([]() {
-            const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+            const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kWalkForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
             if (e != cudaSuccess) return e;
-            return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+            const cudaError_t f = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+            if (f != cudaSuccess) return f;
+            const cudaError_t g = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (g != cudaSuccess) return g;
+            return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kBlocksForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
         }))
         return B200WKV_ELAUNCH;
     *range_flag = wkv_call_flag(range_ticket);
@@ -831,6 +1085,28 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
     StreamMaps out_maps;                         // m[0]: the outputs, with the 128-byte swizzle of the kernel's output tile
     const void* out_bases[2] = {y, residual ? (const void*)((char*)residual + lay.rbar) : y};   // m[1]: the R- rows
     if (!make_stream_maps(&out_maps, out_bases, 2, B, T, H, /*swizzle128=*/true)) return B200WKV_ELAUNCH;
+    // (a workspace that is there has the bytes of the one form or the other)
+    const int ring = workspace != nullptr && ring_bytes(B, T, H, residual != nullptr) <= ((size_t)2 << 30) ? ring_size(B, T, H, residual != nullptr) : 1;
+    if (ring > 1) {
+        BlockParts parts = {};
+        parts.sa = (float4*)workspace;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ring; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(B * H * ring));
+        cfg.blockDim = dim3(256);
+        cfg.dynamicSmemBytes = SMEM_BYTES;
+        cfg.stream = st;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, wkv7_chunk_fwd_kernel<kRingForm>, T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a,
+                                  (const bf*)b, (const bf*)s0, length, ns, (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : (float*)nullptr, maps,
+                                  out_maps.m[0], out_maps.m[1], residual ? (unsigned char*)(base + lay.saved) : (unsigned char*)nullptr, *range_flag,
+                                  *range_ticket, residual_mark, residual ? (bf*)(base + lay.mprime) : (bf*)nullptr,
+                                  residual ? (bf*)(base + lay.rbar) : (bf*)workspace,
+                                  residual ? (float*)(base + lay.lam) : (float*)nullptr, 1, parts) == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+    }
     if (workspace != nullptr) {   // the blocks side by side (see wkv7_blocks_bytes)
         const BlocksLayout bl = blocks_layout(B, T, H, residual != nullptr);
         char* const ws = static_cast<char*>(workspace);
@@ -843,7 +1119,7 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
         c.s0_tiles = residual ? c.saved + (size_t)SAVED_S0 * GTILE : (unsigned char*)(ws + bl.s0);
         c.s0_stride = residual ? kSavedBytes : (size_t)GTILE;
         const long long units = (long long)B * H * (block_slots(T) - 1), slots = 2LL * sm_count_of_current_device();
-        wkv7_chunk_fwd_kernel<true><<<(int)(units < slots ? units : slots), 256, SMEM_BYTES, st>>>(
+        wkv7_chunk_fwd_kernel<kBlocksForm><<<(int)(units < slots ? units : slots), 256, SMEM_BYTES, st>>>(
             T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a, (const bf*)b, (const bf*)s0, length, ns, (bf*)y,
             (bf*)s_out, nullptr, maps, out_maps.m[0], out_maps.m[1], c.saved, *range_flag, *range_ticket, residual_mark, c.mprime, c.rbar, c.lam, 1,
             c.parts);
@@ -861,7 +1137,7 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
         if (pieces > T / 128) pieces = T / 128;
         if (pieces < 1 || T / pieces >= 32768) pieces = 1;
     }
-    wkv7_chunk_fwd_kernel<false><<<B * H * pieces, 256, SMEM_BYTES, st>>>(T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v,
+    wkv7_chunk_fwd_kernel<kWalkForm><<<B * H * pieces, 256, SMEM_BYTES, st>>>(T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v,
                                                           (const bf*)a, (const bf*)b, (const bf*)s0, length, ns,
                                                           (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : nullptr,
                                                           maps, out_maps.m[0], out_maps.m[1],
