@@ -124,8 +124,10 @@ __global__ void token_shift_fwd_kernel(int B, int Tlen, int D, int M, const T* _
 // The mix gradients leave as one fp32 partial sum per (batch row, tile): deterministic, no atomics.
 //   gx[t] = sum_m g_m[t] (1 - c_m) + [t+1 < T and not start[t+1]] sum_m g_m[t+1] c_m + [t == last] gstate
 // grid (ceil(D / V / kLanes), tiles, B)
-template <typename T, int V, int MM, int kLanes, int kParts>
-__global__ void __launch_bounds__(kLanes * kParts)
+// Tokens are taken G at a time: the G x (MM + 1) loads of a group are all issued, in packed form, before the first token of the group
+// is worked on.  kThreads per SM, which bounds the registers (0: 255).
+template <typename T, int V, int MM, int kLanes, int kParts, int G, int kThreads>
+__global__ void __launch_bounds__(kLanes * kParts, kThreads / (kLanes * kParts))
 token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T* __restrict__ prev,
                        const MixPtrs mix, const uint32_t* __restrict__ length,
                        const uint8_t* __restrict__ new_starts, const T* __restrict__ gout,
@@ -165,9 +167,6 @@ token_shift_bwd_kernel(int B, int Tlen, int D, const T* __restrict__ x, const T*
     }
     Vec<V> xc = zerov<V>();
     if (any) xc = loadv<V>(x + base + (size_t)(t1 - 1) * D);
-    // Tokens are taken four at a time: the 4 x (MM + 1) loads of a group are all issued, in packed form, before
-    // the first token of the group is worked on, so a thread has ~450 bytes in flight at 255 registers.
-    constexpr int G = 4;
     for (int tg = t1 - 1; tg >= t0; tg -= G) {
         RawVec<V, T> rg[G][MM], rx[G];
 #pragma unroll
@@ -255,11 +254,29 @@ void launch_bwd_m(cudaStream_t st, int B, int Tlen, int D, const void* x, const 
         kernel<<<grid, lanes * parts, 0, st>>>(B, Tlen, D, (const T*)x, (const T*)prev, mix, length, ns, (const T*)gout, (const T*)gstate, (T*)gx,
                                                (T*)gprev, (float*)gmix);
     };
-    // Fewer blocks than SMs: four parts per tile instead, of 32 x V channels (B=1, T=512, D=768, M=6, bf16: 35 -> 13 us).  With
-    // more, whole tiles keep more of a row together (B=8, T=2048, D=768: 59 us against 70; B=8, T=4096, D=2048: 230 against 306).
-    const long long blocks = (long long)((D / V + 63) / 64) * tiles * B;
-    if (blocks <= sm_count_of_current_device()) launch(token_shift_bwd_kernel<T, V, MM, 32, 4>, 32, 4);
-    else launch(token_shift_bwd_kernel<T, V, MM, 64, 1>, 64, 1);
+    const long long sms = sm_count_of_current_device();
+    auto fits = [&](int lanes, int per_sm) { return (long long)((D / V + lanes - 1) / lanes) * tiles * B <= per_sm * sms; };
+    if constexpr (sizeof(T) == 4) {
+        // Fewer blocks than SMs: four parts per tile instead, of 32 x V channels.  With more, whole tiles keep more of a row together.
+        if (fits(64, 1)) launch(token_shift_bwd_kernel<T, V, MM, 32, 4, 4, 0>, 32, 4);
+        else launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 4, 0>, 64, 1);
+    } else {
+        // A thread's walk is a chain of groups, 2.7 us each, and what hides it is what is in flight besides: threads with four channels
+        // (with eight, 255 registers held groups of four tokens), and of the splits the finest whose blocks are all resident at once;
+        // once that is many threads anyway, they need less in flight each.  us, eight channels (whole tiles or four parts) / here, M=6:
+        //   D=768   T=256  B=1  15 / 8.5    T=512  B=8 26 / 13.6                   D=2048  T=831  B=1  17 / 12
+        //   D=2048  T=1024 B=2  30 / 18 by 64 lanes, 2 parts of groups of 8 (23 by 32 lanes and 4 parts, which do not fit at once)
+        //   D=2048  T=1000 B=3  48 / 24 by 2 parts, groups of 4 (8: 32)
+        //   D=2048  T=1024 B=4  50 / 33 by whole tiles, groups of 8 (42 by 2 parts)
+        //   D=768   T=2048 B=8  61 / 42, groups of 5 (8: 58, 3: 49)
+        //   D=2048  T=1024 B=8  74 / 57, groups of 3 (5: 70)
+        if (fits(32, 3)) launch(token_shift_bwd_kernel<T, V, MM, 32, 4, 4, 384>, 32, 4);
+        else if (fits(64, 2)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 8, 256>, 64, 2);
+        else if (fits(64, 3)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 4, 384>, 64, 2);
+        else if (fits(64, 4)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 8, 256>, 64, 1);
+        else if (fits(64, 6)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 5, 384>, 64, 1);
+        else launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 3, 512>, 64, 1);
+    }
 }
 
 template <typename T, int V>
@@ -292,7 +309,6 @@ int token_shift_bwd(cudaStream_t st, int dtype, int B, int T, int D, int M, cons
     MixPtrs rows;
     for (int m = 0; m < 8; ++m) rows.p[m] = mix[m < M ? m : 0];
     if (dtype == B200WKV_F32) launch_bwd<float, 4>(st, B, T, D, M, x, prev, rows, length, ns, gout, gstate, gx, gprev, gmix);
-    else if (D % 8 == 0) launch_bwd<__nv_bfloat16, 8>(st, B, T, D, M, x, prev, rows, length, ns, gout, gstate, gx, gprev, gmix);
     else launch_bwd<__nv_bfloat16, 4>(st, B, T, D, M, x, prev, rows, length, ns, gout, gstate, gx, gprev, gmix);
     return cudaGetLastError() == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
 }
