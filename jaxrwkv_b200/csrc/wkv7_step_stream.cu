@@ -6,7 +6,7 @@
 // asynchronous copies (an mbarrier per stage counts the bytes).  The current state is updated in
 // registers, four rows of sixteen columns per thread (64 elements: the fixed cost of an iteration and
 // the reads of the six vectors are spread over them).  A stage is handed back to the copy thread as soon
-// as its state is in registers, so the whole ring is loads in flight; results leave the registers as
+// as its state has been used once, so the whole ring is loads in flight; results leave the registers as
 // 32-byte stores (one full sector per lane).  The six vectors of a pair travel into its stage with the
 // state and the start / length flags are fetched 64 pairs at a time: no iteration waits for a global
 // load of its own, which under a saturated memory system would cost microseconds each.
@@ -83,7 +83,7 @@ struct StepSmem {
     alignas(16) float vec[2][6][kN];   // decay, r, k, v, a, b of the current and the next pair
     unsigned char flags[2][kFlagBatch];
     uint64_t full[Tile<T>::kStages];   // the stage's bytes have arrived
-    uint64_t done[Tile<T>::kStages];   // both computing warps have taken the stage into registers
+    uint64_t done[Tile<T>::kStages];   // both computing warps have used what they read of the stage
 };
 
 template <typename T>
@@ -213,8 +213,6 @@ wkv7_step_stream_kernel(int BH, int H, const T* __restrict__ w, const T* __restr
         for (int g = 0; g < 4; ++g)
 #pragma unroll
             for (int q = 0; q < kChunks; ++q) TL::unpack(*reinterpret_cast<const uint4*>(stage + chunk_off(g, q)), &S[g][q * kCE]);
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&sm.done[s]);   // this warp has its half of the stage in registers
         T* const out = s_out + state_off(bh) + (size_t)row0 * kN + 16 * p;
         // register slot q of a lane of odd rsel holds chunk q ^ 1: such a lane stores its slots swapped
         auto write_state = [&]() {
@@ -253,6 +251,12 @@ wkv7_step_stream_kernel(int BH, int H, const T* __restrict__ w, const T* __restr
             sa[g] = sum4(sa[g]);
             vv[g] = vec[3][row0 + 8 * g];
         }
+        // Every value of this warp's half of the stage has gone into a sum that the shuffles above have passed on, so nothing of the
+        // stage is still to be read when it is handed back.  With the hand-back right behind the loads and nothing in between
+        // that needs their values, the last ones of a warp (its upper 16 rows) now and then returned the pair that was loaded next:
+        // fp32, 5120 pairs, one pair in some 150000.  The later place costs nothing (32 layers at 10240 bf16 pairs 1082 / 1081 us).
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&sm.done[s]);
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
             const int c = vgroup(cc);
