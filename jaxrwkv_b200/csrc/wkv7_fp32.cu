@@ -634,6 +634,9 @@ wkv7_fp32_chain_kernel(const Operands op, const Tiles tiles, const float* __rest
         const typename Smem::Stage& s = sm.st[stage];
         if (kForward && kind == kFresh) x.clear();
         x.store(slots + at.slot(it) + in_state);
+        // (the stage of the chunk before: what was read of it went into the state that has just been stored)
+        __syncwarp();
+        if (it > 0 && lane == 0) tc::mbar_arrive(&sm.empty[(it - 1) % Smem::kStages]);
         if (kind != kWalked) {
             if (!kForward && at.L == t0 + kC && x0 != nullptr) x.add(x0 + state_at);
             // Slot i of a lane holds token i ^ l, so that the sums over the 16 lanes need no exchange of halves: what a lane keeps
@@ -690,8 +693,6 @@ wkv7_fp32_chain_kernel(const Operands op, const Tiles tiles, const float* __rest
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(&sm.raw_empty);
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&sm.empty[stage]);
     }
     if (!kForward) {
         if (at.L == 0 && x0 != nullptr) x.add(x0 + state_at);
