@@ -715,8 +715,9 @@ wkv7_fp32_outputs_kernel(const Operands op, const Tiles tiles, const float* slot
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t0 = c * kC;
     const int L = min((int)op.length[bi], op.T);
     const bool flag = tid > 0 && tid < kC && t0 + tid < op.T && op.new_starts[(size_t)bi * op.T + t0 + tid] != 0;
-    if (__syncthreads_or(flag) || kind_of(0, t0, op.T, L) == kWalked) return;
-    wait_for_grid_in_front();
+    const bool walked = __syncthreads_or(flag) || kind_of(0, t0, op.T, L) == kWalked;
+    wait_for_grid_in_front();                        // (also where there is nothing to do: see launch_in_chain)
+    if (walked) return;
     const float* const state = slots + ((size_t)bh * nC + c) * (kN * kN);
     const float* const rbar = tiles.rbar + bh * tiles.head_stride + c * tiles.chunk_stride;
 #pragma unroll
