@@ -104,9 +104,9 @@ int b200wkv7_step_inplace(void* stream, int dtype, int B, int H, int N,
  * streams and of the initial state out (the reference's result order is
  * gw, gr, gk, gv, ga, gb, gs — rwkv7.py:406).  dy or ds_out may be NULL (= zeros).
  * Unlike the reference kernels (README "CudaRWKV" caveats), gradients flow from
- * s_out and into s0, and start flags cut the dependency exactly.  The fp32
- * backward keeps tiles in the gradient buffers until it writes the gradients:
- * they must not overlap an operand. */
+ * s_out and into s0, and start flags cut the dependency exactly.  In fp32
+ * a gradient may be written over an operand of its size (the same address), dy
+ * and ds_out among them; such a call takes the slower token-by-token kernels. */
 int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N,
                  const void* w, const void* r, const void* k, const void* v,
                  const void* a, const void* b, const void* s0,

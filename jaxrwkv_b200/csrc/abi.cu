@@ -103,6 +103,11 @@ static bool aligned(size_t bytes, std::initializer_list<const void*> ps) {
     for (const void* p : ps) bits |= reinterpret_cast<uintptr_t>(p);
     return bits % bytes == 0;
 }
+// Whether `n` bytes at x and `m` bytes at y have any in common (NULL: none).
+static bool meet(const void* x, size_t n, const void* y, size_t m) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
+    return a != 0 && b != 0 && a < b + m && b < a + n;
+}
 // four elements, what the token-sequential kernels access at a time
 static size_t vec4_bytes(int dtype) { return dtype == B200WKV_F32 ? 16 : 8; }
 
@@ -277,7 +282,20 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
         return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
                             residual, b200wkv7_residual_bytes(dtype, B, T, H, N) - kResidualMarkBytes, dw, dr, dk, dv, da, db, ds0, mark);
     }
-    if (dtype == B200WKV_F32 && wkv7_fp32_takes(B, T, H) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H))
+    // Gradients written over operands: the token-by-token kernels read a chunk's rows before they write them, where those for 16 tokens
+    // at a time keep tiles in the gradients' buffers first.  ds0 over ds_out: without a carry between runs, which would be written
+    // before the last read.  (The forward's checkpoints are the same for both.)
+    bool in_place = false;
+    const size_t stream_bytes = (size_t)B * T * H * kN * sizeof(float), state_bytes = (size_t)B * H * kN * kN * sizeof(float);
+    if (dtype == B200WKV_F32) {
+        for (const void* g : {dw, dr, dk, dv, da, db})
+            for (const void* x : {w, r, k, v, a, b, dy}) in_place |= meet(g, stream_bytes, x, stream_bytes);
+        if (meet(ds0, state_bytes, ds_out, state_bytes)) {
+            in_place = true;
+            residual_bytes = wkv7_seq_residual_bytes(B, T, H);
+        }
+    }
+    if (dtype == B200WKV_F32 && !in_place && wkv7_fp32_takes(B, T, H) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H))
         return wkv7_fp32_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, ds_out, residual, dw, dr, dk, dv, da, db, ds0);
     return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
                         residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, nullptr);
