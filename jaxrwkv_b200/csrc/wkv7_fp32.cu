@@ -376,7 +376,7 @@ wkv7_fp32_prepare_kernel(const Operands op, const Tiles tiles, float* __restrict
 // ------------------------------------------------------------------ the chain --------
 // Rows of the state never meet, so a (sequence, head) is spread over CTAs of 2 R W rows: W computing warps of two groups of 16
 // lanes, each group R rows, four columns of each row in a lane, and a warp that fetches the chunks' tiles (of a chunk that is
-// walked: its raw rows) by bulk copies.  A step is latency: dot products, their sums over the lanes, the way of the sums back to all
+// walked: its raw rows) by bulk copies, five to eight chunks ahead.  A step is latency: dot products, their sums over the lanes, the way of the sums back to all
 // lanes, the update, 0.65 us for one row, 0.8 for two, 1.1 for four (dealing a step's products out to more threads, with the state
 // in shared memory and barriers in between, was no faster).
 //
@@ -388,13 +388,12 @@ wkv7_fp32_prepare_kernel(const Operands op, const Tiles tiles, float* __restrict
 template <int W, int R>
 struct ChainSmem {
     static constexpr int kRows = 2 * R * W, kWarps = W;              // rows, computing warps of a CTA
-    static constexpr int kStages = kRows <= 8 ? 8 : kRows <= 16 ? 6 : 5;
-    struct Stage {
-        float left[kC][kN], right[kC][kN], decay[kN], d[kRows][kN];
-    } st[kStages];
-    float raw[6][kC][kN];                            // decay, a, b, r, v, k of a chunk that is walked
+    static constexpr int kStages = kRows <= 8 ? 8 : kRows <= 16 ? 6 : 5;      // (five of 22 KB: two CTAs per SM)
+    struct Whole { float left[kC][kN], right[kC][kN], decay[kN], d[kRows][kN]; };
+    struct Walked { float decay[kC][kN], a[kC][kN], b[kC][kN], r[kC][kN], k[kC][kN], v[kC][kRows]; };      // raw rows of tokens
+    union Stage { Whole whole; Walked walked; } st[kStages];
     float s[kRows][kC];
-    uint64_t full[kStages], empty[kStages], raw_full, raw_empty;
+    uint64_t full[kStages], empty[kStages];
     int kind[kStages];
     uint32_t starts[kStages];
 
@@ -404,8 +403,6 @@ struct ChainSmem {
             tc::mbar_init(&full[i], 1);
             tc::mbar_init(&empty[i], kWarps);
         }
-        tc::mbar_init(&raw_full, 1);
-        tc::mbar_init(&raw_empty, kWarps);
         tc::mbar_init_fence();
     }
 };
@@ -430,10 +427,8 @@ template <bool kForward, class Smem>
 __device__ __forceinline__ bool fetch_chunks(Smem& sm, const Operands& op, const Tiles& tiles, const Place<kForward>& at, const float* slots) {
     const int lane = threadIdx.x & 31;
     const uint8_t* const ns = op.new_starts + (size_t)at.bi * op.T;
-    const float* const raw[5] = {op.a, op.b, op.r, op.v, op.k};
-    const int n_raw = kForward ? 6 : op.v != nullptr ? 5 : 4;
+    constexpr int kRaw = kForward ? 4 : 3;           // streams fetched whole: a, b, r, forward k
     uint32_t ahead = 0;                              // flags of 32 chunks, one per lane
-    int walked = 0;
     for (int it = 0; it < at.nC; ++it) {
         const int stage = it % Smem::kStages, t0 = at.chunk(it) * kC, n = min(kC, op.T - t0);
         if ((it & 31) == 0) {
@@ -447,27 +442,29 @@ __device__ __forceinline__ bool fetch_chunks(Smem& sm, const Operands& op, const
         const int kind = kind_of(starts, t0, op.T, at.L);
         if (it == 0) wait_for_grid_in_front();
         if (it >= Smem::kStages && !tc::mbar_wait(&sm.empty[stage], (it / Smem::kStages - 1) & 1)) return false;
-        if (kind == kWalked && walked > 0 && !tc::mbar_wait(&sm.raw_empty, (walked - 1) & 1)) return false;
-        typename Smem::Stage& s = sm.st[stage];
         uint64_t* const bar = &sm.full[stage];
         if (lane == 0) {
             sm.kind[stage] = kind;
             sm.starts[stage] = starts;
-            if (kind == kWalked) {
-                tc::mbar_arrive(bar);
-                tc::mbar_expect_tx(&sm.raw_full, (uint32_t)(n_raw * n * kN * 4));
-            } else {
-                tc::mbar_expect_tx(bar, (uint32_t)((2 * kTile + kN + Smem::kRows * kN) * 4));
-            }
+            tc::mbar_expect_tx(bar, (uint32_t)((kind == kWalked ? n * ((kRaw + 1) * kN + (op.v != nullptr ? Smem::kRows : 0))
+                                                                : 2 * kTile + kN + Smem::kRows * kN) * 4));
         }
         __syncwarp();
         const size_t tile = at.bh * tiles.head_stride + at.chunk(it) * tiles.chunk_stride;
-        if (kind == kWalked) {
-            ++walked;
-            if (lane == 0) tc::bulk_load(sm.raw[0], tiles.left + tile, (uint32_t)(n * kN * 4), &sm.raw_full);
-            for (int i = lane; i < (n_raw - 1) * n; i += 32)
-                tc::bulk_load(sm.raw[1 + i / n][i % n], raw[i / n] + at.seq + (size_t)(t0 + i % n) * at.tok, kN * 4, &sm.raw_full);
+        if (kind == kWalked) {                       // a lane one token of two of the streams
+            typename Smem::Walked& s = sm.st[stage].walked;
+            const int t = lane & 15;
+            const size_t row = at.seq + (size_t)(t0 + t) * at.tok;
+            if (lane == 0) tc::bulk_load(s.decay, tiles.left + tile, (uint32_t)(n * kN * 4), bar);
+            if (t < n) {
+                const bool even = lane < 16;
+                tc::bulk_load(even ? s.a[t] : s.b[t], (even ? op.a : op.b) + row, kN * 4, bar);
+                if (even) tc::bulk_load(s.r[t], op.r + row, kN * 4, bar);
+                else if (kForward) tc::bulk_load(s.k[t], op.k + row, kN * 4, bar);
+                if (!even && op.v != nullptr) tc::bulk_load(s.v[t], op.v + row + at.part * Smem::kRows, Smem::kRows * 4, bar);
+            }
         } else {
+            typename Smem::Whole& s = sm.st[stage].whole;
             if (lane == 0) tc::bulk_load(s.left, tiles.left + tile, kTile * 4, bar);
             else if (lane == 1) tc::bulk_load(s.right, tiles.right + tile, kTile * 4, bar);
             else if (lane == 2) tc::bulk_load(s.decay, tiles.decay + tile, kN * 4, bar);
@@ -503,10 +500,13 @@ struct Slice {
     }
 };
 
-// A chunk token by token.  What a token waits for is one sum over 16 lanes, 150 cycles, which all rows of a lane take together; the
-// operands of four tokens are in registers before the first of them, and the outputs' sums, which nothing waits for, are
-// taken for four tokens at once.  A flag in 300 tokens of 4 heads costs 4.4 us so, 12.1 where every lane takes its own decays and
-// the sums one after the other (T=2048 with a flag every 256 tokens 144 and 168 us, 64 heads, T=300, forward and backward 254 and 268).
+// A chunk token by token.  What a token waits for is one sum over 16 lanes, which all rows of a lane take together; the operands of four
+// tokens are in registers before the first of them, and the outputs' sums, which nothing waits for, are taken for four tokens at
+// once.  Its rows come through the stages that whole chunks' tiles come through, so that they are fetched as far ahead: with one
+// buffer for them apart, asked for when the walked chunk in front was done, a chunk was 5.4 us, and is 2.5 (4 heads; 81 copies to issue
+// for it take as long as its tokens; four rows per lane and two CTAs per SM: 3.3 a chunk and SM).  us of a forward, before / now: 4 heads,
+// T=2048, all chunks walked 701 / 332, a flag every 16 tokens 469 / 255 (the token-by-token kernel 235); 24 heads 890 / 413 and 631 / 345;
+// 128 heads, T=512 319 / 214 and 283 / 210.  Fetched by 16-byte asynchronous copies: 321, but 2 % more where no chunk is walked.
 template <int R>
 __device__ __forceinline__ void sum16(float* x) {
 #pragma unroll
@@ -514,72 +514,84 @@ __device__ __forceinline__ void sum16(float* x) {
 #pragma unroll
         for (int m = 0; m < R; ++m) x[m] += __shfl_xor_sync(0xffffffffu, x[m], bit);
 }
-template <bool kForward, int R, class Smem>
-__device__ __forceinline__ void walk(Slice<R>& x, const Smem& sm, const Operands& op, const Place<kForward>& at, int t0, uint32_t starts, int row, int col,
-                                     const float* x0, float* sums, float* y, float* out) {
+template <bool kForward, int R, class Walked>
+__device__ __forceinline__ void walk(Slice<R>& x, const Walked& s, const Operands& op, const Place<kForward>& at, int t0, uint32_t starts, int row, int own,
+                                     int col, const float* x0, float* sums, float* y, float* out) {
     constexpr int kStep = 4;
     const int n = min(kC, op.T - t0), l = col >> 2;
     const size_t state_at = ((size_t)at.bh * kN + row) * kN + col;
+    const int stop = kForward || x0 != nullptr ? at.L - 1 - t0 : -1;     // the token behind which the returned state lies
     auto axpy = [](Pair f, const Row4& a, const Row4& b) { return Row4{fma2(f, a.lo, b.lo), fma2(f, a.hi, b.hi)}; };
+    auto keep_if = [](bool c, const Row4& a, const Row4& b) { return Row4{Pair{c ? a.lo.u : b.lo.u}, Pair{c ? a.hi.u : b.hi.u}}; };
+    const Row4 none{Pair{0}, Pair{0}};
 #pragma unroll 1
     for (int i0 = 0; i0 < n; i0 += kStep) {
         Row4 w[kStep], a[kStep], b[kStep], r[kStep], k[kStep];
-        float v[kStep][R], o[R][kStep];
+        float v[kStep][R], o[R][kStep], sum[R][kStep];
 #pragma unroll
         for (int e = 0; e < kStep; ++e) {
             const int i = min(i0 + e, n - 1), t = kForward ? i : n - 1 - i;
-            w[e] = row4(&sm.raw[0][t][col]);
-            a[e] = row4(&sm.raw[1][t][col]);
-            b[e] = row4(&sm.raw[2][t][col]);
-            r[e] = row4(&sm.raw[3][t][col]);
-            if (kForward) k[e] = row4(&sm.raw[5][t][col]);
+            w[e] = row4(&s.decay[t][col]);
+            a[e] = row4(&s.a[t][col]);
+            b[e] = row4(&s.b[t][col]);
+            r[e] = row4(&s.r[t][col]);
+            if (kForward) k[e] = row4(&s.k[t][col]);
 #pragma unroll
-            for (int m = 0; m < R; ++m) {
-                v[e][m] = op.v != nullptr ? sm.raw[4][t][row + m] : 0.f;
-                o[m][e] = 0.f;
-            }
+            for (int m = 0; m < R; ++m) v[e][m] = op.v != nullptr ? s.v[t][own + m] : 0.f;
+        }
+        if (i0 + kStep > n) {                        // tokens behind the end change nothing
+#pragma unroll
+            for (int e = 1; e < kStep; ++e)
+                if (i0 + e >= n) {
+                    w[e].lo = w[e].hi = pair(1.f, 1.f);
+                    a[e] = b[e] = r[e] = none;
+                    if (kForward) k[e] = none;
+#pragma unroll
+                    for (int m = 0; m < R; ++m) v[e][m] = 0.f;
+                }
         }
 #pragma unroll
-        for (int e = 0; e < kStep; ++e) {
-            if (i0 + e >= n) break;
+        for (int e = 0; e < kStep; ++e) {            // (without branches: a token's worth of them takes as long as its sum)
             const int t = kForward ? i0 + e : n - 1 - i0 - e;
-            float sum[R];
+            const bool first = t >= 0 && ((starts >> t) & 1u);
+            float f[R];
             if (kForward) {
-                if ((starts >> t) & 1u) x.clear();
 #pragma unroll
-                for (int m = 0; m < R; ++m) sum[m] = dot(x.x[m], a[e]);
-                sum16<R>(sum);
+                for (int m = 0; m < R; ++m) {
+                    x.x[m] = keep_if(first, none, x.x[m]);
+                    f[m] = dot(x.x[m], a[e]);
+                }
+                sum16<R>(f);
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
                     const Pair V = pair(v[e][m], v[e][m]);
                     const Row4 kept{fma2(x.x[m].lo, w[e].lo, mul2(V, k[e].lo)), fma2(x.x[m].hi, w[e].hi, mul2(V, k[e].hi))};
-                    x.x[m] = axpy(pair(sum[m], sum[m]), b[e], kept);
+                    x.x[m] = axpy(pair(f[m], f[m]), b[e], kept);
                     o[m][e] = dot(x.x[m], r[e]);
                 }
-                if (t0 + t == at.L - 1) x.store(out + state_at);
+                if (t == stop) x.store(out + state_at);
             } else {
-                if (t0 + t == at.L - 1 && x0 != nullptr) x.add(x0 + state_at);
+                if (t == stop && t >= 0) x.add(x0 + state_at);
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
                     x.x[m] = axpy(pair(v[e][m], v[e][m]), r[e], x.x[m]);
-                    sum[m] = dot(x.x[m], b[e]);
+                    f[m] = dot(x.x[m], b[e]);
                 }
-                sum16<R>(sum);
+                sum16<R>(f);
 #pragma unroll
                 for (int m = 0; m < R; ++m) {
-                    const Pair S = pair(sum[m], sum[m]);
-                    x.x[m] = Row4{fma2(x.x[m].lo, w[e].lo, mul2(S, a[e].lo)), fma2(x.x[m].hi, w[e].hi, mul2(S, a[e].hi))};
+                    const Pair S = pair(f[m], f[m]);
+                    x.x[m] = keep_if(first, none, Row4{fma2(x.x[m].lo, w[e].lo, mul2(S, a[e].lo)), fma2(x.x[m].hi, w[e].hi, mul2(S, a[e].hi))});
                 }
-                if ((starts >> t) & 1u) x.clear();
             }
-            if (sums != nullptr && col == 0) {
-                float* const to = sums + at.sum(op, t0 + t) + row;
 #pragma unroll
-                for (int m = 0; m < R; ++m) to[m] = sum[m];
-            }
+            for (int m = 0; m < R; ++m) sum[m][e] = f[m];
         }
+        auto pick = [l](const float* f) { return l & 2 ? (l & 1 ? f[3] : f[2]) : (l & 1 ? f[1] : f[0]); };
+        const bool mine = l < kStep && i0 + l < n;   // lane l: token l of the four
+        const int t = t0 + (kForward ? i0 + l : n - 1 - i0 - l);
+        float q[R];
         if (kForward) {                              // lane l ends with the outputs of token l % 4
-            float q[R];
 #pragma unroll
             for (int m = 0; m < R; ++m) {
                 const bool odd = l & 1;
@@ -591,16 +603,19 @@ __device__ __forceinline__ void walk(Slice<R>& x, const Smem& sm, const Operands
             for (int bit = 4; bit < 16; bit <<= 1)
 #pragma unroll
                 for (int m = 0; m < R; ++m) q[m] += __shfl_xor_sync(0xffffffffu, q[m], bit);
-            if (l < kStep && i0 + l < n) {
+        }
+        if (mine) {
 #pragma unroll
-                for (int m = 0; m < R; ++m) y[at.seq + (size_t)(t0 + i0 + l) * at.tok + row + m] = q[m];
+            for (int m = 0; m < R; ++m) {
+                if (kForward) y[at.seq + (size_t)t * at.tok + row + m] = q[m];
+                if (sums != nullptr) sums[at.sum(op, t) + row + m] = pick(sum[m]);
             }
         }
     }
 }
 
 template <bool kForward, int W, int R>
-__global__ void __launch_bounds__(32 * (W + 1))
+__global__ void __launch_bounds__(32 * (W + 1), R == 4 ? 2 : 1)
 wkv7_fp32_chain_kernel(const Operands op, const Tiles tiles, const float* __restrict__ x0, float* slots, float* sums, float* __restrict__ y,
                        float* __restrict__ out, int* __restrict__ status) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -620,18 +635,13 @@ wkv7_fp32_chain_kernel(const Operands op, const Tiles tiles, const float* __rest
     if (kForward) x.load(x0 + state_at); else x.clear();
     wait_for_grid_in_front();
     if (kForward && at.L == 0) x.store(out + state_at);
-    int walked = 0;
     bool landed = true;
     for (int it = 0; it < at.nC; ++it) {
         const int stage = it % Smem::kStages, t0 = at.chunk(it) * kC;
-        landed = tc::mbar_wait(&sm.full[stage], (it / Smem::kStages) & 1);
+        landed = __all_sync(0xffffffffu, tc::mbar_wait(&sm.full[stage], (it / Smem::kStages) & 1));
+        if (!landed) break;
         const int kind = sm.kind[stage];
-        if (kind == kWalked && landed) landed = tc::mbar_wait(&sm.raw_full, walked++ & 1);
-        if (!__all_sync(0xffffffffu, landed)) {
-            landed = false;
-            break;
-        }
-        const typename Smem::Stage& s = sm.st[stage];
+        const typename Smem::Whole& s = sm.st[stage].whole;
         if (kForward && kind == kFresh) x.clear();
         x.store(slots + at.slot(it) + in_state);
         // (the stage of the chunk before: what was read of it went into the state that has just been stored)
@@ -689,9 +699,7 @@ wkv7_fp32_chain_kernel(const Operands op, const Tiles tiles, const float* __rest
             if (kForward && at.L == t0 + kC) x.store(out + state_at);
             if (!kForward && kind == kFresh) x.clear();
         } else {
-            walk<kForward>(x, sm, op, at, t0, sm.starts[stage], row, 4 * l, x0, sums, y, out);
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&sm.raw_empty);
+            walk<kForward>(x, sm.st[stage].walked, op, at, t0, sm.starts[stage], row, own, 4 * l, x0, sums, y, out);
         }
     }
     if (!kForward) {

@@ -53,6 +53,13 @@ def test_flags_and_lengths_at_chunk_edges(B, H):
     check(wkv7_case(B, T, H, seed=H, s0_scale=0.3, starts=starts, lengths=lengths), H)
 
 
+# each split: chunks walked token by token many times around the stages, among whole ones, and in a row
+@pytest.mark.parametrize("B,H", [(1, 4), (3, 5), (4, 8), (4, 10)])
+@pytest.mark.parametrize("p_start", [0.03, 0.3])
+def test_flags_in_many_chunks(B, H, p_start):
+    check(wkv7_case(B, 16 * 24 + 5, H, seed=B + H, s0_scale=0.3, p_start=p_start, random_length=True), H)
+
+
 @pytest.mark.parametrize("gy,gs", [(True, False), (False, True)])
 def test_one_cotangent(gy, gs):
     check(wkv7_case(2, 340, 2, seed=4, p_start=0.02, random_length=True, s0_scale=0.3), 2, gy, gs)
