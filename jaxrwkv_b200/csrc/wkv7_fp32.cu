@@ -1062,21 +1062,29 @@ int launch_chain(cudaStream_t st, int heads, A... args) {
 }  // namespace
 
 // Whether calls with gradients take these kernels (the rest of wkv7_chain.cu and wkv7_seq.cu: fewer tokens, and residuals without
-// their room).  Where the host's launches take longer than the device (some 100 us for a forward and backward), the four
-// kernels more are 6 us lost; the line is where the token-by-token kernels are at 105-110 us.  Those / here, us: 8 heads 99 / 106
-// at T=256, 125 / 107 at 320; 24 heads 102 / 107 at 160, 134 / 107 at 208; 40 heads 101 / 107 at 104, 129 / 104 at 160; 64 heads 100 / 104
-// at 64, 115 / 105 at 104; 160 heads 177 / 122 at 64, 774 / 480 at 320; 640 heads 534 / 395 at 64.
+// their room).  The device is faster here at every size measured; the line is a host's.  An eager forward and backward takes the host of
+// a B200 some 105 us with the kernels there and 112 with the four more here, so that below the line, where those kernels are done
+// by then, these cost 6 us.  Calls from a captured graph, which have no such floor, would gain from fewer tokens on.  us, there / here, eager (graph):
+// 8 heads, T=192 105 / 112 (70 / 49), 256 106 / 113 (84 / 54), 320 127 / 112 (119 / 67); 24 heads, 96 106 / 113 (57 / 46), 160 108 / 113
+// (94 / 59), 208 135 / 114 (127 / 80); 40 heads, 104 107 / 113 (86 / 62), 160 130 / 113 (123 / 82); 64 heads, 64 106 / 112 (72 / 54), 104 116 / 111
+// (107 / 85); 160 heads, 64 178 / 122; 640 heads, 64 534 / 395.  With a flag every 16 tokens, eager: 8 heads, T=1024 330 / 303; 24 heads, 208
+// 142 / 125, 2048 1104 / 861; 160 heads, 64 179 / 144.
 bool wkv7_fp32_takes(int B, int T, int H) { return chunks_of(T) >= 4 && chunks_of(T) * ((long long)B * H + 16) >= 440; }
 
-// What a forward call without a residual wants as a workspace (0: it takes the token-by-token chain).  Measured, us, that chain /
-// here, and with a flag every 256 tokens and lengths of T / 2 to T: 4 heads 27 / 23 and 27 / 29 at T=200, 37 / 29 and 37 / 33 at
-// 300, 115 / 60 and 115 / 80 at 1000; 32 heads 41 / 37 and 42 / 44 at 256, 76 / 61 and 78 / 82 at 512, 283 / 217 and 289 / 246 at 2000;
-// 48 heads 107 / 95 and 109 / 114 at 600; 64 heads 58 / 60 and 59 / 84 at 300, 176 / 179 and 179 / 216 at 1000.  That chain takes the same
-// time up to a head per SM and doesn't mind flags, this one shares the device with what is done beside it: up to a quarter of a
-// head per SM, from 16 chunks on, and as many as heads.  The last limit bounds the workspace, 2 GiB.
+// What a forward call without a residual wants as a workspace (0: it takes the token-by-token chain).  That chain takes the same
+// time up to a head per SM and doesn't mind flags, this one shares the device with what is done beside it, and a flagged or cut chunk
+// is walked: up to a quarter of a head per SM, and from 13 chunks on, where no count of heads loses at a flag every 256 tokens and
+// lengths of T / 2 to T.  us, that chain / here, without flags, and with those flags and lengths:
+//     4 heads:   T=144 21 / 17, 21 / 21    208 27 / 20, 27 / 23    512 60 / 31, 60 / 37    2000 223 / 97, 224 / 109
+//     16 heads:  T=160 23 / 21, 23 / 27    208 27 / 24, 27 / 27    512 60 / 45, 61 / 52    2000 224 / 146, 224 / 166
+//     24 heads:  T=160 27 / 23, 27 / 27    208 34 / 27, 35 / 31    512 76 / 52, 77 / 56    2000 282 / 179, 288 / 199
+//     36 heads:  T=176 29 / 27, 31 / 33    208 35 / 33, 35 / 33    512 76 / 60, 77 / 67    2000 282 / 220, 287 / 242
+//     48 heads:  T=208 41 / 37, 41 / 42    512 92 / 78, 93 / 99    64 heads:  T=512 92 / 92, 93 / 111
+// With a flag every 64 tokens they are equal at T=256 to 512 (4 heads 33 / 33, 36 heads 82 / 82) and these faster behind that (4 heads, T=2000
+// 225 / 138).  Every 16 tokens 4 heads take 33 / 49 at T=256 and 230 / 230 at 2000, 24 heads 48 / 60 and 330 / 325: the host doesn't know
+// the flags.  The last limit bounds the workspace, 2 GiB.
 size_t wkv7_fp32_workspace_bytes(int B, int T, int H) {
-    const long long heads = (long long)B * H;
-    if (chunks_of(T) < 16 || chunks_of(T) < heads || 4 * heads > sm_count_of_current_device()) return 0;
+    if (chunks_of(T) < 13 || 4 * (long long)B * H > sm_count_of_current_device()) return 0;
     const size_t bytes = (size_t)B * H * chunks_of(T) * (kN * kN + kTileFloats) * sizeof(float);
     return bytes <= ((size_t)2 << 30) ? bytes : 0;
 }
