@@ -71,12 +71,15 @@ int b200wkv_device_status(void);
  * `residual` is an opaque device buffer the forward fills for the backward
  * (the counterpart of the reference's s_restore/sa_restore results,
  * rwkv7.py:363-364).  Pass NULL/0 for inference: nothing is saved then.  The
- * backward must be called with the same dtype and flags as the forward that
- * filled the buffer, and it uses the tail of the buffer as scratch (carries
+ * backward must be called with the same dtype, flags and residual_bytes as the
+ * forward that filled the buffer, and it uses the tail of the buffer as scratch (carries
  * passed between thread blocks), so the buffer must be writable and one
  * buffer must not serve two backward calls that overlap on the GPU.
  */
 size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N);
+/* The least residual that the two calls take (given the same size): in fp32, where memory is short, they
+ * do with the checkpoints alone and are slower; otherwise it is the size above. */
+size_t b200wkv7_residual_min_bytes(int dtype, int B, int T, int H, int N);
 
 int b200wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N,
                  const void* w, const void* r, const void* k, const void* v,

@@ -21,13 +21,14 @@ int wkv7_seq_bwd(cudaStream_t st, int dtype, int B, int T, int H, const void* w,
 // fp32 where wkv7_fp32_takes() says so: 16 tokens at a time (wkv7_fp32.cu)
 bool wkv7_fp32_takes(int B, int T, int H);
 size_t wkv7_fp32_workspace_bytes(int B, int T, int H);
-size_t wkv7_fp32_residual_bytes(int B, int T, int H);
+size_t wkv7_fp32_kept_bytes(int B, int T, int H);
+size_t wkv7_fp32_state_bytes(int B, int T, int H);
 int wkv7_fp32_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
                   const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual,
-                  void* workspace);
+                  size_t residual_bytes, void* workspace);
 int wkv7_fp32_bwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
-                  const void* b, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual, void* dw,
-                  void* dr, void* dk, void* dv, void* da, void* db, void* ds0);
+                  const void* b, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual,
+                  size_t residual_bytes, void* workspace, void* dw, void* dr, void* dk, void* dv, void* da, void* db, void* ds0);
 
 int wkv7_step(cudaStream_t st, int dtype, int B, int H, const void* w, const void* r, const void* k, const void* v,
               const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
@@ -92,9 +93,6 @@ static int* residual_mark_of(void* residual, size_t bytes) {
     return residual ? reinterpret_cast<int*>(static_cast<char*>(residual) + bytes - kResidualMarkBytes) : nullptr;
 }
 
-size_t wkv7_residual_min_bytes(int dtype, int B, int T, int H) {
-    return dtype == B200WKV_F32 ? wkv7_seq_residual_bytes(B, T, H) : b200wkv7_residual_bytes(dtype, B, T, H, kN);
-}
 
 // Whether all of these lie on boundaries of `bytes` (NULL does).  The kernels read and write vectors; an address that does not
 // suit them is refused here, since a misaligned access ends the process's work on the device.
@@ -119,13 +117,20 @@ static int check_dims(int dtype, int B, int T, int H, int N) {
     return B200WKV_OK;
 }
 
+// Whether a call with a residual takes 16 tokens at a time: where the residual has all the room, or keeps what it has to beside a
+// workspace.  The forward and the backward of a residual have to agree on it (the host path sees to that: wkv7_kept_bytes).
+static size_t fp32_full_bytes(int B, int T, int H) { return wkv7_fp32_kept_bytes(B, T, H) + wkv7_fp32_state_bytes(B, T, H); }
+static bool wkv7_fp32_in_chunks(int B, int T, int H, size_t residual_bytes, const void* workspace) {
+    return wkv7_fp32_takes(B, T, H) && residual_bytes >= (workspace != nullptr ? wkv7_fp32_kept_bytes(B, T, H) : fp32_full_bytes(B, T, H));
+}
+
 int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k, const void* v,
              const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
              void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace) {
     int st = check_dims(dtype, B, T, H, N);
     if (st != B200WKV_OK) return st;
     if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !y || !s_out) return B200WKV_ENULL;
-    if (residual != nullptr && residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
+    if (residual != nullptr && residual_bytes < b200wkv7_residual_min_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
     // one token and no residual wanted (recurrent decoding): a single pass over the state
     if (T == 1 && residual == nullptr) {
         if (!aligned(vec4_bytes(dtype), {w, r, k, v, a, b}) || !aligned(16, {s0, s_out})) return B200WKV_EUNSUPPORTED;
@@ -144,17 +149,70 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
         return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual,
                             range_flag, ticket, mark);
     }
-    // 16 tokens at a time where the residual has all its room, or a workspace was brought
     if (dtype == B200WKV_F32 &&
-        (residual != nullptr ? wkv7_fp32_takes(B, T, H) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H) : workspace != nullptr))
-        return wkv7_fp32_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, workspace);
+        (residual != nullptr ? wkv7_fp32_in_chunks(B, T, H, residual_bytes, workspace) : workspace != nullptr))
+        return wkv7_fp32_fwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out, residual, residual_bytes, workspace);
     return wkv7_seq_fwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, y, s_out,
                         residual, nullptr, 0, nullptr);
 }
 
+int wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k, const void* v,
+             const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, const void* dy,
+             const void* ds_out, void* residual, size_t residual_bytes, void* dw, void* dr, void* dk, void* dv, void* da, void* db,
+             void* ds0, unsigned flags, void* workspace) {
+    int st = check_dims(dtype, B, T, H, N);
+    if (st != B200WKV_OK) return st;
+    if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !residual || !dw || !dr || !dk || !dv ||
+        !da || !db || !ds0)
+        return B200WKV_ENULL;
+    if (residual_bytes < b200wkv7_residual_min_bytes(dtype, B, T, H, N)) return B200WKV_ERESIDUAL;
+    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
+    if (!aligned(sequential ? vec4_bytes(dtype) : 16, {w, r, k, v, a, b, dy, dw, dr, dk, dv, da, db}) ||
+        !aligned(vec4_bytes(dtype), {s0, ds_out, ds0}) || !aligned(16, {residual, workspace}))
+        return B200WKV_EUNSUPPORTED;
+    // must match the kernel family that filled the residual in b200wkv7_fwd (same dtype and flags)
+    if (!sequential) {
+        const int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
+        // the sequential state-gradient carry, then the gradients of all blocks in parallel; the sequential kernels behind
+        // them return at once unless the forward fell back to them
+        st = wkv7_carry_bwd((cudaStream_t)stream, B, T, H, length, dy, ds_out, residual, mark, ds0);
+        if (st != B200WKV_OK) return st;
+        st = wkv7_grad_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, residual, mark, dw, dr, dk, dv, da, db);
+        if (st != B200WKV_OK) return st;
+        return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
+                            residual, b200wkv7_residual_bytes(dtype, B, T, H, N) - kResidualMarkBytes, dw, dr, dk, dv, da, db, ds0, mark);
+    }
+    // Gradients written over operands: the token-by-token kernels read a chunk's rows before they write them, where those for 16 tokens
+    // at a time keep tiles in the gradients' buffers first.  ds0 over ds_out: without a carry between runs, which would be written
+    // before the last read.  (The forward's checkpoints are the same for both.)
+    bool in_place = false;
+    const size_t stream_bytes = (size_t)B * T * H * kN * sizeof(float), state_bytes = (size_t)B * H * kN * kN * sizeof(float);
+    if (dtype == B200WKV_F32) {
+        for (const void* g : {dw, dr, dk, dv, da, db})
+            for (const void* x : {w, r, k, v, a, b, dy}) in_place |= meet(g, stream_bytes, x, stream_bytes);
+        if (meet(ds0, state_bytes, ds_out, state_bytes)) {
+            in_place = true;
+            residual_bytes = wkv7_seq_residual_bytes(B, T, H);
+        }
+    }
+    if (dtype == B200WKV_F32 && !in_place && wkv7_fp32_in_chunks(B, T, H, residual_bytes, workspace))
+        return wkv7_fp32_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, ds_out, residual, residual_bytes, workspace, dw, dr,
+                             dk, dv, da, db, ds0);
+    return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
+                        residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, nullptr);
+}
+
 size_t wkv7_workspace_bytes(int dtype, int B, int T, int H, bool residual) {
-    if (dtype == B200WKV_F32) return residual ? 0 : wkv7_fp32_workspace_bytes(B, T, H);
+    if (dtype == B200WKV_F32) return !residual ? wkv7_fp32_workspace_bytes(B, T, H) : wkv7_fp32_takes(B, T, H) ? wkv7_fp32_state_bytes(B, T, H) : 0;
     return wkv7_blocks_bytes(B, T, H, residual);
+}
+size_t wkv7_kept_bytes(int dtype, int B, int T, int H, bool workspace) {
+    if (dtype != B200WKV_F32 || !wkv7_fp32_takes(B, T, H)) return b200wkv7_residual_bytes(dtype, B, T, H, kN);
+    return workspace ? wkv7_fp32_kept_bytes(B, T, H) : b200wkv7_residual_min_bytes(dtype, B, T, H, kN);
+}
+size_t wkv7_bwd_workspace_bytes(int dtype, int B, int T, int H, size_t residual_bytes) {
+    if (dtype != B200WKV_F32 || !wkv7_fp32_takes(B, T, H) || residual_bytes < wkv7_fp32_kept_bytes(B, T, H)) return 0;
+    return residual_bytes < fp32_full_bytes(B, T, H) ? wkv7_fp32_state_bytes(B, T, H) : 0;
 }
 
 size_t wkv6_workspace_bytes(int dtype, bool per_token, int B, int T, int H) {
@@ -235,14 +293,22 @@ int b200wkv_abi_version(void) { return 2; }
 
 int b200wkv_device_status(void) { return wkv7_chunk_status(); }
 
+size_t b200wkv7_residual_min_bytes(int dtype, int B, int T, int H, int N) {
+    if (check_dims(dtype, B, T, H, N) != B200WKV_OK) return 0;
+    return dtype == B200WKV_F32 ? wkv7_seq_residual_bytes(B, T, H) : b200wkv7_residual_bytes(dtype, B, T, H, N);
+}
+
 size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N) {
     if (check_dims(dtype, B, T, H, N) != B200WKV_OK) return 0;
     // fp32 keeps a state every 16 tokens; bf16 uses the chunked tensor-core
     // kernels (a state every 64 tokens) unless B200WKV_FLAG_SEQUENTIAL asks otherwise, so size for both
-    // (fp32: and for what the backward that works on all chunks side by side wants besides, where it does)
-    if (dtype == B200WKV_F32 && wkv7_fp32_takes(B, T, H)) return wkv7_fp32_residual_bytes(B, T, H);
+    // (fp32: and for what the backward that works on all chunks side by side wants besides, where it does.  Where the sequences fill
+    // their waves of CTAs it doesn't without a workspace: 36 KB per 16 tokens and head for 16 is more memory than the time is worth.)
     const size_t seq = wkv7_seq_residual_bytes(B, T, H);
-    if (dtype == B200WKV_F32) return seq + wkv7_seq_carry_bytes(B, T, H);
+    if (dtype == B200WKV_F32) {
+        const size_t carry = wkv7_seq_carry_bytes(B, T, H);
+        return carry != 0 && wkv7_fp32_takes(B, T, H) ? fp32_full_bytes(B, T, H) : seq + carry;
+    }
     const size_t chk = wkv7_chunk_residual_bytes(B, T, H);
     // + one word at the end that says which of the two formats the forward left (see residual_mark_of)
     return (seq > chk ? seq : chk) + kResidualMarkBytes;
@@ -260,45 +326,8 @@ int b200wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void
                  const uint8_t* new_starts, const void* dy, const void* ds_out, void* residual,
                  size_t residual_bytes, void* dw, void* dr, void* dk, void* dv, void* da, void* db, void* ds0,
                  unsigned flags) {
-    int st = check_dims(dtype, B, T, H, N);
-    if (st != B200WKV_OK) return st;
-    if (!w || !r || !k || !v || !a || !b || !s0 || !length || !new_starts || !residual || !dw || !dr || !dk || !dv ||
-        !da || !db || !ds0)
-        return B200WKV_ENULL;
-    if (residual_bytes < wkv7_residual_min_bytes(dtype, B, T, H)) return B200WKV_ERESIDUAL;
-    const bool sequential = dtype == B200WKV_F32 || (flags & B200WKV_FLAG_SEQUENTIAL);
-    if (!aligned(sequential ? vec4_bytes(dtype) : 16, {w, r, k, v, a, b, dy, dw, dr, dk, dv, da, db}) ||
-        !aligned(vec4_bytes(dtype), {s0, ds_out, ds0}) || !aligned(16, {residual}))
-        return B200WKV_EUNSUPPORTED;
-    // must match the kernel family that filled the residual in b200wkv7_fwd (same dtype and flags)
-    if (!sequential) {
-        const int* mark = residual_mark_of(residual, b200wkv7_residual_bytes(dtype, B, T, H, N));
-        // the sequential state-gradient carry, then the gradients of all blocks in parallel; the sequential kernels behind
-        // them return at once unless the forward fell back to them
-        st = wkv7_carry_bwd((cudaStream_t)stream, B, T, H, length, dy, ds_out, residual, mark, ds0);
-        if (st != B200WKV_OK) return st;
-        st = wkv7_grad_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, residual, mark, dw, dr, dk, dv, da, db);
-        if (st != B200WKV_OK) return st;
-        return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
-                            residual, b200wkv7_residual_bytes(dtype, B, T, H, N) - kResidualMarkBytes, dw, dr, dk, dv, da, db, ds0, mark);
-    }
-    // Gradients written over operands: the token-by-token kernels read a chunk's rows before they write them, where those for 16 tokens
-    // at a time keep tiles in the gradients' buffers first.  ds0 over ds_out: without a carry between runs, which would be written
-    // before the last read.  (The forward's checkpoints are the same for both.)
-    bool in_place = false;
-    const size_t stream_bytes = (size_t)B * T * H * kN * sizeof(float), state_bytes = (size_t)B * H * kN * kN * sizeof(float);
-    if (dtype == B200WKV_F32) {
-        for (const void* g : {dw, dr, dk, dv, da, db})
-            for (const void* x : {w, r, k, v, a, b, dy}) in_place |= meet(g, stream_bytes, x, stream_bytes);
-        if (meet(ds0, state_bytes, ds_out, state_bytes)) {
-            in_place = true;
-            residual_bytes = wkv7_seq_residual_bytes(B, T, H);
-        }
-    }
-    if (dtype == B200WKV_F32 && !in_place && wkv7_fp32_takes(B, T, H) && residual_bytes >= wkv7_fp32_residual_bytes(B, T, H))
-        return wkv7_fp32_bwd((cudaStream_t)stream, B, T, H, w, r, k, v, a, b, length, new_starts, dy, ds_out, residual, dw, dr, dk, dv, da, db, ds0);
-    return wkv7_seq_bwd((cudaStream_t)stream, dtype, B, T, H, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out,
-                        residual, residual_bytes, dw, dr, dk, dv, da, db, ds0, nullptr);
+    return b200wkv::wkv7_bwd(stream, dtype, B, T, H, N, w, r, k, v, a, b, s0, length, new_starts, dy, ds_out, residual, residual_bytes, dw, dr, dk, dv, da,
+                             db, ds0, flags, nullptr);
 }
 
 size_t b200wkv6_residual_bytes(int dtype, int B, int T, int H, int N) {

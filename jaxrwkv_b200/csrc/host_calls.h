@@ -12,6 +12,16 @@ int wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w,
              const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, void* y,
              void* s_out, void* residual, size_t residual_bytes, unsigned flags, void* workspace);
 
+// b200wkv7_bwd with a workspace of wkv7_bwd_workspace_bytes() (0: it wants none, NULL).
+size_t wkv7_bwd_workspace_bytes(int dtype, int B, int T, int H, size_t residual_bytes);
+int wkv7_bwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k, const void* v,
+             const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* new_starts, const void* dy,
+             const void* ds_out, void* residual, size_t residual_bytes, void* dw, void* dr, void* dk, void* dv, void* da, void* db,
+             void* ds0, unsigned flags, void* workspace);
+// What is to be kept for the backward (N = 64) where the forward has its workspace or, where it wants one, doesn't.  The size tells the
+// backward which kernels filled it.
+size_t wkv7_kept_bytes(int dtype, int B, int T, int H, bool workspace);
+
 // b200wkv6_fwd; a call without a residual may bring a workspace of wkv6_workspace_bytes() (0: it wants none, NULL) and then has
 // the arithmetic of a call with one.
 size_t wkv6_workspace_bytes(int dtype, bool per_token, int B, int T, int H);

@@ -169,17 +169,41 @@ variable_list gradients_of(AutogradContext* ctx, const variable_list& grads) {
 
 // ------------------------------------------------------------------------------------------------- RWKV-7
 // Streams (lead, T, H, N), state (lead, H, N, N), any number of leading batch axes.
-// the workspace of a forward call (NULL: it wants none); `scratch` keeps it until the call is enqueued
-static void* wkv7_workspace(Tensor& scratch, const Tensor& like, int B, int T, int H, int N, bool residual) {
-    if (N != 64 || B < 1 || T < 2 || H < 1) return nullptr;
-    const size_t n = b200wkv::wkv7_workspace_bytes(dtype_code(like), B, T, H, residual);
-    if (n == 0) return nullptr;
+// `n` bytes, or an undefined tensor where the device has no room for them
+static Tensor bytes_if_room(size_t n, const Tensor& like) {
     try {
-        scratch = bytes(n, like);
+        return bytes(n, like);
     } catch (const c10::OutOfMemoryError&) {
-        return nullptr;                           // no room for it (up to 2 GiB): the walk needs none
+        return Tensor();
     }
-    return out(scratch);
+}
+// What a forward call wants beside its results: a workspace until it is enqueued, and, where asked for, what its backward reads.  Without
+// room for the one or the other (up to 2 GiB; 16 and 20 KB per 16 tokens and head in fp32) there are kernels that need less.
+struct Wkv7Room {
+    Tensor workspace, residual;
+    size_t residual_bytes = 0;
+    Wkv7Room(const Tensor& like, int B, int T, int H, int N, bool keep) {
+        const int code = dtype_code(like);
+        const bool known = N == 64 && B > 0 && T > 0 && H > 0;       // (the call says what is wrong with others)
+        const size_t n = known && T > 1 ? b200wkv::wkv7_workspace_bytes(code, B, T, H, keep) : 0;
+        if (n != 0) workspace = bytes_if_room(n, like);
+        if (!keep) return;
+        const auto fits = [&](size_t size) {
+            residual_bytes = size;
+            return (residual = bytes_if_room(size, like)).defined();
+        };
+        const size_t least = b200wkv7_residual_min_bytes(code, B, T, H, N);
+        if (known && fits(b200wkv::wkv7_kept_bytes(code, B, T, H, workspace.defined()))) return;
+        workspace.reset();
+        if (known && fits(b200wkv::wkv7_kept_bytes(code, B, T, H, false))) return;
+        residual_bytes = least;
+        residual = bytes(least, like);
+    }
+    void* ws() const { return workspace.defined() ? workspace.mutable_data_ptr() : nullptr; }
+};
+static Tensor wkv7_bwd_workspace(const Tensor& like, int B, int T, int H, const Tensor& residual) {
+    const size_t n = b200wkv::wkv7_bwd_workspace_bytes(dtype_code(like), B, T, H, (size_t)residual.numel());
+    return n != 0 ? bytes_if_room(n, like) : Tensor();               // (without it a sequence is walked in longer runs)
 }
 
 struct Wkv7 {
@@ -202,13 +226,11 @@ struct Wkv7 {
         Tensor c[kIn];
         for (int i = 0; i < kIn; ++i) c[i] = t[i].contiguous();
         Tensor y = fresh_like(k), s_out = fresh_like(t[6]);
-        const size_t rbytes = residual ? b200wkv7_residual_bytes(dtype_code(k), B, T, H, N) : 0;
-        if (residual) *residual = bytes(rbytes, k);
-        Tensor scratch;
-        void* const ws = wkv7_workspace(scratch, k, B, T, H, N, residual != nullptr);
+        const Wkv7Room room(k, B, T, H, N, residual != nullptr);
+        if (residual) *residual = room.residual;
         check(b200wkv::wkv7_fwd(stream_of(k), dtype_code(k), B, T, H, N, in(c[1]), in(c[0]), in(c[2]), in(c[3]), in(c[4]), in(c[5]),
                            in(c[6]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), out(y), out(s_out),
-                           residual ? out(*residual) : nullptr, rbytes, 0, ws));
+                           out(room.residual), room.residual_bytes, 0, room.ws()));
         return {s_out, y};
     }
     // saved: the seven operands, length, new_starts, residual; grads: of the returned state and of the output
@@ -224,9 +246,10 @@ struct Wkv7 {
             c[i] = saved[i].contiguous();
             g[i] = fresh_like(saved[i]);
         }
-        check(b200wkv7_bwd(stream_of(k), dtype_code(k), B, T, H, N, in(c[1]), in(c[0]), in(c[2]), in(c[3]), in(c[4]), in(c[5]),
-                           in(c[6]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), in(gy), in(gs), out(res),
-                           (size_t)res.numel(), out(g[1]), out(g[0]), out(g[2]), out(g[3]), out(g[4]), out(g[5]), out(g[6]), 0));
+        const Tensor ws = wkv7_bwd_workspace(k, B, T, H, res);
+        check(b200wkv::wkv7_bwd(stream_of(k), dtype_code(k), B, T, H, N, in(c[1]), in(c[0]), in(c[2]), in(c[3]), in(c[4]), in(c[5]),
+                                in(c[6]), (const uint32_t*)in(f.length), (const uint8_t*)in(f.starts), in(gy), in(gs), out(res),
+                                (size_t)res.numel(), out(g[1]), out(g[0]), out(g[2]), out(g[3]), out(g[4]), out(g[5]), out(g[6]), 0, out(ws)));
         return {g[0], g[1], g[2], g[3], g[4], g[5], g[6]};
     }
 };
@@ -692,12 +715,10 @@ struct Layer {
         lora(3, kG1, m[5], b200wkv::kSigmoid, q.g);
         check(b200wkv7_mix_pre_fwd(st, code, d.rows, H, (int)kN, !d.first, q.k, q.wl, q.al, v, in(kept.v_first), d.first ? nullptr : q.vl, in(p[kW0]),
                                    in(p[kA0]), in(p[kV0]), in(p[kKk]), in(p[kKa]), q.w, q.kp, q.vp, q.ai, q.bi));
-        const size_t rbytes = residual ? b200wkv7_residual_bytes(code, B, T, H, (int)kN) : 0;
-        if (residual) kept.residual = bytes(rbytes, x);
-        Tensor scratch;
-        void* const ws = wkv7_workspace(scratch, x, B, T, H, (int)kN, residual);
+        const Wkv7Room room(x, B, T, H, (int)kN, residual);
+        kept.residual = room.residual;
         check(b200wkv::wkv7_fwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(f.length),
-                           (const uint8_t*)in(f.starts), q.y, s_out.p, out(kept.residual), rbytes, 0, ws));
+                           (const uint8_t*)in(f.starts), q.y, s_out.p, out(kept.residual), room.residual_bytes, 0, room.ws()));
         s_out.finish(st);
         check(b200wkv7_mix_post_fwd(st, code, d.rows, H, (int)kN, kEps, q.y, q.r, q.kp, q.vp, q.g, in(p[kLnW]), in(p[kLnB]), in(p[kRk]), q.xo));
         gemm.nt(d.rows, d.C, d.C, q.xo, in(p[kWo]), out(o));
@@ -752,8 +773,10 @@ struct Layer {
         if (wanted[1]) g[1] = fresh_like(kept.state);
         const Tensor state_room = wanted[1] ? g[1] : fresh_like(kept.state);
         const Landing gprev(state_room, 0, 1), gs0(state_room, 1, kN);
-        check(b200wkv7_bwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(kept.length),
-                           (const uint8_t*)in(kept.starts), dy, gs, out(kept.residual), (size_t)kept.residual.numel(), gw, gr, gk, gv, ga, gb, gs0.p, 0));
+        const Tensor ws = wkv7_bwd_workspace(x, B, T, H, kept.residual);
+        check(b200wkv::wkv7_bwd(st, code, B, T, H, (int)kN, q.w, q.r, q.kp, q.vp, q.ai, q.bi, s0, (const uint32_t*)in(kept.length),
+                                (const uint8_t*)in(kept.starts), dy, gs, out(kept.residual), (size_t)kept.residual.numel(), gw, gr, gk, gv, ga, gb, gs0.p, 0,
+                                out(ws)));
         if (wanted[1]) gs0.finish(st);
         // r, k' and v' also feed the stage behind the operator: its shares (dr, dkp, dvp) are added where the next kernel reads
         // anyway (gr in place)

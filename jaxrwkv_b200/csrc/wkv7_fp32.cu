@@ -1088,22 +1088,22 @@ size_t wkv7_fp32_workspace_bytes(int B, int T, int H) {
     const size_t bytes = (size_t)B * H * chunks_of(T) * (kN * kN + kTileFloats) * sizeof(float);
     return bytes <= ((size_t)2 << 30) ? bytes : 0;
 }
-// Of the residual: the checkpoints, as much again for the state gradients between the chunks (the forward keeps its tiles there), and
-// s of every token.
-size_t wkv7_fp32_residual_bytes(int B, int T, int H) {
-    const size_t heads = (size_t)B * H;
-    return (2 * heads * chunks_of(T) * kN * kN + heads * T * kN) * sizeof(float);
-}
+// What a forward leaves for its backward: the checkpoints and s of every token.  Besides, both want as much room as the checkpoints
+// have while they run (the forward for its tiles, the backward for the state gradients between the chunks): a workspace of each, or
+// the residual's middle.
+size_t wkv7_fp32_state_bytes(int B, int T, int H) { return (size_t)B * H * chunks_of(T) * kN * kN * sizeof(float); }
+size_t wkv7_fp32_kept_bytes(int B, int T, int H) { return wkv7_fp32_state_bytes(B, T, H) + (size_t)B * H * T * kN * sizeof(float); }
 
 int wkv7_fp32_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
                   const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y, void* s_out, void* residual,
-                  void* workspace) {
+                  size_t residual_bytes, void* workspace) {
     const int heads = B * H, nC = chunks_of(T);
     const Operands op{T, H, (const float*)w, (const float*)r, (const float*)k, (const float*)v, (const float*)a, (const float*)b, length, ns};
     const size_t states = (size_t)heads * nC * kN * kN, stride = residual != nullptr ? (size_t)kN * kN : (size_t)kTileFloats;
+    const bool room = residual != nullptr && residual_bytes >= wkv7_fp32_kept_bytes(B, T, H) + wkv7_fp32_state_bytes(B, T, H);
     float* const slots = (float*)(residual != nullptr ? residual : workspace);
-    float* const base = slots + states;
-    float* const sums = residual != nullptr ? base + states : nullptr;
+    float* const base = residual == nullptr || room ? slots + states : (float*)workspace;
+    float* const sums = residual == nullptr ? nullptr : room ? base + states : slots + states;
     const Tiles tiles{base, base + kTile, base + 2 * kTile, base + 3 * kTile, stride * nC, stride};
     int s = launch_prepare<true>(st, heads, op, tiles, slots, sums, (float*)y);
     if (s != B200WKV_OK) return s;
@@ -1115,12 +1115,13 @@ int wkv7_fp32_fwd(cudaStream_t st, int B, int T, int H, const void* w, const voi
 // The tiles of the chain lie in the buffers of the gradients, as [head][token][64], until the last kernel writes these; g lies in
 // dv's, where the last kernel's CTAs write over their own.
 int wkv7_fp32_bwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v, const void* a,
-                  const void* b, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual, void* dw,
-                  void* dr, void* dk, void* dv, void* da, void* db, void* ds0) {
+                  const void* b, const uint32_t* length, const uint8_t* ns, const void* dy, const void* ds_out, void* residual,
+                  size_t residual_bytes, void* workspace, void* dw, void* dr, void* dk, void* dv, void* da, void* db, void* ds0) {
     const int heads = B * H, nC = chunks_of(T);
     const Operands op{T, H, (const float*)w, (const float*)r, (const float*)k, (const float*)dy, (const float*)a, (const float*)b, length, ns};
     const size_t states = (size_t)heads * nC * kN * kN;
-    float *const ckpt = (float*)residual, *const carry = ckpt + states, *const sums = carry + states;
+    const bool room = residual_bytes >= wkv7_fp32_kept_bytes(B, T, H) + wkv7_fp32_state_bytes(B, T, H);
+    float *const ckpt = (float*)residual, *const carry = room ? ckpt + states : (float*)workspace, *const sums = ckpt + (room ? 2 : 1) * states;
     const Tiles tiles{(float*)dk, (float*)da, nullptr, (float*)dw, (size_t)T * kN, (size_t)kTile};
     int s = launch_prepare<false>(st, heads, op, tiles, carry, (float*)dv, nullptr);
     if (s != B200WKV_OK) return s;

@@ -17,11 +17,11 @@
 namespace b200wkv {
 size_t wkv7_seq_residual_bytes(int B, int T, int H);
 size_t wkv7_chunk_residual_bytes(int B, int T, int H);
-size_t wkv7_residual_min_bytes(int dtype, int B, int T, int H);
 }
 
 extern "C" {
 size_t b200wkv7_residual_bytes(int dtype, int B, int T, int H, int N);
+size_t b200wkv7_residual_min_bytes(int dtype, int B, int T, int H, int N);
 int b200wkv7_fwd(void* stream, int dtype, int B, int T, int H, int N, const void* w, const void* r, const void* k,
                  const void* v, const void* a, const void* b, const void* s0, const uint32_t* length,
                  const uint8_t* new_starts, void* y, void* s_out, void* residual, size_t residual_bytes,
@@ -85,7 +85,7 @@ int b200wkv7_fwd_bwd_static(void* stream, int dtype, int B, int T, int H, int N,
         return b200wkv7_fwd(stream, dtype, B, T, H, N, w, r, k, v, a, b, s0, length, new_starts, y, s_out, nullptr, 0, flags);
     }
     // more than the array has, but enough without the room that lets the backward walk a sequence's chunks side by side
-    if (need > kStaticScratchBytes && b200wkv::wkv7_residual_min_bytes(dtype, B, T, H) <= kStaticScratchBytes) need = kStaticScratchBytes;
+    if (need > kStaticScratchBytes && b200wkv7_residual_min_bytes(dtype, B, T, H, N) <= kStaticScratchBytes) need = kStaticScratchBytes;
     if (need > kStaticScratchBytes) return B200WKV_ESCRATCH;
     // everything either kernel pair could refuse is checked here, so that a bad argument of the
     // backward is reported before the forward has been enqueued

@@ -72,9 +72,14 @@ def batched_wkv7_fwd(r, w, k, v, a, b, s, length, new_starts, B, need_residual=T
         rbytes = lib.b200wkv7_residual_bytes(code, B, T, H, N)
         residual = buffers.get("residual")
         if residual is None:
-            residual = torch.empty(rbytes, dtype=torch.uint8, device=k.device)
+            try:
+                residual = torch.empty(rbytes, dtype=torch.uint8, device=k.device)
+            except torch.OutOfMemoryError:                        # fp32 does with the checkpoints alone
+                rbytes = lib.b200wkv7_residual_min_bytes(code, B, T, H, N)
+                residual = torch.empty(rbytes, dtype=torch.uint8, device=k.device)
         elif residual.numel() * residual.element_size() < rbytes or not residual.is_contiguous():
             raise _lib.B200WKVError("wkv7: the preallocated residual is too small")
+        rbytes = residual.numel() * residual.element_size()                   # as the backward is told
     _lib.check(lib.b200wkv7_fwd(_stream(), code, B, T, H, N, _ptr(w), _ptr(r), _ptr(k), _ptr(v), _ptr(a), _ptr(b),
                                 _ptr(s), _ptr(length), _ptr(new_starts), _ptr(out), _ptr(new_s),
                                 _ptr(residual), rbytes, flags))
