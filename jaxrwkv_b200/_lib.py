@@ -23,6 +23,7 @@ PROTOTYPES = {
     "b200wkv_abi_version": (_I, []),
     "b200wkv_device_status": (_I, []),
     "b200wkv_debug_step_residency": (_I, [_I, _P, _P]),
+    "b200wkv_debug_wkv7_fwd_form": (_I, [_I, _I, _I, _I, _I, _I]),
     "b200wkv7_residual_bytes": (_SZ, [_I, _I, _I, _I, _I]),
     "b200wkv7_residual_min_bytes": (_SZ, [_I, _I, _I, _I, _I]),
     "b200wkv7_fwd": (_I, [_P, _I, _I, _I, _I, _I] + [_P] * 9 + [_P, _P, _P, _SZ, _U]),

@@ -505,6 +505,11 @@ int b200wkv_debug_step_residency(int dtype, int* grid_per_sm, int* fit_per_sm) {
     return wkv7_step_stream_residency(dtype, grid_per_sm, fit_per_sm);
 }
 
+int b200wkv_debug_wkv7_fwd_form(int sms, int largest_cluster, int B, int T, int H, int residual) {
+    if (sms < 1 || check_dims(B200WKV_BF16, B, T, H, kN) != B200WKV_OK) return B200WKV_ESHAPE;
+    return wkv7_fwd_form(sms, largest_cluster, B, T, H, residual != 0);
+}
+
 static int check_shift(int dtype, int B, int T, int D, int M) {
     if (dtype != B200WKV_F32 && dtype != B200WKV_BF16) return B200WKV_EDTYPE;
     if (B < 1 || T < 1 || D < 4 || (D % 4) != 0 || M < 1 || M > 8 || (long long)B * T > 2147483647LL || B > 65535) return B200WKV_ESHAPE;

@@ -38,7 +38,9 @@ struct BlocksCall {
     size_t s0_stride;
     unsigned char* saved;
 };
-// Bytes of workspace with which a call takes this form (0: it does not)
+// Bytes of workspace with which a call takes this form or a ring (0: neither), and which it is on a given device: 0 the walk, 1 this
+// one, else a ring of so many CTAs
+int wkv7_fwd_form(int sms, int largest, int B, int T, int H, bool residual);
 size_t wkv7_blocks_bytes(int B, int T, int H, bool residual);
 int wkv7_blocks_finish(cudaStream_t st, int B, int T, int H, const uint32_t* length, const uint8_t* ns, const void* s0, int* range_flag, int range_ticket,
                        const BlocksCall& call, void* y,

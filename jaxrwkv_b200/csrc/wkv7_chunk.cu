@@ -1036,9 +1036,9 @@ int* wkv_call_flag(int* ticket) {
 //     BH=80:  T=1024 112 / 94, 124 / 97    2000 216 / 171, 138 / 180     BH=72 (side by side):  T=2000 158 / 170, 153 / 183
 // From three blocks on (T=192: 25.3 / 19; two: 19.2 / 17-21), with a residual from four: there the host, who has a workspace to
 // allocate, is what such a call waits for.
-static int ring_size(int B, int T, int H, bool residual) {
-    const long long sms = sm_count_of_current_device(), seqs = (long long)B * H, blocks = block_slots(T) - 1;
-    const long long n = 16 * seqs <= sms ? 16 : std::min(7 * sms / 4 / seqs, 9LL);
+static int ring_size(long long sms, int largest, int B, int T, int H, bool residual) {
+    const long long seqs = (long long)B * H, blocks = block_slots(T) - 1;
+    const long long n = std::min(16 * seqs <= sms ? 16 : std::min(7 * sms / 4 / seqs, 9LL), (long long)largest);
     const long long longest = n * seqs < 4 * sms / 3 ? 24 : n >= 7 ? 65535 : n == 6 ? 48 : n > 3 ? 32 : 2 * seqs > sms ? 16 : 0;
     if (n < 3 || blocks < (residual ? 4 : 3) || blocks > longest) return 1;
     return (int)std::min(n, blocks);
@@ -1049,32 +1049,73 @@ static size_t ring_bytes(int B, int T, int H, bool residual) {
     return (size_t)B * H * (residual ? (size_t)block_slots(T) * (kC * kN * sizeof(float)) : (size_t)T * (kN * sizeof(__nv_bfloat16)));
 }
 
-size_t wkv7_blocks_bytes(int B, int T, int H, bool residual) {
+// The form for a device of `sms` SMs that takes clusters of up to `largest` CTAs: the CTAs of a ring, or kWalkForm, kBlocksForm
+int wkv7_fwd_form(int sms, int largest, int B, int T, int H, bool residual) {
     const size_t most = (size_t)2 << 30;
-    if (ring_size(B, T, H, residual) > 1 && ring_bytes(B, T, H, residual) <= most) return ring_bytes(B, T, H, residual);
-    const long long sms = sm_count_of_current_device(), seqs = (long long)B * H, blocks = block_slots(T) - 1;
-    if (blocks < 4 || blocks >= 65536) return 0;
-    if (2 * seqs > sms && !(residual && blocks >= 24 && 3 * seqs <= 2 * sms)) return 0;
-    if (!residual && seqs * blocks > 9 * 2 * sms) return 0;
-    const size_t bytes = blocks_layout(B, T, H, residual).end;
-    return bytes <= most ? bytes : 0;
+    const int ring = ring_size(sms, largest, B, T, H, residual);
+    if (ring > 1 && ring_bytes(B, T, H, residual) <= most) return ring;
+    const long long seqs = (long long)B * H, blocks = block_slots(T) - 1;
+    if (blocks < 4 || blocks >= 65536) return kWalkForm;
+    if (2 * seqs > sms && !(residual && blocks >= 24 && 3 * seqs <= 2 * sms)) return kWalkForm;
+    if (!residual && seqs * blocks > 9LL * 2 * sms) return kWalkForm;
+    return blocks_layout(B, T, H, residual).end <= most ? kBlocksForm : kWalkForm;
+}
+
+static cudaLaunchConfig_t ring_config(cudaLaunchAttribute* attr, int heads, int ring, cudaStream_t st) {
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = ring; attr->val.clusterDim.y = 1; attr->val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(heads * ring));
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = SMEM_BYTES;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+static bool forms_set_up() {       // the opt-in to large dynamic shared memory is a per-device function attribute
+    static DeviceOnce once;
+    return once.ok([]() {
+        const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kWalkForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (e != cudaSuccess) return e;
+        const cudaError_t f = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        if (f != cudaSuccess) return f;
+        const cudaError_t g = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (g != cudaSuccess) return g;
+        return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kBlocksForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    });
+}
+// CTAs of the largest ring that the current device takes: 16 of a whole B200 (seven such clusters at once), fewer, down to none, where
+// the process has been given a share of its SMs.
+static int largest_ring() {
+    static DeviceOnce once;
+    static int largest[kMaxDevices];
+    const int dev = current_device();
+    if (dev < 0 || !forms_set_up()) return 0;
+    once.ok([dev]() {
+        for (int n = 16; n > 2 && largest[dev] == 0; --n) {
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = ring_config(&attr, 1, n, nullptr);
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, wkv7_chunk_fwd_kernel<kRingForm>, &cfg) != cudaSuccess) (void)cudaGetLastError();
+            else if (clusters > 0) largest[dev] = n;
+        }
+        return cudaSuccess;
+    });
+    return largest[dev];
+}
+static int form_here(int B, int T, int H, bool residual) { return wkv7_fwd_form(sm_count_of_current_device(), largest_ring(), B, T, H, residual); }
+
+size_t wkv7_blocks_bytes(int B, int T, int H, bool residual) {
+    const int form = form_here(B, T, H, residual);
+    return form == kWalkForm ? 0 : form == kBlocksForm ? blocks_layout(B, T, H, residual).end : ring_bytes(B, T, H, residual);
 }
 
 int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const void* r, const void* k, const void* v,
                    const void* a, const void* b, const void* s0, const uint32_t* length, const uint8_t* ns, void* y,
                    void* s_out, void* residual, void* workspace, int* residual_mark, int** range_flag, int* range_ticket) {
     typedef __nv_bfloat16 bf;
-    static DeviceOnce smem_attr;   // the opt-in to large dynamic shared memory is a per-device function attribute
-    if (!smem_attr.ok([]() {
-            const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kWalkForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-            if (e != cudaSuccess) return e;
-            const cudaError_t f = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-            if (f != cudaSuccess) return f;
-            const cudaError_t g = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-            if (g != cudaSuccess) return g;
-            return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kBlocksForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        }))
-        return B200WKV_ELAUNCH;
+    if (!forms_set_up()) return B200WKV_ELAUNCH;
     *range_flag = wkv_call_flag(range_ticket);
     if (*range_flag == nullptr) return B200WKV_ELAUNCH;
     const ResidualLayout lay = residual_layout(B, T, H);
@@ -1085,29 +1126,22 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
     StreamMaps out_maps;                         // m[0]: the outputs, with the 128-byte swizzle of the kernel's output tile
     const void* out_bases[2] = {y, residual ? (const void*)((char*)residual + lay.rbar) : y};   // m[1]: the R- rows
     if (!make_stream_maps(&out_maps, out_bases, 2, B, T, H, /*swizzle128=*/true)) return B200WKV_ELAUNCH;
-    // (a workspace that is there has the bytes of the one form or the other)
-    const int ring = workspace != nullptr && ring_bytes(B, T, H, residual != nullptr) <= ((size_t)2 << 30) ? ring_size(B, T, H, residual != nullptr) : 1;
-    if (ring > 1) {
+    const int form = workspace != nullptr ? form_here(B, T, H, residual != nullptr) : (int)kWalkForm;      // (the workspace has the form's bytes)
+    if (form > kBlocksForm) {
         BlockParts parts = {};
         parts.sa = (float4*)workspace;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = ring; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(B * H * ring));
-        cfg.blockDim = dim3(256);
-        cfg.dynamicSmemBytes = SMEM_BYTES;
-        cfg.stream = st;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, wkv7_chunk_fwd_kernel<kRingForm>, T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a,
-                                  (const bf*)b, (const bf*)s0, length, ns, (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : (float*)nullptr, maps,
-                                  out_maps.m[0], out_maps.m[1], residual ? (unsigned char*)(base + lay.saved) : (unsigned char*)nullptr, *range_flag,
-                                  *range_ticket, residual_mark, residual ? (bf*)(base + lay.mprime) : (bf*)nullptr,
-                                  residual ? (bf*)(base + lay.rbar) : (bf*)workspace,
-                                  residual ? (float*)(base + lay.lam) : (float*)nullptr, 1, parts) == cudaSuccess ? B200WKV_OK : B200WKV_ELAUNCH;
+        cudaLaunchAttribute attr;
+        const cudaLaunchConfig_t cfg = ring_config(&attr, B * H, form, st);
+        if (cudaLaunchKernelEx(&cfg, wkv7_chunk_fwd_kernel<kRingForm>, T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a,
+                               (const bf*)b, (const bf*)s0, length, ns, (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : (float*)nullptr, maps,
+                               out_maps.m[0], out_maps.m[1], residual ? (unsigned char*)(base + lay.saved) : (unsigned char*)nullptr, *range_flag,
+                               *range_ticket, residual_mark, residual ? (bf*)(base + lay.mprime) : (bf*)nullptr,
+                               residual ? (bf*)(base + lay.rbar) : (bf*)workspace,
+                               residual ? (float*)(base + lay.lam) : (float*)nullptr, 1, parts) == cudaSuccess)
+            return B200WKV_OK;
+        (void)cudaGetLastError();  // (a share of SMs that this stream alone has: the walk below needs no cluster)
     }
-    if (workspace != nullptr) {   // the blocks side by side (see wkv7_blocks_bytes)
+    if (form == kBlocksForm) {     // the blocks side by side
         const BlocksLayout bl = blocks_layout(B, T, H, residual != nullptr);
         char* const ws = static_cast<char*>(workspace);
         BlocksCall c;
