@@ -1024,22 +1024,35 @@ int* wkv_call_flag(int* ticket) {
 // slot.  The last limit bounds the workspace, 2 GiB.
 //
 // Rings take precedence.  A ring has as many CTAs as the device has room for: seven eighths of the two slots per SM, because a
-// cluster stays within a GPC (BH=32, T=2048: 83 us by six, 72 by seven, 68 by eight; 114 by nine, which do not fit at once;
-// BH=80: three, and two CTAs only wait for one another).  Nine are enough to keep a state moving (17 k cycles for a block, 2.7 k for
-// a hop); up to a sixteenth of a sequence per SM there is room for sixteen, which halves the time between start flags.  Without
-// flags a ring is never slower than the other two.  With many, blocks side by side and the walk in pieces are cut into shorter
-// chains, a ring isn't, and its few CTAs lose in long sequences.  The limits in blocks are where both are equal at a flag every
-// 256 tokens (us, walk or side by side / ring, without flags and with):
-//     BH=4:   T=2048 60 / 56, 42 / 42      4096 99 / 99, 52 / 60         BH=16:  T=1600 68 / 54, 54 / 50    4096 137 / 110, 85 / 104
-//     BH=32:  T=4096 185 / 123, 130 / 125                                BH=40:  T=3000 157 / 119, 124 / 124  4096 201 / 157, 158 / 163
-//     BH=48:  T=2000 126 / 101, 115 / 106  4096 418 / 187, 161 / 201     BH=64:  T=2000 145 / 127, 133 / 136  4096 419 / 242, 170 / 258
-//     BH=80:  T=1024 112 / 94, 124 / 97    2000 216 / 171, 138 / 180     BH=72 (side by side):  T=2000 158 / 170, 153 / 183
-// From three blocks on (T=192: 25.3 / 19; two: 19.2 / 17-21), with a residual from four: there the host, who has a workspace to
+// cluster stays within a GPC (BH=32, T=2048: 83 us by six, 72 by seven, 68 by eight; 114 by nine, which do not fit at once; two
+// CTAs only wait for one another).  Nine are enough to keep a state moving (17 k cycles for a block, 2.7 k for a hop); up to a
+// sixteenth of a sequence per SM there is room for sixteen, which halves the time between start flags.  Of four and more, a ring
+// is the fastest without flags; a ring of three is slower than blocks side by side (which go up to half a sequence per SM) from eight
+// blocks on.  With flags, blocks side by side and the walk in pieces are cut into shorter chains, a ring isn't, and loses in long
+// sequences.  With a residual the walk is not cut, and a ring lasts longer.  The host doesn't know the flags: a limit in blocks lies where a
+// ring and what is taken behind it are equal at a flag every 256 tokens, or where it loses 2-9 % with those and gains 7-24 % without
+// (rings of four and six).  us, that form / ring, without flags and with (rings of seven and more are the faster ones up to T=4096
+// except of few heads, which don't fill the device):
+//     no residual  BH=4, 8:   T=1536 52 / 46, 36 / 31 and 54 / 51, 43 / 39      2000 60 / 56, 34 / 36 and 64 / 62, 44 / 45     4096 112 / 108, 58 / 73
+//                  BH=16:     T=1536 66 / 52, 54 / 50    1792 73 / 59, 55 / 55    4096 136 / 111, 89 / 104
+//                  BH=24, 36: T=3072 125 / 92, 83 / 85 and 154 / 102, 119 / 108    4096 163 / 118, 112 / 112 and 196 / 132, 149 / 135
+//                  BH=40:     T=2304 126 / 94, 100 / 95    2560 137 / 103, 108 / 109    3072 158 / 120, 121 / 125
+//                  BH=48:     T=2304 139 / 113, 117 / 117    2560 150 / 124, 129 / 128    3072 178 / 143, 145 / 150
+//                  BH=64:     T=1472 110 / 95, 104 / 100    1600 120 / 102, 111 / 106    1792 132 / 114, 118 / 118    2000 145 / 126, 126 / 133
+//                  BH=56:     T=1600 112 / 100, 102 / 102    1792 122 / 113, 111 / 115    2000 136 / 127, 120 / 131
+//                  BH=65-74:  T=192 25 / 22, 27 / 22    384 46 / 40, 46 / 42    448 50 / 44, 49 / 45    512 51 / 51, 50 / 53    1024 87 / 93, 82 / 96
+//                  BH=80:     T=768 85 / 72, 76 / 74    1024 112 / 95, 102 / 95 (walked)    1280 138 / 114, 117 / 117    1536 165 / 133, 104 / 136
+//     residual     BH=40, 48, 64: T=3072 177 / 136, 140 / 138 and 198 / 164, 167 / 167 and 232 / 207, 209 / 213      4096 224 / 174, 179 / 178 and
+//                             251 / 206, 209 / 217 and 303 / 274, 265 / 279
+//                  BH=65-74:  T=320 48 / 38, 50 / 38    384 52 / 46, 53 / 47    512 60 / 58, 59 / 60    1024 100 / 105, 95 / 107
+//                  BH=80:     T=1024 121 / 105, 125 / 107 (walked)    1472 169 / 141, 174 / 145    1536 153 / 145, 141 / 149 (side by side from here on)
+// From three blocks on (T=192: 25 / 19; two: 19 / 17-21), with a residual from four: there the host, who has a workspace to
 // allocate, is what such a call waits for.
 static int ring_size(long long sms, int largest, int B, int T, int H, bool residual) {
     const long long seqs = (long long)B * H, blocks = block_slots(T) - 1;
     const long long n = std::min(16 * seqs <= sms ? 16 : std::min(7 * sms / 4 / seqs, 9LL), (long long)largest);
-    const long long longest = n * seqs < 4 * sms / 3 ? 24 : n >= 7 ? 65535 : n == 6 ? 48 : n > 3 ? 32 : 2 * seqs > sms ? 16 : 0;
+    const bool few = 9 * seqs < 4 * sms / 3;                  // rings at their largest leave a third of the device idle
+    const long long longest = few ? 24 : n >= 7 ? 65535 : n > 3 && residual ? 48 : n == 6 ? 48 : n == 5 ? 40 : n == 4 ? 32 : 2 * seqs <= sms ? 7 : residual ? 23 : 16;
     if (n < 3 || blocks < (residual ? 4 : 3) || blocks > longest) return 1;
     return (int)std::min(n, blocks);
 }
