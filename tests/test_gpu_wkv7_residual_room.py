@@ -33,18 +33,32 @@ def backward(case, leaves, out):
 
 
 class Room:
-    """The device as full as it is, but for pieces of `n` bytes."""
+    """The device as full as it is, but for pieces of `n` bytes; free parts of the allocator's segments are filled as well."""
     def __init__(self, n, pieces=1):
         torch.cuda.synchronize()
         torch.cuda.empty_cache()
+        self.limit()
+        self.fill = []
+        for size in (64 * MB, 16 * MB, 4 * MB, MB + 512):
+            try:
+                while True:
+                    self.fill.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                pass
+        torch.cuda.set_per_process_memory_fraction(1.0)
         self.blocks = [torch.empty(n, dtype=torch.uint8, device="cuda") for _ in range(pieces)]
 
-    def __enter__(self):
+    @staticmethod
+    def limit():
         torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+
+    def __enter__(self):
+        self.limit()
         del self.blocks
 
     def __exit__(self, *_):
         torch.cuda.set_per_process_memory_fraction(1.0)
+        del self.fill
 
 
 def test_what_is_kept_and_what_does_without(case):
