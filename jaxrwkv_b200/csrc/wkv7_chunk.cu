@@ -79,6 +79,8 @@ constexpr int OFF_SB = OFF_SA;                   // the same in bf16         64-
 constexpr int OFF_MH = OFF_V;                    // M', its bf16 part        64-row slab
 constexpr int OFF_ML = OFF_G;                    // M', what that rounds off 64-row slab (over W~)
 constexpr int OFF_WR = OFF_TP;                   // [W~ ; R-]                128-row slab
+// ... of kExactRingForm: [W~ ; R~], without a residual [P_rb W~ ; R~], and
+constexpr int OFF_PW = OFF_ML;                   // with one P_rb W~         64-row slab, once the state products are done
 static_assert(OFF_IN + kN * kN * 4 <= OFF_SB, "the entering state lies over B^ and K^");
 struct Small {
     float h1[kN];        // cumulative log-decay of tokens 0..31, stored [e][jb] for channel 8 jb + e
@@ -203,7 +205,12 @@ __device__ __forceinline__ void load_part(const float4* tiles, size_t slot, int 
 // CTA takes 2700 cycles (330 to the operand slab, 870 products, 400 results, 1000 to the next CTA), a block 17 k of its CTA's, 13 k of
 // them before the state is needed.  One sequence of 40 heads, T=1999: 114 us in kBlocks, 83 by rings of six; 80 sequences,
 // T=1024: 111 walked, 96 by rings of three.
-enum Form { kWalkForm, kBlocksForm, kRingForm };
+// R- = R~ + P_rb W~ is rounded once more than R~ and sa are before they meet in the walk, which makes the outputs' errors 0.15 % larger
+// than the walk's (4.090e-3 of them against 4.084e-3, 80 sequences, T=1000), in blocks side by side as in a ring.  kExactRing, for
+// calls that without rings would be walked: R~ and P_rb W~ each meet the state in a product (4.084e-3).  A product of 64 deep takes
+// some 350 cycles that a block of a full device waits for, so that all other rings leave it out (us, B=5, H=16, T=1000: 93.6 / 97.7; 40
+// heads, T=1999: 83.8 / 90).
+enum Form { kWalkForm, kBlocksForm, kRingForm, kExactRingForm };
 //
 // 256 threads: warp = (quad, hsel); quad selects the 32 TMEM lanes (tile rows) the warp may access,
 // hsel the column half it works on, so every accumulator tile is shared by two warps per row group.
@@ -220,7 +227,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                       int* __restrict__ range_flag, int range_ticket, int* __restrict__ residual_mark,
                       __nv_bfloat16* __restrict__ mprime, __nv_bfloat16* __restrict__ rbar, float* __restrict__ lam_out, int pieces,
                       const BlockParts parts) {
-    constexpr bool kBlocks = kForm == kBlocksForm, kRing = kForm == kRingForm, kZero = kBlocks || kRing;
+    constexpr bool kBlocks = kForm == kBlocksForm, kExactRing = kForm == kExactRingForm, kRing = kForm == kRingForm || kExactRing, kZero = kBlocks || kRing;
     if (kZero) let_next_in();
     extern __shared__ __align__(1024) unsigned char smem[];   // (the swizzle of the output tile is a function of the address)
     Small& sm = *reinterpret_cast<Small*>(smem + OFF_SMALL);
@@ -757,6 +764,7 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 tc::mbar_arrive_in_cta(tc::in_cta(&sm.ring[3], left));
             }
             float x[32];
+            uint4 pw[4];                                               // P_rb W~ (kExactRing)
             if (quad < 2) {
                 tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);          // M'[j][j'], row j = this thread's lane, as high + low parts
                 tc::tmem_wait_ld();
@@ -789,8 +797,12 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
 #pragma unroll
                     for (int e = 0; e < 8; ++e) rf[e] += x[c * 8 + e];
                     const uint4 r_bar = pack8(rf);
-                    slab_store(smem + OFF_WR, CB128, row, hsel * 4 + c, r_bar);
+                    slab_store(smem + OFF_WR, CB128, row, hsel * 4 + c, kExactRing ? rt[c] : r_bar);
                     if (keep != nullptr && t < n) to[c] = r_bar;
+                    if constexpr (kExactRing) {
+                        pw[c] = pack8(&x[c * 8]);
+                        if (keep == nullptr) slab_store(smem + OFF_WR, CB128, t, hsel * 4 + c, pw[c]);
+                    }
                 }
             }
             // ---- the leaving state: of a flagged block U, which waits for nothing, otherwise what becomes of the entering one
@@ -848,12 +860,31 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 tc::commit(&sm.ring[0]);
             } else if (tid == kIssuer2) {      // what no other CTA waits for
                 tc::fence_after_sync();
-                mma_k64(tbase + D1, kmaj128(tc::smem_u32(smem + OFF_WR)), kmaj64(tc::smem_u32(smem + OFF_SB)), ID_128x64_KK, false);
-                tc::commit(&sm.ring[1]);
+                const bool onto_y = kExactRing && keep == nullptr;     // (nobody wants W~ S0^T)
+                mma_k64(tbase + (onto_y ? D2 : D1), kmaj128(tc::smem_u32(smem + OFF_WR)), kmaj64(tc::smem_u32(smem + OFF_SB)), ID_128x64_KK, onto_y);
+                if (!kExactRing) tc::commit(&sm.ring[1]);
             }
             if (keep != nullptr && warp == 7 && lane < 8) {   // the bf16 entering state goes to the residual
                 tc::bulk_store(keep + (size_t)SAVED_S0 * GTILE + lane * GCB, smem + OFF_SB + lane * CB64, 64 * 16);
                 tc::bulk_commit();
+            }
+            // P_rb W~ behind the state products, as rows 64..127 of an operand that begins 64 rows in front of it (nobody reads the results of
+            // rows 0..63).  With a residual W~ has the rows that it has without, and it goes where the low part of M' was read.
+            if (kExactRing && quad >= 2) {
+                if (!flagged && !tc::mbar_wait(&sm.ring[0], ring_par)) failed = true;
+                if (keep != nullptr) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) slab_store(smem + OFF_PW, CB64, row - 64, hsel * 4 + c, pw[c]);
+                    tc::fence_async_smem();
+                    tc::fence_before_sync();
+                    asm volatile("bar.sync 1, 128;" ::: "memory");
+                }
+                if (tid == kIssuer2) {
+                    tc::fence_after_sync();
+                    mma_k64(tbase + D2, keep == nullptr ? kmaj128(tc::smem_u32(smem + OFF_WR) - 64 * 16) : kmaj64(tc::smem_u32(smem + OFF_PW) - 64 * 16),
+                            kmaj64(tc::smem_u32(smem + OFF_SB)), ID_128x64_KK, true);
+                    tc::commit(&sm.ring[1]);
+                }
             }
             if (!flagged) {
                 // (meanwhile: whether the next CTA can take the state, what remains of the entering one)
@@ -885,10 +916,14 @@ wkv7_chunk_fwd_kernel(int Tlen, int H, int n_seq, const __nv_bfloat16* __restric
                 const int t = row - 64;
                 float yv[32];
                 tc::tmem_ld32(lane_addr + D2 + hsel * 32, yv);
-                tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);
-                tc::tmem_wait_ld();
+                if (!kExactRing || keep != nullptr) {
+                    tc::tmem_ld32(lane_addr + D1 + hsel * 32, x);
+                    tc::tmem_wait_ld();
 #pragma unroll
-                for (int c = 0; c < 32; ++c) yv[c] += x[c];
+                    for (int c = 0; c < 32; ++c) yv[c] += x[c];
+                } else {
+                    tc::tmem_wait_ld();
+                }
                 if (n == kC) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c)
@@ -1031,7 +1066,8 @@ int* wkv_call_flag(int* ticket) {
 // blocks on.  With flags, blocks side by side and the walk in pieces are cut into shorter chains, a ring isn't, and loses in long
 // sequences.  With a residual the walk is not cut, and a ring lasts longer.  The host doesn't know the flags: a limit in blocks lies where a
 // ring and what is taken behind it are equal at a flag every 256 tokens, or where it loses 2-9 % with those and gains 7-24 % without
-// (rings of four and six).  us, that form / ring, without flags and with (rings of seven and more are the faster ones up to T=4096
+// (rings of four and six).  us, that form / ring (kRing; where that form is the walk the call takes kExactRing, 4 % above the figure
+// here), without flags and with (rings of seven and more are the faster ones up to T=4096
 // except of few heads, which don't fill the device):
 //     no residual  BH=4, 8:   T=1536 52 / 46, 36 / 31 and 54 / 51, 43 / 39      2000 60 / 56, 34 / 36 and 64 / 62, 44 / 45     4096 112 / 108, 58 / 73
 //                  BH=16:     T=1536 66 / 52, 54 / 50    1792 73 / 59, 55 / 55    4096 136 / 111, 89 / 104
@@ -1063,15 +1099,17 @@ static size_t ring_bytes(int B, int T, int H, bool residual) {
 }
 
 // The form for a device of `sms` SMs that takes clusters of up to `largest` CTAs: the CTAs of a ring, or kWalkForm, kBlocksForm
-int wkv7_fwd_form(int sms, int largest, int B, int T, int H, bool residual) {
-    const size_t most = (size_t)2 << 30;
-    const int ring = ring_size(sms, largest, B, T, H, residual);
-    if (ring > 1 && ring_bytes(B, T, H, residual) <= most) return ring;
+constexpr size_t kMostWorkspace = (size_t)2 << 30;
+static int form_without_rings(int sms, int B, int T, int H, bool residual) {
     const long long seqs = (long long)B * H, blocks = block_slots(T) - 1;
     if (blocks < 4 || blocks >= 65536) return kWalkForm;
     if (2 * seqs > sms && !(residual && blocks >= 24 && 3 * seqs <= 2 * sms)) return kWalkForm;
     if (!residual && seqs * blocks > 9LL * 2 * sms) return kWalkForm;
-    return blocks_layout(B, T, H, residual).end <= most ? kBlocksForm : kWalkForm;
+    return blocks_layout(B, T, H, residual).end <= kMostWorkspace ? kBlocksForm : kWalkForm;
+}
+int wkv7_fwd_form(int sms, int largest, int B, int T, int H, bool residual) {
+    const int ring = ring_size(sms, largest, B, T, H, residual);
+    return ring > 1 && ring_bytes(B, T, H, residual) <= kMostWorkspace ? ring : form_without_rings(sms, B, T, H, residual);
 }
 
 static cudaLaunchConfig_t ring_config(cudaLaunchAttribute* attr, int heads, int ring, cudaStream_t st) {
@@ -1089,13 +1127,12 @@ static cudaLaunchConfig_t ring_config(cudaLaunchAttribute* attr, int heads, int 
 static bool forms_set_up() {       // the opt-in to large dynamic shared memory is a per-device function attribute
     static DeviceOnce once;
     return once.ok([]() {
-        const cudaError_t e = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kWalkForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (e != cudaSuccess) return e;
-        const cudaError_t f = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-        if (f != cudaSuccess) return f;
-        const cudaError_t g = cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kRingForm>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (g != cudaSuccess) return g;
-        return cudaFuncSetAttribute(wkv7_chunk_fwd_kernel<kBlocksForm>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        cudaError_t e = cudaSuccess;
+        for (const auto kernel : {wkv7_chunk_fwd_kernel<kWalkForm>, wkv7_chunk_fwd_kernel<kBlocksForm>, wkv7_chunk_fwd_kernel<kRingForm>, wkv7_chunk_fwd_kernel<kExactRingForm>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+        for (const auto kernel : {wkv7_chunk_fwd_kernel<kRingForm>, wkv7_chunk_fwd_kernel<kExactRingForm>})
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return e;
     });
 }
 // CTAs of the largest ring that the current device takes: 16 of a whole B200 (seven such clusters at once), fewer, down to none, where
@@ -1145,7 +1182,8 @@ int wkv7_chunk_fwd(cudaStream_t st, int B, int T, int H, const void* w, const vo
         parts.sa = (float4*)workspace;
         cudaLaunchAttribute attr;
         const cudaLaunchConfig_t cfg = ring_config(&attr, B * H, form, st);
-        if (cudaLaunchKernelEx(&cfg, wkv7_chunk_fwd_kernel<kRingForm>, T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a,
+        const bool walked = form_without_rings(sm_count_of_current_device(), B, T, H, residual != nullptr) == kWalkForm;
+        if (cudaLaunchKernelEx(&cfg, walked ? wkv7_chunk_fwd_kernel<kExactRingForm> : wkv7_chunk_fwd_kernel<kRingForm>, T, H, B * H, (const bf*)w, (const bf*)r, (const bf*)k, (const bf*)v, (const bf*)a,
                                (const bf*)b, (const bf*)s0, length, ns, (bf*)y, (bf*)s_out, residual ? (float*)(base + lay.s_at_len) : (float*)nullptr, maps,
                                out_maps.m[0], out_maps.m[1], residual ? (unsigned char*)(base + lay.saved) : (unsigned char*)nullptr, *range_flag,
                                *range_ticket, residual_mark, residual ? (bf*)(base + lay.mprime) : (bf*)nullptr,

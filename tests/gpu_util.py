@@ -3,6 +3,7 @@ import numpy as np
 import torch
 
 import oracle
+from jaxrwkv_b200 import _lib
 
 NAMES7 = ("r", "w", "k", "v", "a", "b", "s0")
 # Stated tolerances (Frobenius-relative): fp32 against the float64 oracle, bf16 against the
@@ -37,3 +38,12 @@ def wkv7_case(B, T, H, seed, p_start=0.0, random_length=False, s0_scale=0.0, sta
     if lengths is not None:
         d["length"] = np.asarray(lengths, dtype=np.uint32)
     return d
+
+
+WALK, BLOCKS = 0, 1
+
+
+def forward_form(B, T, H, train):
+    """The form that a bf16 RWKV-7 forward takes on this device: WALK, BLOCKS, or a ring of so many CTAs."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return _lib.load().b200wkv_debug_wkv7_fwd_form(sms, 16, B, T, H, int(train))
