@@ -1,5 +1,6 @@
-"""GPU tests of the block-parallel RWKV-7 forward (few sequences of four blocks or more): the blocks of all sequences over the
-CTAs, the chain over the blocks and its cuts behind flagged blocks, `length` inside and between blocks, ragged last blocks."""
+"""GPU tests of the block-parallel RWKV-7 forward (few sequences, longer than rings take): the blocks of all sequences over the
+CTAs, the chain over the blocks and its cuts behind flagged blocks, `length` inside and between blocks, ragged last blocks; and the
+same inputs at the shorter sizes that rings take."""
 import numpy as np
 import pytest
 import torch
@@ -7,7 +8,7 @@ import torch
 import oracle
 from jaxrwkv_b200 import rwkv7
 from conftest import rel_err
-from gpu_util import NAMES7, TOL, flags, npf, rounded, to_dev, wkv7_case
+from gpu_util import BLOCKS, NAMES7, TOL, flags, forward_form, npf, rounded, to_dev, wkv7_case
 
 pytestmark = pytest.mark.gpu
 
@@ -15,6 +16,19 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("train", [False, True])
 @pytest.mark.parametrize("T,H,p_start", [(193, 1, 0.0), (256, 2, 0.0), (700, 1, 0.01), (1100, 5, 1 / 128)])
 def test_forward_and_backward(T, H, p_start, train):
+    assert forward_form(4, T, H, train) > BLOCKS                    # a ring
+    check(T, H, p_start, train)
+
+
+# a chain in one piece and in eight; several heads; more sequences than rings of four take
+@pytest.mark.parametrize("train", [False, True])
+@pytest.mark.parametrize("T,H,p_start", [(1601, 1, 0.0), (1664, 2, 0.02), (2111, 1, 1 / 128), (1700, 2, 1 / 256), (520, 17, 1 / 128)])
+def test_forward_and_backward_side_by_side(T, H, p_start, train):
+    assert forward_form(4, T, H, train) == BLOCKS
+    check(T, H, p_start, train)
+
+
+def check(T, H, p_start, train):
     B = 4
     d = wkv7_case(B, T, H, seed=T, p_start=p_start, s0_scale=0.5)
     d["length"][:] = [T, 0, 128, T - 37]
@@ -39,8 +53,10 @@ def test_forward_and_backward(T, H, p_start, train):
         assert rel_err(npf(got[n]), b) < tol, n
 
 
-def test_decay_outside_the_range_is_redone():
-    d = wkv7_case(2, 320, 1, seed=3)
+@pytest.mark.parametrize("T,blocks", [(320, False), (1700, True)])
+def test_decay_outside_the_range_is_redone(T, blocks):
+    assert (forward_form(2, T, 1, False) == BLOCKS) == blocks
+    d = wkv7_case(2, T, 1, seed=3)
     d["w"][1, 70:90] = 3.0                     # exp(-20) per token
     t = to_dev(d, torch.bfloat16)
     length, ns = flags(d)

@@ -5,10 +5,16 @@ import torch
 
 from jaxrwkv_b200 import rwkv7
 from conftest import rel_err
-from gpu_util import NAMES7, TOL, flags, npf, to_dev, wkv7_case
+from gpu_util import BLOCKS, NAMES7, TOL, flags, forward_form, npf, to_dev, wkv7_case
 
 pytestmark = pytest.mark.gpu
 BAD = ("w", "k", "v", "a", "b", "s0")
+FORMS = ["walk", "ring", "side by side"]
+LONG = 1700                                       # blocks side by side are taken where a ring is not, above 24 blocks
+
+
+def takes(form, T, H, train):
+    return forward_form(1, T, H, train) == BLOCKS if form == "side by side" else forward_form(1, T, H, train) > BLOCKS
 
 
 def operands(T, H, starts, bad, at, value):
@@ -33,9 +39,10 @@ def outside_equals(clean, odd, lo, hi):
 # the value lies in front of a flag of its own 64-token block; a block and more in front of one; behind another one
 @pytest.mark.parametrize("lo,at,hi", [(0, 66, 70), (0, 10, 140), (70, 100, 200), (128, 128, 192)])
 @pytest.mark.parametrize("bad", BAD)
-@pytest.mark.parametrize("form", ["walk", "side by side"])
+@pytest.mark.parametrize("form", FORMS)
 def test_forward(form, bad, lo, at, hi):
-    T, H, value = 600, 3, float("inf") if bad in ("k", "v") else float("nan")
+    T, H, value = LONG if form == "side by side" else 600, 3, float("inf") if bad in ("k", "v") else float("nan")
+    assert takes(form, T, H, False)
     if bad == "s0":
         lo = 0
     clean, odd, (length, ns) = operands(T, H, sorted({lo, hi} - {0}), bad, at, value)
@@ -51,9 +58,10 @@ def test_forward(form, bad, lo, at, hi):
 
 @pytest.mark.parametrize("lo,at,hi", [(70, 100, 200), (128, 150, 192), (64, 190, 256)])
 @pytest.mark.parametrize("bad", BAD)
-@pytest.mark.parametrize("form", ["walk", "side by side"])
+@pytest.mark.parametrize("form", FORMS)
 def test_gradients_of_what_lies_outside(form, bad, lo, at, hi):
-    T, H = 400, 2
+    T, H = LONG if form == "side by side" else 400, 2
+    assert takes(form, T, H, True)
     if bad == "s0":
         lo = 0
     clean, odd, (length, ns) = operands(T, H, sorted({lo, hi} - {0}), bad, at, float("nan"))
