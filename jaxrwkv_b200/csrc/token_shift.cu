@@ -249,8 +249,8 @@ void launch_bwd_m(cudaStream_t st, int B, int Tlen, int D, const void* x, const 
                   const uint32_t* length, const uint8_t* ns, const void* gout, const void* gstate, void* gx, void* gprev,
                   void* gmix) {
     const int tiles = (Tlen + B200WKV_SHIFT_TILE - 1) / B200WKV_SHIFT_TILE;
-    auto launch = [&](auto kernel, int lanes, int parts) {
-        const dim3 grid((D / V + lanes - 1) / lanes, tiles, B);
+    auto launch = [&](auto kernel, int lanes, int parts, int channels = V) {
+        const dim3 grid((D / channels + lanes - 1) / lanes, tiles, B);
         kernel<<<grid, lanes * parts, 0, st>>>(B, Tlen, D, (const T*)x, (const T*)prev, mix, length, ns, (const T*)gout, (const T*)gstate, (T*)gx,
                                                (T*)gprev, (float*)gmix);
     };
@@ -264,18 +264,39 @@ void launch_bwd_m(cudaStream_t st, int B, int Tlen, int D, const void* x, const 
         // A thread's walk is a chain of groups, 2.7 us each, and what hides it is what is in flight besides: threads with four channels
         // (with eight, 255 registers held groups of four tokens), and of the splits the finest whose blocks are all resident at once;
         // once that is many threads anyway, they need less in flight each.  us, eight channels (whole tiles or four parts) / here, M=6:
-        //   D=768   T=256  B=1  15 / 8.5    T=512  B=8 26 / 13.6                   D=2048  T=831  B=1  17 / 12
-        //   D=2048  T=1024 B=2  30 / 18 by 64 lanes, 2 parts of groups of 8 (23 by 32 lanes and 4 parts, which do not fit at once)
-        //   D=2048  T=1000 B=3  48 / 24 by 2 parts, groups of 4 (8: 32)
-        //   D=2048  T=1024 B=4  50 / 33 by whole tiles, groups of 8 (42 by 2 parts)
-        //   D=768   T=2048 B=8  61 / 42, groups of 5 (8: 58, 3: 49)
-        //   D=2048  T=1024 B=8  74 / 57, groups of 3 (5: 70)
-        if (fits(32, 3)) launch(token_shift_bwd_kernel<T, V, MM, 32, 4, 4, 384>, 32, 4);
-        else if (fits(64, 2)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 8, 256>, 64, 2);
-        else if (fits(64, 3)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 4, 384>, 64, 2);
-        else if (fits(64, 4)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 8, 256>, 64, 1);
-        else if (fits(64, 6)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 5, 384>, 64, 1);
-        else launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 3, 512>, 64, 1);
+        //   D=768   T=256  B=1  15 / 8.3    T=512  B=8 28 / 16.5                   D=2048  T=831  B=1  20 / 14
+        //   D=2048  T=1024 B=2  32 / 20 by 64 lanes, 2 parts of groups of 8 (23 by 32 lanes and 4 parts, which do not fit at once)
+        //   D=2048  T=1000 B=3  49 / 27 by 2 parts, groups of 4 (8: 32)
+        //   D=2048  T=1024 B=4  52 / 35 by whole tiles, groups of 8 (42 by 2 parts)
+        //   D=768   T=2048 B=8  63 / 43, groups of 5 (8: 58, 3: 49)
+        //   D=2048  T=1024 B=8  73 / 57, groups of 3 (5: 70)    T=4096 B=8 234 / 200
+        // Fewer rows of mix leave registers for more threads and longer groups, and with what six rows take they have too little in flight
+        // (one row, D=2048, T=4096, B=8: 92).  us as above, M=1, 2, 3, 4 (two rows of 9-12 blocks per SM: by eight channels):
+        //   D=2048  T=1024 B=2  11 / 10.4   12.8 / 12.4   14.4 / 14.4   16.5 / 16.5        B=4  25 / 15   28 / 18   31 / 23   35 / 27
+        //   D=768   T=2048 B=8  29 / 23   33 / 27   39 / 31   42 / 33
+        //   D=2048  T=1024 B=8  31 / 25   35 / 30   41 / 35   45 / 41     B=16 41 / 41   68 / 55   75 / 65   83 / 77
+        //   D=2048  T=4096 B=8  76 / 76   107 / 99   143 / 119   157 / 143
+        if constexpr (MM >= 5) {
+            if (fits(32, 3)) launch(token_shift_bwd_kernel<T, V, MM, 32, 4, 4, 384>, 32, 4);
+            else if (fits(64, 2)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 8, 256>, 64, 2);
+            else if (fits(64, 3)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 4, 384>, 64, 2);
+            else if (fits(64, 4)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 8, 256>, 64, 1);
+            else if (fits(64, 6)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 5, 384>, 64, 1);
+            else launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 3, 512>, 64, 1);
+        } else if constexpr (MM >= 3) {
+            if (fits(32, 4)) launch(token_shift_bwd_kernel<T, V, MM, 32, 4, 4, 512>, 32, 4);
+            else if (fits(64, 3)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 4, 384>, 64, 2);
+            else if (fits(64, 4)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 4, 512>, 64, 2);
+            else if (fits(64, 6)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 8, 384>, 64, 1);
+            else launch(token_shift_bwd_kernel<T, V, MM, 64, 1, MM == 3 ? 6 : 4, 512>, 64, 1);
+        } else {
+            if (fits(32, MM == 1 ? 6 : 4)) launch(token_shift_bwd_kernel<T, V, MM, 32, 4, 4, MM == 1 ? 768 : 512>, 32, 4);
+            else if (fits(64, 4)) launch(token_shift_bwd_kernel<T, V, MM, 64, 2, 8, 512>, 64, 2);
+            else if (fits(64, 8)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 8, 512>, 64, 1);
+            else if (MM == 2 && fits(64, 12) && D % 8 == 0) launch(token_shift_bwd_kernel<T, 8, 2, 64, 1, 4, 0>, 64, 1, 8);
+            else if (fits(64, 12)) launch(token_shift_bwd_kernel<T, V, MM, 64, 1, 4, 768>, 64, 1);
+            else launch(token_shift_bwd_kernel<T, V, MM, 64, 1, MM == 1 ? 4 : 8, MM == 1 ? 1024 : 512>, 64, 1);
+        }
     }
 }
 

@@ -8,9 +8,11 @@ from jaxrwkv_b200.token_shift import token_shift
 pytestmark = pytest.mark.gpu
 
 
-# on 148 SMs: 4 parts; 2 parts by groups of 8; of 4; whole tiles by groups of 8; of 5; of 3
-@pytest.mark.parametrize("B,T,D", [(2, 129, 264), (130, 65, 256), (111, 150, 256), (250, 70, 256), (100, 129, 512), (500, 70, 252)])
-@pytest.mark.parametrize("M", [2, 6, 8])
+# on 148 SMs, with five rows and more: 4 parts; 2 parts by groups of 8; of 4; whole tiles by groups of 8; of 5; of 3; with fewer the
+# splits change at other counts: 2 parts in front of whole tiles, up to 12 blocks per SM and above, each with channels that 8 do not divide
+@pytest.mark.parametrize("B,T,D", [(2, 129, 264), (130, 65, 256), (111, 150, 256), (250, 70, 256), (100, 129, 512), (500, 70, 252),
+                                   (190, 70, 512), (700, 70, 256), (700, 70, 252), (900, 70, 256)])
+@pytest.mark.parametrize("M", [1, 2, 3, 4, 6, 8])
 def test_backward(B, T, D, M):
     g = torch.Generator().manual_seed(T + D)
     x, prev, mix = (torch.randn(*s, generator=g).bfloat16() for s in ((B, T, D), (B, D), (M, D)))
