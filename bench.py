@@ -50,7 +50,7 @@ METRIC = "wkv7_fwd_bwd_tokens_per_s"
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of ONE launch at B=8, T=4096, H=32 from the
 # ncu captures summarised under profiles/, with the hash of the kernel sources they were taken from.
 # Traffic is proportional to B; the figure is dropped (null) when the sources no longer match.
-NCU_TRAFFIC = {"sources": "65d31a7bf3c2", "B": 8, "wkv7_fwd": 1975.2e6, "wkv7_bwd": 524.4e6 + 2674.0e6}
+NCU_TRAFFIC = {"sources": "12c319953578", "B": 8, "wkv7_fwd": 1978.2e6, "wkv7_bwd": 518.5e6 + 2665.9e6}
 # The backward call is timed as a whole (CUDA events around the call): its device time is the sequential
 # state-gradient carry followed by the block-parallel gradient kernel; the launch list under profiles/
 # gives each kernel's share.  Traffic of the backward is the sum over both kernels.

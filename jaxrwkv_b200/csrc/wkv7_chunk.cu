@@ -204,12 +204,12 @@ __device__ __forceinline__ void load_part(const float4* tiles, size_t slot, int 
 // the CTA with the block in front has put it, passes S_C on to the next one and then finishes its outputs.  A state's way through a
 // CTA takes 2700 cycles (330 to the operand slab, 870 products, 400 results, 1000 to the next CTA), a block 17 k of its CTA's, 13 k of
 // them before the state is needed.  One sequence of 40 heads, T=1999: 114 us in kBlocks, 83 by rings of six; 80 sequences,
-// T=1024: 111 walked, 96 by rings of three.
+// T=1024: 111 walked, 99 by rings of three (kExactRing).
 // R- = R~ + P_rb W~ is rounded once more than R~ and sa are before they meet in the walk, which makes the outputs' errors 0.15 % larger
 // than the walk's (4.090e-3 of them against 4.084e-3, 80 sequences, T=1000), in blocks side by side as in a ring.  kExactRing, for
-// calls that without rings would be walked: R~ and P_rb W~ each meet the state in a product (4.084e-3).  A product of 64 deep takes
-// some 350 cycles that a block of a full device waits for, so that all other rings leave it out (us, B=5, H=16, T=1000: 93.6 / 97.7; 40
-// heads, T=1999: 83.8 / 90).
+// calls that without rings would be walked: R~ and P_rb W~ each meet the state in a product (4.084e-3).  That product costs a block of a
+// full device some 5 % (us, B=5, H=16, T=1000: 93.6 / 97.7; 40 heads, T=1999: 83.8 / 90), so that rings in the place of blocks side by
+// side leave it out.
 enum Form { kWalkForm, kBlocksForm, kRingForm, kExactRingForm };
 //
 // 256 threads: warp = (quad, hsel); quad selects the 32 TMEM lanes (tile rows) the warp may access,

@@ -17,13 +17,14 @@
 // token: wkv7_fp32_grads_kernel walks S forward and dS back elementwise.
 //
 // The token-by-token chain (wkv7_chain.cu) takes 0.12-0.15 us per token whatever else the device does, the chain here 0.6-1.1 us per
-// 16 tokens, and what is taken out of it fills the device.  Forward of 8 heads, T=256: 32.8 -> 24.6 us (6.4 before the chain, 14
-// in it, 3 behind); forward and backward of 24 heads, T=512: 280 -> 162 us (20 + 30 + 7, 17 + 33 + 58), where the gradients
-// were 131 us of sums over rows and columns that every token waited for.  Errors against 64 bits, forward / backward: 0.98e-7 /
-// 0.96-1.41e-7, token by token 1.02e-7 / 0.96-1.39e-7.
+// 16 tokens, and what is taken out of it fills the device.  Forward of 8 heads, T=256: 32.8 -> 22.5 us (6 before the chain, 13
+// in it, 3 behind); forward and backward of 24 heads, T=512: 280 -> 155 us, where the gradients
+// were 131 us of sums over rows and columns that every token waited for.  Errors against 64 bits (without flags / a flag every 128
+// tokens), token by token and here: outputs 1.02e-7 / 1.02e-7 and 0.98e-7 / 0.98e-7, state 0.77e-7 / 0.76e-7 and 0.79e-7 / 0.76e-7, the
+// nearest and the farthest gradient 0.96-1.39e-7 / 0.95-1.39e-7 and 0.96-1.41e-7 / 0.96-1.40e-7.
 //
 // Chunks with a start flag behind their first token, those that `length` cuts and those of fewer than
-// 16 tokens are walked token by token inside the chain kernel, exactly as that one does it: a flag drops the state whatever it
+// 16 tokens are walked token by token inside the chain kernel (its sums in another order than wkv7_chain.cu's): a flag drops the state whatever it
 // holds.  Semantics: BaseRWKV.inner_loop of jaxrwkv (src/jaxrwkv/rwkv7.py:199-220) and its reverse.
 #include "common.cuh"
 #include "device_once.cuh"
