@@ -15,7 +15,7 @@ GRADS = ("dr", "dw", "dk", "dv", "da", "db", "ds0")
 TOL = 1e-5
 
 
-def check(d, H, gy=True, gs=True):
+def check(d, H, gy=True, gs=True, tol=TOL):
     B, T = d["k"].shape[:2]
     t = to_dev(d, torch.float32)
     length, ns = (x.cuda() for x in flags(d))
@@ -29,13 +29,13 @@ def check(d, H, gy=True, gs=True):
     leaves = [t[n].requires_grad_(True) for n in NAMES7]
     s1, y1 = rwkv7.CudaRWKV.inner_loop(*leaves, length, ns)  # with a residual
     for got in ((s, y), (s1, y1)):
-        assert rel_err(npf(got[0]), so) < TOL and rel_err(npf(got[1]), yo) < TOL
+        assert rel_err(npf(got[0]), so) < tol and rel_err(npf(got[1]), yo) < tol
     outs = [(y1, gy), (s1, gs)]
     grads = torch.autograd.grad([o for o, c in outs if c is not None], leaves, [c for _, c in outs if c is not None])
     ref = oracle.wkv7_bwd_batched(*ins, d["length"], d["new_starts"], npf(gy) if gy is not None else np.zeros_like(yo),
                                   npf(gs) if gs is not None else np.zeros_like(so))
     for n, a, b in zip(GRADS, grads, ref):
-        assert rel_err(npf(a), b) < TOL, n
+        assert rel_err(npf(a), b) < tol, n
 
 
 # each split of a head's rows on 148 SMs; token by token, whole chunks, ragged ones; without gradients from 13 chunks on
@@ -107,3 +107,10 @@ def test_walked_chunks_are_the_same_every_time(B, H):
     first = once()
     for _ in range(60):
         assert all(torch.equal(a, b) for a, b in zip(once(), first))
+
+
+# The common bound leaves room for what decays that vanish and lone cotangents lose; of the model's own distributions the worst gradient
+# is 1.41e-7 off, as token by token (1.39e-7), the outputs 0.98e-7 (1.02e-7): within four roundings to 24 bits
+@pytest.mark.parametrize("T,p_start", [(512, 0.0), (512, 1 / 128), (333, 1 / 16)])
+def test_errors_are_those_of_a_few_roundings(T, p_start):
+    check(wkv7_case(2, T, 12, seed=T, p_start=p_start, random_length=p_start > 0, s0_scale=0.3), 12, tol=2.0 ** -22)
